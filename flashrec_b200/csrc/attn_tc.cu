@@ -190,13 +190,16 @@ decode_attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   const uint32_t bar_vfull = bar0 + 40;     // [2]
   const uint32_t bar_vempty = bar0 + 56;    // [2]
   const uint32_t bar_sfull = bar0 + 72;     // [2] S tile complete in TMEM buffer (tile & 1)
-  const uint32_t bar_pfull = bar0 + 88;     // P tile written into TMEM (128 arrivals)
-  const uint32_t bar_ofull = bar0 + 96;     // P.V accumulated (one phase per tile; waited for by the rare O rescale)
+  // [2] P tile written into TMEM buffer (tile & 1), 128 arrivals. One barrier per buffer: S of tile j + 1 is issued before
+  // P of tile j is waited for, so the softmax warps may finish both while the issuing thread is held up, and a parity
+  // wait on a barrier that has gone through two phases does not return. A buffer's next S is issued after its P was seen.
+  const uint32_t bar_pfull = bar0 + 88;
+  const uint32_t bar_ofull = bar0 + 104;    // P.V accumulated (one phase per tile; waited for by the rare O rescale)
   // Last P.V accumulated. Its own one-phase barrier: the softmax of the last tile can finish while the
   // P.V before the last is still pending (S of tile j + 1 is issued before P.V of tile j), and a parity
   // wait on bar_ofull two phases ahead of the barrier would pass at once.
   const uint32_t bar_done = bar0 + 112;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   constexpr int kBeams = kM / G;
@@ -228,6 +231,7 @@ decode_attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     ptx::mbar_init(bar_sfull, 1);
     ptx::mbar_init(bar_sfull + 8, 1);
     ptx::mbar_init(bar_pfull, 128);
+    ptx::mbar_init(bar_pfull + 8, 128);
     ptx::mbar_init(bar_ofull, 1);
     ptx::mbar_init(bar_done, 1);
     *abort_flag = 0;
@@ -309,7 +313,7 @@ decode_attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
           ok = issue_s(j + 1);
           if (!ok) break;
         }
-        ok = ptx::mbar_wait(bar_pfull, j & 1, abort_flag, status, 15);
+        ok = ptx::mbar_wait(bar_pfull + 8 * (j & 1), (j >> 1) & 1, abort_flag, status, 15);
         if (!ok) break;
         ok = ptx::mbar_wait(bar_vfull + 8 * (j & 1), (j >> 1) & 1, abort_flag, status, 16);
         if (!ok) break;
@@ -412,7 +416,7 @@ decode_attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       ptx::tmem_st_32x32(t_lane + kColS + (j & 1) * kTileN, w);
       ptx::tmem_st_wait();
       ptx::tc_fence_before();
-      ptx::mbar_arrive(bar_pfull);
+      ptx::mbar_arrive(bar_pfull + 8 * (j & 1));
     }
     if (ok && n_tiles > 0) {
       int okw = 0;
