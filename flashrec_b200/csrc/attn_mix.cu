@@ -5,8 +5,8 @@
 // a sliding window that keeps the first tokens or with chunks, and an optional linear distance bias.
 //
 // Because the mixture is linear, sum_s coef[o, s] (P_s V) = (sum_s coef[o, s] P_s) V:
-//   * mix_scores_kernel + mix_values_kernel (fr_mix_attn_rows: decode, f32, any head size) write the scores of
-//     every visible key, mix the normalised weights and pass over V once; keys may be split over CTAs;
+//   * mix_scores_kernel + mix_values_kernel (fr_mix_attn_rows: f32, and bf16 heads that attn_rows.cu does not take) write
+//     the scores of every visible key, mix the normalised weights and pass over V once; keys may be split over CTAs;
 //   * mix_tc_kernel (fr_mix_attn_tc: bf16 prompts, tcgen05) runs one flash pass per source map and adds
 //     coef[o, s] / l_s times its result to the outputs' accumulators, which stay in TMEM beside S and O.
 #include "attn_mix.cuh"
@@ -18,6 +18,9 @@ int talk_tc(const fr_mix_attn& a, const int32_t* tiles, int n_tiles, int n_rows,
 int64_t talk_tc_tile_bytes(const fr_mix_attn& a, int max_pos);
 
 namespace mix {
+
+bool fused_rows_fit(const fr_mix_attn& a, int max_keys);  // attn_rows.cu
+int fused_rows(const fr_mix_attn& a, int row0, int n_rows, int max_keys, cudaStream_t stream);
 
 constexpr int kKeyBlock = 64;
 constexpr int kMaxPer = 4;  // key blocks per CTA of the scores kernel when the batch fills the GPU anyway
@@ -884,6 +887,7 @@ extern "C" int fr_mix_attn_rows(const fr_mix_attn* a, int row0, int n_rows, int 
   FR_CHECK_ARG(scratch && aligned16(scratch) && (splits == 1 || counters));
   FR_CHECK_ARG(scratch_bytes >= fr_mix_attn_rows_scratch(a->mix, a->heads, a->vdim, n_rows, max_keys, splits));
   FR_CHECK_SUPPORTED(a->vdim <= 1024 && n_rows <= 65535);
+  if (mix::fused_rows_fit(*a, max_keys)) return mix::fused_rows(*a, row0, n_rows, max_keys, stream);
   const int64_t src = static_cast<int64_t>(n_rows) * (a->mix == FR_MIX_DIFF ? 2 * a->heads : a->heads);
   float2* stats = static_cast<float2*>(scratch);
   float* scores = reinterpret_cast<float*>(stats + src * ceil_div(max_keys, mix::kKeyBlock));

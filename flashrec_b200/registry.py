@@ -49,9 +49,9 @@ def _load_kotipel(path: str, cfg: dict, dtype: torch.dtype, device):
 FAMILIES: List[ModelFamily] = [
     ModelFamily("qwen3-fp8", _is_qwen3, _load_qwen3, (torch.bfloat16,)),
     ModelFamily("dibepel", lambda c: c.get("architecture") == "Dibepel", _load_dibepel, (torch.bfloat16, torch.float32),
-                ("capi", "dense_proj", "lm_rows", "attn_mix", "attn_talk")),
+                ("capi", "dense_proj", "lm_rows", "attn_mix", "attn_rows", "attn_talk")),
     ModelFamily("kotipel", lambda c: c.get("architecture") == "Kotipel", _load_kotipel, (torch.bfloat16, torch.float32),
-                ("capi", "dense_proj", "lm_rows", "attn_mix", "attn_talk", "linear_scan", "linear_chunk")),
+                ("capi", "dense_proj", "lm_rows", "attn_mix", "attn_rows", "attn_talk", "linear_scan", "linear_chunk")),
 ]
 
 

@@ -1,0 +1,55 @@
+"""Row attention of bf16 heads up to 128 (one launch) against the general kernels, which the same call takes in float32:
+every mixture over rows of unequal length, at the edges of its key blocks, warps, shares and clusters."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+PAGE = 64
+
+
+def _run(kind, dtype, heads, kv, dim, vdim, lens, window, keep, seed):
+    """One query per request, at the last of its ``lens`` tokens; [rows, heads * vdim] as float."""
+    from flashrec_b200.core import ForwardBatch
+    from flashrec_b200.kvcache import CacheSpec
+    from flashrec_b200.lm_layers import MixAttention, alibi_slopes
+
+    maps = 2 if kind == "diff" else 1
+    g = torch.Generator().manual_seed(seed)
+    rnd = lambda *s: torch.randn(*s, generator=g).bfloat16()  # noqa: E731
+    n, pages = len(lens), [(m + PAGE - 1) // PAGE for m in lens]
+    perm, table, at = torch.randperm(sum(pages), generator=g), torch.zeros((n + 1, max(pages) * PAGE), dtype=torch.int32), 0
+    for r, p in enumerate(pages):
+        table[r + 1, :p * PAGE] = (perm[at:at + p, None] * PAGE + torch.arange(PAGE)).reshape(-1).to(torch.int32)
+        at += p
+    slots = sum(pages) * PAGE
+    q, k, v = rnd(n, heads * maps * dim), rnd(slots, kv * maps * dim), rnd(slots, kv * vdim)
+    coef, gate = 0.5 * torch.randn(heads, heads, generator=g), torch.randn(n, heads, generator=g)
+    spec = CacheSpec(0, 0, mask="chunk" if kind == "talk" else "window", size=window, keep_first=keep)
+    attn = MixAttention(kind, heads, kv, dim, vdim, dim ** -0.5, spec, eps=1e-5, lam=0.4, out_scale=0.8,
+                        coef=coef if kind == "talk" else None, slopes=torch.tensor(alibi_slopes(heads)) if kind == "talk" else None)
+    attn.bind("cuda")
+    pos = torch.tensor([m - 1 for m in lens])
+    b = ForwardBatch(input_ids=None, req_pool_indices=torch.arange(1, n + 1).cuda(), seq_lens=None, positions=pos.cuda(),
+                     tok_req=torch.arange(n, dtype=torch.int32).cuda(), n_row_tokens=n, max_pos=max(lens) - 1)
+    counters = torch.zeros(4096, dtype=torch.int32, device="cuda")
+    y = attn.forward(*(x.to(dtype).cuda() for x in (q, k, v)), table.cuda(), b, counters,
+                     head_gate=gate.cuda() if kind == "plain" else None)
+    assert not counters.any()
+    return y.float().cpu()
+
+
+@pytest.mark.parametrize("kind", ["diff", "talk", "plain"])
+@pytest.mark.parametrize("heads,kv,dim,vdim", [(16, 8, 128, 128), (4, 4, 64, 128), (8, 2, 64, 64), (8, 1, 128, 48), (4, 2, 64, 48), (6, 2, 80, 128), (5, 1, 16, 16)])
+@pytest.mark.parametrize("lens,window,keep", [
+    ((1,), 4096, 0), ((1100,), 4096, 0), ((3000,), 1024, 4), ((31, 32, 33, 1, 127, 128, 129, 257), 200, 3),
+    (tuple(range(5, 400, 9)), 300, 1)])
+def test_rows_match_the_general_kernels(kind, heads, kv, dim, vdim, lens, window, keep):
+    if kind != "diff" and keep:
+        keep = 0
+    got, ref = (_run(kind, d, heads, kv, dim, vdim, lens, window, keep, 3) for d in (torch.bfloat16, torch.float32))
+    # both compute in fp32 from the same values; rounding to the 8 significant bits of bf16 moves each element by at most half
+    # a unit in the last place, 2^-8 of it, and sums in another order move the norm by a few 1e-6
+    err = (got - ref).norm(dim=1) / ref.norm(dim=1)
+    assert err.max() < 2 ** -8 + 1e-4, (int(err.argmax()), float(err.max()))
