@@ -207,6 +207,7 @@ _SIGNATURES = {
     "fr_dense_proj_split": [_I, P, _L, P, _L, _I, _I, _I, P, _I, P, _I, P],
     "fr_dense_gated_add": [_I, P, _I, P, _L, _I, _I, P, _I, P, _L, _I, P],
     "fr_dense_gated_add_splits": [_I] * 5,
+    "fr_dense_few_row_splits": [_I] * 5,
     "fr_lm_embed": [_I, P, _L, P, P, _L, _I, _I, _I, _F, P, _L, P, P, P, P],
     "fr_lm_norm": [_I, P, _L, P, _F, _F, P, _I, _L, P, P, _L, _I, _I, P],
     "fr_lm_update_norm": [P, _I, _I, P],

@@ -10,8 +10,8 @@
 //   dense_tc_kernel    bf16, persistent and warp-specialised like gemm_fp8.cu: warp 0 = TMA producer (128-byte
 //                      swizzle, 64 bf16 per row), warp 1 = tcgen05.mma issuer (kind::f16, M = 128, fp32
 //                      accumulators in TMEM, two buffers), warps 2..9 = epilogue
-//   dense_rows_kernel  M <= 8 (decode): a warp streams four weight rows against all M activations, so the
-//                      weights cross HBM once; the warps of a CTA may split K
+//   dense_rows_kernel  M <= 8 (decode of one or two rows, few columns, f32): a warp streams four weight rows against all
+//                      M activations, so the weights cross HBM once; the warps of a CTA may split K
 //   dense_simt_kernel  f32 with more rows: 64 x 64 tiles, plain fp32 FMAs
 #include "fr_common.cuh"
 #include "sm100_ptx.cuh"
@@ -414,17 +414,38 @@ enum Epi { kEpiSegs = 0, kEpiAdd = 1, kEpiPartial = 2 };
 
 template <int BLOCK_N>
 struct Cfg {
-  static constexpr int kStageA = kBlockM * kBlockK * 2;
-  static constexpr int kStageB = BLOCK_N * kBlockK * 2;
-  static constexpr int kStageBytes = kStageA + kStageB;
+  static constexpr int kStageBytes = (kBlockM + BLOCK_N) * kBlockK * 2;
   static constexpr int kStages = BLOCK_N == 256 ? 4 : (BLOCK_N == 128 ? 6 : 8);
-  static constexpr int kTmemCols = 2 * BLOCK_N;
-  static constexpr int kBarBytes = (2 * kStages + 4) * 8 + 16;
-  static constexpr int kSmemBytes = 1024 + kStages * kStageBytes + kBarBytes;
+  static constexpr int kTmemCols = BLOCK_N <= 64 ? 128 : (BLOCK_N == 128 ? 256 : 512);  // a power of two
+};
+
+// Operand stages of a few rows (one row block). They bring in only themselves: an SM pulls operands at about 48 bytes per
+// clock, and a whole tile of A would be two thirds of that traffic beside 64 weight rows. The product still reads 128 rows
+// of A; what lies behind the loaded ones goes into accumulator rows that nobody stores.
+// A hand-over between the loading and the issuing thread costs about 400 clocks whatever the tile's width, 0.29 us per
+// k-block with its four products, while the products of 64 columns need 0.07: narrow tiles hand over up to four k-blocks at
+// a time, as long as three stages remain (0.17 us per k-block then; 64 rows x 4096 x 12288: 59.5 -> 37.2 us).
+constexpr int kTileA = kBlockM * kBlockK * 2;
+constexpr int kMaxStages = 12;
+constexpr int kOperandBytes = 200 * 1024;
+constexpr int kBarBytes = (2 * kMaxStages + 4) * 8 + 16;
+struct Stages {
+  int a_rows, a_bytes, block_bytes, blocks, n, smem;  // blocks: k-blocks of a stage, each [A rows | weight rows]
+  __host__ Stages(int M, int block_n) {  // M <= 128
+    a_rows = (M + 7) / 8 * 8;
+    a_bytes = a_rows * kBlockK * 2;
+    block_bytes = a_bytes + block_n * kBlockK * 2;
+    blocks = block_n > 128 ? 1 : 4;
+    while (blocks > 1 && 3 * blocks * block_bytes > kOperandBytes) blocks /= 2;
+    n = kOperandBytes / (blocks * block_bytes);
+    n = n < kMaxStages ? n : kMaxStages;
+    smem = 1024 + n * blocks * block_bytes + (kTileA - a_bytes) + kBarBytes;
+  }
 };
 
 struct TcArgs {
   int M, N;
+  int a_bytes, block_bytes, stage_blocks, stages;  // as planned by Stages
   int n_parts;
   int kb[2];         // k-blocks per part
   int splits[2];     // kEpiPartial: K splits per part
@@ -508,7 +529,9 @@ __device__ __forceinline__ void store32_f32(float* dst, const float (&v)[32], in
   }
 }
 
-template <int BLOCK_N, int EPI>
+// FEW: at most 128 rows, stages as planned at launch; otherwise their sizes are constants (a full tile's products take
+// longer than the hand-over, and the issuing thread has no time to spare: run-time sizes cost 8192 rows 4 %).
+template <int BLOCK_N, int EPI, bool FEW>
 __global__ void __launch_bounds__(kThreads, 1)
 dense_tc_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUtensorMap tb0,
                 const __grid_constant__ CUtensorMap ta1, const __grid_constant__ CUtensorMap tb1,
@@ -518,12 +541,16 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
   const uint32_t raw = ptx::smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* smem = smem_raw + (base - raw);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kStages * C::kStageBytes);
+  const uint32_t n_stages = FEW ? g.stages : C::kStages, block_bytes = FEW ? g.block_bytes : C::kStageBytes;
+  const uint32_t a_bytes = FEW ? g.a_bytes : kTileA;
+  const int stage_blocks = FEW && BLOCK_N <= 128 ? g.stage_blocks : 1;
+  const uint32_t stage_bytes = stage_blocks * block_bytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + n_stages * stage_bytes + (kTileA - a_bytes));
   const uint32_t bar_full = ptx::smem_u32(bars);
-  const uint32_t bar_empty = bar_full + 8 * C::kStages;
-  const uint32_t bar_tfull = bar_empty + 8 * C::kStages;
+  const uint32_t bar_empty = bar_full + 8 * kMaxStages;
+  const uint32_t bar_tfull = bar_empty + 8 * kMaxStages;
   const uint32_t bar_tempty = bar_tfull + 16;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * C::kStages + 4);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kMaxStages + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -533,7 +560,7 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
   const int num_units = m_blocks * n_blocks * (EPI == kEpiPartial ? g.splits[0] + g.splits[1] : 1);
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < C::kStages; ++s) {
+    for (int s = 0; s < static_cast<int>(n_stages); ++s) {
       ptx::mbar_init(bar_full + 8 * s, 1);
       ptx::mbar_init(bar_empty + 8 * s, 1);
     }
@@ -566,14 +593,17 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
           const Job j = job_at<EPI>(g, unit, sub, m_blocks, n_blocks);
           const CUtensorMap* ta = j.part == 0 ? &ta0 : &ta1;
           const CUtensorMap* tb = j.part == 0 ? &tb0 : &tb1;
-          for (int kb = j.kb0; kb < j.kb1; ++kb) {
+          for (int kb0 = j.kb0; kb0 < j.kb1; kb0 += stage_blocks) {
             ok = ptx::mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag, status, 61);
             if (!ok) break;
-            const uint32_t sa = base + stage * C::kStageBytes;
-            ptx::mbar_expect_tx(bar_full + 8 * stage, C::kStageBytes);
-            ptx::tma_load_2d(sa, ta, kb * kBlockK, j.mb * kBlockM, bar_full + 8 * stage);
-            ptx::tma_load_2d(sa + C::kStageA, tb, kb * kBlockK, j.nb * BLOCK_N, bar_full + 8 * stage);
-            if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
+            uint32_t sa = base + stage * stage_bytes;
+            const int kb1 = stage_blocks == 1 ? kb0 + 1 : min(kb0 + stage_blocks, j.kb1);
+            ptx::mbar_expect_tx(bar_full + 8 * stage, (kb1 - kb0) * block_bytes);
+            for (int kb = kb0; kb < kb1; ++kb, sa += block_bytes) {
+              ptx::tma_load_2d(sa, ta, kb * kBlockK, j.mb * kBlockM, bar_full + 8 * stage);
+              ptx::tma_load_2d(sa + a_bytes, tb, kb * kBlockK, j.nb * BLOCK_N, bar_full + 8 * stage);
+            }
+            if (++stage == n_stages) { stage = 0; phase ^= 1u; }
           }
         }
       }
@@ -593,18 +623,21 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
           if (!ok) break;
           ptx::tc_fence_after();
           const uint32_t d_tmem = tmem_base + buf * BLOCK_N;
-          for (int kb = j.kb0; kb < j.kb1; ++kb) {
+          for (int kb0 = j.kb0; kb0 < j.kb1; kb0 += stage_blocks) {
             ok = ptx::mbar_wait(bar_full + 8 * stage, phase, abort_flag, status, 63);
             if (!ok) break;
             ptx::tc_fence_after();
-            const uint32_t sa = base + stage * C::kStageBytes;
-            const uint64_t a_desc = ptx::smem_desc_sw128(sa);
-            const uint64_t b_desc = ptx::smem_desc_sw128(sa + C::kStageA);
+            uint32_t sa = base + stage * stage_bytes;
+            const int kb1 = stage_blocks == 1 ? kb0 + 1 : min(kb0 + stage_blocks, j.kb1);
+            for (int kb = kb0; kb < kb1; ++kb, sa += block_bytes) {
+              const uint64_t a_desc = ptx::smem_desc_sw128(sa);
+              const uint64_t b_desc = ptx::smem_desc_sw128(sa + a_bytes);
 #pragma unroll
-            for (int k = 0; k < kBlockK / kUmmaK; ++k)
-              ptx::mma_f16(d_tmem, a_desc + 2u * k, b_desc + 2u * k, idesc, (kb > j.kb0 || k > 0) ? 1u : 0u);
+              for (int k = 0; k < kBlockK / kUmmaK; ++k)
+                ptx::mma_f16(d_tmem, a_desc + 2u * k, b_desc + 2u * k, idesc, (kb > j.kb0 || k > 0) ? 1u : 0u);
+            }
             ptx::tc_commit(bar_empty + 8 * stage);
-            if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
+            if (++stage == n_stages) { stage = 0; phase ^= 1u; }
           }
           if (ok) ptx::tc_commit(bar_tfull + 8 * buf);
         }
@@ -622,6 +655,7 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
         const uint32_t buf = it & 1;
         const int row = j.mb * kBlockM + quad * 32 + lane;
         const int n0 = j.nb * BLOCK_N;
+        const bool any_row = row - lane < g.M;
         int okw = 0;
         if (lane == 0) okw = ptx::mbar_wait(bar_tfull + 8 * buf, (it >> 1) & 1, abort_flag, status, 64) ? 1 : 0;
         okw = __shfl_sync(0xffffffffu, okw, 0);
@@ -630,7 +664,7 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + buf * BLOCK_N;
         if constexpr (EPI == kEpiSegs) {
 #pragma unroll 1
-          for (int c = part_of_cols; c < BLOCK_N / 64; c += 2) {  // pairs of 32-column chunks
+          for (int c = part_of_cols; any_row && c < BLOCK_N / 64; c += 2) {  // pairs of 32-column chunks
             const int col = n0 + c * 64;
             if (col >= g.N) break;
             uint32_t r0[32], r1[32];
@@ -686,7 +720,7 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
           }
         } else {
 #pragma unroll 1
-          for (int c = part_of_cols; c < BLOCK_N / 32; c += 2) {
+          for (int c = part_of_cols; any_row && c < BLOCK_N / 32; c += 2) {
             const int col = n0 + c * 32;
             const int nvalid = g.N - col;
             if (nvalid <= 0) break;
@@ -792,40 +826,59 @@ int make_tmap_bf16_2d(CUtensorMap* map, const void* ptr, uint64_t cols, uint64_t
   return r == CUDA_SUCCESS ? FR_OK : FR_ERR_CUDA;
 }
 
-template <int BLOCK_N, int EPI>
-static int launch_tc(const TcArgs& g, const fr_gated_part* parts, cudaStream_t stream) {
+template <int BLOCK_N, int EPI, bool FEW>
+static int launch_tc(TcArgs g, const fr_gated_part* parts, cudaStream_t stream) {
+  using C = Cfg<BLOCK_N>;
+  const Stages few(FEW ? g.M : kBlockM, BLOCK_N);
+  g.a_bytes = few.a_bytes;
+  g.block_bytes = few.block_bytes;
+  g.stage_blocks = few.blocks;
+  g.stages = few.n;
+  const int smem = FEW ? few.smem : 1024 + C::kStages * C::kStageBytes + kBarBytes;
   CUtensorMap ta[2], tb[2];
   for (int p = 0; p < 2; ++p) {
     const fr_gated_part& q = parts[p < g.n_parts ? p : 0];
-    int st = make_tmap_bf16_2d(&ta[p], q.a, q.K, g.M, q.lda, kBlockM);
+    int st = make_tmap_bf16_2d(&ta[p], q.a, q.K, g.M, q.lda, FEW ? few.a_rows : kBlockM);
     if (st == FR_OK) st = make_tmap_bf16_2d(&tb[p], q.w, q.K, g.N, q.ldw, BLOCK_N);
     if (st != FR_OK) return st;
   }
-  auto kern = dense_tc_kernel<BLOCK_N, EPI>;
+  auto kern = dense_tc_kernel<BLOCK_N, EPI, FEW>;
   static PerDeviceFlag attr_done;
-  if (ensure_dyn_smem(attr_done, kern, Cfg<BLOCK_N>::kSmemBytes) != FR_OK) return FR_ERR_CUDA;
+  if (ensure_dyn_smem(attr_done, kern, FEW ? 1024 + kOperandBytes + kTileA + kBarBytes : smem) != FR_OK) return FR_ERR_CUDA;
   int* status = device_status_ptr();
   if (!status) return FR_ERR_CUDA;
   const int64_t units = static_cast<int64_t>(ceil_div(g.M, kBlockM)) * ceil_div(g.N, BLOCK_N) *
                         (EPI == kEpiPartial ? g.splits[0] + g.splits[1] : 1);
   const int grid = static_cast<int>(units < device_sm_count() ? units : device_sm_count());
-  return launch_kernel(kern, grid, kThreads, Cfg<BLOCK_N>::kSmemBytes, stream, g.M <= kPdlRows, ta[0], tb[0], ta[1], tb[1], g,
-                       status);
+  return launch_kernel(kern, grid, kThreads, smem, stream, g.M <= kPdlRows, ta[0], tb[0], ta[1], tb[1], g, status);
 }
 
 // Tile width with the least work on the busiest SM: rounds of tiles times the rows of A and B that a tile brings in.
-static int pick_block_n(int M, int N) {
-  const int64_t sms = device_sm_count(), mb = ceil_div(M, kBlockM);
+// 192 is for a single row block only: there it fills one round of SMs where 256 leaves many idle and 128 begins a second
+// (64 rows x 20480 x 2048: 17.9 us; 28 with 80 tiles of 256 and whole tiles of A).
+static int pick_block_n(int M, int N, bool any_width) {
+  const int64_t sms = device_sm_count(), mb = ceil_div(M, kBlockM), a_rows = M <= kBlockM ? Stages(M, 64).a_rows : kBlockM;
   int best = 0;
   int64_t best_cost = 0;
-  for (int bn = 256; bn >= 64; bn /= 2) {
-    const int64_t cost = (mb * ceil_div(N, bn) + sms - 1) / sms * (kBlockM + bn);
+  for (int bn = 256; bn >= 64; bn -= bn == 128 ? 64 : (any_width && M <= kBlockM ? 64 : 128)) {
+    const int64_t cost = (mb * ceil_div(N, bn) + sms - 1) / sms * (a_rows + bn);
     if (best == 0 || cost < best_cost) {
       best = bn;
       best_cost = cost;
     }
   }
   return best;
+}
+
+// Whether a few-row product streams the weights through the row kernel. There a weight costs an FMA per row: one or two rows
+// hide them behind the loads, more do not, and the tensor cores take those where there are columns enough for tiles
+// (us for 20480 x 2048, rows 1 / 2 / 4 / 8: 15.6 / 19.4 / 30.5 / 60.0 here, 17.7 for any of them there).
+// Fewer columns than 64 tiles of 64 leave the tensor cores' loads to few SMs: three or four rows stay here up to that
+// (2048 x 2048: 5.4 against 9.0 us) unless K can be split over the SMs too.
+static bool use_rows(int dtype, int M, int N, bool split_k) {
+  if (M > 8) return false;
+  if (dtype != 0 || M <= 2 || N <= 1024) return true;
+  return !split_k && M <= 4 && N <= 4096;
 }
 
 static int rows_ks(int N, int K) {
@@ -922,7 +975,7 @@ extern "C" int fr_dense_proj(int dtype, const void* a, int64_t lda, const void* 
   FR_CHECK_ARG(dense::operand_ok(a, lda, K) && dense::operand_ok(w, ldw, K) && N % 4 == 0);
   dense::Segs sg{};
   if (check_segs(segs, n_segs, N, &sg) != FR_OK) return FR_ERR_BAD_ARG;
-  if (algo == 0) algo = M <= 8 ? 1 : 2;
+  if (algo == 0) algo = dense::use_rows(dtype, M, N, false) ? 1 : 2;
   if (algo == 1) {
     FR_CHECK_SUPPORTED(M <= 8);
     return dtype == 0 ? dense::launch_rows_proj<__nv_bfloat16>(a, lda, w, ldw, M, N, K, sg, stream)
@@ -941,10 +994,19 @@ extern "C" int fr_dense_proj(int dtype, const void* a, int64_t lda, const void* 
   g.kb[0] = ceil_div(K, dense::kBlockK);
   g.segs = sg;
   fr_gated_part part{a, w, nullptr, lda, ldw, 0, K, 0};
-  switch (dense::pick_block_n(M, N)) {
-    case 256: return dense::launch_tc<256, dense::kEpiSegs>(g, &part, stream);
-    case 128: return dense::launch_tc<128, dense::kEpiSegs>(g, &part, stream);
-    default: return dense::launch_tc<64, dense::kEpiSegs>(g, &part, stream);
+  const int block_n = dense::pick_block_n(M, N, true);
+  if (M <= dense::kBlockM) {
+    switch (block_n) {
+      case 256: return dense::launch_tc<256, dense::kEpiSegs, true>(g, &part, stream);
+      case 192: return dense::launch_tc<192, dense::kEpiSegs, true>(g, &part, stream);
+      case 128: return dense::launch_tc<128, dense::kEpiSegs, true>(g, &part, stream);
+      default: return dense::launch_tc<64, dense::kEpiSegs, true>(g, &part, stream);
+    }
+  }
+  switch (block_n) {
+    case 256: return dense::launch_tc<256, dense::kEpiSegs, false>(g, &part, stream);
+    case 128: return dense::launch_tc<128, dense::kEpiSegs, false>(g, &part, stream);
+    default: return dense::launch_tc<64, dense::kEpiSegs, false>(g, &part, stream);
   }
 }
 
@@ -961,7 +1023,11 @@ extern "C" int fr_dense_proj_split(int dtype, const void* a, int64_t lda, const 
 }
 
 extern "C" int fr_dense_gated_add_splits(int dtype, int M, int N, int K0, int K1) {
-  if (dtype != 0 || M <= 8 || N <= 0 || K0 <= 0) return 0;
+  return M <= 8 ? 0 : fr_dense_few_row_splits(dtype, M, N, K0, K1);
+}
+
+extern "C" int fr_dense_few_row_splits(int dtype, int M, int N, int K0, int K1) {
+  if (dtype != 0 || M <= 0 || N <= 0 || K0 <= 0 || dense::use_rows(dtype, M, N, true)) return 0;
   int a, b;
   dense::plan_splits(M, N, ceil_div(K0, dense::kBlockK), K1 > 0 ? ceil_div(K1, dense::kBlockK) : 0, &a, &b);
   return a + b;
@@ -1009,11 +1075,12 @@ extern "C" int fr_dense_gated_add(int dtype, const fr_gated_part* parts, int n_p
     dense::plan_splits(M, N, g.kb[0], n_parts > 1 ? g.kb[1] : 0, &g.splits[0], &g.splits[1]);
     FR_CHECK_ARG(g.splits[0] > 0 && g.splits[0] + g.splits[1] == n_splits && (n_parts == 1 || g.splits[1] > 0));
     g.partials = partials;
-    return dense::launch_tc<64, dense::kEpiPartial>(g, parts, stream);
+    return M <= dense::kBlockM ? dense::launch_tc<64, dense::kEpiPartial, true>(g, parts, stream)
+                               : dense::launch_tc<64, dense::kEpiPartial, false>(g, parts, stream);
   }
-  switch (dense::pick_block_n(M, N)) {
-    case 256: return dense::launch_tc<256, dense::kEpiAdd>(g, parts, stream);
-    case 128: return dense::launch_tc<128, dense::kEpiAdd>(g, parts, stream);
-    default: return dense::launch_tc<64, dense::kEpiAdd>(g, parts, stream);
+  switch (dense::pick_block_n(M, N, false)) {
+    case 256: return dense::launch_tc<256, dense::kEpiAdd, false>(g, parts, stream);
+    case 128: return dense::launch_tc<128, dense::kEpiAdd, false>(g, parts, stream);
+    default: return dense::launch_tc<64, dense::kEpiAdd, false>(g, parts, stream);
   }
 }

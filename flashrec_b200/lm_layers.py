@@ -153,9 +153,10 @@ class Partials:
 
 
 def gated_add(x: torch.Tensor, parts: Sequence[Tuple[torch.Tensor, torch.Tensor, Optional[torch.Tensor]]],
-              algo: int = 0, split: bool = True, copy: Optional[torch.Tensor] = None) -> Optional[Partials]:
+              algo: int = 0, split: bool = True, copy: Optional[torch.Tensor] = None, few_rows: bool = False) -> Optional[Partials]:
     """``x += sum gate * (a @ w.T)`` over one or two ``(a, w, gate)`` parts; few-row products may come back as
-    partials for the following ``rms_norm`` instead. ``copy`` gets the new x in its own type (not with partials)."""
+    partials for the following ``rms_norm`` instead, with ``few_rows`` also those of 3 to 8 rows. ``copy`` gets the new x in
+    its own type (not with partials)."""
     require_cuda(x)
     m, n = int(x.shape[0]), int(x.shape[1])
     arr = (FrGatedPart * len(parts))()
@@ -164,7 +165,9 @@ def gated_add(x: torch.Tensor, parts: Sequence[Tuple[torch.Tensor, torch.Tensor,
                              int(w.shape[1]), 0)
     code = dtype_code(parts[0][1].dtype)
     k = [int(p[1].shape[1]) for p in parts] + [0]
-    n_splits = _lib.load().fr_dense_gated_add_splits(code, m, n, k[0], k[1]) if split and algo == 0 else 0
+    lib = _lib.load()
+    splits = lib.fr_dense_few_row_splits if few_rows else lib.fr_dense_gated_add_splits
+    n_splits = splits(code, m, n, k[0], k[1]) if split and algo == 0 else 0
     buf = torch.empty((n_splits, m, n), dtype=torch.float32, device=x.device) if n_splits > 0 else None
     if n_splits > 0:
         copy = None
@@ -190,7 +193,7 @@ def split_product(a: torch.Tensor, w: torch.Tensor) -> Optional[Partials]:
     """``a @ w.T`` as K shares when it has so few tiles that they would leave SMs idle, else None."""
     require_cuda(a)
     m, n, code = int(a.shape[0]), int(w.shape[0]), dtype_code(w.dtype)
-    n_splits = _lib.load().fr_dense_gated_add_splits(code, m, n, int(w.shape[1]), 0)
+    n_splits = _lib.load().fr_dense_few_row_splits(code, m, n, int(w.shape[1]), 0)
     if n_splits < 2:
         return None
     buf = torch.empty((n_splits, m, n), dtype=torch.float32, device=a.device)

@@ -567,11 +567,13 @@ struct fr_gated_part {
 /* x[m, n] += sum_p gate_p[m, n] * (a_p . w_p^T)[m, n], one or two parts. With `partials` (f32
  * [splits, M, N]) the K extent is split instead: partial s receives its share of the sum, x is left alone
  * and fr_lm_norm adds the partials in order. n_splits: 0 without partials; else as returned by
- * fr_dense_gated_add_splits for the same shape. copy (or null, without partials): the new x rounded to dtype as well;
+ * fr_dense_gated_add_splits or fr_dense_few_row_splits for the same shape. copy (or null, without partials): the new x rounded to dtype as well;
  * columns [N, ldc) are zeroed up to a multiple of 8. */
 int fr_dense_gated_add(int dtype, const struct fr_gated_part* parts, int n_parts, float* x, int64_t ldx, int M, int N,
                        float* partials, int n_splits, void* copy, int64_t ldc, int algo, cudaStream_t stream);
 int fr_dense_gated_add_splits(int dtype, int M, int N, int K0, int K1);
+/* The same, but also for 3 to 8 rows where the split product is the faster one (fr_dense_gated_add_splits says 0 there). */
+int fr_dense_few_row_splits(int dtype, int M, int N, int K0, int K1);
 
 /* x[t, :] = table[ids[t], :] * scale, and the slot table entry of the token: req_to_token[rows[t], pos[t]] = loc[t]
  * (skipped when req_to_token is null). */
