@@ -12,7 +12,7 @@
 //                      accumulators in TMEM, two buffers), warps 2..9 = epilogue
 //   dense_rows_kernel  M <= 8 (decode of one or two rows, few columns, f32): a warp streams four weight rows against all
 //                      M activations, so the weights cross HBM once; the warps of a CTA may split K
-//   dense_simt_kernel  f32 with more rows: 64 x 64 tiles, plain fp32 FMAs
+//   dense_simt_kernel  f32 with more rows: tiles of 64 or 128 x 64, fp32 FMAs
 #include "fr_common.cuh"
 #include "sm100_ptx.cuh"
 
@@ -280,95 +280,149 @@ dense_rows_gated_kernel(const __grid_constant__ Parts pt, float* __restrict__ x,
 }
 
 // ---------------------------------------------------------------------------
-// f32, more rows: 64 x 64 tiles, 256 threads, 4 x 4 outputs per thread. Columns of a thread: two in the
-// first half of the tile and the two 32 further on, so that a SwiGLU pair meets in one thread.
+// f32, more rows: TM x 64 tiles, 256 threads of TM / 16 x 4 outputs. Bound by the fp32 units where there are tiles enough:
+// operands arrive by cp.async two steps of 16 ahead and stay as they lie in memory, rows of k, so that one fma.rn.f32x2
+// takes two consecutive k of an output without any rearranging (an output is the sum of its even and its odd chain).
+// us for 64 / 351 rows of 2048: 20480 columns 286 / 1153 before (64 x 64 tiles through transposed copies, one step ahead), 220 /
+// 863 now (34 TFLOP/s); 2048 columns 133 / 226 and 92 / 155. The gated update's 192 tiles of K = 8192 stay a chain per SM:
+// 679 and 659.
 // ---------------------------------------------------------------------------
-constexpr int kSimtK = 16;
+constexpr int kSimtK = 16, kSimtStages = 3;
+constexpr int kSimtPitch = kSimtK + 4;  // floats: eight consecutive rows of 16 bytes meet in no bank
 
-__device__ __forceinline__ void simt_tile(const float* __restrict__ a, int64_t lda, const float* __restrict__ w, int64_t ldw,
-                                          int M, int N, int K, int m0, int n0, float (&as)[kSimtK][68],
-                                          float (&ws)[kSimtK][68], float (&acc)[4][4]) {
-  const int tid = threadIdx.x, lr = tid >> 2, lk = (tid & 3) * 4;
-  const int tx = tid & 15, ty = tid >> 4;
-  for (int k0 = 0; k0 < K; k0 += kSimtK) {
-    float4 av = make_float4(0, 0, 0, 0), wv = av;
-    if (k0 + lk < K) {  // K is a multiple of 8
-      if (m0 + lr < M) av = *reinterpret_cast<const float4*>(a + (m0 + lr) * lda + k0 + lk);
-      if (n0 + lr < N) wv = *reinterpret_cast<const float4*>(w + (n0 + lr) * ldw + k0 + lk);
-    }
-    __syncthreads();
-    as[lk][lr] = av.x; as[lk + 1][lr] = av.y; as[lk + 2][lr] = av.z; as[lk + 3][lr] = av.w;
-    ws[lk][lr] = wv.x; ws[lk + 1][lr] = wv.y; ws[lk + 2][lr] = wv.z; ws[lk + 3][lr] = wv.w;
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < kSimtK; ++k) {
-      float ar[4], wr[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) ar[i] = as[k][ty * 4 + i];
-      wr[0] = ws[k][tx * 2]; wr[1] = ws[k][tx * 2 + 1];
-      wr[2] = ws[k][32 + tx * 2]; wr[3] = ws[k][33 + tx * 2];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(ar[i], wr[j], acc[i][j]);
-    }
-  }
+__device__ __forceinline__ uint64_t f32x2_fma(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ float f32x2_sum(uint64_t v) {
+  float lo, hi;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+  return lo + hi;
 }
 
-__global__ void __launch_bounds__(256)
+template <int TM>
+struct Simt {
+  static constexpr int RM = TM / 16, CN = 4;
+  float as[kSimtStages][TM][kSimtPitch], ws[kSimtStages][64][kSimtPitch];
+
+  // row r of a thread's RM and column c of its four (of a [32 gate | 32 up] block two gates, then their ups), within the tile
+  static __device__ __forceinline__ int row_of(int ty, int r) { return ty * RM + r; }
+  static __device__ __forceinline__ int col_of(int tx, int c) { return c * 16 + tx; }
+
+  __device__ __forceinline__ void tile(const float* __restrict__ a, int64_t lda, const float* __restrict__ w, int64_t ldw, int M,
+                                       int N, int K, int m0, int n0, float (&out)[RM][CN]) {
+    const int tid = threadIdx.x, lr = tid >> 2, lk = (tid & 3) * 4, tx = tid & 15, ty = tid >> 4;
+    auto copy = [](float* dst, const float* src, bool in) {  // zeros outside; `src` is a valid address either way
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ptx::smem_u32(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
+    };
+    const int steps = (K + kSimtK - 1) / kSimtK;
+    auto fetch = [&](int step) {
+      if (step < steps) {
+        const int st = step % kSimtStages, k = step * kSimtK + lk;
+        const bool in = k < K;  // K is a multiple of 8
+#pragma unroll
+        for (int i = 0; i < TM / 64; ++i) {
+          const bool row = m0 + lr + 64 * i < M;
+          copy(&as[st][lr + 64 * i][lk], a + static_cast<int64_t>(row ? m0 + lr + 64 * i : 0) * lda + (in ? k : 0), in && row);
+        }
+        const bool col = n0 + lr < N;
+        copy(&ws[st][lr][lk], w + static_cast<int64_t>(col ? n0 + lr : 0) * ldw + (in ? k : 0), in && col);
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    uint64_t acc[RM][CN] = {};
+    __syncthreads();  // the tile before, if any, has been read
+    for (int i = 0; i < kSimtStages - 1; ++i) fetch(i);
+    for (int step = 0; step < steps; ++step) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(kSimtStages - 2) : "memory");
+      __syncthreads();  // this step's operands are there, the last one's are read
+      fetch(step + kSimtStages - 1);
+      const int st = step % kSimtStages;
+#pragma unroll
+      for (int k = 0; k < kSimtK; k += 4) {
+        ulonglong2 wv[CN];
+#pragma unroll
+        for (int c = 0; c < CN; ++c) wv[c] = *reinterpret_cast<const ulonglong2*>(&ws[st][col_of(tx, c)][k]);
+#pragma unroll
+        for (int r = 0; r < RM; ++r) {
+          const ulonglong2 av = *reinterpret_cast<const ulonglong2*>(&as[st][row_of(ty, r)][k]);
+#pragma unroll
+          for (int c = 0; c < CN; ++c) {
+            acc[r][c] = f32x2_fma(av.x, wv[c].x, acc[r][c]);
+            acc[r][c] = f32x2_fma(av.y, wv[c].y, acc[r][c]);
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < RM; ++r)
+#pragma unroll
+      for (int c = 0; c < CN; ++c) out[r][c] = f32x2_sum(acc[r][c]);
+  }
+};
+
+template <int TM>
+__global__ void __launch_bounds__(256, TM == 64 ? 3 : 2)
 dense_simt_proj_kernel(const float* __restrict__ a, int64_t lda, const float* __restrict__ w, int64_t ldw, int M, int N, int K,
                        const __grid_constant__ Segs sg) {
-  __shared__ float as[kSimtK][68], ws[kSimtK][68];
-  const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-  float acc[4][4] = {};
-  simt_tile(a, lda, w, ldw, M, N, K, m0, n0, as, ws, acc);
+  using S = Simt<TM>;
+  __shared__ __align__(16) S sm;
+  const int m0 = blockIdx.y * TM, n0 = blockIdx.x * 64;
+  float acc[S::RM][S::CN];
+  sm.tile(a, lda, w, ldw, M, N, K, m0, n0, acc);
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+#pragma unroll
   for (int half = 0; half < 2; ++half) {
     const int col0 = n0 + half * 32;  // a 32-column chunk lies in one range
     if (col0 >= N) break;
     const fr_out_segment& s = sg.s[seg_of(sg, col0)];
-    if (paired(s)) {
-      if (half == 1) continue;
-      const int ch = (col0 - s.n0) / 2 + tx * 2;
-      for (int i = 0; i < 4; ++i) {
-        const int row = m0 + ty * 4 + i;
-        if (row >= M) break;
-        for (int j = 0; j < 2; ++j) seg_write<float, false>(s, row, ch + j, pair_act<false>(s, acc[i][j], acc[i][2 + j]));
-      }
-    } else {
-      for (int i = 0; i < 4; ++i) {
-        const int row = m0 + ty * 4 + i;
-        if (row >= M) break;
-        for (int j = 0; j < 2; ++j) seg_write<float, false>(s, row, col0 - s.n0 + tx * 2 + j, acc[i][half * 2 + j]);
+    const bool pair = paired(s);
+    if (pair && half == 1) continue;
+#pragma unroll
+    for (int r = 0; r < S::RM; ++r) {
+      const int row = m0 + S::row_of(ty, r);
+      if (row >= M) continue;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const float v = acc[r][2 * half + e];
+        if (pair)
+          seg_write<float, false>(s, row, (col0 - s.n0) / 2 + e * 16 + tx, pair_act<false>(s, v, acc[r][2 + e]));
+        else
+          seg_write<float, false>(s, row, col0 - s.n0 + e * 16 + tx, v);
       }
     }
   }
 }
 
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 3)
 dense_simt_gated_kernel(const __grid_constant__ Parts pt, float* __restrict__ x, int64_t ldx, int M, int N, float* __restrict__ copy,
                         int64_t ldc) {
-  __shared__ float as[kSimtK][68], ws[kSimtK][68];
+  using S = Simt<64>;
+  __shared__ __align__(16) S sm;
   const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  float sum[4][4] = {};
+  float sum[S::RM][S::CN] = {};
   for (int p = 0; p < pt.n; ++p) {
     const fr_gated_part& part = pt.p[p];
-    float acc[4][4] = {};
-    simt_tile(static_cast<const float*>(part.a), part.lda, static_cast<const float*>(part.w), part.ldw, M, N, part.K, m0, n0,
-              as, ws, acc);
+    float acc[S::RM][S::CN];
+    sm.tile(static_cast<const float*>(part.a), part.lda, static_cast<const float*>(part.w), part.ldw, M, N, part.K, m0, n0, acc);
     const float* g = static_cast<const float*>(part.gate);
-    for (int i = 0; i < 4; ++i)
-      for (int j = 0; j < 4; ++j) {
-        const int row = m0 + ty * 4 + i, col = n0 + (j >> 1) * 32 + tx * 2 + (j & 1);
-        if (row < M && col < N) sum[i][j] += (g != nullptr ? g[row * part.ldg + col] : 1.0f) * acc[i][j];
+#pragma unroll
+    for (int r = 0; r < S::RM; ++r)
+#pragma unroll
+      for (int c = 0; c < S::CN; ++c) {
+        const int row = m0 + S::row_of(ty, r), col = n0 + S::col_of(tx, c);
+        if (row < M && col < N) sum[r][c] += (g != nullptr ? g[row * part.ldg + col] : 1.0f) * acc[r][c];
       }
   }
-  for (int i = 0; i < 4; ++i)
-    for (int j = 0; j < 4; ++j) {
-      const int row = m0 + ty * 4 + i, col = n0 + (j >> 1) * 32 + tx * 2 + (j & 1);
+#pragma unroll
+  for (int r = 0; r < S::RM; ++r)
+#pragma unroll
+    for (int c = 0; c < S::CN; ++c) {
+      const int row = m0 + S::row_of(ty, r), col = n0 + S::col_of(tx, c);
       if (row < M && col < N) {
-        const float v = x[row * ldx + col] + sum[i][j];
+        const float v = x[row * ldx + col] + sum[r][c];
         x[row * ldx + col] = v;
         if (copy != nullptr) copy[row * ldc + col] = v;
       } else if (copy != nullptr && row < M && col < (N + 7) / 8 * 8 && col < ldc) {
@@ -982,9 +1036,14 @@ extern "C" int fr_dense_proj(int dtype, const void* a, int64_t lda, const void* 
                       : dense::launch_rows_proj<float>(a, lda, w, ldw, M, N, K, sg, stream);
   }
   if (dtype == 1) {
-    dim3 grid(ceil_div(N, 64), ceil_div(M, 64));
-    dense::dense_simt_proj_kernel<<<grid, 256, 0, stream>>>(static_cast<const float*>(a), lda, static_cast<const float*>(w),
-                                                            ldw, M, N, K, sg);
+    const float* A = static_cast<const float*>(a);
+    const float* W = static_cast<const float*>(w);
+    // 128 rows per tile take every weight from shared memory half as often; with fewer than a tile per SM 64 spread better
+    const int64_t large = static_cast<int64_t>(ceil_div(N, 64)) * ceil_div(M, 128);
+    if (M > 64 && large >= device_sm_count())
+      dense::dense_simt_proj_kernel<128><<<dim3(ceil_div(N, 64), ceil_div(M, 128)), 256, 0, stream>>>(A, lda, W, ldw, M, N, K, sg);
+    else
+      dense::dense_simt_proj_kernel<64><<<dim3(ceil_div(N, 64), ceil_div(M, 64)), 256, 0, stream>>>(A, lda, W, ldw, M, N, K, sg);
     return launch_status();
   }
   dense::TcArgs g{};
@@ -1054,8 +1113,8 @@ extern "C" int fr_dense_gated_add(int dtype, const fr_gated_part* parts, int n_p
   }
   if (dtype == 1) {
     FR_CHECK_SUPPORTED(n_splits == 0);
-    dim3 grid(ceil_div(N, 64), ceil_div(M, 64));
-    dense::dense_simt_gated_kernel<<<grid, 256, 0, stream>>>(pt, x, ldx, M, N, static_cast<float*>(copy), ldc);
+    dense::dense_simt_gated_kernel<<<dim3(ceil_div(N, 64), ceil_div(M, 64)), 256, 0, stream>>>(
+        pt, x, ldx, M, N, static_cast<float*>(copy), ldc);
     return launch_status();
   }
   dense::TcArgs g{};
