@@ -32,6 +32,19 @@ class StepEntry:
     want: Sequence[int] = ()
 
 
+def _token_array(tokens: Sequence[int], vocab: int) -> np.ndarray:
+    """``tokens`` as int64, all of them within the vocabulary."""
+    a = np.asarray(tokens) if isinstance(tokens, (list, tuple, range, np.ndarray)) else None
+    if a is None or a.ndim != 1 or a.dtype.kind not in "iu":  # tensors, mixed or foreign integers: one by one
+        ids = [int(t) for t in tokens]
+        if any(not 0 <= t < vocab for t in ids):
+            raise ValueError("token id outside the vocabulary")
+        return np.array(ids, dtype=np.int64)
+    if a.size and (a.min() < 0 or a.max() >= vocab):
+        raise ValueError("token id outside the vocabulary")
+    return a.astype(np.int64, copy=False)
+
+
 @dataclass
 class _DecodeGraph:
     graph: torch.cuda.CUDAGraph
@@ -88,8 +101,12 @@ class LMEngine:
         if any(self.seqs.length(e.req) + len(e.tokens) > self.max_seq for e in entries):
             raise RuntimeError(f"a request would exceed {self.max_seq} tokens")
         vocab = self.model.vocab
-        if any(not 0 <= int(t) < vocab for e in entries for t in e.tokens):
-            raise ValueError("token id outside the vocabulary")
+        one = all(len(e.tokens) == 1 for e in entries)
+        if one:
+            if any(not 0 <= int(e.tokens[0]) < vocab for e in entries):
+                raise ValueError("token id outside the vocabulary")
+        else:  # prompts: columns of thousands of numbers are arrays
+            ids = [_token_array(e.tokens, vocab) for e in entries]
         if any(not 0 <= int(w) < len(e.tokens) for e in entries for w in e.want):
             raise ValueError("want: place outside the entry's tokens")
         # short portions first: their attention runs row by row, the rest in tiles
@@ -97,19 +114,24 @@ class LMEngine:
         start: Dict[int, int] = {}
         toks, pos, loc, tok_req, rows, req_rows, qo, pre, ext = [], [], [], [], [], [], [0], [], []
         tiles: List[Tuple[int, int, int]] = []
-        n_row = 0
+        n_row = t0 = 0
         for b, i in enumerate(order):
             e = entries[i]
             if e.req not in self.seqs.live:
                 self.seqs.open(e.req)
             seq = self.seqs.live[e.req]
-            n, first, t0 = len(e.tokens), seq.length, len(toks)
+            n, first = len(e.tokens), seq.length
             start[i] = t0
-            toks += [int(t) for t in e.tokens]
-            loc += self.seqs.extend(e.req, n)
-            pos += range(first, first + n)
-            tok_req += [b] * n
-            rows += [seq.row] * n
+            if one:
+                toks.append(int(e.tokens[0]))
+                loc += self.seqs.extend(e.req, 1)
+                pos.append(first)
+                tok_req.append(b)
+                rows.append(seq.row)
+            else:
+                toks.append(ids[i])
+                loc.append(self.seqs.extend_array(e.req, n))
+                pos.append(np.arange(first, first + n, dtype=np.int64))
             req_rows.append(seq.row)
             qo.append(t0 + n)
             pre.append(first)
@@ -118,8 +140,11 @@ class LMEngine:
                 n_row = t0 + n
             else:
                 tiles += [(b, t0 + s, min(TILE_ROWS, n - s)) for s in range(0, n, TILE_ROWS)]
+            t0 += n
+        if not one:
+            toks, loc, pos = np.concatenate(toks), np.concatenate(loc), np.concatenate(pos)
+            tok_req, rows = np.repeat(np.arange(len(ext)), ext), np.repeat(req_rows, ext)
         want = [start[i] + int(w) for i, e in enumerate(entries) for w in e.want]
-        one = len(toks) == len(entries)
         if one and self.use_graphs and on_layer is None and len(entries) <= self.GRAPH_SIZES[-1]:
             out = self._decode(toks, pos, loc, rows, want)
         else:
@@ -136,7 +161,7 @@ class LMEngine:
         n64 = [len(c) for c in cols64]
         n32 = [(len(c) + 1) // 2 * 2 for c in cols32]
         total = sum(n64) + sum(n32) // 2
-        host = torch.empty(total, dtype=torch.int64).pin_memory() if total else torch.empty(0, dtype=torch.int64)
+        host = torch.empty(total, dtype=torch.int64, pin_memory=True) if total else torch.empty(0, dtype=torch.int64)
         flat = host.numpy()
         o = 0
         for c, n in zip(cols64, n64):
@@ -166,7 +191,8 @@ class LMEngine:
             [tok_req, qo, [v for t in tiles for v in t], [p + n for p, n in zip(pre, ext)]])
         batch = ForwardBatch(input_ids=d_tok, req_pool_indices=d_req, seq_lens=d_len, positions=d_pos,
                              out_cache_loc=d_loc, is_prefill=not one, extend_prefix_lens=pre, extend_seq_lens=ext, qo_indptr=d_qo, tok_req=d_tr, tok_rows=d_rows,
-                             n_row_tokens=n_row, tiles=d_tiles.view(-1, 3), one_token=one, max_pos=max(pos))
+                             n_row_tokens=n_row, tiles=d_tiles.view(-1, 3), one_token=one,
+                             max_pos=max(p + n for p, n in zip(pre, ext)) - 1)
         return batch, d_want
 
     # -- captured decode steps --------------------------------------------------------------------------

@@ -11,6 +11,7 @@ from __future__ import annotations
 from dataclasses import dataclass, field
 from typing import Dict, List, Optional, Sequence
 
+import numpy as np
 import torch
 
 PAGE = 64
@@ -111,21 +112,33 @@ class SequenceManager:
         self.live[req] = seq
         return seq
 
-    def extend(self, req, n: int) -> List[int]:
-        """Slots of the next ``n`` positions of ``req``; raises (and changes nothing) when the pool is short."""
+    def _take(self, req, n: int) -> SequenceState:
+        """Pages for the next ``n`` positions of ``req``, whose length stays; raises (and changes nothing) when the pool is
+        short."""
         seq = self.live[req]
         if seq.length + n > self.max_seq:
             raise RuntimeError(f"request {req!r} would exceed {self.max_seq} tokens")
         if self.pages_needed(seq.length, n) > len(self._free_pages):
             raise RuntimeError("out of cache pages")
-        out = []
-        for pos in range(seq.length, seq.length + n):
-            p = pos // PAGE
+        for p in range(seq.length // PAGE, (seq.length + n + PAGE - 1) // PAGE if n > 0 else 0):
             if p not in seq.pages:
                 seq.pages[p] = self._free_pages.pop()
-            out.append(seq.pages[p] * PAGE + pos % PAGE)
-        seq.length += n
-        return out
+        return seq
+
+    def extend(self, req, n: int) -> List[int]:
+        """Slots of the next ``n`` positions of ``req``; raises (and changes nothing) when the pool is short."""
+        seq = self._take(req, n)
+        first, seq.length = seq.length, seq.length + n
+        return [seq.pages[pos // PAGE] * PAGE + pos % PAGE for pos in range(first, first + n)]
+
+    def extend_array(self, req, n: int) -> np.ndarray:
+        """:meth:`extend` of many positions at once, int64 [n]."""
+        seq = self._take(req, n)
+        first, seq.length = seq.length, seq.length + n
+        p0 = first // PAGE
+        pages = np.array([seq.pages[p] for p in range(p0, (first + n + PAGE - 1) // PAGE)], dtype=np.int64)
+        pos = np.arange(first, first + n, dtype=np.int64)
+        return pages[pos // PAGE - p0] * PAGE + pos % PAGE
 
     def trim(self, req) -> int:
         """Give back the pages that the next position sees in no layer. Returns how many."""

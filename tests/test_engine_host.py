@@ -1,0 +1,44 @@
+"""Host side of the step function: slots of many positions at once as one by one, tokens in every form."""
+
+import random
+
+import numpy as np
+import pytest
+import torch
+
+from flashrec_b200.engine import _token_array
+from flashrec_b200.kvcache import PAGE, CacheSpec, SequenceManager
+
+
+def test_slots_of_many_positions_are_those_of_one_after_the_other():
+    r = random.Random(0)
+    one, many = (SequenceManager([CacheSpec(8, 8)], 60, 4, 2000, "cpu") for _ in range(2))
+    for m in (one, many):
+        for q in range(3):
+            m.open(q)
+    for _ in range(200):
+        q, n = r.randrange(3), r.choice([0, 1, 2, PAGE - 1, PAGE, PAGE + 1, 130])
+        try:
+            slots = one.extend(q, n)
+        except RuntimeError:
+            with pytest.raises(RuntimeError):
+                many.extend_array(q, n)
+            for m in (one, many):
+                m.close(q)
+                m.open(q)
+            continue
+        assert slots == many.extend_array(q, n).tolist()
+        assert one.length(q) == many.length(q) and one._free_pages == many._free_pages
+
+
+@pytest.mark.parametrize("tokens", [[1, 99], (0, 4), range(5), np.array([1, 2], np.uint8), np.array([7], np.int32), torch.tensor([1, 2]),
+                                    [np.int32(4), 7], [torch.tensor(3), 4], [1.0, 2], [True, 5]])
+def test_tokens_in_every_form(tokens):
+    a = _token_array(tokens, 100)
+    assert a.dtype == np.int64 and a.tolist() == [int(t) for t in tokens]
+
+
+@pytest.mark.parametrize("tokens", [[1, -1], [5, 100], (2 ** 70, 1), np.array([3, 200]), torch.tensor([1, 100]), np.array([2 ** 63], np.uint64)])
+def test_tokens_outside_the_vocabulary(tokens):
+    with pytest.raises(ValueError):
+        _token_array(tokens, 100)
