@@ -34,7 +34,12 @@ class StepEntry:
 
 def _token_array(tokens: Sequence[int], vocab: int) -> np.ndarray:
     """``tokens`` as int64, all of them within the vocabulary."""
-    a = np.asarray(tokens) if isinstance(tokens, (list, tuple, range, np.ndarray)) else None
+    a = None
+    if type(tokens) in (list, tuple, range, np.ndarray):
+        try:
+            a = np.asarray(tokens)
+        except (TypeError, ValueError, RuntimeError):  # elements that are no arrays but have an ``int``: tensors on a GPU
+            pass
     if a is None or a.ndim != 1 or a.dtype.kind not in "iu":  # tensors, mixed or foreign integers: one by one
         ids = [int(t) for t in tokens]
         if any(not 0 <= t < vocab for t in ids):

@@ -42,3 +42,9 @@ def test_tokens_in_every_form(tokens):
 def test_tokens_outside_the_vocabulary(tokens):
     with pytest.raises(ValueError):
         _token_array(tokens, 100)
+
+
+@pytest.mark.parametrize("tokens", [[torch.tensor(3.0, requires_grad=True), 4], (torch.tensor([3]), torch.tensor([4]))])
+def test_tokens_that_are_no_arrays(tokens):
+    a = _token_array(tokens, 100)  # NumPy takes neither list as a column of integers, the first not at all
+    assert a.dtype == np.int64 and a.tolist() == [3, 4]

@@ -525,3 +525,14 @@ def test_qwen3_runs_through_the_same_engine():
         assert err.max() < 0.15, (portions, float(err.max()))  # e4m3 roundings flip with the summation order
     out = generate(eng, [toks[:20], toks[20:90], toks[:1]], 5)
     assert [len(o) for o in out] == [5, 5, 5] and not eng.seqs.live
+
+
+@pytest.mark.parametrize("form", [lambda t: list(t), lambda t: tuple(t[:, None]), lambda t: t])
+def test_tokens_on_the_gpu(form):
+    from flashrec_b200.engine import StepEntry
+
+    eng = engine("equal", torch.float32, reqs=2)
+    toks = torch.tensor([5, 199, 0, 17], device="cuda")
+    want = eng.step([StepEntry(0, toks.tolist(), [1, 3])])
+    assert torch.equal(eng.step([StepEntry(1, form(toks), [1, 3])]), want)
+    assert torch.equal(eng.step([StepEntry(0, form(toks[:1]), [0])]), eng.step([StepEntry(1, [5], [0])]))
