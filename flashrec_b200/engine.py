@@ -107,8 +107,9 @@ class LMEngine:
             raise RuntimeError(f"a request would exceed {self.max_seq} tokens")
         vocab = self.model.vocab
         one = all(len(e.tokens) == 1 for e in entries)
-        if one:
-            if any(not 0 <= int(e.tokens[0]) < vocab for e in entries):
+        if one:  # `tokens` need not be subscripted from 0: a set, a column of a table
+            ids = [int(t) for e in entries for t in e.tokens]
+            if any(not 0 <= t < vocab for t in ids):
                 raise ValueError("token id outside the vocabulary")
         else:  # prompts: columns of thousands of numbers are arrays
             ids = [_token_array(e.tokens, vocab) for e in entries]
@@ -127,14 +128,13 @@ class LMEngine:
             seq = self.seqs.live[e.req]
             n, first = len(e.tokens), seq.length
             start[i] = t0
+            toks.append(ids[i])
             if one:
-                toks.append(int(e.tokens[0]))
                 loc += self.seqs.extend(e.req, 1)
                 pos.append(first)
                 tok_req.append(b)
                 rows.append(seq.row)
             else:
-                toks.append(ids[i])
                 loc.append(self.seqs.extend_array(e.req, n))
                 pos.append(np.arange(first, first + n, dtype=np.int64))
             req_rows.append(seq.row)

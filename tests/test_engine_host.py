@@ -48,3 +48,16 @@ def test_tokens_outside_the_vocabulary(tokens):
 def test_tokens_that_are_no_arrays(tokens):
     a = _token_array(tokens, 100)  # NumPy takes neither list as a column of integers, the first not at all
     assert a.dtype == np.int64 and a.tolist() == [3, 4]
+
+
+def test_single_tokens_in_every_container(monkeypatch):
+    from types import SimpleNamespace
+
+    from flashrec_b200.engine import LMEngine, StepEntry
+
+    model = SimpleNamespace(device="cpu", vocab=100, cache_specs=[CacheSpec(8, 8)], new_caches=lambda *_: None)
+    eng = LMEngine(model, 256, 4)
+    got = []
+    monkeypatch.setattr(LMEngine, "_decode", lambda self, toks, *_: got.append(list(toks)) or torch.zeros(0, 100))
+    eng.step([StepEntry(i, t) for i, t in enumerate(([7], {8}, {9: "x"}.keys(), torch.tensor([10])))])
+    assert got == [[7, 8, 9, 10]]
