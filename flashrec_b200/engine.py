@@ -21,6 +21,10 @@ from flashrec_b200.lm_layers import ROW_PORTION
 from flashrec_b200.sampling import Sampler, SamplingParams
 
 TILE_ROWS = 128          # tokens per tensor-core attention tile
+# Tokens from which an entry's columns are arrays of its own; shorter ones share lists, steps without a longer one altogether. An
+# array costs 8 us to set up and a step with any 20 us more, a place in the lists 0.2 (255 entries of one token beside a prompt of
+# 512: 0.9 ms, 3.0 with an array each; one prompt of 64: 28 us, 53 with an array).
+ARRAY_TOKENS = 128
 
 
 @dataclass
@@ -90,6 +94,12 @@ class LMEngine:
             return False
         return length + n <= self.max_seq and self.seqs.pages_needed(length, n) <= self.seqs.free_pages
 
+    @staticmethod
+    def _close_run(parts: List[Tuple[np.ndarray, np.ndarray]], toks: List[int], loc: List[int]) -> Tuple[List[int], List[int]]:
+        if toks:
+            parts.append((np.array(toks, dtype=np.int64), np.array(loc, dtype=np.int64)))
+        return [], []
+
     # -- one step ---------------------------------------------------------------------------------------
     def step(self, entries: Sequence[StepEntry], on_layer=None) -> torch.Tensor:
         """Runs the entries' tokens; fp32 logits [wanted, vocab] in the order of entries and of ``want``. New
@@ -107,18 +117,18 @@ class LMEngine:
             raise RuntimeError(f"a request would exceed {self.max_seq} tokens")
         vocab = self.model.vocab
         one = all(len(e.tokens) == 1 for e in entries)
-        if one:  # `tokens` need not be subscripted from 0: a set, a column of a table
-            ids = [int(t) for e in entries for t in e.tokens]
-            if any(not 0 <= t < vocab for t in ids):
-                raise ValueError("token id outside the vocabulary")
-        else:  # prompts: columns of thousands of numbers are arrays
-            ids = [_token_array(e.tokens, vocab) for e in entries]
+        arrays = any(len(e.tokens) >= ARRAY_TOKENS for e in entries)
+        # tokens need not be subscripted from 0: a set, a column of a table
+        ids = [_token_array(e.tokens, vocab) if len(e.tokens) >= ARRAY_TOKENS else [int(t) for t in e.tokens] for e in entries]
+        if any(not 0 <= t < vocab for i in ids if type(i) is list for t in i):
+            raise ValueError("token id outside the vocabulary")
         if any(not 0 <= int(w) < len(e.tokens) for e in entries for w in e.want):
             raise ValueError("want: place outside the entry's tokens")
         # short portions first: their attention runs row by row, the rest in tiles
         order = sorted(range(len(entries)), key=lambda i: len(entries[i].tokens) > ROW_PORTION)
         start: Dict[int, int] = {}
         toks, pos, loc, tok_req, rows, req_rows, qo, pre, ext = [], [], [], [], [], [], [0], [], []
+        parts: List[Tuple[np.ndarray, np.ndarray]] = []  # tokens and slots: an entry that is an array, or a run of short ones
         tiles: List[Tuple[int, int, int]] = []
         n_row = t0 = 0
         for b, i in enumerate(order):
@@ -128,15 +138,16 @@ class LMEngine:
             seq = self.seqs.live[e.req]
             n, first = len(e.tokens), seq.length
             start[i] = t0
-            toks.append(ids[i])
-            if one:
-                loc += self.seqs.extend(e.req, 1)
-                pos.append(first)
-                tok_req.append(b)
-                rows.append(seq.row)
+            if n >= ARRAY_TOKENS:
+                toks, loc = self._close_run(parts, toks, loc)
+                parts.append((ids[i], self.seqs.extend_array(e.req, n)))
             else:
-                loc.append(self.seqs.extend_array(e.req, n))
-                pos.append(np.arange(first, first + n, dtype=np.int64))
+                toks += ids[i]
+                loc += self.seqs.extend(e.req, n)
+                if not arrays:
+                    pos += range(first, first + n)
+                    tok_req += [b] * n
+                    rows += [seq.row] * n
             req_rows.append(seq.row)
             qo.append(t0 + n)
             pre.append(first)
@@ -146,8 +157,10 @@ class LMEngine:
             else:
                 tiles += [(b, t0 + s, min(TILE_ROWS, n - s)) for s in range(0, n, TILE_ROWS)]
             t0 += n
-        if not one:
-            toks, loc, pos = np.concatenate(toks), np.concatenate(loc), np.concatenate(pos)
+        if arrays:
+            self._close_run(parts, toks, loc)
+            toks, loc = (np.concatenate([p[c] for p in parts]) for c in (0, 1))
+            pos = np.arange(t0) + np.repeat(np.array(pre) - np.array(qo[:-1]), ext)
             tok_req, rows = np.repeat(np.arange(len(ext)), ext), np.repeat(req_rows, ext)
         want = [start[i] + int(w) for i, e in enumerate(entries) for w in e.want]
         if one and self.use_graphs and on_layer is None and len(entries) <= self.GRAPH_SIZES[-1]:

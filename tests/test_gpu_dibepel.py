@@ -527,12 +527,13 @@ def test_qwen3_runs_through_the_same_engine():
     assert [len(o) for o in out] == [5, 5, 5] and not eng.seqs.live
 
 
+@pytest.mark.parametrize("n", [4, 200])
 @pytest.mark.parametrize("form", [lambda t: list(t), lambda t: tuple(t[:, None]), lambda t: t])
-def test_tokens_on_the_gpu(form):
+def test_tokens_on_the_gpu(form, n):
     from flashrec_b200.engine import StepEntry
 
     eng = engine("equal", torch.float32, reqs=2)
-    toks = torch.tensor([5, 199, 0, 17], device="cuda")
-    want = eng.step([StepEntry(0, toks.tolist(), [1, 3])])
-    assert torch.equal(eng.step([StepEntry(1, form(toks), [1, 3])]), want)
+    toks = (torch.arange(n, device="cuda") * 67 + 5) % 200
+    want = eng.step([StepEntry(0, toks.tolist(), [1, n - 1])])
+    assert torch.equal(eng.step([StepEntry(1, form(toks), [1, n - 1])]), want)
     assert torch.equal(eng.step([StepEntry(0, form(toks[:1]), [0])]), eng.step([StepEntry(1, [5], [0])]))
