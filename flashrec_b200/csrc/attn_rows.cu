@@ -202,8 +202,9 @@ flash_rows_kernel(const __grid_constant__ fr_mix_attn a, int row0, int max_keys,
       if (a.slopes != nullptr && s % REP < rep) v -= a.slopes[source_of(a, MAPS * g + s / REP, s % REP)] * dist;
       v = lane < nk ? v : -INFINITY;
       const float mn = fmaxf(m[s], warp_max(v));
-      const float corr = expf(m[s] - mn);  // 0 for the first block
-      p[s] = lane < nk ? expf(v - mn) : 0.f;
+      // scores of -inf (behind the last key, or an infinite key) weigh nothing, also while no finite one has been seen
+      const float corr = m[s] == -INFINITY ? 0.f : expf(m[s] - mn);
+      p[s] = v == -INFINITY ? 0.f : expf(v - mn);
       l[s] = l[s] * corr + p[s];
       m[s] = mn;
 #pragma unroll
@@ -231,7 +232,8 @@ flash_rows_kernel(const __grid_constant__ fr_mix_attn a, int row0, int max_keys,
     }
   }
   __syncthreads();
-  auto weight = [](float mw, float mx) { return mw == -INFINITY ? 0.f : expf(mw - mx); };  // no keys: no share
+  // no key above -inf: no share. Its sums are zero then, or NaN from a NaN score, which has to reach the output.
+  auto weight = [](float mw, float mx) { return mw == -INFINITY ? 0.f : expf(mw - mx); };
   if (tid < NS) {
     float mx = m_w[0][tid], ls = 0.f;
     for (int w = 1; w < kFlashWarps; ++w) mx = fmaxf(mx, m_w[w][tid]);
@@ -247,10 +249,7 @@ flash_rows_kernel(const __grid_constant__ fr_mix_attn a, int row0, int max_keys,
   for (int c = tid; c < NS * VP; c += kFlashWarps * 32) {
     float v = 0.f;
 #pragma unroll
-    for (int w = 0; w < kFlashWarps; ++w) {
-      const float f = m_w[w][c / VP];
-      v += f == 0.f ? 0.f : o_w[w][c] * f;
-    }
+    for (int w = 0; w < kFlashWarps; ++w) v += o_w[w][c] * m_w[w][c / VP];
     o_w[0][c] = v;
   }
   if (splits > 1) cluster_sync(); else __syncthreads();
@@ -284,10 +283,8 @@ flash_rows_kernel(const __grid_constant__ fr_mix_attn a, int row0, int max_keys,
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
           const float w = weight(mc[c], mx);
-          if (w != 0.f) {
-            ls += lc[c] * w;
-            os += oc[c] * w;
-          }
+          ls += lc[c] * w;
+          os += oc[c] * w;
         }
         f += (mp == 0 ? 1.0f : -a.lambda) * (os / ls);
       }

@@ -9,7 +9,7 @@ pytestmark = pytest.mark.gpu
 PAGE = 64
 
 
-def _run(kind, dtype, heads, kv, dim, vdim, lens, window, keep, seed):
+def _run(kind, dtype, heads, kv, dim, vdim, lens, window, keep, seed, edit=None):
     """One query per request, at the last of its ``lens`` tokens; [rows, heads * vdim] as float."""
     from flashrec_b200.core import ForwardBatch
     from flashrec_b200.kvcache import CacheSpec
@@ -25,6 +25,8 @@ def _run(kind, dtype, heads, kv, dim, vdim, lens, window, keep, seed):
         at += p
     slots = sum(pages) * PAGE
     q, k, v = rnd(n, heads * maps * dim), rnd(slots, kv * maps * dim), rnd(slots, kv * vdim)
+    if edit is not None:
+        edit(q, k, table[1:].long())
     coef, gate = 0.5 * torch.randn(heads, heads, generator=g), torch.randn(n, heads, generator=g)
     spec = CacheSpec(0, 0, mask="chunk" if kind == "talk" else "window", size=window, keep_first=keep)
     attn = MixAttention(kind, heads, kv, dim, vdim, dim ** -0.5, spec, eps=1e-5, lam=0.4, out_scale=0.8,
@@ -53,3 +55,20 @@ def test_rows_match_the_general_kernels(kind, heads, kv, dim, vdim, lens, window
     # a unit in the last place, 2^-8 of it, and sums in another order move the norm by a few 1e-6
     err = (got - ref).norm(dim=1) / ref.norm(dim=1)
     assert err.max() < 2 ** -8 + 1e-4, (int(err.argmax()), float(err.max()))
+
+
+@pytest.mark.parametrize("kind", ["diff", "talk", "plain"])
+@pytest.mark.parametrize("value", [float("-inf"), float("nan")])
+@pytest.mark.parametrize("n,at", [(33, [32]), (97, [96]), (100, list(range(32))), (300, [40, 299]), (1100, [1099]), (1100, list(range(160, 192)))])
+def test_keys_that_are_not_finite(kind, value, n, at):
+    """Keys whose score is -inf weigh nothing, wherever the first of them stands in the walk; a NaN reaches the output."""
+    def edit(q, k, slots):
+        q[:, ::64] = q[:, ::64].abs() + 0.5
+        for p in at:
+            k[slots[0][p], ::64] = value
+
+    got, ref = (_run(kind, d, 4, 2, 64, 64, (n, 20), 4096, 0, 5, edit) for d in (torch.bfloat16, torch.float32))
+    bad = torch.isnan(ref[0]).all() if value != value else torch.isfinite(ref[0]).all()
+    assert bad and torch.equal(torch.isnan(got), torch.isnan(ref))
+    got, ref = got.nan_to_num(0.0), ref.nan_to_num(0.0)
+    assert ((got - ref).norm(dim=1) <= (2 ** -8 + 1e-4) * ref.norm(dim=1)).all()
