@@ -467,8 +467,8 @@ update_norm_kernel(const __grid_constant__ fr_norm_update u, int W) {
     float4 v[NV], y[kP][NV];
     float ss[kP] = {};
     // EARLY (few rows, bound by the chain of loads and sums): every load of the row goes out before the first sum, without a
-    // branch between them; what is not there is read from the row itself and dropped (one row of 2048 with a part: 6.3 -> 3.1 us,
-    // 48 rows 4.1 -> 2.4)
+    // branch between them; what is not there is read from the row itself and dropped (2048 columns of bf16, a part, operands in
+    // L2: one row 2.56 -> 1.80 us, 48 rows 2.78 -> 1.93)
     float4 pw[EARLY ? kP : 1][EARLY ? NV : 1], ww[EARLY ? NV : 1], ad[EARLY ? NV : 1];
     if constexpr (EARLY) {
       const float* wp = u.weight != nullptr ? u.weight : xr;
@@ -615,13 +615,21 @@ update_norm_kernel(const __grid_constant__ fr_norm_update u, int W) {
 template <typename T, int NP, bool SHARES, bool EARLY>
 static int launch_update_norm_vec(const fr_norm_update& u, int M, int W, cudaStream_t stream) {
   const bool pdl = M <= kPdlRows;
-  if (W <= 512) return launch_kernel(update_norm_kernel<T, 128, 1, NP, SHARES, EARLY>, M, 128, 0, stream, pdl, u, W);
-  // few rows: latency; two parts: registers
-  if ((pdl || NP > 0) && W <= 2048) return launch_kernel(update_norm_kernel<T, 256, 2, NP, SHARES, EARLY>, M, 256, 0, stream, pdl, u, W);
-  if (W <= 2048) return launch_kernel(update_norm_kernel<T, 128, 4, NP, SHARES, EARLY>, M, 128, 0, stream, pdl, u, W);
-  if (NP > 0 && W <= 4096) return launch_kernel(update_norm_kernel<T, 512, 2, NP, SHARES, EARLY>, M, 512, 0, stream, pdl, u, W);
-  if (W <= 4096) return launch_kernel(update_norm_kernel<T, 256, 4, NP, SHARES, EARLY>, M, 256, 0, stream, pdl, u, W);
-  return launch_kernel(update_norm_kernel<T, 512, 4, NP, SHARES, EARLY>, M, 512, 0, stream, pdl, u, W);
+  auto run = [&](auto kern, int threads) { return launch_kernel(kern, M, threads, 0, stream, pdl, u, W); };
+  if (W <= 512) return run(update_norm_kernel<T, 128, 1, NP, SHARES, EARLY>, 128);
+  if constexpr (EARLY || NP > 0) {  // few rows: latency; parts: registers
+    if (W <= 2048) return run(update_norm_kernel<T, 256, 2, NP, SHARES, EARLY>, 256);
+  } else {
+    if (W <= 2048 && pdl) return run(update_norm_kernel<T, 256, 2, NP, SHARES, EARLY>, 256);
+    if (W <= 2048) return run(update_norm_kernel<T, 128, 4, NP, SHARES, EARLY>, 128);
+  }
+  if constexpr (NP > 0) {
+    if (W <= 4096) return run(update_norm_kernel<T, 512, 2, NP, SHARES, EARLY>, 512);
+  } else {
+    if (W <= 4096) return run(update_norm_kernel<T, 256, 4, NP, SHARES, EARLY>, 256);
+  }
+  if constexpr (!EARLY || NP < 2) return run(update_norm_kernel<T, 512, 4, NP, SHARES, EARLY>, 512);
+  return FR_ERR_UNSUPPORTED;  // early loads of two parts are not taken above 4096 columns
 }
 
 template <typename T>
@@ -633,7 +641,15 @@ static int launch_update_norm(const fr_norm_update& u, int M, int W, cudaStream_
     vec = vec && u.parts[p].ldy % 4 == 0 && aligned16(u.parts[p].y) && aligned16(u.parts[p].weight);
     shares = shares || u.parts[p].n_splits > 0;
   }
-  if (vec && !shares && M <= kPdlRows) {
+  // Early loads hold a whole row in registers: they pay while the chain of loads is what costs, not where other rows of the SM
+  // would hide it. us before / with them:
+  //   no part     2048 columns: 512 rows 2.87 / 2.56, 2048 rows 7.30 / 6.65; 5120: 128 rows 2.69 / 2.32, 256 rows 2.96 / 3.71
+  //   one part    (its instance has no second part) 2048 columns, 2048 rows: 14.56 / 13.00; 8192: 69.84 / 48.05
+  //   two parts   512 columns, 2048 rows: 4.74 / 4.24; 2048: 256 rows 3.33 / 2.81, 512 rows 3.97 / 4.61; above 4096 they spill
+  //               (8192 columns of float, a row with partials: 6.05 / 7.33)
+  const int any_rows = u.n_parts == 0 ? 2048 : (u.n_parts == 1 ? INT32_MAX : 512);  // columns up to which rows do not matter
+  const bool early = M <= kPdlRows && (u.n_parts < 2 || W <= 4096) && (W <= any_rows || M <= 128 || static_cast<int64_t>(M) * W <= 1 << 19);
+  if (vec && !shares && early) {
     if (u.n_parts == 0) return launch_update_norm_vec<T, 0, false, true>(u, M, W, stream);
     if (u.n_parts == 1) return launch_update_norm_vec<T, 1, false, true>(u, M, W, stream);
     return launch_update_norm_vec<T, 2, false, true>(u, M, W, stream);

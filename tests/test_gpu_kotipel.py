@@ -112,6 +112,32 @@ def test_update_and_norm(dtype, w):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("m", [3, 128, 129, 300, 2049])
+@pytest.mark.parametrize("w", [512, 2048, 2052, 4096, 4100, 5120, 8192, 8196])
+def test_update_and_norm_at_the_lines_between_its_kernels(dtype, m, w):
+    from flashrec_b200.lm_layers import Partials, Pending, update_norm
+
+    g = torch.Generator(device="cuda").manual_seed(m + w)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    eps, wt, pend = 1e-3, r(w), r(2, m, w)
+    ys, wy, shares = [r(m, w).to(dtype) for _ in range(2)], [r(w) for _ in range(2)], r(4, m, w)
+    rms = lambda v: v * torch.rsqrt(v.pow(2).mean(-1, keepdim=True) + eps)  # noqa: E731
+    # parts of the update; a part given as shares of a split product; partials of the stream
+    for n_parts, as_shares, use_p in ((0, None, False), (0, None, True), (1, None, False), (1, 0, True), (2, None, True), (2, 0, False), (2, 1, False)):
+        x = r(m, w)
+        want = x.double() + (pend.double().sum(0) if use_p else 0)
+        parts = []
+        for i in range(n_parts):
+            y = Partials(shares, 4) if i == as_shares else ys[i]
+            want = want + (0.5, 1.0)[i] * rms(shares.double().sum(0) if i == as_shares else ys[i].double()) * wy[i].double()
+            parts.append((y, wy[i], (0.5, 1.0)[i]))
+        out = torch.empty((m, w), dtype=dtype, device="cuda")
+        update_norm(x, eps, out, wt, 0.25, Pending(Partials(pend, 2) if use_p else None, parts))
+        assert rel(x, want) < 3e-6
+        assert rel(out, rms(want) * (0.25 + wt.double())) < tol(dtype)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("m", [1, 7, 8, 9, 40, 200, 1500])
 @pytest.mark.parametrize("n,k", [(90, 96), (130, 1040), (2048, 512)])
 def test_products_that_update_copy_or_come_in_shares(dtype, m, n, k):
