@@ -907,14 +907,15 @@ static int launch_tc(TcArgs g, const fr_gated_part* parts, cudaStream_t stream) 
   return launch_kernel(kern, grid, kThreads, smem, stream, g.M <= kPdlRows, ta[0], tb[0], ta[1], tb[1], g, status);
 }
 
-// Tile width with the least work on the busiest SM: rounds of tiles times the rows of A and B that a tile brings in.
+// Tile width with the least work on the busiest SM: rounds of tiles times the rows of A and B that a tile brings in (`few`: of a
+// single row block only its own rows; the update in place brings in whole ones, 16 rows x 20480 x 2048: 32.0 us, 38.4 as if it did not).
 // 192 is for a single row block only: there it fills one round of SMs where 256 leaves many idle and 128 begins a second
 // (64 rows x 20480 x 2048: 17.9 us; 28 with 80 tiles of 256 and whole tiles of A).
-static int pick_block_n(int M, int N, bool any_width) {
-  const int64_t sms = device_sm_count(), mb = ceil_div(M, kBlockM), a_rows = M <= kBlockM ? Stages(M, 64).a_rows : kBlockM;
+static int pick_block_n(int M, int N, bool few) {
+  const int64_t sms = device_sm_count(), mb = ceil_div(M, kBlockM), a_rows = few && M <= kBlockM ? Stages(M, 64).a_rows : kBlockM;
   int best = 0;
   int64_t best_cost = 0;
-  for (int bn = 256; bn >= 64; bn -= bn == 128 ? 64 : (any_width && M <= kBlockM ? 64 : 128)) {
+  for (int bn = 256; bn >= 64; bn -= bn == 128 ? 64 : (few && M <= kBlockM ? 64 : 128)) {
     const int64_t cost = (mb * ceil_div(N, bn) + sms - 1) / sms * (a_rows + bn);
     if (best == 0 || cost < best_cost) {
       best = bn;
