@@ -13,6 +13,8 @@
 #include "linear_scan.cuh"
 #include "sm100_ptx.cuh"
 
+#include <algorithm>
+
 namespace fr {
 namespace scan {
 
@@ -26,7 +28,9 @@ struct RowsPlan {
   int smem;
 };
 
-// MAXT: threads of a CTA at most; 256 leaves the registers that keep the state's loads in flight
+// MAXT: threads of a CTA at most. 256 (80 registers) keeps the state's loads in flight while the first tokens are staged; 1024 (64
+// registers) waits for them first: held longer they spill, and rows of 1024 x 32 took 10.83 -> 11.30 us, f32 prompts of 512 x 64
+// with channel decays 7.17 -> 7.35 ms.
 template <typename T, bool CHANNEL, int MAXT>
 __global__ void __launch_bounds__(MAXT, MAXT == 256 ? 3 : 1)
 scan_rows_kernel(const __grid_constant__ fr_linear_scan a, const RowsPlan pl, int min_tokens, int max_tokens,
@@ -44,7 +48,7 @@ scan_rows_kernel(const __grid_constant__ fr_linear_scan a, const RowsPlan pl, in
   const int b = blockIdx.z, h = blockIdx.y, c0 = blockIdx.x * pl.vb, tid = threadIdx.x, nt = blockDim.x;
   // One token per request (decode) is bound by the state, read and written once, so everything that leads to its loads and
   // the loads themselves go out before anything is waited for; whether position 0 makes the state zero is decided after
-  // (48 requests, 64 heads of 128 x 64: 47.7 -> 36.4 us, 5.5 TB/s; 16 heads of 64 x 128 with channel decays 18.8 -> 16.1).
+  // (48 requests, 64 heads of 128 x 64: 54.3 -> 42.1 us; 16 heads of 64 x 128 with channel decays 21.3 -> 18.2).
   const int64_t state_row = a.state_slots[b];
   const int q0 = a.qo_indptr[b], q1 = a.qo_indptr[b + 1];
   if (q0 >= q1 || q1 - q0 > max_tokens || q1 - q0 < min_tokens) return;
@@ -54,11 +58,24 @@ scan_rows_kernel(const __grid_constant__ fr_linear_scan a, const RowsPlan pl, in
   const bool active = rg < rg_n;
   const float skip = a.skip != nullptr ? a.skip[h] : 0.f;
   float* st = a.state + ((state_row * a.heads + h) * np + rg * kRows) * static_cast<int64_t>(vp) + c0 + cq * kCols;
+  constexpr bool kEarly = MAXT == 256;
+  const bool load = active && (kEarly || a.pos[q0] > 0);
   float4 s_in[kRows];
 #pragma unroll
   for (int r = 0; r < kRows; ++r)
-    s_in[r] = active ? *reinterpret_cast<const float4*>(st + static_cast<int64_t>(r) * vp) : make_float4(0, 0, 0, 0);
-  const bool fresh = a.pos[q0] <= 0;
+    s_in[r] = load ? *reinterpret_cast<const float4*>(st + static_cast<int64_t>(r) * vp) : make_float4(0, 0, 0, 0);
+  uint64_t s2[kRows / 2][kCols];  // pairs of rows
+  auto pack = [&](bool fresh) {
+    const float4 zero = make_float4(0, 0, 0, 0);
+#pragma unroll
+    for (int r = 0; r < kRows / 2; ++r) {
+      const float4 lo = fresh ? zero : s_in[2 * r], hi = fresh ? zero : s_in[2 * r + 1];
+      s2[r][0] = pack2(lo.x, hi.x); s2[r][1] = pack2(lo.y, hi.y);
+      s2[r][2] = pack2(lo.z, hi.z); s2[r][3] = pack2(lo.w, hi.w);
+    }
+  };
+  const bool fresh = kEarly && a.pos[q0] <= 0;
+  if constexpr (!kEarly) pack(false);
   const T* qp = static_cast<const T*>(a.q);
   const T* kp = static_cast<const T*>(a.k);
   const T* vpt = static_cast<const T*>(a.v);
@@ -82,18 +99,13 @@ scan_rows_kernel(const __grid_constant__ fr_linear_scan a, const RowsPlan pl, in
       for (int tt = tid; tt < n; tt += nt) s_a[tt] = expf(-a.rate[h] * head_step(a, t0 + tt, h));
     __syncthreads();
   };
-  stage(q0, min(pl.tb, q1 - q0));
-  uint64_t s2[kRows / 2][kCols];  // pairs of rows
-#pragma unroll
-  for (int r = 0; r < kRows / 2; ++r) {
-    const float4 zero = make_float4(0, 0, 0, 0);
-    const float4 lo = fresh ? zero : s_in[2 * r], hi = fresh ? zero : s_in[2 * r + 1];
-    s2[r][0] = pack2(lo.x, hi.x); s2[r][1] = pack2(lo.y, hi.y);
-    s2[r][2] = pack2(lo.z, hi.z); s2[r][3] = pack2(lo.w, hi.w);
+  if constexpr (kEarly) {
+    stage(q0, min(pl.tb, q1 - q0));
+    pack(fresh);
   }
   for (int t0 = q0; t0 < q1; t0 += pl.tb) {
     const int n = min(pl.tb, q1 - t0);
-    if (t0 != q0) stage(t0, n);
+    if (!kEarly || t0 != q0) stage(t0, n);
     if (active) {
       for (int tt = 0; tt < n; ++tt) {
         const ulonglong2* kr = reinterpret_cast<const ulonglong2*>(s_k + tt * np + rg * kRows);
@@ -175,7 +187,13 @@ static int launch_rows(const fr_linear_scan& a, int n_req, int min_tokens, int m
   FR_CHECK_SUPPORTED(plan_rows(a, max_tokens, &pl));
   static PerDeviceFlag f, f1;
   const dim3 grid(state_cols(a.vdim) / pl.vb, a.heads, n_req);
-  if (pl.threads <= 256) {
+  // With channel decays arithmetic counts too, and a second round of CTAs costs more than what the wider instance gains: 64 heads of
+  // 128 x 64, 8 requests of 8 tokens, 1024 CTAs of 128 threads: 44.2 us at 64 registers, 52.1 at 80; 16 heads of 256 x 128, 8
+  // requests of one token, 512 CTAs of 256 threads: 14.1 and 15.0.
+  const int64_t ctas = static_cast<int64_t>(grid.x) * grid.y * grid.z, sms = device_sm_count();
+  auto at_once = [&](int regs) { return sms * std::min(65536 / (regs * pl.threads), (227 * 1024) / (pl.smem + 1024)); };
+  const bool one_round_at_64 = CHANNEL && ctas > at_once(80) && ctas <= at_once(64);
+  if (pl.threads <= 256 && !one_round_at_64) {
     auto kern = scan_rows_kernel<T, CHANNEL, 256>;
     if (ensure_dyn_smem(f, kern, 200 * 1024) != FR_OK) return FR_ERR_CUDA;
     return launch_kernel(kern, grid, pl.threads, pl.smem, stream, pdl, a, pl, min_tokens, max_tokens, flags);

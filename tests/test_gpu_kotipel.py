@@ -333,6 +333,13 @@ def test_recurrences_in_segments(case):
     _check_scan(torch.bfloat16, case, [2100, 700, 1030], ((2100,), (1200, 9, 1500)))
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("case", [("head", 2, 1, 320, 32, 0.1), ("head", 1, 1, 1024, 32, 0.05), ("channel", 2, 2, 384, 64, 0.05), ("channel", 160, 160, 128, 64, 0.05)])
+def test_recurrences_of_large_states_and_of_many_heads(dtype, case):
+    """CTAs of more than 256 threads, and as many CTAs as fit at once only with fewer registers each."""
+    _check_scan(dtype, case, [8, 8, 5], ((8,), (3, 1, 4)))
+
+
 def _check_scan(dtype, case, lens, cuts):
     from flashrec_b200.kvcache import CacheSpec
     from flashrec_b200.lm_layers import LinearScan
