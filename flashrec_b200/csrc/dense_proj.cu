@@ -466,11 +466,19 @@ constexpr int kEpiWarps = 8;
 constexpr int kThreads = 64 + kEpiWarps * 32;
 enum Epi { kEpiSegs = 0, kEpiAdd = 1, kEpiPartial = 2 };
 
-template <int BLOCK_N>
+// Rows a kernel is made for. kAny: stage sizes are constants (a full tile's products take longer than the hand-over, and the
+// issuing thread has no time to spare: run-time sizes cost 8192 rows 4 %). kFew: at most 128 rows, stages as planned at launch.
+// kOctet: at most 8 rows, which the row kernel sums in fp32 FMAs otherwise. The tensor cores' accumulation loses bits with
+// every product added (2.1e-6 of the norm at K = 2048, 1.4e-5 at 12288, where the row kernel has 8e-8 and 9e-8), so here it
+// spans one k-block only: the four blocks of a stage go to four accumulators, which a warp adds up in fp32 registers.
+enum Rows { kAny = 0, kFew = 1, kOctet = 2 };
+
+template <int BLOCK_N, int ROWS>
 struct Cfg {
   static constexpr int kStageBytes = (kBlockM + BLOCK_N) * kBlockK * 2;
   static constexpr int kStages = BLOCK_N == 256 ? 4 : (BLOCK_N == 128 ? 6 : 8);
-  static constexpr int kTmemCols = BLOCK_N <= 64 ? 128 : (BLOCK_N == 128 ? 256 : 512);  // a power of two
+  static constexpr int kAcc = ROWS == kOctet ? 8 : 2;  // accumulators in TMEM
+  static constexpr int kTmemCols = kAcc * BLOCK_N <= 128 ? 128 : (kAcc * BLOCK_N <= 256 ? 256 : 512);  // a power of two
 };
 
 // Operand stages of a few rows (one row block). They bring in only themselves: an SM pulls operands at about 48 bytes per
@@ -483,6 +491,8 @@ constexpr int kTileA = kBlockM * kBlockK * 2;
 constexpr int kMaxStages = 12;
 constexpr int kOperandBytes = 200 * 1024;
 constexpr int kBarBytes = (2 * kMaxStages + 4) * 8 + 16;
+constexpr int kOctetBlocks = 4;  // k-blocks of a stage of kOctet
+constexpr int kOctetBytes = 2 * 8 * 64 * 4 + 16;  // its finished tiles on their way out, two of [8][64], and whether they are whole
 struct Stages {
   int a_rows, a_bytes, block_bytes, blocks, n, smem;  // blocks: k-blocks of a stage, each [A rows | weight rows]
   __host__ Stages(int M, int block_n) {  // M <= 128
@@ -583,21 +593,42 @@ __device__ __forceinline__ void store32_f32(float* dst, const float (&v)[32], in
   }
 }
 
-// FEW: at most 128 rows, stages as planned at launch; otherwise their sizes are constants (a full tile's products take
-// longer than the hand-over, and the issuing thread has no time to spare: run-time sizes cost 8192 rows 4 %).
-template <int BLOCK_N, int EPI, bool FEW>
+// Stores the 64 columns of kOctet's tile ([8][64] in shared memory) that begin at n0; thread `t` of `nt`.
+template <int EPI>
+__device__ __forceinline__ void finish_octet(const TcArgs& g, const Job& j, int n0, const float* v, int t, int nt) {
+#pragma unroll 1
+  for (int e = t; e < g.M * 64; e += nt) {
+    const int row = e / 64, c = e % 64, col = n0 + c;
+    if (col >= g.N) continue;
+    if constexpr (EPI == kEpiSegs) {
+      const fr_out_segment& s = g.segs.s[seg_of(g.segs, col)];
+      if (!paired(s))
+        seg_write<__nv_bfloat16, true>(s, row, col - s.n0, v[e]);
+      else if (c < 32)
+        seg_write<__nv_bfloat16, true>(s, row, (n0 - s.n0) / 2 + c, pair_act<true>(s, v[e], v[e + 32]));
+    } else {
+      const __nv_bfloat16* gp = g.gate[j.part];
+      const float gt = gp != nullptr ? __bfloat162float(gp[row * g.ldg[j.part] + col]) : 1.0f;
+      g.partials[(static_cast<int64_t>(j.slot) * g.M + row) * g.N + col] = gt * v[e];
+    }
+  }
+}
+
+template <int BLOCK_N, int EPI, int ROWS>
 __global__ void __launch_bounds__(kThreads, 1)
 dense_tc_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUtensorMap tb0,
                 const __grid_constant__ CUtensorMap ta1, const __grid_constant__ CUtensorMap tb1,
                 const __grid_constant__ TcArgs g, int* status) {
-  using C = Cfg<BLOCK_N>;
+  using C = Cfg<BLOCK_N, ROWS>;
+  constexpr bool FEW = ROWS != kAny;
+  static_assert(ROWS != kOctet || (BLOCK_N == 64 && EPI != kEpiAdd), "");
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = ptx::smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* smem = smem_raw + (base - raw);
   const uint32_t n_stages = FEW ? g.stages : C::kStages, block_bytes = FEW ? g.block_bytes : C::kStageBytes;
   const uint32_t a_bytes = FEW ? g.a_bytes : kTileA;
-  const int stage_blocks = FEW && BLOCK_N <= 128 ? g.stage_blocks : 1;
+  const int stage_blocks = ROWS == kOctet ? kOctetBlocks : (FEW && BLOCK_N <= 128 ? g.stage_blocks : 1);
   const uint32_t stage_bytes = stage_blocks * block_bytes;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + n_stages * stage_bytes + (kTileA - a_bytes));
   const uint32_t bar_full = ptx::smem_u32(bars);
@@ -606,6 +637,7 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
   const uint32_t bar_tempty = bar_tfull + 16;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kMaxStages + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  float* octet = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + kBarBytes);  // kOctet
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m_blocks = (g.M + kBlockM - 1) / kBlockM;
@@ -620,7 +652,7 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
     }
     for (int b = 0; b < 2; ++b) {
       ptx::mbar_init(bar_tfull + 8 * b, 1);
-      ptx::mbar_init(bar_tempty + 8 * b, kEpiWarps);
+      ptx::mbar_init(bar_tempty + 8 * b, ROWS == kOctet ? 1 : kEpiWarps);
     }
     *abort_flag = 0;
     ptx::mbar_init_fence();
@@ -670,14 +702,22 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
       bool ok = true;
       int it = 0;
       for (int unit = blockIdx.x; unit < num_units && ok; unit += gridDim.x) {
-        for (int sub = 0; sub < subs && ok; ++sub, ++it) {
+        for (int sub = 0; sub < subs && ok; ++sub) {
           const Job j = job_at<EPI>(g, unit, sub, m_blocks, n_blocks);
-          const uint32_t buf = it & 1;
-          ok = ptx::mbar_wait(bar_tempty + 8 * buf, ((it >> 1) & 1) ^ 1u, abort_flag, status, 62);
+          // a set of accumulators: of the whole job, or (kOctet) of one stage, one per k-block
+          uint32_t set = 0, d_tmem = 0;
+          auto next_set = [&]() {
+            set = it & 1;
+            d_tmem = tmem_base + set * (C::kAcc / 2 * BLOCK_N);
+            ok = ptx::mbar_wait(bar_tempty + 8 * set, ((it >> 1) & 1) ^ 1u, abort_flag, status, 62);
+            ++it;
+            if (ok) ptx::tc_fence_after();
+          };
+          if (ROWS != kOctet) next_set();
           if (!ok) break;
-          ptx::tc_fence_after();
-          const uint32_t d_tmem = tmem_base + buf * BLOCK_N;
           for (int kb0 = j.kb0; kb0 < j.kb1; kb0 += stage_blocks) {
+            if (ROWS == kOctet) next_set();
+            if (!ok) break;
             ok = ptx::mbar_wait(bar_full + 8 * stage, phase, abort_flag, status, 63);
             if (!ok) break;
             ptx::tc_fence_after();
@@ -688,16 +728,82 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
               const uint64_t b_desc = ptx::smem_desc_sw128(sa + a_bytes);
 #pragma unroll
               for (int k = 0; k < kBlockK / kUmmaK; ++k)
-                ptx::mma_f16(d_tmem, a_desc + 2u * k, b_desc + 2u * k, idesc, (kb > j.kb0 || k > 0) ? 1u : 0u);
+                ptx::mma_f16(d_tmem, a_desc + 2u * k, b_desc + 2u * k, idesc, ((ROWS != kOctet && kb > j.kb0) || k > 0) ? 1u : 0u);
+              if (ROWS == kOctet) d_tmem += BLOCK_N;
             }
             ptx::tc_commit(bar_empty + 8 * stage);
+            if (ROWS == kOctet) ptx::tc_commit(bar_tfull + 8 * set);
             if (++stage == n_stages) { stage = 0; phase ^= 1u; }
           }
-          if (ok) ptx::tc_commit(bar_tfull + 8 * buf);
+          if (ok && ROWS != kOctet) ptx::tc_commit(bar_tfull + 8 * set);
         }
       }
     }
     __syncwarp();
+  } else if (ROWS == kOctet) {
+    // Warp 4 adds up: TMEM lanes 0 .. 31 are open to it, and all rows lie in lanes 0 .. 7. The other seven store the tile that
+    // it has left in shared memory while it goes on with the next one; all eight meet once per tile.
+    bool ok = true;
+    int it = 0, tile = 0;
+    for (int unit = blockIdx.x; unit < num_units && ok; unit += gridDim.x) {
+      for (int sub = 0; sub < subs && ok; ++sub, ++tile) {
+        const Job j = job_at<EPI>(g, unit, sub, m_blocks, n_blocks);
+        float* out = octet + (tile & 1) * (8 * 64);
+        volatile int* whole = reinterpret_cast<volatile int*>(octet + 2 * 8 * 64) + (tile & 1);
+        if (warp == 4) {
+          float v[16] = {}, lost[16] = {};
+          for (int kb0 = j.kb0; kb0 < j.kb1; kb0 += kOctetBlocks, ++it) {
+            const uint32_t set = it & 1;
+            int okw = 0;
+            if (lane == 0) okw = ptx::mbar_wait(bar_tfull + 8 * set, (it >> 1) & 1, abort_flag, status, 64) ? 1 : 0;
+            okw = __shfl_sync(0xffffffffu, okw, 0);
+            if (!okw) { ok = false; break; }
+            ptx::tc_fence_after();
+            float sum[16];
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+              const int n = j.kb1 - kb0 - 2 * half;  // blocks left; what lies behind them is old and not added
+              if (n <= 0) break;
+              uint32_t r0[32], r1[32];
+              const uint32_t taddr = tmem_base + (set * kOctetBlocks + 2 * half) * BLOCK_N;
+              ptx::tmem_ld_16x256(taddr, r0);
+              ptx::tmem_ld_16x256(taddr + BLOCK_N, r1);
+              ptx::tmem_ld_wait();
+#pragma unroll
+              for (int i = 0; i < 16; ++i) {  // registers 4 x + 2 and 4 x + 3 hold rows 8 .. 15
+                const int x = i / 2 * 4 + i % 2;
+                const float two = __uint_as_float(r0[x]) + (n > 1 ? __uint_as_float(r1[x]) : 0.f);
+                sum[i] = half == 0 ? two : sum[i] + two;
+              }
+            }
+            ptx::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) ptx::mbar_arrive(bar_tempty + 8 * set);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {  // Knuth's two-sum: what the addition rounds away is kept beside it
+              const float t = v[i] + sum[i], z = t - v[i];
+              lost[i] += (v[i] - (t - z)) + (sum[i] - z);
+              v[i] = t;
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {  // row lane / 4, columns 8 i + 2 (lane % 4) and the one after
+            const float x = fabsf(v[2 * i]) < INFINITY ? v[2 * i] + lost[2 * i] : v[2 * i];
+            const float y = fabsf(v[2 * i + 1]) < INFINITY ? v[2 * i + 1] + lost[2 * i + 1] : v[2 * i + 1];
+            *reinterpret_cast<float2*>(out + (lane >> 2) * 64 + 8 * i + 2 * (lane & 3)) = make_float2(x, y);
+          }
+          if (lane == 0) *whole = ok ? 1 : 0;
+          __syncwarp();
+        }
+        // a tile that was given up (a wait that ran out) ends the loop for all eight warps alike
+        asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
+        ok = *whole != 0;
+        if (ok && warp != 4) {
+          const int w = warp - 2 - (warp > 4 ? 1 : 0);
+          finish_octet<EPI>(g, j, j.nb * BLOCK_N, out, w * 32 + lane, (kEpiWarps - 1) * 32);
+        }
+      }
+    }
   } else {
     const int quad = warp & 3;
     const int part_of_cols = (warp - 2) >> 2;  // two warps per lane quadrant: even / odd chunks
@@ -880,15 +986,16 @@ int make_tmap_bf16_2d(CUtensorMap* map, const void* ptr, uint64_t cols, uint64_t
   return r == CUDA_SUCCESS ? FR_OK : FR_ERR_CUDA;
 }
 
-template <int BLOCK_N, int EPI, bool FEW>
+template <int BLOCK_N, int EPI, int ROWS>
 static int launch_tc(TcArgs g, const fr_gated_part* parts, cudaStream_t stream) {
-  using C = Cfg<BLOCK_N>;
+  using C = Cfg<BLOCK_N, ROWS>;
+  constexpr bool FEW = ROWS != kAny;
   const Stages few(FEW ? g.M : kBlockM, BLOCK_N);
   g.a_bytes = few.a_bytes;
   g.block_bytes = few.block_bytes;
   g.stage_blocks = few.blocks;
   g.stages = few.n;
-  const int smem = FEW ? few.smem : 1024 + C::kStages * C::kStageBytes + kBarBytes;
+  const int smem = FEW ? few.smem + (ROWS == kOctet ? kOctetBytes : 0) : 1024 + C::kStages * C::kStageBytes + kBarBytes;
   CUtensorMap ta[2], tb[2];
   for (int p = 0; p < 2; ++p) {
     const fr_gated_part& q = parts[p < g.n_parts ? p : 0];
@@ -896,9 +1003,9 @@ static int launch_tc(TcArgs g, const fr_gated_part* parts, cudaStream_t stream) 
     if (st == FR_OK) st = make_tmap_bf16_2d(&tb[p], q.w, q.K, g.N, q.ldw, BLOCK_N);
     if (st != FR_OK) return st;
   }
-  auto kern = dense_tc_kernel<BLOCK_N, EPI, FEW>;
+  auto kern = dense_tc_kernel<BLOCK_N, EPI, ROWS>;
   static PerDeviceFlag attr_done;
-  if (ensure_dyn_smem(attr_done, kern, FEW ? 1024 + kOperandBytes + kTileA + kBarBytes : smem) != FR_OK) return FR_ERR_CUDA;
+  if (ensure_dyn_smem(attr_done, kern, FEW ? 1024 + kOperandBytes + kTileA + kBarBytes + kOctetBytes : smem) != FR_OK) return FR_ERR_CUDA;
   int* status = device_status_ptr();
   if (!status) return FR_ERR_CUDA;
   const int64_t units = static_cast<int64_t>(ceil_div(g.M, kBlockM)) * ceil_div(g.N, BLOCK_N) *
@@ -1054,19 +1161,20 @@ extern "C" int fr_dense_proj(int dtype, const void* a, int64_t lda, const void* 
   g.kb[0] = ceil_div(K, dense::kBlockK);
   g.segs = sg;
   fr_gated_part part{a, w, nullptr, lda, ldw, 0, K, 0};
+  if (M <= 8) return dense::launch_tc<64, dense::kEpiSegs, dense::kOctet>(g, &part, stream);
   const int block_n = dense::pick_block_n(M, N, true);
   if (M <= dense::kBlockM) {
     switch (block_n) {
-      case 256: return dense::launch_tc<256, dense::kEpiSegs, true>(g, &part, stream);
-      case 192: return dense::launch_tc<192, dense::kEpiSegs, true>(g, &part, stream);
-      case 128: return dense::launch_tc<128, dense::kEpiSegs, true>(g, &part, stream);
-      default: return dense::launch_tc<64, dense::kEpiSegs, true>(g, &part, stream);
+      case 256: return dense::launch_tc<256, dense::kEpiSegs, dense::kFew>(g, &part, stream);
+      case 192: return dense::launch_tc<192, dense::kEpiSegs, dense::kFew>(g, &part, stream);
+      case 128: return dense::launch_tc<128, dense::kEpiSegs, dense::kFew>(g, &part, stream);
+      default: return dense::launch_tc<64, dense::kEpiSegs, dense::kFew>(g, &part, stream);
     }
   }
   switch (block_n) {
-    case 256: return dense::launch_tc<256, dense::kEpiSegs, false>(g, &part, stream);
-    case 128: return dense::launch_tc<128, dense::kEpiSegs, false>(g, &part, stream);
-    default: return dense::launch_tc<64, dense::kEpiSegs, false>(g, &part, stream);
+    case 256: return dense::launch_tc<256, dense::kEpiSegs, dense::kAny>(g, &part, stream);
+    case 128: return dense::launch_tc<128, dense::kEpiSegs, dense::kAny>(g, &part, stream);
+    default: return dense::launch_tc<64, dense::kEpiSegs, dense::kAny>(g, &part, stream);
   }
 }
 
@@ -1135,12 +1243,13 @@ extern "C" int fr_dense_gated_add(int dtype, const fr_gated_part* parts, int n_p
     dense::plan_splits(M, N, g.kb[0], n_parts > 1 ? g.kb[1] : 0, &g.splits[0], &g.splits[1]);
     FR_CHECK_ARG(g.splits[0] > 0 && g.splits[0] + g.splits[1] == n_splits && (n_parts == 1 || g.splits[1] > 0));
     g.partials = partials;
-    return M <= dense::kBlockM ? dense::launch_tc<64, dense::kEpiPartial, true>(g, parts, stream)
-                               : dense::launch_tc<64, dense::kEpiPartial, false>(g, parts, stream);
+    if (M <= 8) return dense::launch_tc<64, dense::kEpiPartial, dense::kOctet>(g, parts, stream);
+    return M <= dense::kBlockM ? dense::launch_tc<64, dense::kEpiPartial, dense::kFew>(g, parts, stream)
+                               : dense::launch_tc<64, dense::kEpiPartial, dense::kAny>(g, parts, stream);
   }
   switch (dense::pick_block_n(M, N, false)) {
-    case 256: return dense::launch_tc<256, dense::kEpiAdd, false>(g, parts, stream);
-    case 128: return dense::launch_tc<128, dense::kEpiAdd, false>(g, parts, stream);
-    default: return dense::launch_tc<64, dense::kEpiAdd, false>(g, parts, stream);
+    case 256: return dense::launch_tc<256, dense::kEpiAdd, dense::kAny>(g, parts, stream);
+    case 128: return dense::launch_tc<128, dense::kEpiAdd, dense::kAny>(g, parts, stream);
+    default: return dense::launch_tc<64, dense::kEpiAdd, dense::kAny>(g, parts, stream);
   }
 }

@@ -48,3 +48,67 @@ def test_gated_update(m, n, ks):
     p = gated_add(x, parts, few_rows=True)
     got = x.double() + (p.buf.double().sum(0) if p is not None else 0)
     assert float((got - want).abs().max()) < 8 * max(ks) ** 0.5 * 2 ** -24 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("m", [3, 4, 5, 7, 8])
+@pytest.mark.parametrize("k", [2048, 2056, 12296])
+@pytest.mark.parametrize("n,pairs", [(2052, 0), (3080, 0), (4100, 0), (5156, 544), (9476, 0), (32, 4128)])
+def test_up_to_eight_rows_are_summed_in_fp32(m, k, n, pairs):
+    """Long products of few rows, on either side of the line between the row kernel and the tensor cores."""
+    from flashrec_b200 import device_status
+    from flashrec_b200.lm_layers import MergedProjection, interleave_rows
+
+    a, w = _rand(m, k, seed=m), _rand(n, k, seed=1) * k ** -0.5
+    proj = MergedProjection(k)
+    proj.add("store_f32", w)
+    outs = [torch.full((m, n), float("nan"), device="cuda")]
+    if pairs:
+        gate, up = _rand(pairs, k, seed=2) * k ** -0.5, _rand(pairs, k, seed=3) * k ** -0.5
+        proj.add("swiglu", interleave_rows(gate, up), n=pairs)
+        outs.append(torch.full((m, pairs), float("nan"), device="cuda").bfloat16())
+    proj.finish(torch.bfloat16, "cuda")
+    proj(a, outs)
+    ref = a.double() @ w.double().T
+    # the result's own rounding is 2^-24 of an element at most, 0.6 of that in the norm; sums of k products in fp32 add about as
+    # much, whatever k; accumulated in the tensor cores they would add 1e-9 of the norm per element of k, 2e-6 at the least here
+    assert float((outs[0].double() - ref).norm() / ref.norm()) < 2 * 2 ** -24
+    if pairs:
+        g, u = a.double() @ gate.double().T, a.double() @ up.double().T
+        want = torch.nn.functional.silu(g) * u
+        assert float(((outs[1].double() - want).abs() - 2 ** -8 * want.abs()).max()) < 1e-4
+    assert device_status() == (0, 0)
+
+
+@pytest.mark.parametrize("m", [5, 8])
+@pytest.mark.parametrize("n,ks", [(1056, (2056,)), (2048, (2048, 6144)), (4100, (12288,))])
+def test_updates_of_up_to_eight_rows_are_summed_in_fp32(m, n, ks):
+    from flashrec_b200 import device_status
+    from flashrec_b200.lm_layers import gated_add, split_product
+
+    parts = [(_rand(m, k, seed=k), _rand(n, k, seed=k + 1) * k ** -0.5, _rand(m, n + (-n) % 8, seed=k + 2)[:, :n]) for k in ks]
+    x = torch.zeros(m, n, device="cuda")
+    want = sum(g.double() * (a.double() @ w.double().T) for a, w, g in parts)
+    p = gated_add(x, parts, few_rows=True)
+    got = x.double() + (p.buf.double().sum(0) if p is not None else 0)
+    assert float((got - want).norm() / want.norm()) < 2 * 2 ** -24
+    p = split_product(*parts[0][:2])
+    want = parts[0][0].double() @ parts[0][1].double().T
+    assert p is None or float((p.buf.double().sum(0) - want).norm() / want.norm()) < 2 * 2 ** -24
+    assert device_status() == (0, 0)
+
+
+@pytest.mark.parametrize("m", [3, 8])
+@pytest.mark.parametrize("n", [1056, 6148])
+def test_few_rows_with_infinities_and_nan(m, n):
+    from flashrec_b200.lm_layers import MergedProjection
+
+    k = 4096
+    a, w = _rand(m, k, seed=m), (_rand(n, k, seed=1).abs() + 0.5) * k ** -0.5
+    a[0, 5], a[1, k - 1], a[2, 70], a[2, 4000] = float("inf"), float("-inf"), float("inf"), float("nan")
+    proj = MergedProjection(k)
+    proj.add("store_f32", w)
+    proj.finish(torch.bfloat16, "cuda")
+    out = torch.zeros((m, n), device="cuda")
+    proj(a, [out])
+    assert (out[0] == float("inf")).all() and (out[1] == float("-inf")).all() and out[2].isnan().all()
+    assert out[3:].isfinite().all()
