@@ -10,7 +10,7 @@
 //   dense_tc_kernel    bf16, persistent and warp-specialised like gemm_fp8.cu: warp 0 = TMA producer (128-byte
 //                      swizzle, 64 bf16 per row), warp 1 = tcgen05.mma issuer (kind::f16, M = 128, fp32
 //                      accumulators in TMEM, two buffers), warps 2..9 = epilogue
-//   dense_rows_kernel  M <= 8 (decode of one or two rows, few columns, f32): a warp streams four weight rows against all
+//   dense_rows_kernel  M <= 8 (decode of one or two rows, few columns, short K, f32): a warp streams four weight rows against all
 //                      M activations, so the weights cross HBM once; the warps of a CTA may split K
 //   dense_simt_kernel  f32 with more rows: tiles of 64 or 128 x 64, fp32 FMAs
 #include "fr_common.cuh"
@@ -1032,15 +1032,24 @@ static int pick_block_n(int M, int N, bool few) {
   return best;
 }
 
-// Whether a few-row product streams the weights through the row kernel. There a weight costs an FMA per row: one or two rows
-// hide them behind the loads, more do not, and the tensor cores take those where there are columns enough for tiles
-// (us for 20480 x 2048, rows 1 / 2 / 4 / 8: 15.6 / 19.4 / 30.5 / 60.0 here, 17.7 for any of them there).
-// Fewer columns than 64 tiles of 64 leave the tensor cores' loads to few SMs: three or four rows stay here up to that
-// (2048 x 2048: 5.4 against 9.0 us) unless K can be split over the SMs too.
-static bool use_rows(int dtype, int M, int N, bool split_k) {
+// Whether a few-row product streams the weights through the row kernel. There a weight costs an FMA per row, rows counted as 1, 2, 4
+// or 8: one or two hide them behind the loads, eight do not, four hardly. The tensor cores (kOctet) take 0.18 us per k-block and
+// round of tiles and 3 us more, whatever the rows. us, row kernel / tensor cores:
+//   8 rows   K = 2048: N = 1536 8.7 / 9.7, 4096 14.2 / 10.3, 20480 60 / 24; K = 4096: 2048 14.2 / 15.9, 2560 17.4 / 15.9; K = 8192:
+//            2560 25.7 / 27.7, 4096 35.6 / 28.1; K = 12288: 3072 37.6 / 39.2, 4096 44.7 / 39.6
+//   4 rows   K = 2048: 5120 10.2 / 10.2, 8192 14.1 / 10.9, 10240 (two rounds, the second nearly empty) 17.5 / 16.9, 20480 31 / 23;
+//            K = 8192: 6144 30.2 / 28.3, 10240 44.6 / 52.1, 14336 57.9 / 52.6
+// Below K = 2048 the row kernel's sums are the more accurate ones (6e-8 of the norm at 512, 8e-8 here; 7.5e-8 and 8e-8 at 2048,
+// 9.4e-8 and 8e-8 at 12288). With K split over the SMs (a launch that reads the shares follows; K is the sum over the parts):
+//   8 rows   K = 2048: 1056 7.9 / 7.2, 4096 16.6 / 11.8; K = 12288: 1056 16.5 / 12.9, 4096 48.6 / 30.6
+//   4 rows   K = 2048: 2048 7.7 / 8.4, 4096 9.1 / 11.5; K = 12288: 2048 17.0 / 18.4, 4096 29.1 / 30.4
+static bool use_rows(int dtype, int M, int N, int64_t K, bool split_k) {
   if (M > 8) return false;
-  if (dtype != 0 || M <= 2 || N <= 1024) return true;
-  return !split_k && M <= 4 && N <= 4096;
+  if (dtype != 0 || M <= 2 || N <= 1024 || K < 2048) return true;
+  if (split_k) return M <= 4;
+  if (M > 4) return N <= (K <= 6144 ? 2048 : 3072);
+  const int64_t tiles = ceil_div(N, 64), sms = device_sm_count(), rounds = ceil_div(tiles, sms);
+  return N <= 4096 || tiles * 5 < rounds * sms * 3;  // less than three fifths of the SMs busy
 }
 
 static int rows_ks(int N, int K) {
@@ -1137,7 +1146,7 @@ extern "C" int fr_dense_proj(int dtype, const void* a, int64_t lda, const void* 
   FR_CHECK_ARG(dense::operand_ok(a, lda, K) && dense::operand_ok(w, ldw, K) && N % 4 == 0);
   dense::Segs sg{};
   if (check_segs(segs, n_segs, N, &sg) != FR_OK) return FR_ERR_BAD_ARG;
-  if (algo == 0) algo = dense::use_rows(dtype, M, N, false) ? 1 : 2;
+  if (algo == 0) algo = dense::use_rows(dtype, M, N, K, false) ? 1 : 2;
   if (algo == 1) {
     FR_CHECK_SUPPORTED(M <= 8);
     return dtype == 0 ? dense::launch_rows_proj<__nv_bfloat16>(a, lda, w, ldw, M, N, K, sg, stream)
@@ -1195,7 +1204,7 @@ extern "C" int fr_dense_gated_add_splits(int dtype, int M, int N, int K0, int K1
 }
 
 extern "C" int fr_dense_few_row_splits(int dtype, int M, int N, int K0, int K1) {
-  if (dtype != 0 || M <= 0 || N <= 0 || K0 <= 0 || dense::use_rows(dtype, M, N, true)) return 0;
+  if (dtype != 0 || M <= 0 || N <= 0 || K0 <= 0 || dense::use_rows(dtype, M, N, static_cast<int64_t>(K0) + (K1 > 0 ? K1 : 0), true)) return 0;
   int a, b;
   dense::plan_splits(M, N, ceil_div(K0, dense::kBlockK), K1 > 0 ? ceil_div(K1, dense::kBlockK) : 0, &a, &b);
   return a + b;

@@ -155,7 +155,7 @@ class Partials:
 def gated_add(x: torch.Tensor, parts: Sequence[Tuple[torch.Tensor, torch.Tensor, Optional[torch.Tensor]]],
               algo: int = 0, split: bool = True, copy: Optional[torch.Tensor] = None, few_rows: bool = False) -> Optional[Partials]:
     """``x += sum gate * (a @ w.T)`` over one or two ``(a, w, gate)`` parts; few-row products may come back as
-    partials for the following ``rms_norm`` instead, with ``few_rows`` also those of 3 to 8 rows. ``copy`` gets the new x in
+    partials for the following ``rms_norm`` instead, with ``few_rows`` also those of up to 8 rows. ``copy`` gets the new x in
     its own type (not with partials)."""
     require_cuda(x)
     m, n = int(x.shape[0]), int(x.shape[1])

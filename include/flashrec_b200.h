@@ -550,7 +550,7 @@ int fr_dense_proj(int dtype, const void* a, int64_t lda, const void* w, int64_t 
                   const struct fr_out_segment* segs, int n_segs, int algo, cudaStream_t stream);
 
 /* The same with the K extent split over CTAs, for few rows and columns: n_splits as returned by
- * fr_dense_gated_add_splits(dtype, M, N, K, 0), partials [n_splits, M, N] f32 scratch. */
+ * fr_dense_gated_add_splits(dtype, M, N, K, 0) or fr_dense_few_row_splits, partials [n_splits, M, N] f32 scratch. */
 int fr_dense_proj_split(int dtype, const void* a, int64_t lda, const void* w, int64_t ldw, int M, int N, int K,
                         const struct fr_out_segment* segs, int n_segs, float* partials, int n_splits, cudaStream_t stream);
 
@@ -572,7 +572,7 @@ struct fr_gated_part {
 int fr_dense_gated_add(int dtype, const struct fr_gated_part* parts, int n_parts, float* x, int64_t ldx, int M, int N,
                        float* partials, int n_splits, void* copy, int64_t ldc, int algo, cudaStream_t stream);
 int fr_dense_gated_add_splits(int dtype, int M, int N, int K0, int K1);
-/* The same, but also for 3 to 8 rows where the split product is the faster one (fr_dense_gated_add_splits says 0 there). */
+/* The same, but also for up to 8 rows where the split product is the faster one (fr_dense_gated_add_splits says 0 there). */
 int fr_dense_few_row_splits(int dtype, int M, int N, int K0, int K1);
 
 /* x[t, :] = table[ids[t], :] * scale, and the slot table entry of the token: req_to_token[rows[t], pos[t]] = loc[t]
