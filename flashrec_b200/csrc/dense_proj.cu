@@ -1014,6 +1014,11 @@ static int launch_tc(TcArgs g, const fr_gated_part* parts, cudaStream_t stream) 
   return launch_kernel(kern, grid, kThreads, smem, stream, g.M <= kPdlRows, ta[0], tb[0], ta[1], tb[1], g, status);
 }
 
+// Whether kFew pays: of more than 64 rows little of a row block is left out, and a short product is over before that repays the
+// run-time sizes (128 rows x 2048 x 256: 4.46 us with constants, 4.65 with sizes; K = 2048: 12.5 and 11.9; 64 rows x 2048 x 128:
+// 3.72 and 3.87; K = 512: 5.5 and 5.2).
+static bool few_rows(int M, int64_t K) { return M <= kBlockM && K >= (M <= 64 ? 256 : 1024); }
+
 // Tile width with the least work on the busiest SM: rounds of tiles times the rows of A and B that a tile brings in (`few`: of a
 // single row block only its own rows; the update in place brings in whole ones, 16 rows x 20480 x 2048: 32.0 us, 38.4 as if it did not).
 // 192 is for a single row block only: there it fills one round of SMs where 256 leaves many idle and 128 begins a second
@@ -1171,8 +1176,9 @@ extern "C" int fr_dense_proj(int dtype, const void* a, int64_t lda, const void* 
   g.segs = sg;
   fr_gated_part part{a, w, nullptr, lda, ldw, 0, K, 0};
   if (M <= 8) return dense::launch_tc<64, dense::kEpiSegs, dense::kOctet>(g, &part, stream);
-  const int block_n = dense::pick_block_n(M, N, true);
-  if (M <= dense::kBlockM) {
+  const bool few = dense::few_rows(M, K);
+  const int block_n = dense::pick_block_n(M, N, few);
+  if (few) {
     switch (block_n) {
       case 256: return dense::launch_tc<256, dense::kEpiSegs, dense::kFew>(g, &part, stream);
       case 192: return dense::launch_tc<192, dense::kEpiSegs, dense::kFew>(g, &part, stream);
@@ -1217,7 +1223,9 @@ extern "C" int fr_dense_gated_add(int dtype, const fr_gated_part* parts, int n_p
   FR_CHECK_ARG(x && ldx >= N && (copy == nullptr || (ldc >= N && partials == nullptr)));
   dense::Parts pt{};
   pt.n = n_parts;
+  int64_t K = 0;
   for (int p = 0; p < n_parts; ++p) {
+    K += parts[p].K;
     FR_CHECK_ARG(dense::operand_ok(parts[p].a, parts[p].lda, parts[p].K) &&
                  dense::operand_ok(parts[p].w, parts[p].ldw, parts[p].K));
     pt.p[p] = parts[p];
@@ -1253,8 +1261,8 @@ extern "C" int fr_dense_gated_add(int dtype, const fr_gated_part* parts, int n_p
     FR_CHECK_ARG(g.splits[0] > 0 && g.splits[0] + g.splits[1] == n_splits && (n_parts == 1 || g.splits[1] > 0));
     g.partials = partials;
     if (M <= 8) return dense::launch_tc<64, dense::kEpiPartial, dense::kOctet>(g, parts, stream);
-    return M <= dense::kBlockM ? dense::launch_tc<64, dense::kEpiPartial, dense::kFew>(g, parts, stream)
-                               : dense::launch_tc<64, dense::kEpiPartial, dense::kAny>(g, parts, stream);
+    return dense::few_rows(M, K) ? dense::launch_tc<64, dense::kEpiPartial, dense::kFew>(g, parts, stream)
+                                 : dense::launch_tc<64, dense::kEpiPartial, dense::kAny>(g, parts, stream);
   }
   switch (dense::pick_block_n(M, N, false)) {
     case 256: return dense::launch_tc<256, dense::kEpiAdd, dense::kAny>(g, parts, stream);
