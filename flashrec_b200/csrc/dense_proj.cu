@@ -1160,9 +1160,11 @@ extern "C" int fr_dense_proj(int dtype, const void* a, int64_t lda, const void* 
   if (dtype == 1) {
     const float* A = static_cast<const float*>(a);
     const float* W = static_cast<const float*>(w);
-    // 128 rows per tile take every weight from shared memory half as often; with fewer than a tile per SM 64 spread better
+    // 128 rows per tile take every weight from shared memory half as often; with fewer than a tile per SM 64 spread better, and
+    // short products are mostly beginnings and ends of tiles, of which two CTAs per SM hide fewer than three
+    // (us, 64 / 128 rows per tile: 128 x 20480 x 64 22.6 / 29.0, 351 x 20480 x 2048 see the kernel)
     const int64_t large = static_cast<int64_t>(ceil_div(N, 64)) * ceil_div(M, 128);
-    if (M > 64 && large >= device_sm_count())
+    if (M > 64 && K >= 512 && large >= device_sm_count())
       dense::dense_simt_proj_kernel<128><<<dim3(ceil_div(N, 64), ceil_div(M, 128)), 256, 0, stream>>>(A, lda, W, ldw, M, N, K, sg);
     else
       dense::dense_simt_proj_kernel<64><<<dim3(ceil_div(N, 64), ceil_div(M, 64)), 256, 0, stream>>>(A, lda, W, ldw, M, N, K, sg);

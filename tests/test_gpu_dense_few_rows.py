@@ -112,3 +112,24 @@ def test_few_rows_with_infinities_and_nan(m, n):
     proj(a, [out])
     assert (out[0] == float("inf")).all() and (out[1] == float("-inf")).all() and out[2].isnan().all()
     assert out[3:].isfinite().all()
+
+
+@pytest.mark.parametrize("m", [65, 129, 351])
+@pytest.mark.parametrize("k", [504, 512, 1048])
+def test_f32_tiles_of_128_rows(m, k):
+    """Columns enough for a tile of 128 rows per SM, with pairs, rows left over, and K on either side of the line."""
+    from flashrec_b200.lm_layers import MergedProjection, interleave_rows
+
+    g = torch.Generator(device="cuda").manual_seed(k)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    plain, pairs = 8228, 912
+    a, w, gate, up = r(m, k), r(plain, k) * k ** -0.5, r(pairs, k) * k ** -0.5, r(pairs, k) * k ** -0.5
+    proj = MergedProjection(k)
+    proj.add("store", w)
+    proj.add("swiglu", interleave_rows(gate, up), n=pairs)
+    proj.finish(torch.float32, "cuda")
+    outs = [torch.full((m, plain), float("nan"), device="cuda"), torch.full((m, pairs), float("nan"), device="cuda")]
+    proj(a, outs)
+    for got, want in zip(outs, (a.double() @ w.double().T, torch.nn.functional.silu(a.double() @ gate.double().T) * (a.double() @ up.double().T))):
+        # k roundings of 2^-24 of a sum of about 1 in random order, and a few more of the activation's
+        assert float((got.double() - want).norm() / want.norm()) < (k ** 0.5 + 8) * 2 ** -24
