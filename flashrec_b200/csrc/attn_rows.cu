@@ -11,15 +11,18 @@
 // queries are one mma.sync per 16 dimensions, with the keys as its 16-row operand straight from global memory: lane t of
 // a quad loads 16 consecutive bytes of a key and the queries are loaded the same way, so both sides see the same
 // permutation of the dimensions and the sum is unchanged. Weights stay fp32; weights times values are fp32 FMAs.
+// An mma.sync cuts off bits of what it adds up, so each begins at zero and fp32 additions join them, and values are summed per block
+// of keys first. With one accumulator throughout a quarter more of the outputs were not the bf16 nearest to the 64-bit result than from
+// the general kernels, 3.3e-4 against 2.4e-4 at 800 keys of unit scores; now 2.2e-4 (64 x 2000 PLAIN 90.9 -> 93.7 us, others within 4 %).
 // Measured against one kernel that writes all scores to global memory and one that mixes them (caches larger than L2):
 //   rows x keys, kv heads          before      here
-//   DIFF   1 x  800, 8            17.5 us    9.3 us
-//   DIFF  64 x  150, 8            38.2      18.9
-//   TALK   1 x  800, 8            24.4      16.8
-//   TALK  64 x  150, 8            43.9      19.3
-//   PLAIN  1 x   60, 8            13.9       4.9
-//   PLAIN  5 x 2000, 8            59.4      23.4
-//   PLAIN 64 x 2000, 8           251.4      88.7  (5.9 TB/s)
+//   DIFF   1 x  800, 8            18.0 us    9.7 us
+//   DIFF  64 x  150, 8            36.4      20.3
+//   TALK   1 x  800, 8            23.0      17.5
+//   TALK  64 x  150, 8            41.0      20.3
+//   PLAIN  1 x   60, 8            13.7       4.8
+//   PLAIN  5 x 2000, 8            59.5      24.4
+//   PLAIN 64 x 2000, 8           256.0      93.7  (5.6 TB/s)
 #include "attn_mix.cuh"
 
 namespace fr {
@@ -84,12 +87,15 @@ struct Scores {
       for (int half = 0; half < 2; ++half)
 #pragma unroll
         for (int m = 0; m < kMaps; ++m) {
-          float d[4] = {0.f, 0.f, 0.f, 0.f};
+          float d[4];
 #pragma unroll
           for (int j = 0; j < NCH; ++j) {
             const uint4 &lo = x[2 * half][m][j], &hi = x[2 * half + 1][m][j];
-            mma(d, lo.x, hi.x, lo.y, hi.y, q[m0 + m][j][0], q[m0 + m][j][1]);
-            mma(d, lo.z, hi.z, lo.w, hi.w, q[m0 + m][j][2], q[m0 + m][j][3]);
+            float e[4] = {0.f, 0.f, 0.f, 0.f}, f[4] = {0.f, 0.f, 0.f, 0.f};
+            mma(e, lo.x, hi.x, lo.y, hi.y, q[m0 + m][j][0], q[m0 + m][j][1]);
+            mma(f, lo.z, hi.z, lo.w, hi.w, q[m0 + m][j][2], q[m0 + m][j][3]);
+#pragma unroll
+            for (int y = 0; y < 4; ++y) d[y] = j == 0 ? e[y] + f[y] : d[y] + (e[y] + f[y]);
           }
           float* s0 = sc + (half * 16 + r) * NS + (m0 + m) * REP + 2 * t;
           if (2 * t < REP) {
@@ -195,7 +201,7 @@ flash_rows_kernel(const __grid_constant__ fr_mix_attn a, int row0, int max_keys,
     scores(a, g, slot, my);
     __syncwarp();
     const float dist = static_cast<float>(i - vis.key(k0 + min(lane, nk - 1)));
-    float p[NS];
+    float p[NS], fade[NS];
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
       float v = my[lane * NS + s] * a.scale;
@@ -207,13 +213,17 @@ flash_rows_kernel(const __grid_constant__ fr_mix_attn a, int row0, int max_keys,
       p[s] = v == -INFINITY ? 0.f : expf(v - mn);
       l[s] = l[s] * corr + p[s];
       m[s] = mn;
-#pragma unroll
-      for (int e = 0; e < 8; ++e) acc[s][e] *= corr;
+      fade[s] = corr;
     }
+    float blk[NS][8] = {};
 #pragma unroll
     for (int s = 0; s < NS; ++s) my[lane * NS + s] = p[s];
     __syncwarp();
-    add_values<NS, VL>(a, g, slot, nk, my, acc);
+    add_values<NS, VL>(a, g, slot, nk, my, blk);
+#pragma unroll
+    for (int s = 0; s < NS; ++s)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[s][e] = fmaf(acc[s][e], fade[s], blk[s][e]);
   }
   // the warps' shares, then the CTAs'
 #pragma unroll
@@ -430,8 +440,14 @@ talk_rows_kernel(const __grid_constant__ fr_mix_attn a, int row0, int max_keys) 
   __syncthreads();
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // done with the others' memory
   float acc[REP][8] = {};
-  for (int k0 = warp * 32; k0 < n; k0 += W * 32)
-    add_values<REP, VL>(a, g, slots[k0 + lane], min(32, n - k0), mw + k0 * REP, acc);
+  for (int k0 = warp * 32; k0 < n; k0 += W * 32) {
+    float blk[REP][8] = {};
+    add_values<REP, VL>(a, g, slots[k0 + lane], min(32, n - k0), mw + k0 * REP, blk);
+#pragma unroll
+    for (int o = 0; o < REP; ++o)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[o][e] += blk[o][e];
+  }
 #pragma unroll
   for (int o = 0; o < REP; ++o)
 #pragma unroll
