@@ -280,8 +280,8 @@ dense_rows_gated_kernel(const __grid_constant__ Parts pt, float* __restrict__ x,
 }
 
 // ---------------------------------------------------------------------------
-// f32, more rows: TM x 64 tiles, 256 threads of TM / 16 x 4 outputs. Bound by the fp32 units where there are tiles enough:
-// operands arrive by cp.async two steps of 16 ahead and stay as they lie in memory, rows of k, so that one fma.rn.f32x2
+// f32, more rows: TM x 64 tiles, 256 threads of TM / 16 x 4 outputs. With tiles enough they reach 34 of the fp32 units' 75 TFLOP/s
+// (loads from shared memory and FMAs share the issue slots). Operands arrive by cp.async two steps of 16 ahead and stay as they lie in memory, rows of k, so that one fma.rn.f32x2
 // takes two consecutive k of an output without any rearranging (an output is the sum of its even and its odd chain).
 // us for 64 / 351 rows of 2048: 20480 columns 286 / 1153 before (64 x 64 tiles through transposed copies, one step ahead), 220 /
 // 863 now (34 TFLOP/s); 2048 columns 133 / 226 and 92 / 155. The gated update's 192 tiles of K = 8192 stay a chain per SM:

@@ -6,6 +6,14 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture(autouse=True)
+def _clean_status():
+    yield
+    from flashrec_b200 import device_status
+
+    assert device_status() == (0, 0)
+
+
 def _rand(*shape, seed):
     g = torch.Generator(device="cuda").manual_seed(seed)
     return torch.randn(*shape, generator=g, device="cuda").bfloat16()
