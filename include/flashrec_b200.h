@@ -710,7 +710,9 @@ struct fr_mix_attn {
   int64_t ld_gate;
 };
 
-/* Any head sizes, bf16 or f32, prompts or decode: scores of every visible key, then the mixture over the values.
+/* Any head sizes, bf16 or f32, prompts or decode: scores of every visible key, then the mixture over the values; bf16 heads of
+ * up to 128, up to 8 of them per kv head (DIFF: 4), take one launch, which asks for
+ * scratch and counters alike but leaves them alone (TALK: kv_heads 1, 2, 4 or 8, and weights that fit into shared memory).
  * Rows [row0, row0 + n_rows) of the batch. max_keys bounds the visible keys of a row; scratch holds
  * fr_mix_attn_rows_scratch(...) bytes, counters n_rows * kv_heads zeroed words (left zeroed). */
 int fr_mix_attn_rows(const struct fr_mix_attn* a, int row0, int n_rows, int max_keys, int splits, void* scratch,
