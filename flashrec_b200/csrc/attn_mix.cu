@@ -469,7 +469,7 @@ mix_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
   const int total = n_tiles * n_src;
   auto k_head = [&](int s) { return diff ? 2 * vh + s : (plain ? vh : s / rep); };
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int i = 0; i < 24; ++i) ptx::mbar_init(bar0 + 8 * i, 1);
     ptx::mbar_init(bar_pfull, 128);
@@ -496,110 +496,103 @@ mix_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CU
   const uint32_t col_acc = col_o + pl.v_cols;
 
   if (warp == 0) {
-    if (lane == 0) {
-      bool ok = true;
-      auto load_q = [&](int s) -> bool {
-        const uint32_t st = s & 1;
-        if (!ptx::mbar_wait(bar_qempty + 8 * st, ((s >> 1) & 1) ^ 1u, abort_flag, status, 71)) return false;
-        ptx::mbar_expect_tx(bar_qfull + 8 * st, q_bytes);
-        for (int b = 0; b < pl.q_boxes; ++b)
-          ptx::tma_load_2d(sm_q + st * q_bytes + b * kM * 128, &tq, (src0 + s) * a.dim + b * 64, row0, bar_qfull + 8 * st);
-        return true;
-      };
-      // stage and parity of the next K and V tile, position of the next K tile (map, tile): counted, not divided
-      int k_st = 0, k_ph = 0, k_j = 0, k_s = 0, next_k = 0;
-      auto load_k = [&]() -> bool {
-        if (k_j == 0 && !load_q(k_s)) return false;
-        if (!ptx::mbar_wait(bar_kempty + 8 * k_st, k_ph ^ 1u, abort_flag, status, 72)) return false;
-        ptx::mbar_expect_tx(bar_kfull + 8 * k_st, k_bytes);
-        const int row = page_at(a, table, kt, pages, k_j), col = k_head(k_s) * a.dim;
-        for (int b = 0; b < pl.q_boxes; ++b)
-          ptx::tma_load_2d(sm_k + k_st * k_bytes + b * kTileN * 128, &tk, col + b * 64, row, bar_kfull + 8 * k_st);
-        if (++k_st == n_st) { k_st = 0; k_ph ^= 1; }
-        if (++k_j == n_tiles) { k_j = 0; ++k_s; }
-        ++next_k;
-        return true;
-      };
-      // K (and at a map's start its Q) runs up to n_st - 1 tiles ahead of V
-      int v_st = 0, v_ph = 0, v_j = 0;
-      for (int it = 0; it < total && ok; ++it) {
-        while (ok && next_k < total && next_k < it + n_st) ok = load_k();
-        if (!ok) break;
-        ok = ptx::mbar_wait(bar_vempty + 8 * v_st, v_ph ^ 1u, abort_flag, status, 73);
-        if (!ok) break;
-        ptx::mbar_expect_tx(bar_vfull + 8 * v_st, v_bytes);
-        const int row = page_at(a, table, kt, pages, v_j);
-        for (int b = 0; b < pl.v_boxes; ++b)
-          ptx::tma_load_2d(sm_v + v_st * v_bytes + b * kTileN * 128, &tv, vh * a.vdim + b * 64, row, bar_vfull + 8 * v_st);
-        if (++v_st == n_st) { v_st = 0; v_ph ^= 1; }
-        if (++v_j == n_tiles) v_j = 0;
-      }
+    bool ok = true;
+    auto load_q = [&](int s) -> bool {
+      const uint32_t st = s & 1;
+      if (!ptx::mbar_wait_warp(bar_qempty + 8 * st, ((s >> 1) & 1) ^ 1u, abort_flag, status, 71)) return false;
+      ptx::mbar_expect_tx_one(bar_qfull + 8 * st, q_bytes);
+      for (int b = 0; b < pl.q_boxes; ++b)
+        ptx::tma_load_2d_one(sm_q + st * q_bytes + b * kM * 128, &tq, (src0 + s) * a.dim + b * 64, row0, bar_qfull + 8 * st);
+      return true;
+    };
+    // stage and parity of the next K and V tile, position of the next K tile (map, tile): counted, not divided
+    int k_st = 0, k_ph = 0, k_j = 0, k_s = 0, next_k = 0;
+    auto load_k = [&]() -> bool {
+      if (k_j == 0 && !load_q(k_s)) return false;
+      if (!ptx::mbar_wait_warp(bar_kempty + 8 * k_st, k_ph ^ 1u, abort_flag, status, 72)) return false;
+      ptx::mbar_expect_tx_one(bar_kfull + 8 * k_st, k_bytes);
+      const int row = page_at(a, table, kt, pages, k_j), col = k_head(k_s) * a.dim;
+      for (int b = 0; b < pl.q_boxes; ++b)
+        ptx::tma_load_2d_one(sm_k + k_st * k_bytes + b * kTileN * 128, &tk, col + b * 64, row, bar_kfull + 8 * k_st);
+      if (++k_st == n_st) { k_st = 0; k_ph ^= 1; }
+      if (++k_j == n_tiles) { k_j = 0; ++k_s; }
+      ++next_k;
+      return true;
+    };
+    // K (and at a map's start its Q) runs up to n_st - 1 tiles ahead of V
+    int v_st = 0, v_ph = 0, v_j = 0;
+    for (int it = 0; it < total && ok; ++it) {
+      while (ok && next_k < total && next_k < it + n_st) ok = load_k();
+      if (!ok) break;
+      ok = ptx::mbar_wait_warp(bar_vempty + 8 * v_st, v_ph ^ 1u, abort_flag, status, 73);
+      if (!ok) break;
+      ptx::mbar_expect_tx_one(bar_vfull + 8 * v_st, v_bytes);
+      const int row = page_at(a, table, kt, pages, v_j);
+      for (int b = 0; b < pl.v_boxes; ++b)
+        ptx::tma_load_2d_one(sm_v + v_st * v_bytes + b * kTileN * 128, &tv, vh * a.vdim + b * 64, row, bar_vfull + 8 * v_st);
+      if (++v_st == n_st) { v_st = 0; v_ph ^= 1; }
+      if (++v_j == n_tiles) v_j = 0;
     }
-    __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc_s = ptx::make_idesc(1u, 1u, kM, kTileN);
-      const int k_steps = a.dim / 16;
-      bool ok = true;
-      int st = 0, ph = 0, j = 0, s = 0;
-      for (int it = 0; it < total && ok; ++it) {
-        const uint32_t sb = it & 1;
-        if (j == 0) ok = ptx::mbar_wait(bar_qfull + 8 * (s & 1), (s >> 1) & 1, abort_flag, status, 74);
-        ok = ok && ptx::mbar_wait(bar_kfull + 8 * st, ph, abort_flag, status, 75);
-        // the buffer held P of tile it - 2
-        if (ok && it >= 2) ok = ptx::mbar_wait(bar_ofull + 8 * sb, ((it >> 1) - 1) & 1, abort_flag, status, 83);
-        if (!ok) break;
-        ptx::tc_fence_after();
-        const uint64_t a_desc = ptx::smem_desc_sw128(sm_q + (s & 1) * q_bytes);
-        const uint64_t b_desc = ptx::smem_desc_sw128(sm_k + st * k_bytes);
-        const uint32_t d = tmem_base + sb * kTileN;
+    const uint32_t idesc_s = ptx::make_idesc(1u, 1u, kM, kTileN);
+    const int k_steps = a.dim / 16;
+    bool ok = true;
+    int st = 0, ph = 0, j = 0, s = 0;
+    for (int it = 0; it < total && ok; ++it) {
+      const uint32_t sb = it & 1;
+      if (j == 0) ok = ptx::mbar_wait_warp(bar_qfull + 8 * (s & 1), (s >> 1) & 1, abort_flag, status, 74);
+      ok = ok && ptx::mbar_wait_warp(bar_kfull + 8 * st, ph, abort_flag, status, 75);
+      // the buffer held P of tile it - 2
+      if (ok && it >= 2) ok = ptx::mbar_wait_warp(bar_ofull + 8 * sb, ((it >> 1) - 1) & 1, abort_flag, status, 83);
+      if (!ok) break;
+      ptx::tc_fence_after();
+      const uint64_t a_desc = ptx::smem_desc_sw128(sm_q + (s & 1) * q_bytes);
+      const uint64_t b_desc = ptx::smem_desc_sw128(sm_k + st * k_bytes);
+      const uint32_t d = tmem_base + sb * kTileN;
 #pragma unroll 1
-        for (int kb = 0; kb < k_steps; kb += 4) {  // 64 columns per box; descriptor addresses count 16-byte units
-          const uint64_t ad = a_desc + (kb >> 2) * (kM * 128 / 16), bd = b_desc + (kb >> 2) * (kTileN * 128 / 16);
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            if (kb + k < k_steps) ptx::mma_f16(d, ad + 2u * k, bd + 2u * k, idesc_s, (kb | k) != 0 ? 1u : 0u);
-        }
-        ptx::tc_commit(bar_sfull + 8 * sb);
-        ptx::tc_commit(bar_kempty + 8 * st);
-        if (++st == n_st) { st = 0; ph ^= 1; }
-        if (++j == n_tiles) {
-          ptx::tc_commit(bar_qempty + 8 * (s & 1));
-          j = 0;
-          ++s;
+      for (int kb = 0; kb < k_steps; kb += 4) {  // 64 columns per box; descriptor addresses count 16-byte units
+        const uint64_t ad = a_desc + (kb >> 2) * (kM * 128 / 16), bd = b_desc + (kb >> 2) * (kTileN * 128 / 16);
+        if (kb + 4 <= k_steps) {
+          ptx::mma_k_block_f16(d, ad, bd, idesc_s, kb != 0 ? 1u : 0u);
+        } else {
+          for (int k = 0; kb + k < k_steps; ++k) ptx::mma_f16_one(d, ad + 2u * k, bd + 2u * k, idesc_s, (kb | k) != 0 ? 1u : 0u);
         }
       }
+      ptx::tc_commit_one(bar_sfull + 8 * sb);
+      ptx::tc_commit_one(bar_kempty + 8 * st);
+      if (++st == n_st) { st = 0; ph ^= 1; }
+      if (++j == n_tiles) {
+        ptx::tc_commit_one(bar_qempty + 8 * (s & 1));
+        j = 0;
+        ++s;
+      }
     }
-    __syncwarp();
   } else if (warp == 6) {
-    if (lane == 0) {
-      const uint32_t idesc_o = ptx::make_idesc(1u, 1u, kM, a.vdim) | (1u << 16);  // B is MN-major
-      bool ok = true;
-      int st = 0, ph = 0, j = 0, s = 0;
-      for (int it = 0; it < total && ok; ++it) {
-        const uint32_t sb = it & 1;
-        ok = ptx::mbar_wait(bar_vfull + 8 * st, ph, abort_flag, status, 77) &&
-             ptx::mbar_wait(bar_pfull + 8 * sb, (it >> 1) & 1, abort_flag, status, 76);
-        // the first P.V of a map overwrites O: the previous map's must have been read
-        if (ok && j == 0 && s > 0) ok = ptx::mbar_wait(bar_oread, (s - 1) & 1, abort_flag, status, 78);
-        if (!ok) break;
-        ptx::tc_fence_after();
-        const uint64_t v_desc = smem_desc_mn(sm_v + st * v_bytes, kTileN * 128);
+    const uint32_t idesc_o = ptx::make_idesc(1u, 1u, kM, a.vdim) | (1u << 16);  // B is MN-major
+    bool ok = true;
+    int st = 0, ph = 0, j = 0, s = 0;
+    for (int it = 0; it < total && ok; ++it) {
+      const uint32_t sb = it & 1;
+      ok = ptx::mbar_wait_warp(bar_vfull + 8 * st, ph, abort_flag, status, 77) &&
+           ptx::mbar_wait_warp(bar_pfull + 8 * sb, (it >> 1) & 1, abort_flag, status, 76);
+      // the first P.V of a map overwrites O: the previous map's must have been read
+      if (ok && j == 0 && s > 0) ok = ptx::mbar_wait_warp(bar_oread, (s - 1) & 1, abort_flag, status, 78);
+      if (!ok) break;
+      ptx::tc_fence_after();
+      const uint64_t v_desc = smem_desc_mn(sm_v + st * v_bytes, kTileN * 128);
 #pragma unroll
-        for (int k = 0; k < kTileN / 16; ++k)  // 16 keys = 8 columns of P, 16 rows of V
-          ptx::mma_f16_ts(col_o, tmem_base + sb * kTileN + 8u * k, v_desc + static_cast<uint64_t>(k * 16 * 128 >> 4), idesc_o,
-                          (j | k) != 0 ? 1u : 0u);
-        ptx::tc_commit(bar_ofull + 8 * sb);
-        ptx::tc_commit(bar_vempty + 8 * st);
-        if (++st == n_st) { st = 0; ph ^= 1; }
-        if (++j == n_tiles) {
-          ptx::tc_commit(bar_done);
-          j = 0;
-          ++s;
-        }
+      for (int k = 0; k < kTileN / 16; ++k)  // 16 keys = 8 columns of P, 16 rows of V
+        ptx::mma_f16_ts_one(col_o, tmem_base + sb * kTileN + 8u * k, v_desc + static_cast<uint64_t>(k * 16 * 128 >> 4), idesc_o,
+                        (j | k) != 0 ? 1u : 0u);
+      ptx::tc_commit_one(bar_ofull + 8 * sb);
+      ptx::tc_commit_one(bar_vempty + 8 * st);
+      if (++st == n_st) { st = 0; ph ^= 1; }
+      if (++j == n_tiles) {
+        ptx::tc_commit_one(bar_done);
+        j = 0;
+        ++s;
       }
     }
-    __syncwarp();
   } else {
     const int quad = warp & 3;
     const int r = quad * 32 + lane;

@@ -61,7 +61,7 @@ talk_maps_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
   const int32_t* table = a.req_to_token + a.req_rows[req] * a.table_stride;
   const mix::KeyTiles kt = mix::key_tiles(a, pos0, pos0 + n_tok - 1);
   const int total = kt.n;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     ptx::mbar_init(bar_q, 1);
     for (int i = 0; i < kKStages; ++i) {
@@ -90,40 +90,41 @@ talk_maps_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
-      ptx::mbar_expect_tx(bar_q, q_bytes);
-      for (int b = 0; b < boxes; ++b) ptx::tma_load_2d(sm_q + b * kM * 128, &tq, head * a.dim + b * 64, row0, bar_q);
-      bool ok = true;
-      for (int it = 0; it < total && ok; ++it) {
-        const int st = it % kKStages;
-        ok = ptx::mbar_wait(bar_kempty + 8 * st, ((it / kKStages) & 1) ^ 1u, abort_flag, status, 91);
-        if (!ok) break;
-        ptx::mbar_expect_tx(bar_kfull + 8 * st, k_bytes);
-        const int row = mix::page_at(a, table, kt, pages, it);
-        for (int b = 0; b < boxes; ++b)
-          ptx::tma_load_2d(sm_k + st * k_bytes + b * kTileN * 128, &tk, kvh * a.dim + b * 64, row, bar_kfull + 8 * st);
-      }
+    ptx::mbar_expect_tx_one(bar_q, q_bytes);
+    for (int b = 0; b < boxes; ++b) ptx::tma_load_2d_one(sm_q + b * kM * 128, &tq, head * a.dim + b * 64, row0, bar_q);
+    bool ok = true;
+    for (int it = 0; it < total && ok; ++it) {
+      const int st = it % kKStages;
+      ok = ptx::mbar_wait_warp(bar_kempty + 8 * st, ((it / kKStages) & 1) ^ 1u, abort_flag, status, 91);
+      if (!ok) break;
+      ptx::mbar_expect_tx_one(bar_kfull + 8 * st, k_bytes);
+      const int row = mix::page_at(a, table, kt, pages, it);
+      for (int b = 0; b < boxes; ++b)
+        ptx::tma_load_2d_one(sm_k + st * k_bytes + b * kTileN * 128, &tk, kvh * a.dim + b * 64, row, bar_kfull + 8 * st);
     }
-    __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = ptx::make_idesc(1u, 1u, kM, kTileN);
-      bool ok = ptx::mbar_wait(bar_q, 0, abort_flag, status, 92);
-      for (int it = 0; it < total && ok; ++it) {
-        const int st = it % kKStages, sb = it % kSBufs;
-        ok = ptx::mbar_wait(bar_sempty + 8 * sb, ((it / kSBufs) & 1) ^ 1u, abort_flag, status, 93) &&
-             ptx::mbar_wait(bar_kfull + 8 * st, (it / kKStages) & 1, abort_flag, status, 94);
-        if (!ok) break;
-        ptx::tc_fence_after();
-        for (int k = 0; k < a.dim / 16; ++k)
-          ptx::mma_f16(tmem_base + sb * kTileN, ptx::smem_desc_sw128(sm_q + (k >> 2) * kM * 128) + 2u * (k & 3),
-                       ptx::smem_desc_sw128(sm_k + st * k_bytes + (k >> 2) * kTileN * 128) + 2u * (k & 3), idesc,
-                       k > 0 ? 1u : 0u);
-        ptx::tc_commit(bar_kempty + 8 * st);
-        ptx::tc_commit(bar_sfull + 8 * sb);
+    const uint32_t idesc = ptx::make_idesc(1u, 1u, kM, kTileN);
+    bool ok = ptx::mbar_wait_warp(bar_q, 0, abort_flag, status, 92);
+    for (int it = 0; it < total && ok; ++it) {
+      const int st = it % kKStages, sb = it % kSBufs;
+      ok = ptx::mbar_wait_warp(bar_sempty + 8 * sb, ((it / kSBufs) & 1) ^ 1u, abort_flag, status, 93) &&
+           ptx::mbar_wait_warp(bar_kfull + 8 * st, (it / kKStages) & 1, abort_flag, status, 94);
+      if (!ok) break;
+      ptx::tc_fence_after();
+      const int k_steps = a.dim / 16;
+      for (int kb = 0; kb < k_steps; kb += 4) {
+        const uint64_t ad = ptx::smem_desc_sw128(sm_q + (kb >> 2) * kM * 128);
+        const uint64_t bd = ptx::smem_desc_sw128(sm_k + st * k_bytes + (kb >> 2) * kTileN * 128);
+        if (kb + 4 <= k_steps) {
+          ptx::mma_k_block_f16(tmem_base + sb * kTileN, ad, bd, idesc, kb != 0 ? 1u : 0u);
+        } else {
+          for (int k = 0; kb + k < k_steps; ++k)
+            ptx::mma_f16_one(tmem_base + sb * kTileN, ad + 2u * k, bd + 2u * k, idesc, (kb | k) != 0 ? 1u : 0u);
+        }
       }
+      ptx::tc_commit_one(bar_kempty + 8 * st);
+      ptx::tc_commit_one(bar_sfull + 8 * sb);
     }
-    __syncwarp();
   } else {
     const int quad = warp & 3, half = (warp - 2) >> 2, r = quad * 32 + lane;
     const int i = pos0 + min(r, n_tok - 1);
@@ -326,7 +327,7 @@ talk_values_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant
   const int pos0 = static_cast<int>(a.pos[row0]);
   const int32_t* table = a.req_to_token + a.req_rows[req] * a.table_stride;
   const mix::KeyTiles kt = mix::key_tiles(a, pos0, pos0 + n_tok - 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int i = 0; i < kStages; ++i) {
       ptx::mbar_init(bar_full + 8 * i, 1);
@@ -349,39 +350,34 @@ talk_values_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   if (warp == 0) {
-    if (lane == 0) {
-      bool ok = true;
-      for (int it = 0; it < kt.n && ok; ++it) {
-        const int st = it % kStages;
-        ok = ptx::mbar_wait(bar_empty + 8 * st, ((it / kStages) & 1) ^ 1u, abort_flag, status, 96);
-        if (!ok) break;
-        ptx::mbar_expect_tx(bar_full + 8 * st, stage);
-        ptx::tma_load_2d(base + st * stage, &tm, it * kTileN, (static_cast<int>(blockIdx.x) * a.heads + head) * kM, bar_full + 8 * st);
-        const int row = mix::page_at(a, table, kt, pages, it);
-        for (int b = 0; b < v_boxes; ++b)
-          ptx::tma_load_2d(base + st * stage + m_bytes + b * kTileN * 128, &tv, vh * a.vdim + b * 64, row, bar_full + 8 * st);
-      }
+    bool ok = true;
+    for (int it = 0; it < kt.n && ok; ++it) {
+      const int st = it % kStages;
+      ok = ptx::mbar_wait_warp(bar_empty + 8 * st, ((it / kStages) & 1) ^ 1u, abort_flag, status, 96);
+      if (!ok) break;
+      ptx::mbar_expect_tx_one(bar_full + 8 * st, stage);
+      ptx::tma_load_2d_one(base + st * stage, &tm, it * kTileN, (static_cast<int>(blockIdx.x) * a.heads + head) * kM, bar_full + 8 * st);
+      const int row = mix::page_at(a, table, kt, pages, it);
+      for (int b = 0; b < v_boxes; ++b)
+        ptx::tma_load_2d_one(base + st * stage + m_bytes + b * kTileN * 128, &tv, vh * a.vdim + b * 64, row, bar_full + 8 * st);
     }
-    __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = ptx::make_idesc(1u, 1u, kM, a.vdim) | (1u << 16);  // B is MN-major
-      bool ok = true;
-      for (int it = 0; it < kt.n && ok; ++it) {
-        const int st = it % kStages;
-        ok = ptx::mbar_wait(bar_full + 8 * st, (it / kStages) & 1, abort_flag, status, 97);
-        if (!ok) break;
-        ptx::tc_fence_after();
-        const uint64_t m_desc = ptx::smem_desc_sw128(base + st * stage);
-        const uint64_t v_desc = mix::smem_desc_mn(base + st * stage + m_bytes, kTileN * 128);
-        for (int k = 0; k < kTileN / 16; ++k)
-          ptx::mma_f16(tmem_base, m_desc + 2u * k, v_desc + static_cast<uint64_t>(k * 16 * 128 >> 4), idesc,
-                       (it | k) != 0 ? 1u : 0u);
-        ptx::tc_commit(bar_empty + 8 * st);
-        if (it + 1 == kt.n) ptx::tc_commit(bar_done);
-      }
+    const uint32_t idesc = ptx::make_idesc(1u, 1u, kM, a.vdim) | (1u << 16);  // B is MN-major
+    bool ok = true;
+    for (int it = 0; it < kt.n && ok; ++it) {
+      const int st = it % kStages;
+      ok = ptx::mbar_wait_warp(bar_full + 8 * st, (it / kStages) & 1, abort_flag, status, 97);
+      if (!ok) break;
+      ptx::tc_fence_after();
+      const uint64_t m_desc = ptx::smem_desc_sw128(base + st * stage);
+      const uint64_t v_desc = mix::smem_desc_mn(base + st * stage + m_bytes, kTileN * 128);
+#pragma unroll
+      for (int k = 0; k < kTileN / 16; ++k)
+        ptx::mma_f16_one(tmem_base, m_desc + 2u * k, v_desc + static_cast<uint64_t>(k * 16 * 128 >> 4), idesc,
+                     (it | k) != 0 ? 1u : 0u);
+      ptx::tc_commit_one(bar_empty + 8 * st);
+      if (it + 1 == kt.n) ptx::tc_commit_one(bar_done);
     }
-    __syncwarp();
   } else {
     const int quad = warp & 3, r = quad * 32 + lane;
     int okw = 0;

@@ -216,7 +216,7 @@ decode_attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   const int n_tiles = (vis + kTileN - 1) / kTileN;
   const int gh = grp * p.hkv + kvh;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     ptx::mbar_init(bar_q, 1);
@@ -251,57 +251,49 @@ decode_attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
 
   if (warp == 0) {
     // ------------------------------ TMA producer ---------------------------
-    if (lane == 0) {
-      // Q is needed by the MMAs and, from shared memory, by the per-row tails
-      ptx::mbar_expect_tx(bar_q, kSmemQ);
-      ptx::tma_load_3d(sm_q, &tmap_q, 0, kvh * G, row0 + beam0, bar_q);
-      ptx::tma_load_3d(sm_q + kSmemQ / 2, &tmap_q, 64, kvh * G, row0 + beam0, bar_q);
-      bool ok = true;
-      auto load_k = [&](int jj) -> bool {
-        const uint32_t st = jj & 1, ph = (jj >> 1) & 1;
-        if (!ptx::mbar_wait(bar_kempty + 8 * st, ph ^ 1u, abort_flag, status, 11)) return false;
-        ptx::mbar_expect_tx(bar_kfull + 8 * st, kSmemK);
-        ptx::tma_load_3d(sm_k + st * kSmemK, &tmap_k, 0, jj * kTileN, gh, bar_kfull + 8 * st);
-        ptx::tma_load_3d(sm_k + st * kSmemK + kSmemK / 2, &tmap_k, 64, jj * kTileN, gh, bar_kfull + 8 * st);
-        return true;
-      };
-      if (n_tiles > 0) ok = load_k(0);
-      for (int j = 0; j < n_tiles && ok; ++j) {
-        // K runs one tile ahead of V so that S of tile j+1 can be issued during the softmax of tile j
-        if (j + 1 < n_tiles) {
-          ok = load_k(j + 1);
-          if (!ok) break;
-        }
-        const uint32_t st = j & 1, ph = (j >> 1) & 1;
-        ok = ptx::mbar_wait(bar_vempty + 8 * st, ph ^ 1u, abort_flag, status, 12);
+    // Q is needed by the MMAs and, from shared memory, by the per-row tails
+    ptx::mbar_expect_tx_one(bar_q, kSmemQ);
+    ptx::tma_load_3d_one(sm_q, &tmap_q, 0, kvh * G, row0 + beam0, bar_q);
+    ptx::tma_load_3d_one(sm_q + kSmemQ / 2, &tmap_q, 64, kvh * G, row0 + beam0, bar_q);
+    bool ok = true;
+    auto load_k = [&](int jj) -> bool {
+      const uint32_t st = jj & 1, ph = (jj >> 1) & 1;
+      if (!ptx::mbar_wait_warp(bar_kempty + 8 * st, ph ^ 1u, abort_flag, status, 11)) return false;
+      ptx::mbar_expect_tx_one(bar_kfull + 8 * st, kSmemK);
+      ptx::tma_load_3d_one(sm_k + st * kSmemK, &tmap_k, 0, jj * kTileN, gh, bar_kfull + 8 * st);
+      ptx::tma_load_3d_one(sm_k + st * kSmemK + kSmemK / 2, &tmap_k, 64, jj * kTileN, gh, bar_kfull + 8 * st);
+      return true;
+    };
+    if (n_tiles > 0) ok = load_k(0);
+    for (int j = 0; j < n_tiles && ok; ++j) {
+      // K runs one tile ahead of V so that S of tile j+1 can be issued during the softmax of tile j
+      if (j + 1 < n_tiles) {
+        ok = load_k(j + 1);
         if (!ok) break;
-        ptx::mbar_expect_tx(bar_vfull + 8 * st, kSmemV);
-        ptx::tma_load_3d(sm_v + st * kSmemV, &tmap_v, j * kTileN, 0, gh, bar_vfull + 8 * st);
       }
+      const uint32_t st = j & 1, ph = (j >> 1) & 1;
+      ok = ptx::mbar_wait_warp(bar_vempty + 8 * st, ph ^ 1u, abort_flag, status, 12);
+      if (!ok) break;
+      ptx::mbar_expect_tx_one(bar_vfull + 8 * st, kSmemV);
+      ptx::tma_load_3d_one(sm_v + st * kSmemV, &tmap_v, j * kTileN, 0, gh, bar_vfull + 8 * st);
     }
-    __syncwarp();
   } else if (warp == 1) {
     // ------------------------------ MMA issuer -----------------------------
-    if (lane == 0 && n_tiles > 0) {
+    if (n_tiles > 0) {
       constexpr uint32_t idesc_s = ptx::make_idesc(1u, 1u, kM, kTileN);  // bf16 x bf16, N = 64 tokens
       constexpr uint32_t idesc_o = ptx::make_idesc(0u, 0u, kM, kD);      // fp16 x fp16, N = 128 dims
-      bool ok = ptx::mbar_wait(bar_q, 0, abort_flag, status, 13);
+      bool ok = ptx::mbar_wait_warp(bar_q, 0, abort_flag, status, 13);
       // S = Q K^T for tile jj into TMEM buffer (jj & 1): 2 k-blocks (64 dims) x 4 instructions of K = 16
       auto issue_s = [&](int jj) -> bool {
         const uint32_t st = jj & 1, ph = (jj >> 1) & 1;
-        if (!ptx::mbar_wait(bar_kfull + 8 * st, ph, abort_flag, status, 14)) return false;
+        if (!ptx::mbar_wait_warp(bar_kfull + 8 * st, ph, abort_flag, status, 14)) return false;
         ptx::tc_fence_after();
 #pragma unroll
-        for (int kb = 0; kb < 2; ++kb) {
-          const uint64_t a_desc = ptx::smem_desc_sw128(sm_q + kb * (kSmemQ / 2));
-          const uint64_t b_desc = ptx::smem_desc_sw128(sm_k + st * kSmemK + kb * (kSmemK / 2));
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            ptx::mma_f16(tmem_base + kColS + st * kTileN, a_desc + 2u * k, b_desc + 2u * k, idesc_s,
-                         (kb | k) != 0 ? 1u : 0u);
-        }
-        ptx::tc_commit(bar_kempty + 8 * st);
-        ptx::tc_commit(bar_sfull + 8 * st);
+        for (int kb = 0; kb < 2; ++kb)
+          ptx::mma_k_block_f16(tmem_base + kColS + st * kTileN, ptx::smem_desc_sw128(sm_q + kb * (kSmemQ / 2)),
+                               ptx::smem_desc_sw128(sm_k + st * kSmemK + kb * (kSmemK / 2)), idesc_s, kb != 0 ? 1u : 0u);
+        ptx::tc_commit_one(bar_kempty + 8 * st);
+        ptx::tc_commit_one(bar_sfull + 8 * st);
         return true;
       };
       if (ok) ok = issue_s(0);
@@ -313,9 +305,9 @@ decode_attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
           ok = issue_s(j + 1);
           if (!ok) break;
         }
-        ok = ptx::mbar_wait(bar_pfull + 8 * (j & 1), (j >> 1) & 1, abort_flag, status, 15);
+        ok = ptx::mbar_wait_warp(bar_pfull + 8 * (j & 1), (j >> 1) & 1, abort_flag, status, 15);
         if (!ok) break;
-        ok = ptx::mbar_wait(bar_vfull + 8 * (j & 1), (j >> 1) & 1, abort_flag, status, 16);
+        ok = ptx::mbar_wait_warp(bar_vfull + 8 * (j & 1), (j >> 1) & 1, abort_flag, status, 16);
         if (!ok) break;
         ptx::tc_fence_after();
         // O (+)= P V: A = P straight from TMEM (bf16 pairs in the first 32 columns of the S
@@ -325,14 +317,13 @@ decode_attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
           const uint64_t b_desc = ptx::smem_desc_sw128(sm_v + (j & 1) * kSmemV);
 #pragma unroll
           for (int k = 0; k < 4; ++k)
-            ptx::mma_f16_ts(tmem_base + kColO, a_tmem + 8u * k, b_desc + 2u * k, idesc_o, (j | k) != 0 ? 1u : 0u);
+            ptx::mma_f16_ts_one(tmem_base + kColO, a_tmem + 8u * k, b_desc + 2u * k, idesc_o, (j | k) != 0 ? 1u : 0u);
         }
-        ptx::tc_commit(bar_vempty + 8 * (j & 1));
-        ptx::tc_commit(bar_ofull);
-        if (j + 1 == n_tiles) ptx::tc_commit(bar_done);
+        ptx::tc_commit_one(bar_vempty + 8 * (j & 1));
+        ptx::tc_commit_one(bar_ofull);
+        if (j + 1 == n_tiles) ptx::tc_commit_one(bar_done);
       }
     }
-    __syncwarp();
   } else {
     // ------------------- softmax / correction / tail / epilogue -------------
     const int quad = warp & 3;

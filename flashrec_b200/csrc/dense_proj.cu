@@ -639,7 +639,7 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* octet = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + kBarBytes);  // kOctet
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
   const int m_blocks = (g.M + kBlockM - 1) / kBlockM;
   const int n_blocks = (g.N + BLOCK_N - 1) / BLOCK_N;
   const int subs = EPI == kEpiPartial ? 1 : g.n_parts;
@@ -671,75 +671,66 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
   ptx::griddep_launch_dependents();
 
   if (warp == 0) {
-    if (lane == 0) {
-      uint32_t stage = 0, phase = 0;
-      bool ok = true;
-      for (int unit = blockIdx.x; unit < num_units && ok; unit += gridDim.x) {
-        for (int sub = 0; sub < subs && ok; ++sub) {
-          const Job j = job_at<EPI>(g, unit, sub, m_blocks, n_blocks);
-          const CUtensorMap* ta = j.part == 0 ? &ta0 : &ta1;
-          const CUtensorMap* tb = j.part == 0 ? &tb0 : &tb1;
-          for (int kb0 = j.kb0; kb0 < j.kb1; kb0 += stage_blocks) {
-            ok = ptx::mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag, status, 61);
-            if (!ok) break;
-            uint32_t sa = base + stage * stage_bytes;
-            const int kb1 = stage_blocks == 1 ? kb0 + 1 : min(kb0 + stage_blocks, j.kb1);
-            ptx::mbar_expect_tx(bar_full + 8 * stage, (kb1 - kb0) * block_bytes);
-            for (int kb = kb0; kb < kb1; ++kb, sa += block_bytes) {
-              ptx::tma_load_2d(sa, ta, kb * kBlockK, j.mb * kBlockM, bar_full + 8 * stage);
-              ptx::tma_load_2d(sa + a_bytes, tb, kb * kBlockK, j.nb * BLOCK_N, bar_full + 8 * stage);
-            }
-            if (++stage == n_stages) { stage = 0; phase ^= 1u; }
-          }
-        }
-      }
-    }
-    __syncwarp();
-  } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = ptx::make_idesc(1u, 1u, kBlockM, BLOCK_N);
-      uint32_t stage = 0, phase = 0;
-      bool ok = true;
-      int it = 0;
-      for (int unit = blockIdx.x; unit < num_units && ok; unit += gridDim.x) {
-        for (int sub = 0; sub < subs && ok; ++sub) {
-          const Job j = job_at<EPI>(g, unit, sub, m_blocks, n_blocks);
-          // a set of accumulators: of the whole job, or (kOctet) of one stage, one per k-block
-          uint32_t set = 0, d_tmem = 0;
-          auto next_set = [&]() {
-            set = it & 1;
-            d_tmem = tmem_base + set * (C::kAcc / 2 * BLOCK_N);
-            ok = ptx::mbar_wait(bar_tempty + 8 * set, ((it >> 1) & 1) ^ 1u, abort_flag, status, 62);
-            ++it;
-            if (ok) ptx::tc_fence_after();
-          };
-          if (ROWS != kOctet) next_set();
+    uint32_t stage = 0, phase = 0;
+    bool ok = true;
+    for (int unit = blockIdx.x; unit < num_units && ok; unit += gridDim.x) {
+      for (int sub = 0; sub < subs && ok; ++sub) {
+        const Job j = job_at<EPI>(g, unit, sub, m_blocks, n_blocks);
+        const CUtensorMap* ta = j.part == 0 ? &ta0 : &ta1;
+        const CUtensorMap* tb = j.part == 0 ? &tb0 : &tb1;
+        for (int kb0 = j.kb0; kb0 < j.kb1; kb0 += stage_blocks) {
+          ok = ptx::mbar_wait_warp(bar_empty + 8 * stage, phase ^ 1u, abort_flag, status, 61);
           if (!ok) break;
-          for (int kb0 = j.kb0; kb0 < j.kb1; kb0 += stage_blocks) {
-            if (ROWS == kOctet) next_set();
-            if (!ok) break;
-            ok = ptx::mbar_wait(bar_full + 8 * stage, phase, abort_flag, status, 63);
-            if (!ok) break;
-            ptx::tc_fence_after();
-            uint32_t sa = base + stage * stage_bytes;
-            const int kb1 = stage_blocks == 1 ? kb0 + 1 : min(kb0 + stage_blocks, j.kb1);
-            for (int kb = kb0; kb < kb1; ++kb, sa += block_bytes) {
-              const uint64_t a_desc = ptx::smem_desc_sw128(sa);
-              const uint64_t b_desc = ptx::smem_desc_sw128(sa + a_bytes);
-#pragma unroll
-              for (int k = 0; k < kBlockK / kUmmaK; ++k)
-                ptx::mma_f16(d_tmem, a_desc + 2u * k, b_desc + 2u * k, idesc, ((ROWS != kOctet && kb > j.kb0) || k > 0) ? 1u : 0u);
-              if (ROWS == kOctet) d_tmem += BLOCK_N;
-            }
-            ptx::tc_commit(bar_empty + 8 * stage);
-            if (ROWS == kOctet) ptx::tc_commit(bar_tfull + 8 * set);
-            if (++stage == n_stages) { stage = 0; phase ^= 1u; }
+          uint32_t sa = base + stage * stage_bytes;
+          const int kb1 = stage_blocks == 1 ? kb0 + 1 : min(kb0 + stage_blocks, j.kb1);
+          ptx::mbar_expect_tx_one(bar_full + 8 * stage, (kb1 - kb0) * block_bytes);
+          for (int kb = kb0; kb < kb1; ++kb, sa += block_bytes) {
+            ptx::tma_load_2d_one(sa, ta, kb * kBlockK, j.mb * kBlockM, bar_full + 8 * stage);
+            ptx::tma_load_2d_one(sa + a_bytes, tb, kb * kBlockK, j.nb * BLOCK_N, bar_full + 8 * stage);
           }
-          if (ok && ROWS != kOctet) ptx::tc_commit(bar_tfull + 8 * set);
+          if (++stage == n_stages) { stage = 0; phase ^= 1u; }
         }
       }
     }
-    __syncwarp();
+  } else if (warp == 1) {
+    constexpr uint32_t idesc = ptx::make_idesc(1u, 1u, kBlockM, BLOCK_N);
+    uint32_t stage = 0, phase = 0;
+    bool ok = true;
+    int it = 0;
+    for (int unit = blockIdx.x; unit < num_units && ok; unit += gridDim.x) {
+      for (int sub = 0; sub < subs && ok; ++sub) {
+        const Job j = job_at<EPI>(g, unit, sub, m_blocks, n_blocks);
+        // a set of accumulators: of the whole job, or (kOctet) of one stage, one per k-block
+        uint32_t set = 0, d_tmem = 0;
+        auto next_set = [&]() {
+          set = it & 1;
+          d_tmem = tmem_base + set * (C::kAcc / 2 * BLOCK_N);
+          ok = ptx::mbar_wait_warp(bar_tempty + 8 * set, ((it >> 1) & 1) ^ 1u, abort_flag, status, 62);
+          ++it;
+          if (ok) ptx::tc_fence_after();
+        };
+        if (ROWS != kOctet) next_set();
+        if (!ok) break;
+        for (int kb0 = j.kb0; kb0 < j.kb1; kb0 += stage_blocks) {
+          if (ROWS == kOctet) next_set();
+          if (!ok) break;
+          ok = ptx::mbar_wait_warp(bar_full + 8 * stage, phase, abort_flag, status, 63);
+          if (!ok) break;
+          ptx::tc_fence_after();
+          uint32_t sa = base + stage * stage_bytes;
+          const int kb1 = stage_blocks == 1 ? kb0 + 1 : min(kb0 + stage_blocks, j.kb1);
+          for (int kb = kb0; kb < kb1; ++kb, sa += block_bytes) {
+            ptx::mma_k_block_f16(d_tmem, ptx::smem_desc_sw128(sa), ptx::smem_desc_sw128(sa + a_bytes), idesc,
+                                 ROWS != kOctet && kb > j.kb0 ? 1u : 0u);
+            if (ROWS == kOctet) d_tmem += BLOCK_N;
+          }
+          ptx::tc_commit_one(bar_empty + 8 * stage);
+          if (ROWS == kOctet) ptx::tc_commit_one(bar_tfull + 8 * set);
+          if (++stage == n_stages) { stage = 0; phase ^= 1u; }
+        }
+        if (ok && ROWS != kOctet) ptx::tc_commit_one(bar_tfull + 8 * set);
+      }
+    }
   } else if (ROWS == kOctet) {
     // Warp 4 adds up: TMEM lanes 0 .. 31 are open to it, and all rows lie in lanes 0 .. 7. The other seven store the tile that
     // it has left in shared memory while it goes on with the next one; all eight meet once per tile.

@@ -12,7 +12,7 @@
 // sm_100a design: a persistent, warp-specialised kernel, one CTA per SM.
 //   warp 0      TMA producer: 128x128-byte A tile + BLOCK_N x128-byte B tile per
 //               stage, 128-byte swizzle, mbarrier complete_tx
-//   warp 1      allocates tensor memory; one lane issues tcgen05.mma
+//   warp 1      allocates tensor memory; an elected lane issues tcgen05.mma
 //               (kind::f8f6f4, M=128, N=BLOCK_N, K=32 per instruction, both
 //               operands K-major straight from shared memory), accumulating
 //               fp32 in TMEM; tcgen05.commit frees the stage / publishes the tile
@@ -35,7 +35,6 @@ namespace gemm {
 
 constexpr int kBlockM = 128;
 constexpr int kBlockK = 128;  // bytes == e4m3 elements: one 128-byte swizzle span
-constexpr int kUmmaK = 32;
 // 2 control warps (TMA, MMA) + epilogue warps. The plain epilogue uses one warp per TMEM lane
 // quadrant; the SwiGLU epilogue does ~40 instructions per element and gets four warps per quadrant
 // (each takes one 32-column chunk) so that it still hides under the main loop.
@@ -162,7 +161,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * C::kStages + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = ptx::warp_index();
   const int lane = threadIdx.x & 31;
   const int m_blocks = (M + kBlockM - 1) / kBlockM;
   const int n_blocks = (N + BLOCK_N - 1) / BLOCK_N;
@@ -198,59 +197,48 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
 
   if (warp == 0) {
     // ------------------------------ TMA producer ---------------------------
-    if (lane == 0) {
-      uint32_t stage = 0, phase = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        const TileCoord tc = tile_coord(tile, m_blocks, n_blocks);
-        const int m0 = tc.mb * kBlockM;
-        const int n0 = tc.nb * BLOCK_N;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          ok = ptx::mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag, status, 1);
-          if (!ok) break;
-          const uint32_t sa = base + stage * C::kStageBytes;
-          const uint32_t sbm = sa + C::kStageA;
-          ptx::mbar_expect_tx(bar_full + 8 * stage, C::kStageBytes);
-          ptx::tma_load_2d(sa, &tmap_a, kb * kBlockK, m0, bar_full + 8 * stage);
-          ptx::tma_load_2d(sbm, &tmap_b, kb * kBlockK, n0, bar_full + 8 * stage);
-          if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
-        }
+    uint32_t stage = 0, phase = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+      const TileCoord tc = tile_coord(tile, m_blocks, n_blocks);
+      const int m0 = tc.mb * kBlockM;
+      const int n0 = tc.nb * BLOCK_N;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        ok = ptx::mbar_wait_warp(bar_empty + 8 * stage, phase ^ 1u, abort_flag, status, 1);
+        if (!ok) break;
+        const uint32_t sa = base + stage * C::kStageBytes;
+        const uint32_t sbm = sa + C::kStageA;
+        ptx::mbar_expect_tx_one(bar_full + 8 * stage, C::kStageBytes);
+        ptx::tma_load_2d_one(sa, &tmap_a, kb * kBlockK, m0, bar_full + 8 * stage);
+        ptx::tma_load_2d_one(sbm, &tmap_b, kb * kBlockK, n0, bar_full + 8 * stage);
+        if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
       }
     }
-    __syncwarp();
   } else if (warp == 1) {
     // ------------------------------ MMA issuer -----------------------------
-    if (lane == 0) {
-      constexpr uint32_t idesc = ptx::make_idesc(0u, 0u, kBlockM, BLOCK_N);
-      uint32_t stage = 0, phase = 0;
-      bool ok = true;
-      int it = 0;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++it) {
-        const uint32_t buf = it & 1;
-        const uint32_t acc_phase = (it >> 1) & 1;
-        ok = ptx::mbar_wait(bar_tempty + 8 * buf, acc_phase ^ 1u, abort_flag, status, 2);
+    constexpr uint32_t idesc = ptx::make_idesc(0u, 0u, kBlockM, BLOCK_N);
+    uint32_t stage = 0, phase = 0;
+    bool ok = true;
+    int it = 0;
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++it) {
+      const uint32_t buf = it & 1;
+      const uint32_t acc_phase = (it >> 1) & 1;
+      ok = ptx::mbar_wait_warp(bar_tempty + 8 * buf, acc_phase ^ 1u, abort_flag, status, 2);
+      if (!ok) break;
+      ptx::tc_fence_after();
+      const uint32_t d_tmem = tmem_base + buf * BLOCK_N;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        ok = ptx::mbar_wait_warp(bar_full + 8 * stage, phase, abort_flag, status, 3);
         if (!ok) break;
         ptx::tc_fence_after();
-        const uint32_t d_tmem = tmem_base + buf * BLOCK_N;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          ok = ptx::mbar_wait(bar_full + 8 * stage, phase, abort_flag, status, 3);
-          if (!ok) break;
-          ptx::tc_fence_after();
-          const uint32_t sa = base + stage * C::kStageBytes;
-          const uint64_t a_desc = ptx::smem_desc_sw128(sa);
-          const uint64_t b_desc = ptx::smem_desc_sw128(sa + C::kStageA);
-#pragma unroll
-          for (int k = 0; k < kBlockK / kUmmaK; ++k) {
-            // +32 bytes along K inside the swizzled 128-byte row == +2 in the (addr >> 4) field
-            ptx::mma_f8f6f4(d_tmem, a_desc + 2u * k, b_desc + 2u * k, idesc, (kb | k) != 0 ? 1u : 0u);
-          }
-          ptx::tc_commit(bar_empty + 8 * stage);  // stage reusable once these MMAs have read it
-          if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
-        }
-        if (ok) ptx::tc_commit(bar_tfull + 8 * buf);  // accumulator complete
+        const uint32_t sa = base + stage * C::kStageBytes;
+        // steps of 32 bytes along K inside the swizzled 128-byte row
+        ptx::mma_k_block_f8(d_tmem, ptx::smem_desc_sw128(sa), ptx::smem_desc_sw128(sa + C::kStageA), idesc, kb != 0 ? 1u : 0u);
+        ptx::tc_commit_one(bar_empty + 8 * stage);  // stage reusable once these MMAs have read it
+        if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
       }
+      if (ok) ptx::tc_commit_one(bar_tfull + 8 * buf);  // accumulator complete
     }
-    __syncwarp();
   } else {
     // ------------------------------ epilogue -------------------------------
     const int quad = warp & 3;  // TMEM lane quadrant this warp may access
@@ -476,7 +464,7 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * C::kStages + 4 + C::kResBars);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = ptx::warp_index();
   const int lane = threadIdx.x & 31;
   const uint32_t rank = ptx::cluster_ctarank();
   const int pair = blockIdx.x >> 1;
@@ -518,29 +506,26 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
 
   if (warp == 0) {
     // ------------------------------ TMA producer (both CTAs) ---------------
-    if (lane == 0) {
-      uint32_t stage = 0, phase = 0;
-      bool ok = true;
-      for (int tile = pair; tile < num_tiles && ok; tile += n_pairs) {
-        const TileCoord tc = tile_coord(tile, m_blocks, n_blocks);
-        const int m0 = tc.mb * (2 * kBlockM) + static_cast<int>(rank) * kBlockM;
-        const int n0 = tc.nb * BLOCK_N + static_cast<int>(rank) * (BLOCK_N / 2);
-        for (int kb = 0; kb < num_kb; ++kb) {
-          ok = ptx::mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag, status, 21);
-          if (!ok) break;
-          const uint32_t sa = base + stage * C::kStageBytes;
-          const uint32_t full0 = ptx::mapa(bar_full + 8 * stage, 0);  // CTA 0 collects both CTAs' bytes
-          if (rank == 0) ptx::mbar_expect_tx(bar_full + 8 * stage, 2 * C::kStageBytes);
-          ptx::tma_load_2d_pair(sa, &tmap_a, kb * kBlockK, m0, full0);
-          ptx::tma_load_2d_pair(sa + C::kStageA, &tmap_b, kb * kBlockK, n0, full0);
-          if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
-        }
+    uint32_t stage = 0, phase = 0;
+    bool ok = true;
+    for (int tile = pair; tile < num_tiles && ok; tile += n_pairs) {
+      const TileCoord tc = tile_coord(tile, m_blocks, n_blocks);
+      const int m0 = tc.mb * (2 * kBlockM) + static_cast<int>(rank) * kBlockM;
+      const int n0 = tc.nb * BLOCK_N + static_cast<int>(rank) * (BLOCK_N / 2);
+      for (int kb = 0; kb < num_kb; ++kb) {
+        ok = ptx::mbar_wait_warp(bar_empty + 8 * stage, phase ^ 1u, abort_flag, status, 21);
+        if (!ok) break;
+        const uint32_t sa = base + stage * C::kStageBytes;
+        const uint32_t full0 = ptx::mapa(bar_full + 8 * stage, 0);  // CTA 0 collects both CTAs' bytes
+        if (rank == 0) ptx::mbar_expect_tx_one(bar_full + 8 * stage, 2 * C::kStageBytes);
+        ptx::tma_load_2d_pair_one(sa, &tmap_a, kb * kBlockK, m0, full0);
+        ptx::tma_load_2d_pair_one(sa + C::kStageA, &tmap_b, kb * kBlockK, n0, full0);
+        if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
       }
     }
-    __syncwarp();
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (CTA 0 only) ----------------
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
       constexpr uint32_t idesc = ptx::make_idesc(0u, 0u, 2 * kBlockM, BLOCK_N);
       uint32_t stage = 0, phase = 0;
       bool ok = true;
@@ -548,31 +533,27 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       for (int tile = pair; tile < num_tiles && ok; tile += n_pairs, ++it) {
         const uint32_t buf = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1;
-        ok = ptx::mbar_wait(bar_tempty + 8 * buf, acc_phase ^ 1u, abort_flag, status, 22);
+        ok = ptx::mbar_wait_warp(bar_tempty + 8 * buf, acc_phase ^ 1u, abort_flag, status, 22);
         if (!ok) break;
         ptx::tc_fence_after();
         const uint32_t d_tmem = tmem_base + buf * BLOCK_N;
         for (int kb = 0; kb < num_kb; ++kb) {
-          ok = ptx::mbar_wait(bar_full + 8 * stage, phase, abort_flag, status, 23);
+          ok = ptx::mbar_wait_warp(bar_full + 8 * stage, phase, abort_flag, status, 23);
           if (!ok) break;
           ptx::tc_fence_after();
           const uint32_t sa = base + stage * C::kStageBytes;
-          const uint64_t a_desc = ptx::smem_desc_sw128(sa);
-          const uint64_t b_desc = ptx::smem_desc_sw128(sa + C::kStageA);
-#pragma unroll
-          for (int k = 0; k < kBlockK / kUmmaK; ++k)
-            ptx::mma_f8f6f4_pair(d_tmem, a_desc + 2u * k, b_desc + 2u * k, idesc, (kb | k) != 0 ? 1u : 0u);
-          ptx::tc_commit_pair(ptx::mapa(bar_empty + 8 * stage, 0));  // stage reusable in both CTAs
-          ptx::tc_commit_pair(ptx::mapa(bar_empty + 8 * stage, 1));
+          ptx::mma_k_block_f8_pair(d_tmem, ptx::smem_desc_sw128(sa), ptx::smem_desc_sw128(sa + C::kStageA), idesc,
+                                   kb != 0 ? 1u : 0u);
+          ptx::tc_commit_pair_one(ptx::mapa(bar_empty + 8 * stage, 0));  // stage reusable in both CTAs
+          ptx::tc_commit_pair_one(ptx::mapa(bar_empty + 8 * stage, 1));
           if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
         }
         if (ok) {
-          ptx::tc_commit_pair(ptx::mapa(bar_tfull + 8 * buf, 0));  // accumulator complete in both CTAs
-          ptx::tc_commit_pair(ptx::mapa(bar_tfull + 8 * buf, 1));
+          ptx::tc_commit_pair_one(ptx::mapa(bar_tfull + 8 * buf, 0));  // accumulator complete in both CTAs
+          ptx::tc_commit_pair_one(ptx::mapa(bar_tfull + 8 * buf, 1));
         }
       }
     }
-    __syncwarp();
   } else {
     // ------------------------------ epilogue (both CTAs) -------------------
     const int quad = warp & 3;
@@ -1136,7 +1117,7 @@ gemm_fp8_splitk_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * C::kStages + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = ptx::warp_index();
   const int lane = threadIdx.x & 31;
   const int rank = static_cast<int>(ptx::cluster_ctarank());
   const int tile = blockIdx.x / S;
@@ -1170,40 +1151,30 @@ gemm_fp8_splitk_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
   ptx::griddep_launch_dependents();
 
   if (warp == 0) {
-    if (lane == 0) {
-      uint32_t stage = 0, phase = 0;
-      for (int i = 0; i < per; ++i) {
-        if (!ptx::mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag, status, 31)) break;
-        const uint32_t sa = base + stage * C::kStageBytes;
-        const int kx = (kb0 + i) * kBlockK;
-        ptx::mbar_expect_tx(bar_full + 8 * stage, C::kStageBytes);
-        ptx::tma_load_2d(sa, &tmap_a, kx, m0, bar_full + 8 * stage);
-        ptx::tma_load_2d(sa + C::kStageA, &tmap_b, kx, n0, bar_full + 8 * stage);
-        if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
-      }
+    uint32_t stage = 0, phase = 0;
+    for (int i = 0; i < per; ++i) {
+      if (!ptx::mbar_wait_warp(bar_empty + 8 * stage, phase ^ 1u, abort_flag, status, 31)) break;
+      const uint32_t sa = base + stage * C::kStageBytes;
+      const int kx = (kb0 + i) * kBlockK;
+      ptx::mbar_expect_tx_one(bar_full + 8 * stage, C::kStageBytes);
+      ptx::tma_load_2d_one(sa, &tmap_a, kx, m0, bar_full + 8 * stage);
+      ptx::tma_load_2d_one(sa + C::kStageA, &tmap_b, kx, n0, bar_full + 8 * stage);
+      if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
     }
-    __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = ptx::make_idesc(0u, 0u, kBlockM, C::kTileN);
-      uint32_t stage = 0, phase = 0;
-      bool ok = true;
-      for (int i = 0; i < per; ++i) {
-        ok = ptx::mbar_wait(bar_full + 8 * stage, phase, abort_flag, status, 32);
-        if (!ok) break;
-        ptx::tc_fence_after();
-        const uint32_t sa = base + stage * C::kStageBytes;
-        const uint64_t a_desc = ptx::smem_desc_sw128(sa);
-        const uint64_t b_desc = ptx::smem_desc_sw128(sa + C::kStageA);
-#pragma unroll
-        for (int k = 0; k < kBlockK / kUmmaK; ++k)
-          ptx::mma_f8f6f4(tmem_base, a_desc + 2u * k, b_desc + 2u * k, idesc, (i | k) != 0 ? 1u : 0u);
-        ptx::tc_commit(bar_empty + 8 * stage);
-        if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
-      }
-      if (ok) ptx::tc_commit(bar_tfull);
+    constexpr uint32_t idesc = ptx::make_idesc(0u, 0u, kBlockM, C::kTileN);
+    uint32_t stage = 0, phase = 0;
+    bool ok = true;
+    for (int i = 0; i < per; ++i) {
+      ok = ptx::mbar_wait_warp(bar_full + 8 * stage, phase, abort_flag, status, 32);
+      if (!ok) break;
+      ptx::tc_fence_after();
+      const uint32_t sa = base + stage * C::kStageBytes;
+      ptx::mma_k_block_f8(tmem_base, ptx::smem_desc_sw128(sa), ptx::smem_desc_sw128(sa + C::kStageA), idesc, i != 0 ? 1u : 0u);
+      ptx::tc_commit_one(bar_empty + 8 * stage);
+      if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
     }
-    __syncwarp();
+    if (ok) ptx::tc_commit_one(bar_tfull);
   }
 
   // ---- cluster-wide reduction. Every thread of every CTA takes part in the cluster barriers;

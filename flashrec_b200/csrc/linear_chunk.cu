@@ -341,8 +341,8 @@ chunk_kernel(const __grid_constant__ ChunkMaps maps, const __grid_constant__ Chu
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + kSets + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const bool compute = tid < kCompute, issuer = tid == kCompute, loader = tid == kCompute + 32;
+  const int tid = threadIdx.x, warp = ptx::warp_index(), lane = tid & 31;
+  const bool compute = warp < kCompute / 32, issuer = warp == kCompute / 32, loader = warp == kCompute / 32 + 1;
   ptx::griddep_wait();
   const int h = blockIdx.x / pl.v_blocks, c0 = (blockIdx.x % pl.v_blocks) * kVb;
   const int b = blockIdx.z, seg = blockIdx.y;
@@ -379,23 +379,23 @@ chunk_kernel(const __grid_constant__ ChunkMaps maps, const __grid_constant__ Chu
   const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
   const Factors* factors = static_cast<const Factors*>(g.factors) + (first_chunk(q0, b) + seg * (pl.seg_len / kChunk)) * a.heads + h;
 
-  // ---- TMA and tcgen05.mma, one thread each --------------------------------------------------------------
+  // ---- TMA and tcgen05.mma, one warp each ----------------------------------------------------------------
   auto load_v = [&](int it) {
     const int set = it % kSets;
-    ptx::mbar_expect_tx(bar_v + 8 * set, kBox + sizeof(Factors));
-    ptx::tma_load_2d(base + off_v + set * kBox, &maps.v, h * a.vdim + c0, t_begin + it * kChunk, bar_v + 8 * set);
-    ptx::bulk_load(ptx::smem_u32(fac + set), factors + static_cast<int64_t>(it) * a.heads, sizeof(Factors), bar_v + 8 * set);
+    ptx::mbar_expect_tx_one(bar_v + 8 * set, kBox + sizeof(Factors));
+    ptx::tma_load_2d_one(base + off_v + set * kBox, &maps.v, h * a.vdim + c0, t_begin + it * kChunk, bar_v + 8 * set);
+    ptx::bulk_load_one(ptx::smem_u32(fac + set), factors + static_cast<int64_t>(it) * a.heads, sizeof(Factors), bar_v + 8 * set);
   };
   auto load_qk = [&](int it) {
     const int t = t_begin + it * kChunk;
-    ptx::mbar_expect_tx(bar_qk, (STATE_ONLY ? 1 : 2) * off_k);
+    ptx::mbar_expect_tx_one(bar_qk, (STATE_ONLY ? 1 : 2) * off_k);
     for (int x = 0; x < pl.boxes; ++x) {
       const int col = kh * a.dim + x * 64;
-      if (!STATE_ONLY) ptx::tma_load_2d(base + off_q + x * kBox, &maps.q, col, t, bar_qk);
-      ptx::tma_load_2d(base + off_k + x * kBox, &maps.k, col, t, bar_qk);
+      if (!STATE_ONLY) ptx::tma_load_2d_one(base + off_q + x * kBox, &maps.q, col, t, bar_qk);
+      ptx::tma_load_2d_one(base + off_k + x * kBox, &maps.k, col, t, bar_qk);
       if (CHANNEL) {
-        if (!STATE_ONLY) ptx::tma_load_2d(base + off_q + kq + x * kBox, &maps.q_lo, col, t, bar_qk);
-        ptx::tma_load_2d(base + off_k + kq + x * kBox, &maps.k_lo, col, t, bar_qk);
+        if (!STATE_ONLY) ptx::tma_load_2d_one(base + off_q + kq + x * kBox, &maps.q_lo, col, t, bar_qk);
+        ptx::tma_load_2d_one(base + off_k + kq + x * kBox, &maps.k_lo, col, t, bar_qk);
       }
     }
   };
@@ -405,13 +405,13 @@ chunk_kernel(const __grid_constant__ ChunkMaps maps, const __grid_constant__ Chu
     const uint64_t lo = kq >> 4;
     steps(a.dim / 16, [&](int k) {
       const uint64_t o = (k >> 2) * (kBox / 16) + 2u * (k & 3);
-      ptx::mma_f16(col_p, qd + o, kd + o, idesc, k > 0 ? 1u : 0u);
+      ptx::mma_f16_one(col_p, qd + o, kd + o, idesc, k > 0 ? 1u : 0u);
       if (CHANNEL) {
-        ptx::mma_f16(col_p, qd + o, kd + lo + o, idesc, 1u);
-        ptx::mma_f16(col_p, qd + lo + o, kd + o, idesc, 1u);
+        ptx::mma_f16_one(col_p, qd + o, kd + lo + o, idesc, 1u);
+        ptx::mma_f16_one(col_p, qd + lo + o, kd + o, idesc, 1u);
       }
     });
-    ptx::tc_commit(bar_g);
+    ptx::tc_commit_one(bar_g);
   };
   auto wait_bar = [&](uint32_t bar, uint32_t parity, int site) {  // whole warps
     if (lane == 0) ptx::mbar_wait(bar, parity, abort_flag, status, site);
@@ -514,8 +514,7 @@ chunk_kernel(const __grid_constant__ ChunkMaps maps, const __grid_constant__ Chu
   // A full chunk's output tile leaves by TMA (a partial one must not touch the rows or columns beside it).
   auto full_tile = [&](int it) { return !STATE_ONLY && vb == kVb && t_end - (t_begin + it * kChunk) >= kChunk; };
   auto store_tile = [&](int it) {
-    ptx::tma_store_2d(&maps.out, base + off_v + (it % kSets) * kBox, h * a.vdim + c0, t_begin + it * kChunk);
-    ptx::bulk_commit();
+    ptx::tma_store_2d_one(&maps.out, base + off_v + (it % kSets) * kBox, h * a.vdim + c0, t_begin + it * kChunk);
   };
   uint32_t x_now[8], x_next[8];
   if (loader) {
@@ -524,7 +523,7 @@ chunk_kernel(const __grid_constant__ ChunkMaps maps, const __grid_constant__ Chu
     if (n_chunks > 1) load_v(1);
   }
   __syncwarp();
-  if (issuer && !STATE_ONLY && ptx::mbar_wait(bar_qk, 0, abort_flag, status, 91)) issue_scores();
+  if (issuer && !STATE_ONLY && ptx::mbar_wait_warp(bar_qk, 0, abort_flag, status, 91)) issue_scores();
   __syncwarp();
   if (compute) operands(0, x_now);
   for (int it = 0; it < n_chunks; ++it) {
@@ -539,7 +538,7 @@ chunk_kernel(const __grid_constant__ ChunkMaps maps, const __grid_constant__ Chu
     if (warp == kCompute / 32 + 1) {
       if (loader) {
         if (it > 0 && full_tile(it - 1)) store_tile(it - 1);
-        if (more && ptx::mbar_wait(bar_su, ph, abort_flag, status, 97)) {  // q's and k's tiles are free
+        if (more && ptx::mbar_wait_warp(bar_su, ph, abort_flag, status, 97)) {  // q's and k's tiles are free
           load_qk(it + 1);
           if (it + 2 < n_chunks) {  // and the v tile of the chunk before, once its output has left
             ptx::bulk_wait_read<0>();
@@ -559,21 +558,21 @@ chunk_kernel(const __grid_constant__ ChunkMaps maps, const __grid_constant__ Chu
         const uint64_t qd = ptx::smem_desc_sw128(base + off_q), qlo = qd + (kq >> 4), sd = desc_mn(base + off_s, s_bytes);
         steps(a.dim / 16, [&](int k) {
           const uint64_t o = (k >> 2) * (kBox / 16) + 2u * (k & 3), so = k * 128u;
-          ptx::mma_f16(col_in, qd + o, sd + so, idesc_pair, k > 0 ? 1u : 0u);
-          if (CHANNEL) ptx::mma_f16(col_in, qlo + o, sd + so, idesc_pair, 1u);
+          ptx::mma_f16_one(col_in, qd + o, sd + so, idesc_pair, k > 0 ? 1u : 0u);
+          if (CHANNEL) ptx::mma_f16_one(col_in, qlo + o, sd + so, idesc_pair, 1u);
         });
       } else {
-        ptx::mbar_wait(bar_qk, ph, abort_flag, status, 96);
+        ptx::mbar_wait_warp(bar_qk, ph, abort_flag, status, 96);
       }
       // A = K^T: rows of S by tokens, a second box of rows for more than 64 (else the first once more, unused)
       const uint64_t kt = desc_mn(base + off_k, pl.boxes > 1 ? kBox : 0);
       const uint64_t ud = desc_mn(base + (CHANNEL ? off_v + set * kBox : off_x), kBox);
       steps(k_tok, [&](int k) {
         const uint64_t o = k * 128u;
-        ptx::mma_f16(col_su, kt + o, ud + o, (CHANNEL ? idesc_one : idesc_pair) | kMnA, k > 0 ? 1u : 0u);
-        if (CHANNEL) ptx::mma_f16(col_su, kt + (kq >> 4) + o, ud + o, idesc_one | kMnA, 1u);
+        ptx::mma_f16_one(col_su, kt + o, ud + o, (CHANNEL ? idesc_one : idesc_pair) | kMnA, k > 0 ? 1u : 0u);
+        if (CHANNEL) ptx::mma_f16_one(col_su, kt + (kq >> 4) + o, ud + o, idesc_one | kMnA, 1u);
       });
-      ptx::tc_commit(bar_su);
+      ptx::tc_commit_one(bar_su);
     }
     __syncwarp();
 
@@ -635,15 +634,15 @@ chunk_kernel(const __grid_constant__ ChunkMaps maps, const __grid_constant__ Chu
         ptx::tc_fence_after();
         constexpr uint32_t idesc_one = ptx::make_idesc(1u, 1u, kChunk, kVb) | (1u << 16);
         const uint64_t vd = desc_mn(base + off_v + set * kBox, kBox);
-        if (CHANNEL) ptx::mbar_wait(bar_su, ph, abort_flag, status, 100);  // Q S' is in place: products of another shape follow
+        if (CHANNEL) ptx::mbar_wait_warp(bar_su, ph, abort_flag, status, 100);  // Q S' is in place: products of another shape follow
         steps(k_tok, [&](int k) {
           const uint32_t pc = col_p + (k >> 1) * 32 + (k & 1) * 8;
-          ptx::mma_f16_ts(col_pu, pc, vd + k * 128u, idesc_one, CHANNEL || k > 0 ? 1u : 0u);
-          ptx::mma_f16_ts(col_pu, pc + 16, vd + k * 128u, idesc_one, 1u);
+          ptx::mma_f16_ts_one(col_pu, pc, vd + k * 128u, idesc_one, CHANNEL || k > 0 ? 1u : 0u);
+          ptx::mma_f16_ts_one(col_pu, pc + 16, vd + k * 128u, idesc_one, 1u);
         });
-        ptx::tc_commit(bar_o);
-        if (more && ptx::mbar_wait(bar_o, ph, abort_flag, status, 99) &&  // the next scores overwrite P
-            ptx::mbar_wait(bar_qk, ph ^ 1, abort_flag, status, 98))
+        ptx::tc_commit_one(bar_o);
+        if (more && ptx::mbar_wait_warp(bar_o, ph, abort_flag, status, 99) &&  // the next scores overwrite P
+            ptx::mbar_wait_warp(bar_qk, ph ^ 1, abort_flag, status, 98))
           issue_scores();
       }
       __syncwarp();
