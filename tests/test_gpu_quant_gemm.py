@@ -277,6 +277,25 @@ def test_gemm_silu_epilogue_corner_inputs(case):
         assert torch.equal(amax.flatten()[finite], want[finite]), (case, mode)
 
 
+@pytest.mark.parametrize("m,n,k", [(1500, 2048, 512), (700, 4104, 256), (3000, 1000, 2064), (257, 304, 6144)])
+def test_gemm_tile_choice_keeps_the_bits(m, n, k):
+    """Every tile and the chosen one (none of these splits K by itself) give the same product and the same update."""
+    from flashrec_b200.kernel.sglops import fp8_scaled_mm, fp8_scaled_mm_add_
+
+    g = torch.Generator().manual_seed(m)
+    aq, asc = O.per_token_quant_fp8(torch.randn(m, k, generator=g).bfloat16())
+    wq, wsc = O.quantize_weight_fp8(0.05 * torch.randn(n, k, generator=g))
+    aq, asc, wq, wsc = aq.to(DEV), asc.to(DEV), wq.to(DEV), wsc.to(DEV)
+    bias = torch.randn(n, generator=g).bfloat16().to(DEV)  # with a bias K is never split
+    res = torch.randn(m, (n + 15) // 8 * 8, generator=g).bfloat16().to(DEV)
+    ref = fp8_scaled_mm(aq, wq.t(), asc, wsc, torch.bfloat16, bias, block_n=64)
+    upd = fp8_scaled_mm_add_(aq, wq.t(), asc, wsc, res.clone()[:, :n], block_n=64)
+    for tile in (128, 256, 512, 0):
+        assert torch.equal(fp8_scaled_mm(aq, wq.t(), asc, wsc, torch.bfloat16, bias, block_n=tile), ref), tile
+        if tile != 0 or m > 1024 or k < 4096:
+            assert torch.equal(fp8_scaled_mm_add_(aq, wq.t(), asc, wsc, res.clone()[:, :n], block_n=tile), upd), tile
+
+
 @pytest.mark.parametrize("m,n,k,block_n", [(300, 512, 256, 0), (37, 200, 128, 64), (128, 256, 2048, 256),
                                            (700, 1024, 384, 512), (513, 200, 512, 512), (4100, 2048, 256, 0),
                                            (512, 2048, 6144, 1024), (300, 200, 384, 1024), (512, 2048, 2048, 0),
