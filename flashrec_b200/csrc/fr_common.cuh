@@ -304,6 +304,101 @@ __device__ __forceinline__ uint32_t silu_mul_pack(uint32_t g, uint32_t u, const 
   return pack_bf16(a, b);
 }
 
+// two fp32 operations per instruction, each rounded as the scalar one is
+__device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ void unpack_f32x2(uint64_t v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint32_t pack_bf16_f32x2(uint64_t v) {
+  float lo, hi;
+  unpack_f32x2(v, lo, hi);
+  return pack_bf16(lo, hi);
+}
+__device__ __forceinline__ uint32_t min_bf16x2(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("min.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
+__device__ __forceinline__ uint32_t max_bf16x2(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("max.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
+__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
+
+// y = bf16(silu(g) * u) of 2 N gate and up values in bf16 pairs, silu rounded to bf16 as silu_bf16 does; returns the pairs' largest
+// |y| (NaN left out). The rounding is known when the fast result, 24 fp32 ulp less and 24 ulp more, rounds to the same value both
+// times; pairs where it does not, and all pairs of a call with a gate below -60 (the exponential overflows from -88 on) or above 1e38 (its exponent does),
+// are read from the table. The products equal those of silu_mul_pack, except that results below 2^-126 are rounded once, not twice.
+template <int N>
+__device__ __forceinline__ uint32_t swiglu_pairs(const uint32_t (&g)[N], const uint32_t (&u)[N], const uint16_t* __restrict__ table,
+                                                 uint32_t (&y)[N]) {
+  constexpr double kLog2e = 1.4426950408889634074;
+  constexpr float kHi = static_cast<float>(kLog2e), kLo = static_cast<float>(kLog2e - static_cast<double>(kHi));
+  constexpr float kUlps = 24.0f / 8388608.0f;
+  const uint64_t hi2 = pack_f32x2(kHi, kHi), neg_hi2 = pack_f32x2(-kHi, -kHi), neg_lo2 = pack_f32x2(-kLo, -kLo);
+  const uint64_t ln2 = pack_f32x2(0.693147182f, 0.693147182f), one = pack_f32x2(1.0f, 1.0f);
+  const uint64_t down = pack_f32x2(1.0f - kUlps, 1.0f - kUlps), up = pack_f32x2(1.0f + kUlps, 1.0f + kUlps);
+  uint32_t unsure = 0u, least = g[0], most = g[0];
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    least = min_bf16x2(least, g[j]);
+    most = max_bf16x2(most, g[j]);
+    const uint64_t gv = pack_f32x2(bf16lo(g[j]), bf16hi(g[j]));
+    // -g log2 e as a sum of two floats, then 2^ of it: ex2 of the first and a first-order correction for the second
+    const uint64_t th = mul_f32x2(gv, hi2);
+    const uint64_t tl = fma_f32x2(gv, neg_lo2, fma_f32x2(gv, neg_hi2, th));
+    float t0, t1;
+    unpack_f32x2(th, t0, t1);
+    uint64_t e = pack_f32x2(ex2_approx(-t0), ex2_approx(-t1));
+    e = add_f32x2(fma_f32x2(e, mul_f32x2(tl, ln2), e), one);
+    float d0, d1, r0, r1;
+    unpack_f32x2(e, d0, d1);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(d0));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(d1));
+    const uint64_t s = mul_f32x2(gv, pack_f32x2(r0, r1));
+    y[j] = pack_bf16_f32x2(mul_f32x2(s, down));
+    if (y[j] != pack_bf16_f32x2(mul_f32x2(s, up))) unsure |= 1u << j;
+  }
+  if (fminf(bf16lo(least), bf16hi(least)) < -60.0f || fmaxf(bf16lo(most), bf16hi(most)) > 1e38f) unsure = 0xffffffffu;
+  if (unsure != 0u) {
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+      if ((unsure >> j) & 1u)
+        y[j] = static_cast<uint32_t>(__ldg(table + (g[j] & 0xffffu))) | static_cast<uint32_t>(__ldg(table + (g[j] >> 16))) << 16;
+  }
+  uint32_t amax = 0u;
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    y[j] = mul_bf16x2(y[j], u[j]);
+    amax = max_bf16x2(amax, y[j] & 0x7fff7fffu);
+  }
+  return amax;
+}
+
 // e4m3 byte -> fp32 (exact).
 __device__ __forceinline__ float e4m3_to_float(uint8_t b) {
   __half_raw h = __nv_cvt_fp8_to_halfraw(static_cast<__nv_fp8_storage_t>(b), __NV_E4M3);

@@ -277,6 +277,29 @@ def test_gemm_silu_epilogue_corner_inputs(case):
         assert torch.equal(amax.flatten()[finite], want[finite]), (case, mode)
 
 
+@pytest.mark.parametrize("mode", [1, 2])
+def test_gemm_silu_epilogue_every_gate(mode):
+    """All 65536 bf16 gates, as channel scales of a product of ones, times one and times -3: the unfused kernel's results, which
+    come from fp64, bit for bit (NaN as NaN)."""
+    from flashrec_b200.kernel.sglops import fp8_scaled_mm_silu_mul, interleave_gate_up, silu_and_mul
+
+    d, k = 65536, 16
+    gates = torch.arange(d, dtype=torch.int32, device=DEV).to(torch.int16).view(torch.bfloat16)
+    a = torch.zeros(2, k, device=DEV)
+    a[:, 0] = 1.0
+    w = torch.zeros(2 * d, k, device=DEV)
+    w[:, 0] = 1.0
+    for up in (1.0, -3.0):
+        scales = torch.cat((gates.float(), torch.full((d,), up, device=DEV)))
+        wi, si = interleave_gate_up(w.to(torch.float8_e4m3fn), scales)
+        y, _ = fp8_scaled_mm_silu_mul(a.to(torch.float8_e4m3fn), wi, torch.ones(2, 1, device=DEV), si, mode=mode)
+        rows = gates.view(16, -1)
+        want = silu_and_mul(torch.cat((rows, torch.full_like(rows, up)), dim=1)).reshape(1, d).expand(2, -1)
+        number = ~want.isnan()
+        assert torch.equal(y.isnan(), want.isnan())
+        assert torch.equal(y.view(torch.int16)[number], want.view(torch.int16)[number])
+
+
 @pytest.mark.parametrize("m,n,k", [(1500, 2048, 512), (700, 4104, 256), (3000, 1000, 2064), (257, 304, 6144)])
 def test_gemm_tile_choice_keeps_the_bits(m, n, k):
     """Every tile and the chosen one (none of these splits K by itself) give the same product and the same update."""
