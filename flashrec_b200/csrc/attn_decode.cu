@@ -308,6 +308,7 @@ __global__ void __launch_bounds__(kThreads) decode_attn_kernel(Params p) {
 // every CTA compares its chunk of rows with the group's first row and lowers
 // out[group] with an atomicMin (out is pre-set to the first row's length).
 constexpr int kPlanRowsPerCta = 32;
+constexpr int kPlanFlight = 8;
 
 __global__ void plan_init_kernel(const int32_t* __restrict__ indptr, const int32_t* __restrict__ group_rows,
                                  int32_t* __restrict__ out, int n_groups) {
@@ -332,10 +333,21 @@ __global__ void __launch_bounds__(256) plan_kernel(const int32_t* __restrict__ i
     const int32_t* cur = indices + indptr[r];
     const int len = min(ref_len, indptr[r + 1] - indptr[r]);
     int lcp = len;
-    for (int i = 0; i < len; i += 32) {
-      const bool diff = (i + lane < len) && (cur[i + lane] != ref[i + lane]);
-      const uint32_t bal = __ballot_sync(0xffffffffu, diff);
-      if (bal) { lcp = i + __ffs(bal) - 1; break; }
+    // kPlanFlight loads of each list in flight per lane: one round of latency per 256 keys, not per 32 (512 rows of 640 keys:
+    // 34 -> 8 us)
+    for (int i0 = 0; i0 < len && lcp == len; i0 += 32 * kPlanFlight) {
+      int32_t a[kPlanFlight], b[kPlanFlight];
+#pragma unroll
+      for (int x = 0; x < kPlanFlight; ++x) {
+        const int i = i0 + 32 * x + lane;
+        a[x] = i < len ? cur[i] : 0;
+        b[x] = i < len ? ref[i] : 0;
+      }
+#pragma unroll
+      for (int x = kPlanFlight - 1; x >= 0; --x) {
+        const uint32_t bal = __ballot_sync(0xffffffffu, a[x] != b[x]);
+        if (bal) lcp = i0 + 32 * x + __ffs(bal) - 1;
+      }
     }
     if (lane == 0) atomicMin(out + grp, lcp);
   }

@@ -165,6 +165,28 @@ __global__ void __launch_bounds__(256) shared_kv_prepare_kernel(Params p) {
   }
 }
 
+// Score of one key (e4m3, the thread's own row of it in `kk`) with query row r of the swizzled Q tile.
+__device__ __forceinline__ float tail_score(const uint4 (&kk)[kD / 16], const uint8_t* q_row, int r) {
+  float dot = 0.f;
+#pragma unroll
+  for (int c = 0; c < kD / 16; ++c) {
+    const uint8_t* qb = q_row + (c >> 2) * (kSmemQ / 2);
+    const int ch = (c & 3) * 2;
+    const uint4 q0 = *reinterpret_cast<const uint4*>(qb + (((ch) ^ (r & 7)) << 4));
+    const uint4 q1 = *reinterpret_cast<const uint4*>(qb + (((ch + 1) ^ (r & 7)) << 4));
+    const uint32_t kw[4] = {kk[c].x, kk[c].y, kk[c].z, kk[c].w};
+    const uint32_t qw[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 ka = e4m3x2_to_float2(static_cast<uint16_t>(kw[i] & 0xffffu));
+      const float2 kb2 = e4m3x2_to_float2(static_cast<uint16_t>(kw[i] >> 16));
+      dot += bf16lo(qw[2 * i]) * ka.x + bf16hi(qw[2 * i]) * ka.y + bf16lo(qw[2 * i + 1]) * kb2.x +
+             bf16hi(qw[2 * i + 1]) * kb2.y;
+    }
+  }
+  return dot;
+}
+
 // ---------------------------------------------------------------------------
 // step 2
 // ---------------------------------------------------------------------------
@@ -217,6 +239,32 @@ decode_attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   const int gh = grp * p.hkv + kvh;
 
   const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
+
+  // Softmax threads: the row and its tail, the slots after the shared prefix. What the first kBatch tail keys need (list entries,
+  // then keys) is on its way while the pipeline fills, and the scores are ready before the first tile; all of it after the last
+  // tile took 8.0 of a CTA's 21.5 us (one request of 512 beams and 640 keys). Launches: 22.8 -> 20.9 us there, 32 requests 179 -> 163.
+  constexpr int kBatch = 4;
+  const int r = (warp & 3) * 32 + lane;  // query vector == TMEM lane == P row
+  const int beam = beam0 + r / G;
+  const bool live = beam < rows_in_group;
+  const int row = row0 + (live ? beam : 0);
+  int t_beg = 0, t_len = 0, slot[kBatch];
+  auto load_slots = [&](int t0) {
+#pragma unroll
+    for (int b = 0; b < kBatch; ++b) {
+      slot[b] = 0;
+      if (t0 + b < t_len) slot[b] = max(0, min(p.indices[t_beg + t0 + b], p.num_slots - 1));
+    }
+  };
+  if (!CAUSAL && warp >= 2) {
+    t_beg = p.indptr[row] + ls;
+    t_len = live ? max(p.indptr[row + 1] - t_beg, 0) : 0;
+    load_slots(0);
+#pragma unroll
+    for (int b = 0; b < kBatch; ++b)  // an earlier step's values have left L2 since
+      if (b < t_len)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(p.vc + static_cast<int64_t>(slot[b]) * p.cv_s + kvh * p.cv_h));
+  }
 
   if (threadIdx.x == 0) {
     ptx::mbar_init(bar_q, 1);
@@ -327,14 +375,37 @@ decode_attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   } else {
     // ------------------- softmax / correction / tail / epilogue -------------
     const int quad = warp & 3;
-    const int r = quad * 32 + lane;  // query vector == TMEM lane == P row
-    const int beam = beam0 + r / G;
-    const bool live = beam < rows_in_group;
-    const int row = row0 + (live ? beam : 0);
     const int head = kvh * G + r % G;
     const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
     float m_used = -INFINITY, l_sum = 0.f;
     bool ok = true;
+    // ---- scores of the first tail keys --------------------------------------
+    const uint8_t* q_row = smem + r * 128;  // + k-block * 16 KB + (chunk ^ (r & 7)) * 16
+    int max_len = t_len;                    // warp-uniform
+    float sc[kBatch];
+    auto load_key = [&](int t0, int b, uint4 (&kk)[kD / 16]) {
+      if (t0 + b < t_len) {
+        const uint8_t* kp = p.kc + static_cast<int64_t>(slot[b]) * p.ck_s + kvh * p.ck_h;
+#pragma unroll
+        for (int c = 0; c < kD / 16; ++c) kk[c] = __ldg(reinterpret_cast<const uint4*>(kp + c * 16));
+      }
+    };
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) max_len = max(max_len, __shfl_xor_sync(0xffffffffu, max_len, o));
+    if (!CAUSAL && max_len > 0) {
+      uint4 kk[2][kD / 16];  // two keys in flight
+      load_key(0, 0, kk[0]);
+      load_key(0, 1, kk[1]);
+      int okq = 0;
+      if (lane == 0) okq = ptx::mbar_wait(bar_q, 0, abort_flag, status, 20) ? 1 : 0;
+      okq = __shfl_sync(0xffffffffu, okq, 0);
+      if (!okq) max_len = 0;
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b) {
+        sc[b] = b < t_len ? tail_score(kk[b & 1], q_row, r) * p.scale_log2 : -INFINITY;
+        if (b + 2 < kBatch) load_key(0, b + 2, kk[b & 1]);
+      }
+    }
     for (int j = 0; j < n_tiles; ++j) {
       int okw = 0;
       if (lane == 0) okw = ptx::mbar_wait(bar_sfull + 8 * (j & 1), (j >> 1) & 1, abort_flag, status, 17) ? 1 : 0;
@@ -409,6 +480,20 @@ decode_attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       ptx::tc_fence_before();
       ptx::mbar_arrive(bar_pfull + 8 * (j & 1));
     }
+    // V rows of a batch, 32 dims at a time; the loads of chunk c + 1 are issued before the
+    // arithmetic of chunk c so that their latency is paid once, not once per chunk
+    uint4 vnext[kBatch][2];
+    auto load_v = [&](int t0, int c) {
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b) {
+        if (t0 + b < t_len) {
+          const uint8_t* vp = p.vc + static_cast<int64_t>(slot[b]) * p.cv_s + kvh * p.cv_h + c * 32;
+          vnext[b][0] = __ldg(reinterpret_cast<const uint4*>(vp));
+          vnext[b][1] = __ldg(reinterpret_cast<const uint4*>(vp + 16));
+        }
+      }
+    };
+    if (!CAUSAL && max_len > 0) load_v(0, 0);
     if (ok && n_tiles > 0) {
       int okw = 0;
       if (lane == 0) okw = ptx::mbar_wait(bar_done, 0, abort_flag, status, 19) ? 1 : 0;
@@ -417,135 +502,8 @@ decode_attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       ptx::tc_fence_after();
     }
     if (ok) {
-      // ---- per-row tail: slots after the shared prefix ------------------------
-      const int t_beg = CAUSAL ? 0 : p.indptr[row] + ls;
-      const int t_len = (!CAUSAL && live) ? max(p.indptr[row + 1] - t_beg, 0) : 0;
-      int max_len = t_len;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) max_len = max(max_len, __shfl_xor_sync(0xffffffffu, max_len, o));
       bool o_valid = n_tiles > 0;
-      if (max_len > 0) {  // warp-uniform; Q tile in shared memory (row r, 128-byte swizzle)
-        int okq = 0;
-        if (lane == 0) okq = ptx::mbar_wait(bar_q, 0, abort_flag, status, 20) ? 1 : 0;
-        okq = __shfl_sync(0xffffffffu, okq, 0);
-        if (!okq) max_len = 0;
-      }
-      const uint8_t* q_row = smem + r * 128;  // + k-block * 16 KB + (chunk ^ (r & 7)) * 16
-      constexpr int kBatch = 4;
-      for (int t0 = 0; t0 < max_len; t0 += kBatch) {
-        float sc[kBatch];
-        int64_t slot[kBatch];
-#pragma unroll
-        for (int b = 0; b < kBatch; ++b) {
-          sc[b] = -INFINITY;
-          slot[b] = 0;
-          if (t0 + b < t_len) {
-            int64_t s = p.indices[t_beg + t0 + b];
-            s = s < 0 ? 0 : (s >= p.num_slots ? p.num_slots - 1 : s);
-            slot[b] = s;
-          }
-        }
-#pragma unroll
-        for (int b = 0; b < kBatch; ++b) {
-          if (t0 + b < t_len) {
-            const uint8_t* kp = p.kc + slot[b] * p.ck_s + kvh * p.ck_h;
-            uint4 kk[kD / 16];
-#pragma unroll
-            for (int c = 0; c < kD / 16; ++c) kk[c] = __ldg(reinterpret_cast<const uint4*>(kp + c * 16));  // all in flight
-            float dot = 0.f;
-#pragma unroll
-            for (int c = 0; c < kD / 16; ++c) {
-              const uint8_t* qb = q_row + (c >> 2) * (kSmemQ / 2);
-              const int ch = (c & 3) * 2;
-              const uint4 q0 = *reinterpret_cast<const uint4*>(qb + (((ch) ^ (r & 7)) << 4));
-              const uint4 q1 = *reinterpret_cast<const uint4*>(qb + (((ch + 1) ^ (r & 7)) << 4));
-              const uint32_t kw[4] = {kk[c].x, kk[c].y, kk[c].z, kk[c].w};
-              const uint32_t qw[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                const float2 ka = e4m3x2_to_float2(static_cast<uint16_t>(kw[i] & 0xffffu));
-                const float2 kb2 = e4m3x2_to_float2(static_cast<uint16_t>(kw[i] >> 16));
-                dot += bf16lo(qw[2 * i]) * ka.x + bf16hi(qw[2 * i]) * ka.y + bf16lo(qw[2 * i + 1]) * kb2.x +
-                       bf16hi(qw[2 * i + 1]) * kb2.y;
-              }
-            }
-            sc[b] = dot * p.scale_log2;
-          }
-        }
-        float bmax = sc[0];
-#pragma unroll
-        for (int b = 1; b < kBatch; ++b) bmax = fmaxf(bmax, sc[b]);
-        const float m_new = fmaxf(m_used, bmax);
-        const float c_old = (m_new == -INFINITY) ? 1.0f : exp2f(m_used - m_new);
-        float pr[kBatch];
-#pragma unroll
-        for (int b = 0; b < kBatch; ++b) pr[b] = (sc[b] == -INFINITY) ? 0.f : exp2f(sc[b] - m_new);
-        m_used = m_new;
-        l_sum = l_sum * c_old;
-#pragma unroll
-        for (int b = 0; b < kBatch; ++b) l_sum += pr[b];
-        // V rows of the batch, 32 dims at a time; the loads of chunk c + 1 are issued before the
-        // arithmetic of chunk c so that their latency is paid once, not once per chunk
-        uint4 vnext[kBatch][2];
-        auto load_v = [&](int c) {
-#pragma unroll
-          for (int b = 0; b < kBatch; ++b) {
-            vnext[b][0] = vnext[b][1] = make_uint4(0, 0, 0, 0);
-            if (pr[b] != 0.f) {
-              const uint8_t* vp = p.vc + slot[b] * p.cv_s + kvh * p.cv_h + c * 32;
-              vnext[b][0] = __ldg(reinterpret_cast<const uint4*>(vp));
-              vnext[b][1] = __ldg(reinterpret_cast<const uint4*>(vp + 16));
-            }
-          }
-        };
-        load_v(0);
-#pragma unroll 1
-        for (int c = 0; c < kD / 32; ++c) {
-          uint4 vv[kBatch][2];
-#pragma unroll
-          for (int b = 0; b < kBatch; ++b) {
-            vv[b][0] = vnext[b][0];
-            vv[b][1] = vnext[b][1];
-          }
-          if (c + 1 < kD / 32) load_v(c + 1);
-          uint32_t o[32];
-          if (o_valid) {
-            ptx::tmem_ld_32x32(t_lane + kColO + c * 32, o);
-            ptx::tmem_ld_wait();
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = 0u;
-          }
-#pragma unroll
-          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * c_old);
-#pragma unroll
-          for (int b = 0; b < kBatch; ++b) {
-            if (pr[b] != 0.f) {
-              const uint32_t vw[8] = {vv[b][0].x, vv[b][0].y, vv[b][0].z, vv[b][0].w,
-                                      vv[b][1].x, vv[b][1].y, vv[b][1].z, vv[b][1].w};
-#pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                const float2 va = e4m3x2_to_float2(static_cast<uint16_t>(vw[i] & 0xffffu));
-                const float2 vb = e4m3x2_to_float2(static_cast<uint16_t>(vw[i] >> 16));
-                o[4 * i + 0] = __float_as_uint(__uint_as_float(o[4 * i + 0]) + pr[b] * va.x);
-                o[4 * i + 1] = __float_as_uint(__uint_as_float(o[4 * i + 1]) + pr[b] * va.y);
-                o[4 * i + 2] = __float_as_uint(__uint_as_float(o[4 * i + 2]) + pr[b] * vb.x);
-                o[4 * i + 3] = __float_as_uint(__uint_as_float(o[4 * i + 3]) + pr[b] * vb.y);
-              }
-            }
-          }
-          ptx::tmem_st_32x32(t_lane + kColO + c * 32, o);
-        }
-        ptx::tmem_st_wait();
-        o_valid = true;
-      }
-      // ---- normalise and store ----------------------------------------------------
-      const float inv = l_sum > 0.f ? 1.0f / l_sum : 0.f;
-      __nv_bfloat16* op = p.out + row * p.o_t + head * kD;
-      const bool wide_out = (reinterpret_cast<uintptr_t>(p.out) & 31u) == 0 && (p.o_t & 15) == 0;  // CTA-uniform
-#pragma unroll 1
-      for (int c = 0; c < kD / 32; ++c) {
-        uint32_t o[32];
+      auto load_o = [&](int c, uint32_t (&o)[32]) {
         if (o_valid) {
           ptx::tmem_ld_32x32(t_lane + kColO + c * 32, o);
           ptx::tmem_ld_wait();
@@ -553,6 +511,11 @@ decode_attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
 #pragma unroll
           for (int i = 0; i < 32; ++i) o[i] = 0u;
         }
+      };
+      __nv_bfloat16* op = p.out + row * p.o_t + head * kD;
+      const bool wide_out = (reinterpret_cast<uintptr_t>(p.out) & 31u) == 0 && (p.o_t & 15) == 0;  // CTA-uniform
+      float inv = 0.f;
+      auto store_o = [&](int c, const uint32_t (&o)[32]) {  // normalised
         if (live) {
           uint32_t w[16];
 #pragma unroll
@@ -570,6 +533,86 @@ decode_attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
             for (int i = 0; i < 4; ++i) d4[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
           }
         }
+      };
+      if (CAUSAL || max_len <= 0) {
+        inv = l_sum > 0.f ? 1.0f / l_sum : 0.f;
+#pragma unroll 1
+        for (int c = 0; c < kD / 32; ++c) {
+          uint32_t o[32];
+          load_o(c, o);
+          store_o(c, o);
+        }
+      }
+      // ---- per-row tail: slots after the shared prefix; the last batch's pass over O also stores it ----
+      for (int t0 = 0; !CAUSAL && t0 < max_len; t0 += kBatch) {
+        const bool last = t0 + kBatch >= max_len;
+        if (t0 > 0) {
+          load_slots(t0);
+          uint4 kk[kD / 16];
+#pragma unroll
+          for (int b = 0; b < kBatch; ++b) {
+            load_key(t0, b, kk);
+            sc[b] = t0 + b < t_len ? tail_score(kk, q_row, r) * p.scale_log2 : -INFINITY;
+          }
+          load_v(t0, 0);
+        }
+        float bmax = sc[0];
+#pragma unroll
+        for (int b = 1; b < kBatch; ++b) bmax = fmaxf(bmax, sc[b]);
+        const float m_new = fmaxf(m_used, bmax);
+        const float c_old = (m_new == -INFINITY) ? 1.0f : exp2f(m_used - m_new);
+        float pr[kBatch];
+#pragma unroll
+        for (int b = 0; b < kBatch; ++b) pr[b] = (sc[b] == -INFINITY) ? 0.f : exp2f(sc[b] - m_new);
+        m_used = m_new;
+        l_sum = l_sum * c_old;
+#pragma unroll
+        for (int b = 0; b < kBatch; ++b) l_sum += pr[b];
+        if (last) inv = l_sum > 0.f ? 1.0f / l_sum : 0.f;
+#pragma unroll 1
+        for (int c = 0; c < kD / 32; ++c) {
+          uint4 vv[kBatch][2];
+#pragma unroll
+          for (int b = 0; b < kBatch; ++b) {
+            vv[b][0] = vnext[b][0];
+            vv[b][1] = vnext[b][1];
+          }
+          if (c + 1 < kD / 32) load_v(t0, c + 1);
+          uint32_t o[32];
+          load_o(c, o);
+          uint64_t acc[16];
+          const uint64_t c_old2 = pack_f32x2(c_old, c_old);
+#pragma unroll
+          for (int i = 0; i < 16; ++i) acc[i] = mul_f32x2(pack_f32x2(__uint_as_float(o[2 * i]), __uint_as_float(o[2 * i + 1])), c_old2);
+#pragma unroll
+          for (int b = 0; b < kBatch; ++b) {
+            if (pr[b] != 0.f) {
+              const uint32_t vw[8] = {vv[b][0].x, vv[b][0].y, vv[b][0].z, vv[b][0].w,
+                                      vv[b][1].x, vv[b][1].y, vv[b][1].z, vv[b][1].w};
+              const uint64_t pr2 = pack_f32x2(pr[b], pr[b]);
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const float2 va = e4m3x2_to_float2(static_cast<uint16_t>(vw[i] & 0xffffu));
+                const float2 vb = e4m3x2_to_float2(static_cast<uint16_t>(vw[i] >> 16));
+                acc[2 * i] = fma_f32x2(pr2, pack_f32x2(va.x, va.y), acc[2 * i]);
+                acc[2 * i + 1] = fma_f32x2(pr2, pack_f32x2(vb.x, vb.y), acc[2 * i + 1]);
+              }
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            float lo, hi;
+            unpack_f32x2(acc[i], lo, hi);
+            o[2 * i] = __float_as_uint(lo);
+            o[2 * i + 1] = __float_as_uint(hi);
+          }
+          if (last)
+            store_o(c, o);
+          else
+            ptx::tmem_st_32x32(t_lane + kColO + c * 32, o);
+        }
+        if (!last) ptx::tmem_st_wait();
+        o_valid = true;
       }
     }
   }
