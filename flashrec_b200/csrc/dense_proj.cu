@@ -284,8 +284,8 @@ dense_rows_gated_kernel(const __grid_constant__ Parts pt, float* __restrict__ x,
 // (loads from shared memory and FMAs share the issue slots). Operands arrive by cp.async two steps of 16 ahead and stay as they lie in memory, rows of k, so that one fma.rn.f32x2
 // takes two consecutive k of an output without any rearranging (an output is the sum of its even and its odd chain).
 // us for 64 / 351 rows of 2048: 20480 columns 286 / 1153 before (64 x 64 tiles through transposed copies, one step ahead), 220 /
-// 863 now (34 TFLOP/s); 2048 columns 133 / 226 and 92 / 155. The gated update's 192 tiles of K = 8192 stay a chain per SM:
-// 679 and 659.
+// 863 now (34 TFLOP/s); 2048 columns 133 / 226 and 92 / 155. (128 x 128 tiles of 8 x 8 outputs per thread, half the loads from shared
+// memory per FMA but one CTA per SM: 1131 for 351 rows x 20480.)
 // ---------------------------------------------------------------------------
 constexpr int kSimtK = 16, kSimtStages = 3;
 constexpr int kSimtPitch = kSimtK + 4;  // floats: eight consecutive rows of 16 bytes meet in no bank
@@ -428,6 +428,34 @@ dense_simt_gated_kernel(const __grid_constant__ Parts pt, float* __restrict__ x,
       } else if (copy != nullptr && row < M && col < (N + 7) / 8 * 8 && col < ldc) {
         copy[row * ldc + col] = 0.f;
       }
+    }
+}
+
+// One share of K per blockIdx.z, times the part's gate, into its partial [M, N]: the tiles of an update alone leave SMs with one or
+// two CTAs of three, each with a chain of thousands of K steps (us: 351 rows x 2048 x 8192 669 -> 371, 128 rows 441 -> 141, 1000
+// rows 1241 -> 899; 128 x 4096 x 12288 638 -> 363). Shorter sums are also closer ones: the error against 64 bits goes from 9e-7 of
+// the norm to 3 to 6e-7.
+__global__ void __launch_bounds__(256, 3)
+dense_simt_partial_kernel(const __grid_constant__ Parts pt, int splits0, int splits1, float* __restrict__ partials, int M, int N) {
+  using S = Simt<64>;
+  __shared__ __align__(16) S sm;
+  const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64, slot = blockIdx.z;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const bool second = slot >= splits0;
+  const fr_gated_part& part = pt.p[second ? 1 : 0];
+  const int i = second ? slot - splits0 : slot, n = second ? splits1 : splits0, steps = (part.K + kSimtK - 1) / kSimtK;
+  const int k0 = static_cast<int>(static_cast<int64_t>(steps) * i / n) * kSimtK;
+  const int k1 = min(static_cast<int>(static_cast<int64_t>(steps) * (i + 1) / n) * kSimtK, part.K);
+  float acc[S::RM][S::CN];
+  sm.tile(static_cast<const float*>(part.a) + k0, part.lda, static_cast<const float*>(part.w) + k0, part.ldw, M, N, k1 - k0, m0, n0, acc);
+  const float* g = static_cast<const float*>(part.gate);
+#pragma unroll
+  for (int r = 0; r < S::RM; ++r)
+#pragma unroll
+    for (int c = 0; c < S::CN; ++c) {
+      const int row = m0 + S::row_of(ty, r), col = n0 + S::col_of(tx, c);
+      if (row < M && col < N)
+        partials[(static_cast<int64_t>(slot) * M + row) * N + col] = (g != nullptr ? g[row * part.ldg + col] : 1.0f) * acc[r][c];
     }
 }
 
@@ -1105,6 +1133,19 @@ static void plan_splits(int M, int N, int kb0, int kb1, int* s0, int* s1) {
   *s1 = b;
 }
 
+// The same for f32, more than 8 rows: three rounds of CTAs, three of them per SM, with shares of at least 512 columns. Up to 1024
+// rows, where the partials that the next launch reads are small beside the product.
+static void plan_simt_splits(int M, int N, int K0, int K1, int* s0, int* s1) {
+  *s0 = *s1 = 0;
+  const int64_t tiles = static_cast<int64_t>(ceil_div(M, 64)) * ceil_div(N, 64), slots = 3 * device_sm_count(), K = static_cast<int64_t>(K0) + K1;
+  if (M <= 8 || M > 1024 || tiles >= 2 * slots) return;
+  const int64_t want = std::min((3 * slots + tiles - 1) / tiles, K / 512);
+  if (want < 2) return;
+  const int64_t share = (K / want + kSimtK - 1) / kSimtK * kSimtK;
+  *s0 = static_cast<int>((K0 + share - 1) / share);
+  *s1 = static_cast<int>((K1 + share - 1) / share);
+}
+
 }  // namespace dense
 
 // shared with attn_mix.cu
@@ -1199,12 +1240,16 @@ extern "C" int fr_dense_proj_split(int dtype, const void* a, int64_t lda, const 
 }
 
 extern "C" int fr_dense_gated_add_splits(int dtype, int M, int N, int K0, int K1) {
-  return M <= 8 ? 0 : fr_dense_few_row_splits(dtype, M, N, K0, K1);
+  return M <= 8 || dtype != 0 ? 0 : fr_dense_few_row_splits(dtype, M, N, K0, K1);
 }
 
 extern "C" int fr_dense_few_row_splits(int dtype, int M, int N, int K0, int K1) {
-  if (dtype != 0 || M <= 0 || N <= 0 || K0 <= 0 || dense::use_rows(dtype, M, N, static_cast<int64_t>(K0) + (K1 > 0 ? K1 : 0), true)) return 0;
   int a, b;
+  if (dtype == 1 && M > 0 && N > 0 && K0 > 0) {
+    dense::plan_simt_splits(M, N, K0, K1 > 0 ? K1 : 0, &a, &b);
+    return a + b;
+  }
+  if (dtype != 0 || M <= 0 || N <= 0 || K0 <= 0 || dense::use_rows(dtype, M, N, static_cast<int64_t>(K0) + (K1 > 0 ? K1 : 0), true)) return 0;
   dense::plan_splits(M, N, ceil_div(K0, dense::kBlockK), K1 > 0 ? ceil_div(K1, dense::kBlockK) : 0, &a, &b);
   return a + b;
 }
@@ -1230,8 +1275,14 @@ extern "C" int fr_dense_gated_add(int dtype, const fr_gated_part* parts, int n_p
     return dtype == 0 ? dense::launch_rows_gated<__nv_bfloat16>(pt, x, ldx, M, N, copy, ldc, stream)
                       : dense::launch_rows_gated<float>(pt, x, ldx, M, N, copy, ldc, stream);
   }
+  if (dtype == 1 && n_splits > 0) {
+    int s0, s1;
+    dense::plan_simt_splits(M, N, parts[0].K, n_parts > 1 ? parts[1].K : 0, &s0, &s1);
+    FR_CHECK_SUPPORTED(s0 > 0 && s0 + s1 == n_splits && (n_parts == 1 || s1 > 0));
+    dense::dense_simt_partial_kernel<<<dim3(ceil_div(N, 64), ceil_div(M, 64), n_splits), 256, 0, stream>>>(pt, s0, s1, partials, M, N);
+    return launch_status();
+  }
   if (dtype == 1) {
-    FR_CHECK_SUPPORTED(n_splits == 0);
     dense::dense_simt_gated_kernel<<<dim3(ceil_div(N, 64), ceil_div(M, 64)), 256, 0, stream>>>(
         pt, x, ldx, M, N, static_cast<float*>(copy), ldc);
     return launch_status();

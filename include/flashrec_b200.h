@@ -572,7 +572,8 @@ struct fr_gated_part {
 int fr_dense_gated_add(int dtype, const struct fr_gated_part* parts, int n_parts, float* x, int64_t ldx, int M, int N,
                        float* partials, int n_splits, void* copy, int64_t ldc, int algo, cudaStream_t stream);
 int fr_dense_gated_add_splits(int dtype, int M, int N, int K0, int K1);
-/* The same, but also for up to 8 rows where the split product is the faster one (fr_dense_gated_add_splits says 0 there). */
+/* The same, but also for up to 8 rows where the split product is the faster one, and for f32 of 9 to 1024 rows
+ * (fr_dense_gated_add_splits says 0 there). */
 int fr_dense_few_row_splits(int dtype, int M, int N, int K0, int K1);
 
 /* x[t, :] = table[ids[t], :] * scale, and the slot table entry of the token: req_to_token[rows[t], pos[t]] = loc[t]

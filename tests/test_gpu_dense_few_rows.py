@@ -141,3 +141,20 @@ def test_f32_tiles_of_128_rows(m, k):
     for got, want in zip(outs, (a.double() @ w.double().T, torch.nn.functional.silu(a.double() @ gate.double().T) * (a.double() @ up.double().T))):
         # k roundings of 2^-24 of a sum of about 1 in random order, and a few more of the activation's
         assert float((got.double() - want).norm() / want.norm()) < (k ** 0.5 + 8) * 2 ** -24
+
+
+@pytest.mark.parametrize("m", [9, 64, 65, 300, 1024, 1025])
+@pytest.mark.parametrize("n,ks", [(1060, (520, 1544)), (2048, (2048, 6144)), (4096, (4096,)), (68, (1032,))])
+def test_f32_updates_in_shares(m, n, ks):
+    """K split over CTAs, up to 1024 rows, with rows, columns and steps of K left over."""
+    from flashrec_b200 import lm_layers as L
+
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    x, parts = r(m, n), [(r(m, k), r(n, k) * k ** -0.5, r(m, n)) for k in ks]
+    want = x.double() + sum(gt.double() * (a.double() @ w.double().T) for a, w, gt in parts)
+    p = L.gated_add(x, parts, few_rows=True)
+    assert (p is None) == (m > 1024 or -(-m // 64) * -(-n // 64) >= 888)
+    got = x.double() + (p.buf.double().sum(0) if p is not None else 0)
+    # k roundings of 2^-24 of sums of about 1 in random order, the gate's and the stream's
+    assert float((got - want).norm() / want.norm()) < (max(ks) ** 0.5 + 4) * 2 ** -24
