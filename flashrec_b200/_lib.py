@@ -221,6 +221,7 @@ _SIGNATURES = {
     "fr_linear_scan_chunks_fit": [P],
     "fr_short_conv": [_I, P, _L, P, P, _I, _I, _I, P, _I, P, P, P, P, P, _I, _I, _I, P],
     "fr_mix_attn_rows": [P, _I, _I, _I, _I, P, _L, P, P],
+    "fr_mix_attn_rows_early": [P, _I, _I, _I, _I, P, _L, P, P],
     "fr_mix_attn_rows_scratch": [_I] * 6,
     "fr_mix_attn_tc": [P, P, _I, _I, _I, P, _L, P],
     "fr_mix_attn_tc_scratch": [P, _I, _I, _L],

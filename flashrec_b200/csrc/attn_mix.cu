@@ -20,7 +20,7 @@ int64_t talk_tc_tile_bytes(const fr_mix_attn& a, int max_pos);
 namespace mix {
 
 bool fused_rows_fit(const fr_mix_attn& a, int max_keys);  // attn_rows.cu
-int fused_rows(const fr_mix_attn& a, int row0, int n_rows, int max_keys, cudaStream_t stream);
+int fused_rows(const fr_mix_attn& a, int row0, int n_rows, int max_keys, bool early, cudaStream_t stream);
 
 constexpr int kKeyBlock = 64;
 constexpr int kMaxPer = 4;  // key blocks per CTA of the scores kernel when the batch fills the GPU anyway
@@ -871,8 +871,8 @@ extern "C" int64_t fr_mix_attn_rows_scratch(int mix_kind, int heads, int vdim, i
   return stats + src * max_keys * 4 + part;
 }
 
-extern "C" int fr_mix_attn_rows(const fr_mix_attn* a, int row0, int n_rows, int max_keys, int splits, void* scratch,
-                                int64_t scratch_bytes, int32_t* counters, cudaStream_t stream) {
+static int mix_attn_rows(const fr_mix_attn* a, int row0, int n_rows, int max_keys, int splits, void* scratch,
+                         int64_t scratch_bytes, int32_t* counters, bool early, cudaStream_t stream) {
   const int st = mix::check_args(a);
   if (st != FR_OK) return st;
   FR_CHECK_ARG(row0 >= 0 && n_rows >= 0 && max_keys > 0 && splits > 0);
@@ -880,13 +880,23 @@ extern "C" int fr_mix_attn_rows(const fr_mix_attn* a, int row0, int n_rows, int 
   FR_CHECK_ARG(scratch && aligned16(scratch) && (splits == 1 || counters));
   FR_CHECK_ARG(scratch_bytes >= fr_mix_attn_rows_scratch(a->mix, a->heads, a->vdim, n_rows, max_keys, splits));
   FR_CHECK_SUPPORTED(a->vdim <= 1024 && n_rows <= 65535);
-  if (mix::fused_rows_fit(*a, max_keys)) return mix::fused_rows(*a, row0, n_rows, max_keys, stream);
+  if (mix::fused_rows_fit(*a, max_keys)) return mix::fused_rows(*a, row0, n_rows, max_keys, early, stream);
   const int64_t src = static_cast<int64_t>(n_rows) * (a->mix == FR_MIX_DIFF ? 2 * a->heads : a->heads);
   float2* stats = static_cast<float2*>(scratch);
   float* scores = reinterpret_cast<float*>(stats + src * ceil_div(max_keys, mix::kKeyBlock));
   float* partial = scores + src * max_keys;
   return a->dtype == 0 ? mix::launch_rows<__nv_bfloat16>(*a, row0, n_rows, max_keys, splits, scores, stats, partial, counters, stream)
                        : mix::launch_rows<float>(*a, row0, n_rows, max_keys, splits, scores, stats, partial, counters, stream);
+}
+
+extern "C" int fr_mix_attn_rows(const fr_mix_attn* a, int row0, int n_rows, int max_keys, int splits, void* scratch,
+                                int64_t scratch_bytes, int32_t* counters, cudaStream_t stream) {
+  return mix_attn_rows(a, row0, n_rows, max_keys, splits, scratch, scratch_bytes, counters, false, stream);
+}
+
+extern "C" int fr_mix_attn_rows_early(const fr_mix_attn* a, int row0, int n_rows, int max_keys, int splits, void* scratch,
+                                      int64_t scratch_bytes, int32_t* counters, cudaStream_t stream) {
+  return mix_attn_rows(a, row0, n_rows, max_keys, splits, scratch, scratch_bytes, counters, true, stream);
 }
 
 extern "C" int fr_mix_attn_tc_fits(int mix_kind, int heads, int kv_heads, int dim, int vdim) {

@@ -147,6 +147,33 @@ __device__ __forceinline__ void prefetch_value(const fr_mix_attn& a, int g, int 
   const __nv_bfloat16* p = static_cast<const __nv_bfloat16*>(a.v) + static_cast<int64_t>(slot) * a.ldv + static_cast<int64_t>(g) * a.vdim;
   for (int c = 0; c < a.vdim; c += 64) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + c));
 }
+// and the key row, of the `maps` maps of the kv head
+__device__ __forceinline__ void prefetch_key(const fr_mix_attn& a, int maps, int g, int slot) {
+  const __nv_bfloat16* p = static_cast<const __nv_bfloat16*>(a.k) + static_cast<int64_t>(slot) * a.ldk + static_cast<int64_t>(maps * g) * a.dim;
+  for (int c = 0; c < maps * a.dim; c += 64) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + c));
+}
+
+// A row's place and what it sees. Read through L2: with `early` (fr_mix_attn_rows_early) this happens before the launch waits for
+// the one that precedes it, and the keys and values of a warp's first blocks are on their way into L2 by then. In steps
+// of the 1.7b sizes: one request of 800 keys, DIFF 16.1 -> 15.0 and TALK 18.9 -> 16.6 us behind the projections; 64 requests of 150 keys 26.1
+// -> 23.0 and 25.6 -> 20.0 (TALK also has eight CTAs' weights in flight where it mixes them). Running through the instructions once
+// before the wait, to have them in the caches, cost what it took (15.0 -> 25.5 us): the launch ahead is nearly over when this begins.
+struct Place {
+  const int32_t* table;     // slots of the request's positions
+  int i, lo, n_first, n;    // own position; the first n_first visible keys lie at 0, the others from lo on
+  __device__ __forceinline__ int key(int x) const { return x < n_first ? x : lo + (x - n_first); }
+};
+__device__ __forceinline__ Place place_of(const fr_mix_attn& a, int64_t t, int max_keys) {
+  const int64_t i = __ldcg(a.pos + t);
+  const Visible v = visible_keys(a, i, max_keys);
+  return Place{a.req_to_token + __ldcg(a.req_rows + __ldcg(a.tok_req + t)) * a.table_stride, static_cast<int>(i), static_cast<int>(v.lo),
+               v.n_first, v.n};
+}
+__device__ __forceinline__ int slot_at(const fr_mix_attn& a, const Place& p, int x) {
+  const int s = __ldcg(p.table + p.key(x));
+  return s < 0 ? 0 : (s >= a.num_slots ? static_cast<int>(a.num_slots - 1) : s);
+}
+constexpr int kEarlyBlocks = 2;  // blocks of 32 keys per warp that are brought into L2 before the wait
 
 __device__ __forceinline__ float ld_cluster(uint32_t addr) {
   float v;
@@ -162,7 +189,7 @@ constexpr int kFlashWarps = 4;
 
 template <int REP, int MAPS, int NCH, int VL>
 __global__ void __launch_bounds__(kFlashWarps * 32, REP * MAPS >= 8 ? 2 : (MAPS * NCH > 4 || REP == 4 ? 3 : 4))
-flash_rows_kernel(const __grid_constant__ fr_mix_attn a, int row0, int max_keys, int splits) {
+flash_rows_kernel(const __grid_constant__ fr_mix_attn a, int row0, int max_keys, int splits, int early) {
   constexpr int NS = REP * MAPS, VP = VL * 8;
   __shared__ __align__(16) float sc[kFlashWarps][32 * NS];
   __shared__ float o_w[kFlashWarps][NS * VP];  // per warp; afterwards the CTA's sum in the first
@@ -171,14 +198,31 @@ flash_rows_kernel(const __grid_constant__ fr_mix_attn a, int row0, int max_keys,
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
   const int split = blockIdx.x, g = blockIdx.y;
   const int rep = a.heads / a.kv_heads;
+  const int64_t t = row0 + static_cast<int64_t>(blockIdx.z);
+  Place at;
+  int k_lo, k_hi, k0, next;
+  auto slot = [&](int base) {  // behind the last key: the last one's, loaded and not used
+    return slot_at(a, at, min(base + lane, k_hi - 1));
+  };
+  auto begin = [&] {
+    at = place_of(a, t, max_keys);
+    const int per = ((at.n + splits - 1) / splits + 31) / 32 * 32;  // whole blocks per share
+    k_lo = min(split * per, at.n);
+    k_hi = min(k_lo + per, at.n);
+    k0 = k_lo + warp * 32;
+    next = k0 < k_hi ? slot(k0) : 0;
+  };
+  if (early) {
+    begin();
+    for (int b = 0, k = k0; b < kEarlyBlocks && k < k_hi; ++b, k += kFlashWarps * 32) {
+      const int x = b == 0 ? next : slot(k);
+      prefetch_key(a, MAPS, g, x);
+      prefetch_value(a, g, x);
+    }
+  }
   ptx::griddep_wait();
   ptx::griddep_launch_dependents();
-  const int64_t t = row0 + static_cast<int64_t>(blockIdx.z);
-  const int64_t i = a.pos[t];
-  const int64_t table_row = a.req_rows[a.tok_req[t]];
-  const Visible vis = visible_keys(a, i, max_keys);
-  const int per = ((vis.n + splits - 1) / splits + 31) / 32 * 32;  // whole blocks per share
-  const int k_lo = min(split * per, vis.n), k_hi = min(k_lo + per, vis.n);
+  if (!early) begin();
   Scores<REP, MAPS, NCH> scores;
   scores.load_queries(a, t, g);
   float m[NS], l[NS], acc[NS][8] = {};
@@ -188,19 +232,16 @@ flash_rows_kernel(const __grid_constant__ fr_mix_attn a, int row0, int max_keys,
     l[s] = 0.f;
   }
   float* my = sc[warp];
-  auto slot_at = [&](int base) {  // behind the last key: the last one's, loaded and not used
-    return static_cast<int>(slot_of(a, table_row, vis.key(min(base + lane, k_hi - 1))));
-  };
-  int k0 = k_lo + warp * 32;
-  int next = k0 < k_hi ? slot_at(k0) : 0;
   for (; k0 < k_hi; k0 += kFlashWarps * 32) {
-    const int slot = next, nk = min(32, k_hi - k0);
-    if (k0 + kFlashWarps * 32 < k_hi) next = slot_at(k0 + kFlashWarps * 32);
-    prefetch_value(a, g, slot);
+    const int here = next, nk = min(32, k_hi - k0);
+    const bool more = k0 + kFlashWarps * 32 < k_hi;
+    if (more) next = slot(k0 + kFlashWarps * 32);
+    prefetch_value(a, g, here);
     __syncwarp();
-    scores(a, g, slot, my);
+    scores(a, g, here, my);
     __syncwarp();
-    const float dist = static_cast<float>(i - vis.key(k0 + min(lane, nk - 1)));
+    if (more) prefetch_key(a, MAPS, g, next);
+    const float dist = static_cast<float>(at.i - at.key(k0 + min(lane, nk - 1)));
     float p[NS], fade[NS];
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
@@ -219,7 +260,7 @@ flash_rows_kernel(const __grid_constant__ fr_mix_attn a, int row0, int max_keys,
 #pragma unroll
     for (int s = 0; s < NS; ++s) my[lane * NS + s] = p[s];
     __syncwarp();
-    add_values<NS, VL>(a, g, slot, nk, my, blk);
+    add_values<NS, VL>(a, g, here, nk, my, blk);
 #pragma unroll
     for (int s = 0; s < NS; ++s)
 #pragma unroll
@@ -335,7 +376,7 @@ static int talk_smem(int rep_p, int heads, int max_keys, int warps, int vp) {
 
 template <int REP, int NCH, int VL, int W>
 __global__ void __launch_bounds__(W * 32, W == 4 ? 4 : 1)
-talk_rows_kernel(const __grid_constant__ fr_mix_attn a, int row0, int max_keys) {
+talk_rows_kernel(const __grid_constant__ fr_mix_attn a, int row0, int max_keys, int early) {
   constexpr int VP = VL * 8;
   extern __shared__ __align__(16) float smem[];
   __shared__ __align__(16) float sc[W][32 * REP];
@@ -348,17 +389,28 @@ talk_rows_kernel(const __grid_constant__ fr_mix_attn a, int row0, int max_keys) 
   float* o_w = cf + a.heads * REP;               // [W][REP][VP]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
   const int g = blockIdx.x;
-  ptx::griddep_wait();
-  ptx::griddep_launch_dependents();
   const int64_t t = row0 + static_cast<int64_t>(blockIdx.y);
-  const int64_t i = a.pos[t];
-  const int64_t table_row = a.req_rows[a.tok_req[t]];
-  const Visible vis = visible_keys(a, i, max_keys);
-  const int n = vis.n;
+  Place at;
+  auto begin = [&] {
+    at = place_of(a, t, max_keys);
+    for (int k0 = warp * 32, b = 0; k0 < at.n; k0 += W * 32, ++b) {
+      const int x = slot_at(a, at, min(k0 + lane, at.n - 1));
+      slots[k0 + lane] = x;
+      if (b < kEarlyBlocks) {
+        if (early) prefetch_key(a, 1, g, x);
+        prefetch_value(a, g, x);
+      }
+    }
+  };
   for (int e = tid; e < a.heads * REP; e += W * 32) {  // coefficient of source s in output o of this kv head
     const int s = e / REP, o = e % REP;
     cf[e] = o < rep ? a.coef[static_cast<int64_t>(g * rep + o) * a.heads + s] : 0.f;
   }
+  if (early) begin();
+  ptx::griddep_wait();
+  ptx::griddep_launch_dependents();
+  if (!early) begin();
+  const int n = at.n;
   Scores<REP, 1, NCH> scores;
   scores.load_queries(a, t, g);
   float mx[REP];
@@ -367,13 +419,10 @@ talk_rows_kernel(const __grid_constant__ fr_mix_attn a, int row0, int max_keys) 
   float* my = sc[warp];
   for (int k0 = warp * 32; k0 < n; k0 += W * 32) {
     const int idx = min(k0 + lane, n - 1);
-    const int slot = static_cast<int>(slot_of(a, table_row, vis.key(idx)));
-    slots[k0 + lane] = slot;
-    prefetch_value(a, g, slot);
     __syncwarp();
-    scores(a, g, slot, my);
+    scores(a, g, slots[k0 + lane], my);
     __syncwarp();
-    const float dist = static_cast<float>(i - vis.key(idx));
+    const float dist = static_cast<float>(at.i - at.key(idx));
 #pragma unroll
     for (int s = 0; s < REP; ++s) {
       float v = my[lane * REP + s] * a.scale;
@@ -422,16 +471,27 @@ talk_rows_kernel(const __grid_constant__ fr_mix_attn a, int row0, int max_keys) 
   __syncthreads();
   for (int k = tid; k < n32; k += W * 32) {
     float w[REP] = {};
-#pragma unroll 2
-    for (int c = 0; c < a.kv_heads; ++c) {
-      const uint32_t base = ptx::mapa(ptx::smem_u32(pw + k), c);
+    constexpr int kAhead = REP <= 2 ? 8 : (REP == 4 ? 4 : 2);  // CTAs whose weights are in flight; at most 16 registers
+    for (int c0 = 0; c0 < a.kv_heads; c0 += kAhead) {
+      float e[kAhead][REP];
 #pragma unroll
-      for (int s = 0; s < REP; ++s) {
-        if (s >= rep) break;
-        const float e = ld_cluster(base + s * cap * 4);
-        const float* f = cf + (c * rep + s) * REP;
+      for (int c = 0; c < kAhead; ++c) {
+        if (c0 + c >= a.kv_heads) break;
+        const uint32_t base = ptx::mapa(ptx::smem_u32(pw + k), c0 + c);
 #pragma unroll
-        for (int o = 0; o < REP; ++o) w[o] = fmaf(f[o], e, w[o]);
+        for (int s = 0; s < REP; ++s)
+          if (s < rep) e[c][s] = ld_cluster(base + s * cap * 4);
+      }
+#pragma unroll
+      for (int c = 0; c < kAhead; ++c) {
+        if (c0 + c >= a.kv_heads) break;
+#pragma unroll
+        for (int s = 0; s < REP; ++s) {
+          if (s >= rep) break;
+          const float* f = cf + ((c0 + c) * rep + s) * REP;
+#pragma unroll
+          for (int o = 0; o < REP; ++o) w[o] = fmaf(f[o], e[c][s], w[o]);
+        }
       }
     }
 #pragma unroll
@@ -469,75 +529,45 @@ talk_rows_kernel(const __grid_constant__ fr_mix_attn a, int row0, int max_keys) 
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // nobody leaves while its weights are read
 }
 
-template <class... KArgs, class... Args>
-static int launch_clusters(void (*kern)(KArgs...), dim3 grid, int threads, int smem, int cluster, bool pdl, cudaStream_t stream,
-                           Args... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = threads;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
-  int n = 0;
-  if (cluster > 1) {
-    attr[n].id = cudaLaunchAttributeClusterDimension;
-    attr[n].val.clusterDim.x = cluster;
-    attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
-    ++n;
-  }
-  if (pdl) {
-    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[n].val.programmaticStreamSerializationAllowed = 1;
-    ++n;
-  }
-  cfg.attrs = attr;
-  cfg.numAttrs = n;
-  if (cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...) != cudaSuccess) {
-    cudaGetLastError();
-    return FR_ERR_CUDA;
-  }
-  return FR_OK;
-}
-
 template <int REP, int MAPS, int NCH, int VL>
-static int launch_flash(const fr_mix_attn& a, int row0, int n_rows, int max_keys, cudaStream_t stream) {
+static int launch_flash(const fr_mix_attn& a, int row0, int n_rows, int max_keys, bool early, cudaStream_t stream) {
   // shares of the keys while two CTAs per SM are not reached and a share keeps its four warps busy
   int splits = 1;
   const int64_t ctas = static_cast<int64_t>(n_rows) * a.kv_heads;
   while (splits < 8 && ctas * splits * 2 <= 2 * device_sm_count() && max_keys > splits * 32 * kFlashWarps) splits *= 2;
-  return launch_clusters(flash_rows_kernel<REP, MAPS, NCH, VL>, dim3(splits, a.kv_heads, n_rows), kFlashWarps * 32, 0, splits,
-                         n_rows <= kPdlRows, stream, a, row0, max_keys, splits);
+  return launch_cluster(flash_rows_kernel<REP, MAPS, NCH, VL>, dim3(splits, a.kv_heads, n_rows), kFlashWarps * 32, 0, stream, splits,
+                        n_rows <= kPdlRows, a, row0, max_keys, splits, early ? 1 : 0);
 }
 
 template <int REP, int NCH, int VL, int W>
-static int launch_talk(const fr_mix_attn& a, int row0, int n_rows, int max_keys, cudaStream_t stream) {
+static int launch_talk(const fr_mix_attn& a, int row0, int n_rows, int max_keys, bool early, cudaStream_t stream) {
   const int smem = talk_smem(REP, a.heads, max_keys, W, VL * 8);
   static PerDeviceFlag f;
   if (ensure_dyn_smem(f, talk_rows_kernel<REP, NCH, VL, W>, kTalkSmem) != FR_OK) return FR_ERR_CUDA;
-  return launch_clusters(talk_rows_kernel<REP, NCH, VL, W>, dim3(a.kv_heads, n_rows), W * 32, smem, a.kv_heads, n_rows <= kPdlRows,
-                         stream, a, row0, max_keys);
+  return launch_cluster(talk_rows_kernel<REP, NCH, VL, W>, dim3(a.kv_heads, n_rows), W * 32, smem, stream, a.kv_heads, n_rows <= kPdlRows,
+                        a, row0, max_keys, early ? 1 : 0);
 }
 
 template <int REP, int NCH, int VL>
-static int launch_sizes(const fr_mix_attn& a, int row0, int n_rows, int max_keys, cudaStream_t stream) {
-  if (a.mix == FR_MIX_PLAIN) return launch_flash<REP, 1, NCH, VL>(a, row0, n_rows, max_keys, stream);
+static int launch_sizes(const fr_mix_attn& a, int row0, int n_rows, int max_keys, bool early, cudaStream_t stream) {
+  if (a.mix == FR_MIX_PLAIN) return launch_flash<REP, 1, NCH, VL>(a, row0, n_rows, max_keys, early, stream);
   if (a.mix == FR_MIX_DIFF) {
-    if constexpr (REP <= 4) return launch_flash<REP, 2, NCH, VL>(a, row0, n_rows, max_keys, stream);
+    if constexpr (REP <= 4) return launch_flash<REP, 2, NCH, VL>(a, row0, n_rows, max_keys, early, stream);
     return FR_ERR_UNSUPPORTED;
   }
   // many rows: small CTAs, so that all of them are resident at once; few: more warps per head
-  if (static_cast<int64_t>(n_rows) * a.kv_heads > device_sm_count()) return launch_talk<REP, NCH, VL, 4>(a, row0, n_rows, max_keys, stream);
-  return launch_talk<REP, NCH, VL, kTalkWarps>(a, row0, n_rows, max_keys, stream);
+  if (static_cast<int64_t>(n_rows) * a.kv_heads > device_sm_count()) return launch_talk<REP, NCH, VL, 4>(a, row0, n_rows, max_keys, early, stream);
+  return launch_talk<REP, NCH, VL, kTalkWarps>(a, row0, n_rows, max_keys, early, stream);
 }
 
 template <int REP>
-static int launch_rep(const fr_mix_attn& a, int row0, int n_rows, int max_keys, cudaStream_t stream) {
+static int launch_rep(const fr_mix_attn& a, int row0, int n_rows, int max_keys, bool early, cudaStream_t stream) {
   if (a.dim <= 64) {
-    if (a.vdim <= 64) return launch_sizes<REP, 2, 8>(a, row0, n_rows, max_keys, stream);
-    return launch_sizes<REP, 2, 16>(a, row0, n_rows, max_keys, stream);
+    if (a.vdim <= 64) return launch_sizes<REP, 2, 8>(a, row0, n_rows, max_keys, early, stream);
+    return launch_sizes<REP, 2, 16>(a, row0, n_rows, max_keys, early, stream);
   }
-  if (a.vdim <= 64) return launch_sizes<REP, 4, 8>(a, row0, n_rows, max_keys, stream);
-  return launch_sizes<REP, 4, 16>(a, row0, n_rows, max_keys, stream);
+  if (a.vdim <= 64) return launch_sizes<REP, 4, 8>(a, row0, n_rows, max_keys, early, stream);
+  return launch_sizes<REP, 4, 16>(a, row0, n_rows, max_keys, early, stream);
 }
 
 // Whether one launch does it: bf16, heads of at most 128, up to 8 heads per kv head (DIFF 4: two maps each), and for TALK
@@ -551,12 +581,12 @@ bool fused_rows_fit(const fr_mix_attn& a, int max_keys) {
          talk_smem(rep_p, a.heads, max_keys, kTalkWarps, a.vdim <= 64 ? 64 : 128) <= kTalkSmem;
 }
 
-int fused_rows(const fr_mix_attn& a, int row0, int n_rows, int max_keys, cudaStream_t stream) {
+int fused_rows(const fr_mix_attn& a, int row0, int n_rows, int max_keys, bool early, cudaStream_t stream) {
   const int rep = a.heads / a.kv_heads;
-  if (rep == 1) return launch_rep<1>(a, row0, n_rows, max_keys, stream);
-  if (rep == 2) return launch_rep<2>(a, row0, n_rows, max_keys, stream);
-  if (rep <= 4) return launch_rep<4>(a, row0, n_rows, max_keys, stream);
-  return launch_rep<8>(a, row0, n_rows, max_keys, stream);
+  if (rep == 1) return launch_rep<1>(a, row0, n_rows, max_keys, early, stream);
+  if (rep == 2) return launch_rep<2>(a, row0, n_rows, max_keys, early, stream);
+  if (rep <= 4) return launch_rep<4>(a, row0, n_rows, max_keys, early, stream);
+  return launch_rep<8>(a, row0, n_rows, max_keys, early, stream);
 }
 
 }  // namespace mix

@@ -79,26 +79,41 @@ static inline int device_sm_count() {
   return cache[d];
 }
 
-// Launch with or without programmatic dependence on the previous kernel of the stream: with it the kernel may start
-// while its predecessor is finishing and must execute griddepcontrol.wait before it touches what others write.
+// Launch, in clusters if `cluster` > 1, with or without programmatic dependence on the previous kernel of the stream: with it
+// the kernel may start while its predecessor is finishing and must execute griddepcontrol.wait before it touches what others write.
 template <class... KArgs, class... Args>
-static inline int launch_kernel(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool pdl,
-                                Args... args) {
+static inline int launch_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster, bool pdl,
+                                 Args... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (cluster > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = cluster;
+    attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  if (pdl) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n].val.programmaticStreamSerializationAllowed = 1;
+    ++n;
+  }
   cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
+  cfg.numAttrs = n;
   if (cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...) != cudaSuccess) {
     cudaGetLastError();
     return FR_ERR_CUDA;
   }
   return FR_OK;
+}
+template <class... KArgs, class... Args>
+static inline int launch_kernel(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool pdl,
+                                Args... args) {
+  return launch_cluster(kern, grid, block, smem, stream, 1, pdl, args...);
 }
 constexpr int kPdlRows = 2048;  // batches up to this many rows launch their kernels with the dependence
 

@@ -194,7 +194,7 @@ class DibepelLayer:
             nq, nk = self.attn.q_cols, self.spec.k_cols
             short_conv(u, self.conv_w, [(q, None, 0, nq), (kc, loc, nq, nk), (vc, loc, nq + nk, self.spec.v_cols)],
                        caches.conv[run], batch)
-        o = self.attn.forward(q, kc, vc, req_to_token, batch, counters, max_keys)
+        o = self.attn.forward(q, kc, vc, req_to_token, batch, counters, max_keys, early=True)
         parts = [(o, self.o_w, g1)]
         if self.layer.ff is not None:
             parts.append((act, self.down_w, g2))

@@ -270,7 +270,7 @@ class ParallelMixer(_Mixer):
         if self.rotary not in c.tables:
             c.tables[self.rotary] = rotary_table(self.inv_freq, b.positions)
         qk_norm_rope(q, k, a.heads, a.kv_heads, a.dim, self.q_norm, self.k_norm, self.cfg.eps, c.tables[self.rotary], b, kc)
-        o = self.attn.forward(q, kc, vc, c.req_to_token, b, c.counters, c.max_keys, gate)
+        o = self.attn.forward(q, kc, vc, c.req_to_token, b, c.counters, c.max_keys, gate, early=True)
         left = self.product(o, self.left_o)
         y = self.scan.forward(rq, rk, rv, low, c.caches.state[c.run], b, self.new(t, g.heads * g.vdim))
         group_norm(y, g.heads, g.vdim, self.head_norm, self.cfg.eps, rv, rg)

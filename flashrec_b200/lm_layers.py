@@ -363,8 +363,9 @@ class MixAttention:
 
     def forward(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, req_to_token: torch.Tensor,
                 batch: ForwardBatch, counters: torch.Tensor, max_keys: Optional[int] = None,
-                head_gate: Optional[torch.Tensor] = None) -> torch.Tensor:
-        """q [T, q_cols]; ``head_gate`` fp32 [T, heads], whose sigmoid multiplies the heads ("plain"); ``k`` / ``v`` the layer's caches (the batch's own keys are in already). bf16 prompts take
+                head_gate: Optional[torch.Tensor] = None, early: bool = False) -> torch.Tensor:
+        """q [T, q_cols]; ``early``: the batch's positions and the slot table were written before the launch that precedes this one
+        (``fr_mix_attn_rows_early``). ``head_gate`` fp32 [T, heads], whose sigmoid multiplies the heads ("plain"); ``k`` / ``v`` the layer's caches (the batch's own keys are in already). bf16 prompts take
         the tensor-core kernel, short portions, decode steps and fp32 the row kernels."""
         require_cuda(q, k, v)
         t = int(q.shape[0])
@@ -383,7 +384,7 @@ class MixAttention:
         n_row = batch.n_row_tokens if tc else t
         if n_row > 0:
             keys = self.cache.max_keys(batch.max_pos) if max_keys is None else max_keys
-            self._rows(a, n_row, keys, counters, s, q.device)
+            self._rows(a, n_row, keys, counters, s, q.device, early)
         if n_row < t:
             n_tiles = int(batch.tiles.shape[0])
             size = _lib.load().fr_mix_attn_tc_scratch(ctypes.byref(a), n_tiles, batch.max_pos, _MAP_SCRATCH_BYTES)
@@ -391,7 +392,7 @@ class MixAttention:
             call("fr_mix_attn_tc", ctypes.byref(a), ptr(batch.tiles), n_tiles, t, batch.max_pos, ptr(scratch), max(size, 0), s)
         return out
 
-    def _rows(self, a: FrMixAttn, n_row: int, keys: int, counters: torch.Tensor, stream, device) -> None:
+    def _rows(self, a: FrMixAttn, n_row: int, keys: int, counters: torch.Tensor, stream, device, early: bool = False) -> None:
         lib = _lib.load()
         blocks = (keys + 63) // 64
         splits = max(1, min(blocks, 16, 444 // max(1, n_row * self.kv_heads)))
@@ -401,7 +402,7 @@ class MixAttention:
         step = max(1, min(n_row, 32768, _SCORE_SCRATCH_BYTES // max(1, size(1))))
         scratch = torch.empty(size(step) + 16, dtype=torch.uint8, device=device)
         for r0 in range(0, n_row, step):
-            call("fr_mix_attn_rows", ctypes.byref(a), r0, min(step, n_row - r0), keys, splits, ptr(scratch),
+            call("fr_mix_attn_rows_early" if early else "fr_mix_attn_rows", ctypes.byref(a), r0, min(step, n_row - r0), keys, splits, ptr(scratch),
                  int(scratch.numel()), ptr(counters), stream)
 
 

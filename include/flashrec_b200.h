@@ -718,6 +718,11 @@ struct fr_mix_attn {
  * fr_mix_attn_rows_scratch(...) bytes, counters n_rows * kv_heads zeroed words (left zeroed). */
 int fr_mix_attn_rows(const struct fr_mix_attn* a, int row0, int n_rows, int max_keys, int splits, void* scratch,
                      int64_t scratch_bytes, int32_t* counters, cudaStream_t stream);
+/* The same for callers whose slot table, positions (pos, tok_req, req_rows) and coefficients were written no later than by the
+ * launch before the one that directly precedes this call in the stream (in a decoder layer: the embedding wrote them, the projections
+ * come between). One-launch rows then read them, and bring keys and values into L2, while the preceding launch still runs. */
+int fr_mix_attn_rows_early(const struct fr_mix_attn* a, int row0, int n_rows, int max_keys, int splits, void* scratch,
+                           int64_t scratch_bytes, int32_t* counters, cudaStream_t stream);
 int64_t fr_mix_attn_rows_scratch(int mix, int heads, int vdim, int n_rows, int max_keys, int splits);
 
 /* bf16 prompts on the tensor cores: tiles [n_tiles, 3] of {request, first row in the batch, rows} (at most 128

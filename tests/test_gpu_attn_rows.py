@@ -134,3 +134,21 @@ def test_rows_of_a_batch_that_is_cut(kind, heads, kv, scratch, monkeypatch):
     got = _run(kind, torch.bfloat16, heads, kv, 64, 64, lens, 300, 0, 9)
     assert [n for n, _ in begins].count("fr_mix_attn_rows") > 1 and max(r for _, r in begins) > 20
     assert ((got - ref).norm(dim=1) < (2 ** -8 + 1e-4) * ref.norm(dim=1)).all()
+
+
+@pytest.mark.parametrize("kind", ["diff", "talk", "plain"])
+@pytest.mark.parametrize("heads,kv,dim,vdim", [(16, 8, 128, 128), (8, 2, 64, 64), (5, 1, 16, 16)])
+@pytest.mark.parametrize("lens", [(1,), (1100,), (15, 16, 17, 18, 31, 33, 129, 257)])
+def test_reads_before_the_launch_ahead_has_ended(kind, heads, kv, dim, vdim, lens, monkeypatch):
+    """The early entry, with everything written long before, gives the same bits."""
+    from flashrec_b200 import lm_layers
+
+    ref = _run(kind, torch.bfloat16, heads, kv, dim, vdim, lens, 200, 0, 11)
+    call = lm_layers.call
+
+    def early(name, *a):
+        torch.cuda.synchronize()
+        call(name + "_early" if name == "fr_mix_attn_rows" else name, *a)
+
+    monkeypatch.setattr(lm_layers, "call", early)
+    assert torch.equal(_run(kind, torch.bfloat16, heads, kv, dim, vdim, lens, 200, 0, 11), ref)
