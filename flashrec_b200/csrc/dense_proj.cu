@@ -499,12 +499,14 @@ enum Epi { kEpiSegs = 0, kEpiAdd = 1, kEpiPartial = 2 };
 // kOctet: at most 8 rows, which the row kernel sums in fp32 FMAs otherwise. The tensor cores' accumulation loses bits with
 // every product added (2.1e-6 of the norm at K = 2048, 1.4e-5 at 12288, where the row kernel has 8e-8 and 9e-8), so here it
 // spans one k-block only: the four blocks of a stage go to four accumulators, which a warp adds up in fp32 registers.
-enum Rows { kAny = 0, kFew = 1, kOctet = 2 };
+// kPair: tiles of 256 rows by two CTAs of a cluster, each with its 128 rows of A and half of the weight rows, one tcgen05.mma for both.
+enum Rows { kAny = 0, kFew = 1, kOctet = 2, kPair = 3 };
 
 template <int BLOCK_N, int ROWS>
 struct Cfg {
-  static constexpr int kStageBytes = (kBlockM + BLOCK_N) * kBlockK * 2;
-  static constexpr int kStages = BLOCK_N == 256 ? 4 : (BLOCK_N == 128 ? 6 : 8);
+  static constexpr int kTileM = ROWS == kPair ? 2 * kBlockM : kBlockM, kTileB = ROWS == kPair ? BLOCK_N / 2 : BLOCK_N;  // kTileB: a CTA's
+  static constexpr int kStageBytes = (kBlockM + kTileB) * kBlockK * 2;
+  static constexpr int kStages = kTileB == 256 ? 4 : (kTileB == 128 ? 6 : 8);
   static constexpr int kAcc = ROWS == kOctet ? 8 : 2;  // accumulators in TMEM
   static constexpr int kTmemCols = kAcc * BLOCK_N <= 128 ? 128 : (kAcc * BLOCK_N <= 256 ? 256 : 512);  // a power of two
 };
@@ -512,9 +514,8 @@ struct Cfg {
 // Operand stages of a few rows (one row block). They bring in only themselves: an SM pulls operands at about 48 bytes per
 // clock, and a whole tile of A would be two thirds of that traffic beside 64 weight rows. The product still reads 128 rows
 // of A; what lies behind the loaded ones goes into accumulator rows that nobody stores.
-// A hand-over between the loading and the issuing thread costs about 400 clocks whatever the tile's width, 0.29 us per
-// k-block with its four products, while the products of 64 columns need 0.07: narrow tiles hand over up to four k-blocks at
-// a time, as long as three stages remain (0.17 us per k-block then; 64 rows x 4096 x 12288: 59.5 -> 37.2 us).
+// A hand-over between the loading and the issuing warp costs a few hundred clocks whatever the tile's width, more than the 0.07 us of
+// a k-block's products of 64 columns: narrow tiles hand over up to four k-blocks at a time, as long as three stages remain.
 constexpr int kTileA = kBlockM * kBlockK * 2;
 constexpr int kMaxStages = 12;
 constexpr int kOperandBytes = 200 * 1024;
@@ -648,7 +649,7 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
                 const __grid_constant__ CUtensorMap ta1, const __grid_constant__ CUtensorMap tb1,
                 const __grid_constant__ TcArgs g, int* status) {
   using C = Cfg<BLOCK_N, ROWS>;
-  constexpr bool FEW = ROWS != kAny;
+  constexpr bool FEW = ROWS == kFew || ROWS == kOctet, PAIR = ROWS == kPair;
   static_assert(ROWS != kOctet || (BLOCK_N == 64 && EPI != kEpiAdd), "");
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = ptx::smem_u32(smem_raw);
@@ -668,7 +669,9 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
   float* octet = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + kBarBytes);  // kOctet
 
   const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
-  const int m_blocks = (g.M + kBlockM - 1) / kBlockM;
+  const uint32_t rank = PAIR ? ptx::cluster_ctarank() : 0u;
+  const int unit0 = PAIR ? blockIdx.x >> 1 : blockIdx.x, unit_step = PAIR ? gridDim.x >> 1 : gridDim.x;
+  const int m_blocks = (g.M + C::kTileM - 1) / C::kTileM;
   const int n_blocks = (g.N + BLOCK_N - 1) / BLOCK_N;
   const int subs = EPI == kEpiPartial ? 1 : g.n_parts;
   const int num_units = m_blocks * n_blocks * (EPI == kEpiPartial ? g.splits[0] + g.splits[1] : 1);
@@ -680,7 +683,7 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
     }
     for (int b = 0; b < 2; ++b) {
       ptx::mbar_init(bar_tfull + 8 * b, 1);
-      ptx::mbar_init(bar_tempty + 8 * b, ROWS == kOctet ? 1 : kEpiWarps);
+      ptx::mbar_init(bar_tempty + 8 * b, ROWS == kOctet ? 1 : (PAIR ? 2 * kEpiWarps : kEpiWarps));  // PAIR: of both CTAs, in CTA 0
     }
     *abort_flag = 0;
     ptx::mbar_init_fence();
@@ -688,11 +691,20 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
     ptx::prefetch_tmap(&tb0);
   }
   if (warp == 1) {
-    ptx::tmem_alloc(ptx::smem_u32(tmem_slot), C::kTmemCols);
-    ptx::tmem_relinquish();
+    if constexpr (PAIR) {
+      ptx::tmem_alloc_pair(ptx::smem_u32(tmem_slot), C::kTmemCols);
+      ptx::tmem_relinquish_pair();
+    } else {
+      ptx::tmem_alloc(ptx::smem_u32(tmem_slot), C::kTmemCols);
+      ptx::tmem_relinquish();
+    }
   }
   ptx::tc_fence_before();
   __syncthreads();
+  if constexpr (PAIR) {  // neither CTA may signal the other's barriers before they are set up
+    ptx::cluster_arrive();
+    ptx::cluster_wait();
+  }
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   ptx::griddep_wait();
@@ -701,7 +713,7 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
   if (warp == 0) {
     uint32_t stage = 0, phase = 0;
     bool ok = true;
-    for (int unit = blockIdx.x; unit < num_units && ok; unit += gridDim.x) {
+    for (int unit = unit0; unit < num_units && ok; unit += unit_step) {
       for (int sub = 0; sub < subs && ok; ++sub) {
         const Job j = job_at<EPI>(g, unit, sub, m_blocks, n_blocks);
         const CUtensorMap* ta = j.part == 0 ? &ta0 : &ta1;
@@ -710,22 +722,38 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
           ok = ptx::mbar_wait_warp(bar_empty + 8 * stage, phase ^ 1u, abort_flag, status, 61);
           if (!ok) break;
           uint32_t sa = base + stage * stage_bytes;
-          const int kb1 = stage_blocks == 1 ? kb0 + 1 : min(kb0 + stage_blocks, j.kb1);
-          ptx::mbar_expect_tx_one(bar_full + 8 * stage, (kb1 - kb0) * block_bytes);
-          for (int kb = kb0; kb < kb1; ++kb, sa += block_bytes) {
-            ptx::tma_load_2d_one(sa, ta, kb * kBlockK, j.mb * kBlockM, bar_full + 8 * stage);
-            ptx::tma_load_2d_one(sa + a_bytes, tb, kb * kBlockK, j.nb * BLOCK_N, bar_full + 8 * stage);
+          if constexpr (PAIR) {  // CTA 0 collects both CTAs' bytes
+            const uint32_t full0 = ptx::mapa(bar_full + 8 * stage, 0);
+            if (rank == 0) ptx::mbar_expect_tx_one(bar_full + 8 * stage, 2 * C::kStageBytes);
+            ptx::tma_load_2d_pair_one(sa, ta, kb0 * kBlockK, j.mb * C::kTileM + static_cast<int>(rank) * kBlockM, full0);
+            ptx::tma_load_2d_pair_one(sa + a_bytes, tb, kb0 * kBlockK, j.nb * BLOCK_N + static_cast<int>(rank) * C::kTileB, full0);
+          } else {
+            const int kb1 = stage_blocks == 1 ? kb0 + 1 : min(kb0 + stage_blocks, j.kb1);
+            ptx::mbar_expect_tx_one(bar_full + 8 * stage, (kb1 - kb0) * block_bytes);
+            for (int kb = kb0; kb < kb1; ++kb, sa += block_bytes) {
+              ptx::tma_load_2d_one(sa, ta, kb * kBlockK, j.mb * kBlockM, bar_full + 8 * stage);
+              ptx::tma_load_2d_one(sa + a_bytes, tb, kb * kBlockK, j.nb * BLOCK_N, bar_full + 8 * stage);
+            }
           }
           if (++stage == n_stages) { stage = 0; phase ^= 1u; }
         }
       }
     }
   } else if (warp == 1) {
-    constexpr uint32_t idesc = ptx::make_idesc(1u, 1u, kBlockM, BLOCK_N);
+    constexpr uint32_t idesc = ptx::make_idesc(1u, 1u, C::kTileM, BLOCK_N);
+    // both CTAs of a pair, or this one
+    auto commit = [&](uint32_t bar) {
+      if constexpr (PAIR) {
+        ptx::tc_commit_pair_one(ptx::mapa(bar, 0));
+        ptx::tc_commit_pair_one(ptx::mapa(bar, 1));
+      } else {
+        ptx::tc_commit_one(bar);
+      }
+    };
     uint32_t stage = 0, phase = 0;
     bool ok = true;
     int it = 0;
-    for (int unit = blockIdx.x; unit < num_units && ok; unit += gridDim.x) {
+    for (int unit = unit0; rank == 0 && unit < num_units && ok; unit += unit_step) {  // PAIR: CTA 0 issues for both
       for (int sub = 0; sub < subs && ok; ++sub) {
         const Job j = job_at<EPI>(g, unit, sub, m_blocks, n_blocks);
         // a set of accumulators: of the whole job, or (kOctet) of one stage, one per k-block
@@ -748,15 +776,19 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
           uint32_t sa = base + stage * stage_bytes;
           const int kb1 = stage_blocks == 1 ? kb0 + 1 : min(kb0 + stage_blocks, j.kb1);
           for (int kb = kb0; kb < kb1; ++kb, sa += block_bytes) {
-            ptx::mma_k_block_f16(d_tmem, ptx::smem_desc_sw128(sa), ptx::smem_desc_sw128(sa + a_bytes), idesc,
-                                 ROWS != kOctet && kb > j.kb0 ? 1u : 0u);
+            const uint64_t a_desc = ptx::smem_desc_sw128(sa), b_desc = ptx::smem_desc_sw128(sa + a_bytes);
+            const uint32_t more = ROWS != kOctet && kb > j.kb0 ? 1u : 0u;
+            if constexpr (PAIR)
+              ptx::mma_k_block_f16_pair(d_tmem, a_desc, b_desc, idesc, more);
+            else
+              ptx::mma_k_block_f16(d_tmem, a_desc, b_desc, idesc, more);
             if (ROWS == kOctet) d_tmem += BLOCK_N;
           }
-          ptx::tc_commit_one(bar_empty + 8 * stage);
-          if (ROWS == kOctet) ptx::tc_commit_one(bar_tfull + 8 * set);
+          commit(bar_empty + 8 * stage);
+          if (ROWS == kOctet) commit(bar_tfull + 8 * set);
           if (++stage == n_stages) { stage = 0; phase ^= 1u; }
         }
-        if (ok && ROWS != kOctet) ptx::tc_commit_one(bar_tfull + 8 * set);
+        if (ok && ROWS != kOctet) commit(bar_tfull + 8 * set);
       }
     }
   } else if (ROWS == kOctet) {
@@ -764,7 +796,7 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
     // it has left in shared memory while it goes on with the next one; all eight meet once per tile.
     bool ok = true;
     int it = 0, tile = 0;
-    for (int unit = blockIdx.x; unit < num_units && ok; unit += gridDim.x) {
+    for (int unit = unit0; unit < num_units && ok; unit += unit_step) {
       for (int sub = 0; sub < subs && ok; ++sub, ++tile) {
         const Job j = job_at<EPI>(g, unit, sub, m_blocks, n_blocks);
         float* out = octet + (tile & 1) * (8 * 64);
@@ -828,11 +860,11 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
     const int part_of_cols = (warp - 2) >> 2;  // two warps per lane quadrant: even / odd chunks
     bool ok = true;
     int it = 0;
-    for (int unit = blockIdx.x; unit < num_units && ok; unit += gridDim.x) {
+    for (int unit = unit0; unit < num_units && ok; unit += unit_step) {
       for (int sub = 0; sub < subs && ok; ++sub, ++it) {
         const Job j = job_at<EPI>(g, unit, sub, m_blocks, n_blocks);
         const uint32_t buf = it & 1;
-        const int row = j.mb * kBlockM + quad * 32 + lane;
+        const int row = j.mb * C::kTileM + static_cast<int>(rank) * kBlockM + quad * 32 + lane;
         const int n0 = j.nb * BLOCK_N;
         const bool any_row = row - lane < g.M;
         int okw = 0;
@@ -956,7 +988,12 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
         }
         ptx::tc_fence_before();
         __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(bar_tempty + 8 * buf);
+        if (lane == 0) {
+          if constexpr (PAIR)
+            ptx::mbar_arrive_cluster_relaxed(ptx::mapa(bar_tempty + 8 * buf, 0));
+          else
+            ptx::mbar_arrive(bar_tempty + 8 * buf);
+        }
       }
     }
   }
@@ -967,9 +1004,16 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
     for (int i = 0; i < 200; ++i) __nanosleep(1000);
     __syncthreads();
   }
+  if constexpr (PAIR) {  // both converge before either frees tensor memory or leaves
+    ptx::cluster_arrive();
+    ptx::cluster_wait();
+  }
   if (warp == 1) {
     ptx::tc_fence_after();
-    ptx::tmem_dealloc(tmem_base, C::kTmemCols);
+    if constexpr (PAIR)
+      ptx::tmem_dealloc_pair(tmem_base, C::kTmemCols);
+    else
+      ptx::tmem_dealloc(tmem_base, C::kTmemCols);
   }
 }
 
@@ -1008,7 +1052,7 @@ int make_tmap_bf16_2d(CUtensorMap* map, const void* ptr, uint64_t cols, uint64_t
 template <int BLOCK_N, int EPI, int ROWS>
 static int launch_tc(TcArgs g, const fr_gated_part* parts, cudaStream_t stream) {
   using C = Cfg<BLOCK_N, ROWS>;
-  constexpr bool FEW = ROWS != kAny;
+  constexpr bool FEW = ROWS == kFew || ROWS == kOctet, PAIR = ROWS == kPair;
   const Stages few(FEW ? g.M : kBlockM, BLOCK_N);
   g.a_bytes = few.a_bytes;
   g.block_bytes = few.block_bytes;
@@ -1019,7 +1063,7 @@ static int launch_tc(TcArgs g, const fr_gated_part* parts, cudaStream_t stream) 
   for (int p = 0; p < 2; ++p) {
     const fr_gated_part& q = parts[p < g.n_parts ? p : 0];
     int st = make_tmap_bf16_2d(&ta[p], q.a, q.K, g.M, q.lda, FEW ? few.a_rows : kBlockM);
-    if (st == FR_OK) st = make_tmap_bf16_2d(&tb[p], q.w, q.K, g.N, q.ldw, BLOCK_N);
+    if (st == FR_OK) st = make_tmap_bf16_2d(&tb[p], q.w, q.K, g.N, q.ldw, C::kTileB);
     if (st != FR_OK) return st;
   }
   auto kern = dense_tc_kernel<BLOCK_N, EPI, ROWS>;
@@ -1027,9 +1071,12 @@ static int launch_tc(TcArgs g, const fr_gated_part* parts, cudaStream_t stream) 
   if (ensure_dyn_smem(attr_done, kern, FEW ? 1024 + kOperandBytes + kTileA + kBarBytes + kOctetBytes : smem) != FR_OK) return FR_ERR_CUDA;
   int* status = device_status_ptr();
   if (!status) return FR_ERR_CUDA;
-  const int64_t units = static_cast<int64_t>(ceil_div(g.M, kBlockM)) * ceil_div(g.N, BLOCK_N) *
+  const int64_t units = static_cast<int64_t>(ceil_div(g.M, C::kTileM)) * ceil_div(g.N, BLOCK_N) *
                         (EPI == kEpiPartial ? g.splits[0] + g.splits[1] : 1);
-  const int grid = static_cast<int>(units < device_sm_count() ? units : device_sm_count());
+  const int slots = device_sm_count() / (PAIR ? 2 : 1);
+  const int grid = static_cast<int>(units < slots ? units : slots) * (PAIR ? 2 : 1);
+  if constexpr (PAIR)
+    return launch_cluster(kern, grid, kThreads, smem, stream, 2, g.M <= kPdlRows, ta[0], tb[0], ta[1], tb[1], g, status);
   return launch_kernel(kern, grid, kThreads, smem, stream, g.M <= kPdlRows, ta[0], tb[0], ta[1], tb[1], g, status);
 }
 
@@ -1054,6 +1101,16 @@ static int pick_block_n(int M, int N, bool few) {
     }
   }
   return best;
+}
+
+// Whether tiles of 256 columns are taken by pairs of CTAs: from two rounds of tiles on, unless 256 rows at a time take more rounds. A
+// CTA of a pair brings in 32 KB per 128 x 256 x 64 products, alone 48. us, alone / in pairs (same bits): 20480 x 2048 700 rows 55.9 /
+// 50.9, 2048 rows 134.7 / 118.4, 8192 rows 516 / 454; 24576 x 4096 2048 rows 304 / 270; update 2048 x 8192 8192 rows 296 / 263; one
+// round, 4096 x 2048 700 rows 17.2 / 17.6; three rounds for two, 20480 x 2048 350 rows 33.0 / 36.8.
+static bool use_pair(int M, int N) {
+  const int64_t sms = device_sm_count(), n_blocks = ceil_div(N, 256);
+  const int64_t alone = (ceil_div(M, kBlockM) * n_blocks + sms - 1) / sms, pairs = (ceil_div(M, 2 * kBlockM) * n_blocks + sms / 2 - 1) / (sms / 2);
+  return alone >= 2 && pairs <= alone;
 }
 
 // Whether a few-row product streams the weights through the row kernel. There a weight costs an FMA per row, rows counted as 1, 2, 4
@@ -1220,6 +1277,7 @@ extern "C" int fr_dense_proj(int dtype, const void* a, int64_t lda, const void* 
       default: return dense::launch_tc<64, dense::kEpiSegs, dense::kFew>(g, &part, stream);
     }
   }
+  if (block_n == 256 && dense::use_pair(M, N)) return dense::launch_tc<256, dense::kEpiSegs, dense::kPair>(g, &part, stream);
   switch (block_n) {
     case 256: return dense::launch_tc<256, dense::kEpiSegs, dense::kAny>(g, &part, stream);
     case 128: return dense::launch_tc<128, dense::kEpiSegs, dense::kAny>(g, &part, stream);
@@ -1308,7 +1366,9 @@ extern "C" int fr_dense_gated_add(int dtype, const fr_gated_part* parts, int n_p
     return dense::few_rows(M, K) ? dense::launch_tc<64, dense::kEpiPartial, dense::kFew>(g, parts, stream)
                                  : dense::launch_tc<64, dense::kEpiPartial, dense::kAny>(g, parts, stream);
   }
-  switch (dense::pick_block_n(M, N, false)) {
+  const int block_n = dense::pick_block_n(M, N, false);
+  if (block_n == 256 && dense::use_pair(M, N)) return dense::launch_tc<256, dense::kEpiAdd, dense::kPair>(g, parts, stream);
+  switch (block_n) {
     case 256: return dense::launch_tc<256, dense::kEpiAdd, dense::kAny>(g, parts, stream);
     case 128: return dense::launch_tc<128, dense::kEpiAdd, dense::kAny>(g, parts, stream);
     default: return dense::launch_tc<64, dense::kEpiAdd, dense::kAny>(g, parts, stream);

@@ -222,6 +222,7 @@ __device__ __forceinline__ void tc_commit_one(uint32_t bar) {
 FR_MMA_K_BLOCK(mma_k_block_f8, "cta_group::1", "kind::f8f6f4")
 FR_MMA_K_BLOCK(mma_k_block_f16, "cta_group::1", "kind::f16")
 FR_MMA_K_BLOCK(mma_k_block_f8_pair, "cta_group::2", "kind::f8f6f4")
+FR_MMA_K_BLOCK(mma_k_block_f16_pair, "cta_group::2", "kind::f16")
 #undef FR_MMA_K_BLOCK
 
 // D[tmem] (+)= A[smem] * B[smem], one product.

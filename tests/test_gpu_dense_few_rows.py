@@ -158,3 +158,24 @@ def test_f32_updates_in_shares(m, n, ks):
     got = x.double() + (p.buf.double().sum(0) if p is not None else 0)
     # k roundings of 2^-24 of sums of about 1 in random order, the gate's and the stream's
     assert float((got - want).norm() / want.norm()) < (max(ks) ** 0.5 + 4) * 2 ** -24
+
+
+@pytest.mark.parametrize("m,n,k", [(385, 37888, 72), (700, 20480, 136), (1111, 10016, 520), (1923, 4128, 1096), (5000, 2080, 72)])
+def test_pairs_of_ctas(m, n, k):
+    """Tiles of 256 rows on two SMs, with rows, columns and K left over: a projection and an update in two parts."""
+    from flashrec_b200.lm_layers import MergedProjection, gated_add
+
+    a, w = _rand(m, k, seed=m), _rand(n, k, seed=1) * k ** -0.5
+    proj = MergedProjection(k)
+    proj.add("store_f32", w)
+    proj.finish(torch.bfloat16, "cuda")
+    out = torch.full((m, n), float("nan"), device="cuda")
+    proj(a, [out])
+    ref = a.double() @ w.double().T
+    # as in test_projection: k roundings of 2^-24 of a sum of about 1, in whatever order
+    bound = 8 * k ** 0.5 * 2 ** -24
+    assert float((out.double() - ref).abs().max()) < bound * float(ref.abs().max())
+    x, gate = torch.randn(m, n, device="cuda", generator=torch.Generator(device="cuda").manual_seed(5)), _rand(m, n, seed=2)
+    want = x.double() + gate.double() * ref + ref
+    assert gated_add(x, [(a, w, gate), (a, w, None)], split=False) is None
+    assert float((x.double() - want).abs().max()) < 2 * bound * float(want.abs().max())
