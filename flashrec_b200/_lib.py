@@ -159,6 +159,7 @@ _SIGNATURES = {
     "fr_version": [],
     "fr_device_status": [POINTER(c_int), POINTER(c_int)],
     "fr_rms_quant_fp8": [P, P, P, _F, P, P, _I, _I, P],
+    "fr_rms_quant_zero_fp8": [P, P, P, _F, P, P, P, _I, _I, P],
     "fr_rmsnorm_bf16": [P, P, P, _F, P, _I, _I, P],
     "fr_token_quant_fp8": [P, _I, P, P, _I, _I, P],
     "fr_silu_mul_quant_fp8": [P, P, P, _I, _I, P],

@@ -73,12 +73,12 @@ struct Params {
 // plan; prefill: every key of the request).
 __device__ __forceinline__ int group_keys(const Params& p, int grp, int row0, const int32_t*& idx) {
   if (p.kv_group_indptr != nullptr) {
-    const int b = p.kv_group_indptr[grp];
+    const int b = __ldcg(p.kv_group_indptr + grp);
     idx = p.indices + b;
-    return min(max(p.kv_group_indptr[grp + 1] - b, 0), p.lcap);
+    return min(max(__ldcg(p.kv_group_indptr + grp + 1) - b, 0), p.lcap);
   }
-  idx = p.indices + p.indptr[row0];
-  return min(p.shared_len[grp], p.lcap);
+  idx = p.indices + __ldcg(p.indptr + row0);
+  return min(__ldcg(p.shared_len + grp), p.lcap);
 }
 
 __device__ __forceinline__ __half2 e4m3x2_to_half2(uint16_t v) {
@@ -116,6 +116,8 @@ __device__ __forceinline__ float2 e4m3x2_to_float2(uint16_t v) {
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) shared_kv_prepare_kernel(Params p) {
   const int grp = blockIdx.z, kvh = blockIdx.y;
+  ptx::griddep_wait();
+  ptx::griddep_launch_dependents();
   const int row0 = p.group_rows[grp];
   const int32_t* idx;
   const int ls = group_keys(p, grp, row0, idx);
@@ -136,8 +138,8 @@ __global__ void __launch_bounds__(256) shared_kv_prepare_kernel(Params p) {
   if (tok < ls) {
     int64_t s = idx[tok];
     s = s < 0 ? 0 : (s >= p.num_slots ? p.num_slots - 1 : s);
-    kraw = __ldg(reinterpret_cast<const uint4*>(p.kc + s * p.ck_s + kvh * p.ck_h + ch * 16));
-    vraw = __ldg(reinterpret_cast<const uint4*>(p.vc + s * p.cv_s + kvh * p.cv_h + ch * 16));
+    kraw = __ldcg(reinterpret_cast<const uint4*>(p.kc + s * p.ck_s + kvh * p.ck_h + ch * 16));
+    vraw = __ldcg(reinterpret_cast<const uint4*>(p.vc + s * p.cv_s + kvh * p.cv_h + ch * 16));
   }
   if (tok >= padded || tok < done) return;
   const uint32_t kw[4] = {kraw.x, kraw.y, kraw.z, kraw.w};
@@ -226,10 +228,15 @@ decode_attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
 
   constexpr int kBeams = kM / G;
   const int grp = blockIdx.z, kvh = blockIdx.y;
-  const int row0 = p.group_rows[grp];
-  const int rows_in_group = p.group_rows[grp + 1] - row0;
+  // Launched while shared_kv_prepare_kernel still runs (few rows). What that kernel does not write was finished before it began:
+  // lists, queries and the tails' keys and values are read at once, through L2; only the loads of the widened tiles wait for it.
+  const int row0 = __ldcg(p.group_rows + grp);
+  const int rows_in_group = __ldcg(p.group_rows + grp + 1) - row0;
   const int beam0 = blockIdx.x * kBeams;
-  if (beam0 >= rows_in_group) return;
+  if (beam0 >= rows_in_group) {
+    ptx::griddep_wait();  // no CTA leaves before: the next launch counts on this one's end
+    return;
+  }
   const int32_t* idx_unused;
   const int ls = group_keys(p, grp, row0, idx_unused);
   const int pfx = CAUSAL ? max(ls - rows_in_group, 0) : 0;
@@ -253,12 +260,12 @@ decode_attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
 #pragma unroll
     for (int b = 0; b < kBatch; ++b) {
       slot[b] = 0;
-      if (t0 + b < t_len) slot[b] = max(0, min(p.indices[t_beg + t0 + b], p.num_slots - 1));
+      if (t0 + b < t_len) slot[b] = max(0, min(__ldcg(p.indices + t_beg + t0 + b), p.num_slots - 1));
     }
   };
   if (!CAUSAL && warp >= 2) {
-    t_beg = p.indptr[row] + ls;
-    t_len = live ? max(p.indptr[row + 1] - t_beg, 0) : 0;
+    t_beg = __ldcg(p.indptr + row) + ls;
+    t_len = live ? max(__ldcg(p.indptr + row + 1) - t_beg, 0) : 0;
     load_slots(0);
 #pragma unroll
     for (int b = 0; b < kBatch; ++b)  // an earlier step's values have left L2 since
@@ -303,6 +310,8 @@ decode_attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     ptx::mbar_expect_tx_one(bar_q, kSmemQ);
     ptx::tma_load_3d_one(sm_q, &tmap_q, 0, kvh * G, row0 + beam0, bar_q);
     ptx::tma_load_3d_one(sm_q + kSmemQ / 2, &tmap_q, 64, kvh * G, row0 + beam0, bar_q);
+    ptx::griddep_wait();
+    ptx::griddep_launch_dependents();
     bool ok = true;
     auto load_k = [&](int jj) -> bool {
       const uint32_t st = jj & 1, ph = (jj >> 1) & 1;
@@ -387,7 +396,7 @@ decode_attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       if (t0 + b < t_len) {
         const uint8_t* kp = p.kc + static_cast<int64_t>(slot[b]) * p.ck_s + kvh * p.ck_h;
 #pragma unroll
-        for (int c = 0; c < kD / 16; ++c) kk[c] = __ldg(reinterpret_cast<const uint4*>(kp + c * 16));
+        for (int c = 0; c < kD / 16; ++c) kk[c] = __ldcg(reinterpret_cast<const uint4*>(kp + c * 16));
       }
     };
 #pragma unroll
@@ -488,8 +497,8 @@ decode_attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       for (int b = 0; b < kBatch; ++b) {
         if (t0 + b < t_len) {
           const uint8_t* vp = p.vc + static_cast<int64_t>(slot[b]) * p.cv_s + kvh * p.cv_h + c * 32;
-          vnext[b][0] = __ldg(reinterpret_cast<const uint4*>(vp));
-          vnext[b][1] = __ldg(reinterpret_cast<const uint4*>(vp + 16));
+          vnext[b][0] = __ldcg(reinterpret_cast<const uint4*>(vp));
+          vnext[b][1] = __ldcg(reinterpret_cast<const uint4*>(vp + 16));
         }
       }
     };
@@ -678,11 +687,10 @@ static int launch(const Params& p, int max_group_rows, cudaStream_t stream) {
   int* status = device_status_ptr();
   if (!status) return FR_ERR_CUDA;
   dim3 pgrid(ceil_div(p.lcap, 32), p.hkv, p.n_groups);
-  shared_kv_prepare_kernel<<<pgrid, 256, 0, stream>>>(p);
-  if (launch_status() != FR_OK) return FR_ERR_CUDA;
+  const bool pdl = p.n_rows <= kPdlRows;
+  if (launch_kernel(shared_kv_prepare_kernel, pgrid, 256, 0, stream, pdl, p) != FR_OK) return FR_ERR_CUDA;
   dim3 grid(ceil_div(max_group_rows, kM / G), p.hkv, p.n_groups);
-  kern<<<grid, kThreads, kSmemBytes, stream>>>(tq, tk, tv, p, status);
-  return launch_status();
+  return launch_kernel(kern, grid, kThreads, kSmemBytes, stream, pdl, tq, tk, tv, p, status);
 }
 
 }  // namespace attn_tc

@@ -16,6 +16,7 @@
 // bf16. The only deliberate difference is the sum of squares, accumulated in
 // fp64 and rounded once (order independent), where torch adds in fp32.
 #include "fr_common.cuh"
+#include "sm100_ptx.cuh"
 
 namespace fr {
 
@@ -27,16 +28,22 @@ constexpr int kWarpsPerCta = 4;  // 128-thread CTAs: at ~96 registers per thread
 template <int VPL, bool NORM, bool RESID, bool QUANT>
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
 row_warp_kernel(const uint4* __restrict__ x, uint4* __restrict__ resid, const uint4* __restrict__ w, float eps,
-                uint2* __restrict__ q, float* __restrict__ scale, uint4* __restrict__ y_out, int rows) {
+                uint2* __restrict__ q, float* __restrict__ scale, uint4* __restrict__ y_out, float* __restrict__ zero, int rows) {
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5);
+  // Up to kPdlRows rows: launched while the launch ahead still runs, as the products around it are. With the norms, quantisers, the
+  // rotary step and the attention launched so, and no fill ahead of the SwiGLU product, a wave of 512 rows (84 layers) takes 7.96 ms
+  // where it took 8.67.
+  ptx::griddep_wait();
+  ptx::griddep_launch_dependents();
   if (row >= rows) return;
   constexpr int kVecPerRow = VPL * 32;
   const uint4* xr = x + static_cast<size_t>(row) * kVecPerRow;
 
   uint4 v[VPL];
 #pragma unroll
-  for (int j = 0; j < VPL; ++j) v[j] = __ldg(xr + j * 32 + lane);
+  for (int j = 0; j < VPL; ++j) v[j] = __ldcg(xr + j * 32 + lane);
+  if (zero != nullptr && lane == 0) zero[row] = 0.f;
 
   if constexpr (RESID) {
     uint4* rr = resid + static_cast<size_t>(row) * kVecPerRow;
@@ -151,11 +158,12 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 template <bool NORM, bool RESID, bool QUANT>
 __global__ void __launch_bounds__(kBlockRowThreads)
 row_block_kernel(const uint4* __restrict__ x, uint4* __restrict__ resid, const uint4* __restrict__ w, float eps,
-                 uint2* __restrict__ q, float* __restrict__ scale, uint4* __restrict__ y_out, int hidden) {
+                 uint2* __restrict__ q, float* __restrict__ scale, uint4* __restrict__ y_out, float* __restrict__ zero, int hidden) {
   extern __shared__ uint4 row_smem[];
   __shared__ double red_d[kBlockRowThreads / 32];
   __shared__ float red_f[kBlockRowThreads / 32];
   const int row = blockIdx.x;
+  if (zero != nullptr && threadIdx.x == 0) zero[row] = 0.f;
   const int nvec = hidden >> 3;
   const uint4* xr = x + static_cast<size_t>(row) * nvec;
   double ss = 0.0;
@@ -322,6 +330,8 @@ __global__ void __launch_bounds__(256)
 quant_known_amax_kernel(const uint4* __restrict__ y, const float* __restrict__ row_amax, uint2* __restrict__ q,
                         float* __restrict__ scale, int vec_per_row) {
   const int row = blockIdx.x;
+  ptx::griddep_wait();
+  ptx::griddep_launch_dependents();
   const uint4* yr = y + static_cast<size_t>(row) * vec_per_row;
   uint4 v[NV];
 #pragma unroll
@@ -330,7 +340,7 @@ quant_known_amax_kernel(const uint4* __restrict__ y, const float* __restrict__ r
     v[j] = make_uint4(0, 0, 0, 0);
     if (i < vec_per_row) v[j] = __ldcs(yr + i);
   }
-  const float s = row_scale(__ldg(row_amax + row));
+  const float s = row_scale(__ldcg(row_amax + row));
   const float inv = __fdiv_rn(1.0f, s);
   const float sf = finite_or_zero(s);
   uint2* qr = q + static_cast<size_t>(row) * vec_per_row;
@@ -354,7 +364,7 @@ quant_known_amax_kernel(const uint4* __restrict__ y, const float* __restrict__ r
 // host-side dispatch
 // ---------------------------------------------------------------------------
 template <bool NORM, bool RESID, bool QUANT>
-static int launch_rows(const void* x, void* resid, const void* w, float eps, void* q, float* scale, void* y,
+static int launch_rows(const void* x, void* resid, const void* w, float eps, void* q, float* scale, void* y, float* zero,
                        int rows, int hidden, cudaStream_t stream) {
   if (rows == 0) return FR_OK;
   const uint4* xp = static_cast<const uint4*>(x);
@@ -365,14 +375,14 @@ static int launch_rows(const void* x, void* resid, const void* w, float eps, voi
   const int grid_w = ceil_div(rows, kWarpsPerCta);
   switch (hidden) {
     case 1024:
-      row_warp_kernel<4, NORM, RESID, QUANT><<<grid_w, kWarpsPerCta * 32, 0, stream>>>(xp, rp, wp, eps, qp, scale, yp, rows);
-      return launch_status();
+      return launch_kernel(row_warp_kernel<4, NORM, RESID, QUANT>, grid_w, kWarpsPerCta * 32, 0, stream, rows <= kPdlRows, xp, rp, wp, eps, qp,
+                           scale, yp, zero, rows);
     case 2048:
-      row_warp_kernel<8, NORM, RESID, QUANT><<<grid_w, kWarpsPerCta * 32, 0, stream>>>(xp, rp, wp, eps, qp, scale, yp, rows);
-      return launch_status();
+      return launch_kernel(row_warp_kernel<8, NORM, RESID, QUANT>, grid_w, kWarpsPerCta * 32, 0, stream, rows <= kPdlRows, xp, rp, wp, eps, qp,
+                           scale, yp, zero, rows);
     case 4096:
-      row_warp_kernel<16, NORM, RESID, QUANT><<<grid_w, kWarpsPerCta * 32, 0, stream>>>(xp, rp, wp, eps, qp, scale, yp, rows);
-      return launch_status();
+      return launch_kernel(row_warp_kernel<16, NORM, RESID, QUANT>, grid_w, kWarpsPerCta * 32, 0, stream, rows <= kPdlRows, xp, rp, wp, eps, qp,
+                           scale, yp, zero, rows);
     default:
       break;
   }
@@ -383,7 +393,7 @@ static int launch_rows(const void* x, void* resid, const void* w, float eps, voi
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
       return FR_ERR_CUDA;
   }
-  kern<<<rows, kBlockRowThreads, smem, stream>>>(xp, rp, wp, eps, qp, scale, yp, hidden);
+  kern<<<rows, kBlockRowThreads, smem, stream>>>(xp, rp, wp, eps, qp, scale, yp, zero, hidden);
   return launch_status();
 }
 
@@ -391,14 +401,25 @@ static int launch_rows(const void* x, void* resid, const void* w, float eps, voi
 
 using namespace fr;
 
-extern "C" int fr_rms_quant_fp8(const void* x, void* residual, const void* weight, float eps, void* q_out,
-                                float* scale_out, int rows, int hidden, cudaStream_t stream) {
+static int rms_quant(const void* x, void* residual, const void* weight, float eps, void* q_out, float* scale_out, float* zero, int rows,
+                     int hidden, cudaStream_t stream) {
   FR_CHECK_ARG(rows >= 0 && hidden > 0 && hidden % 8 == 0);
   if (rows == 0) return FR_OK;
   FR_CHECK_ARG(x && weight && q_out && scale_out);
   FR_CHECK_ARG(aligned16(x) && aligned16(weight) && aligned16(q_out) && (!residual || aligned16(residual)));
-  if (residual) return launch_rows<true, true, true>(x, residual, weight, eps, q_out, scale_out, nullptr, rows, hidden, stream);
-  return launch_rows<true, false, true>(x, nullptr, weight, eps, q_out, scale_out, nullptr, rows, hidden, stream);
+  if (residual) return launch_rows<true, true, true>(x, residual, weight, eps, q_out, scale_out, nullptr, zero, rows, hidden, stream);
+  return launch_rows<true, false, true>(x, nullptr, weight, eps, q_out, scale_out, nullptr, zero, rows, hidden, stream);
+}
+
+extern "C" int fr_rms_quant_fp8(const void* x, void* residual, const void* weight, float eps, void* q_out,
+                                float* scale_out, int rows, int hidden, cudaStream_t stream) {
+  return rms_quant(x, residual, weight, eps, q_out, scale_out, nullptr, rows, hidden, stream);
+}
+
+extern "C" int fr_rms_quant_zero_fp8(const void* x, void* residual, const void* weight, float eps, void* q_out, float* scale_out,
+                                     float* zero_out, int rows, int hidden, cudaStream_t stream) {
+  FR_CHECK_ARG(zero_out != nullptr || rows == 0);
+  return rms_quant(x, residual, weight, eps, q_out, scale_out, zero_out, rows, hidden, stream);
 }
 
 extern "C" int fr_rmsnorm_bf16(const void* x, void* residual, const void* weight, float eps, void* y_out, int rows,
@@ -407,8 +428,8 @@ extern "C" int fr_rmsnorm_bf16(const void* x, void* residual, const void* weight
   if (rows == 0) return FR_OK;
   FR_CHECK_ARG(x && weight && y_out);
   FR_CHECK_ARG(aligned16(x) && aligned16(weight) && aligned16(y_out) && (!residual || aligned16(residual)));
-  if (residual) return launch_rows<true, true, false>(x, residual, weight, eps, nullptr, nullptr, y_out, rows, hidden, stream);
-  return launch_rows<true, false, false>(x, nullptr, weight, eps, nullptr, nullptr, y_out, rows, hidden, stream);
+  if (residual) return launch_rows<true, true, false>(x, residual, weight, eps, nullptr, nullptr, y_out, nullptr, rows, hidden, stream);
+  return launch_rows<true, false, false>(x, nullptr, weight, eps, nullptr, nullptr, y_out, nullptr, rows, hidden, stream);
 }
 
 extern "C" int fr_token_quant_fp8(const void* x, int x_is_f32, void* q_out, float* scale_out, int rows, int hidden,
@@ -423,7 +444,7 @@ extern "C" int fr_token_quant_fp8(const void* x, int x_is_f32, void* q_out, floa
     return launch_status();
   }
   FR_CHECK_ARG(hidden % 8 == 0);
-  return launch_rows<false, false, true>(x, nullptr, nullptr, 0.f, q_out, scale_out, nullptr, rows, hidden, stream);
+  return launch_rows<false, false, true>(x, nullptr, nullptr, 0.f, q_out, scale_out, nullptr, nullptr, rows, hidden, stream);
 }
 
 template <bool QUANT>
@@ -470,13 +491,12 @@ extern "C" int fr_quant_known_amax_fp8(const void* y, const float* row_amax, voi
   uint2* qp = static_cast<uint2*>(q_out);
   const int vec = d / 8;
   switch (ceil_div(vec, 256)) {
-    case 1: quant_known_amax_kernel<1><<<rows, 256, 0, stream>>>(yp, row_amax, qp, scale_out, vec); break;
-    case 2: quant_known_amax_kernel<2><<<rows, 256, 0, stream>>>(yp, row_amax, qp, scale_out, vec); break;
-    case 3: quant_known_amax_kernel<3><<<rows, 256, 0, stream>>>(yp, row_amax, qp, scale_out, vec); break;
-    case 4: quant_known_amax_kernel<4><<<rows, 256, 0, stream>>>(yp, row_amax, qp, scale_out, vec); break;
+    case 1: return launch_kernel(quant_known_amax_kernel<1>, rows, 256, 0, stream, rows <= kPdlRows, yp, row_amax, qp, scale_out, vec);
+    case 2: return launch_kernel(quant_known_amax_kernel<2>, rows, 256, 0, stream, rows <= kPdlRows, yp, row_amax, qp, scale_out, vec);
+    case 3: return launch_kernel(quant_known_amax_kernel<3>, rows, 256, 0, stream, rows <= kPdlRows, yp, row_amax, qp, scale_out, vec);
+    case 4: return launch_kernel(quant_known_amax_kernel<4>, rows, 256, 0, stream, rows <= kPdlRows, yp, row_amax, qp, scale_out, vec);
     case 5: case 6: case 7: case 8:
-      quant_known_amax_kernel<8><<<rows, 256, 0, stream>>>(yp, row_amax, qp, scale_out, vec); break;
+      return launch_kernel(quant_known_amax_kernel<8>, rows, 256, 0, stream, rows <= kPdlRows, yp, row_amax, qp, scale_out, vec);
     default: return FR_ERR_UNSUPPORTED;  // d > 16384
   }
-  return launch_status();
 }

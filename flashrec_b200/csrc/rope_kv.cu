@@ -11,6 +11,7 @@
 // All are HBM-bound; a group of D/8 lanes owns one (token, head) pair and moves
 // 8 bf16 per lane (4 from each rotary half) with 8-byte accesses.
 #include "fr_common.cuh"
+#include "sm100_ptx.cuh"
 
 namespace fr {
 
@@ -41,7 +42,7 @@ struct RopeArgs {
 };
 
 __device__ __forceinline__ void load4(const __nv_bfloat16* p, float (&x)[4]) {
-  uint2 u = *reinterpret_cast<const uint2*>(p);
+  const uint2 u = __ldcg(reinterpret_cast<const uint2*>(p));
   x[0] = bf16lo(u.x); x[1] = bf16hi(u.x); x[2] = bf16lo(u.y); x[3] = bf16hi(u.y);
 }
 
@@ -62,6 +63,8 @@ __global__ void __launch_bounds__(256) qk_rope_kv_kernel(RopeArgs a) {
   const int groups_per_tok = heads_all / HPG;
   const int64_t item = (static_cast<int64_t>(blockIdx.x) * (256 / 32) + (threadIdx.x >> 5)) * GPW + lane / LPH;
   const bool live = item < static_cast<int64_t>(a.T) * groups_per_tok;
+  ptx::griddep_wait();
+  ptx::griddep_launch_dependents();
   // dead groups still take part in the shuffles below
   const int t = live ? static_cast<int>(item / groups_per_tok) : 0;
   const int hs0 = live ? static_cast<int>(item % groups_per_tok) * HPG : 0;
@@ -76,8 +79,8 @@ __global__ void __launch_bounds__(256) qk_rope_kv_kernel(RopeArgs a) {
   // The position / slot lookups and the cos / sin row they lead to are independent of the head
   // data: issue them first so that their two dependent round trips overlap the loads of the heads.
   int64_t p = 0, slot = 0;
-  if (live && rotate) p = __ldg(a.pos + t);
-  if (live && !is_q) slot = __ldg(a.loc + t);
+  if (live && rotate) p = __ldcg(a.pos + t);
+  if (live && !is_q) slot = __ldcg(a.loc + t);
   float lo[HPG][4], hi[HPG][4];
 #pragma unroll
   for (int j = 0; j < HPG; ++j) {
@@ -182,16 +185,14 @@ static int launch_rope(const RopeArgs& a, int D, cudaStream_t stream) {
   const int64_t items = static_cast<int64_t>(a.T) * (four ? heads_all / 4 : heads_all);
   if (D == 128) {
     const int per_cta = 8 * 2;
-    if (four) qk_rope_kv_kernel<128, ROPE, 4, NORM><<<ceil_div(items, per_cta), 256, 0, stream>>>(a);
-    else qk_rope_kv_kernel<128, ROPE, 1, NORM><<<ceil_div(items, per_cta), 256, 0, stream>>>(a);
+    if (four) return launch_kernel(qk_rope_kv_kernel<128, ROPE, 4, NORM>, ceil_div(items, per_cta), 256, 0, stream, a.T <= kPdlRows, a);
+    return launch_kernel(qk_rope_kv_kernel<128, ROPE, 1, NORM>, ceil_div(items, per_cta), 256, 0, stream, a.T <= kPdlRows, a);
   } else if (D == 64) {
     const int per_cta = 8 * 4;
-    if (four) qk_rope_kv_kernel<64, ROPE, 4, NORM><<<ceil_div(items, per_cta), 256, 0, stream>>>(a);
-    else qk_rope_kv_kernel<64, ROPE, 1, NORM><<<ceil_div(items, per_cta), 256, 0, stream>>>(a);
-  } else {
-    return FR_ERR_UNSUPPORTED;
+    if (four) return launch_kernel(qk_rope_kv_kernel<64, ROPE, 4, NORM>, ceil_div(items, per_cta), 256, 0, stream, a.T <= kPdlRows, a);
+    return launch_kernel(qk_rope_kv_kernel<64, ROPE, 1, NORM>, ceil_div(items, per_cta), 256, 0, stream, a.T <= kPdlRows, a);
   }
-  return launch_status();
+  return FR_ERR_UNSUPPORTED;
 }
 
 // Scatter of rows that are e4m3 already: cache[loc[t], h, :] = src[t, h, :] as 16-byte pieces.

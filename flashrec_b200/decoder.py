@@ -112,12 +112,12 @@ class Qwen3MLP:
             self.gate_up_proj._fp8_weight = None
             self.gate_up_proj._fp8_scale = None
 
-    def forward(self, x, *, q_fp8, a_scale, residual_inout=None) -> torch.Tensor:
+    def forward(self, x, *, q_fp8, a_scale, residual_inout=None, row_amax=None) -> torch.Tensor:
         """``residual_inout``: the down_proj GEMM adds its output to this bf16 residual stream in
-        place (and returns it) instead of returning the projection."""
+        place (and returns it) instead of returning the projection. ``row_amax``: zeros for the SwiGLU epilogue's maxima."""
         rows = int(q_fp8.shape[0])
         if self.fuse_silu_gemm and self._gu_w is not None:
-            y, amax = fp8_scaled_mm_silu_mul(q_fp8, self._gu_w, a_scale, self._gu_s)
+            y, amax = fp8_scaled_mm_silu_mul(q_fp8, self._gu_w, a_scale, self._gu_s, row_amax=row_amax)
             y_fp8, y_scale = quant_known_amax_fp8(y, amax)
         else:
             gu = self.gate_up_proj.forward_fp8(q_fp8, a_scale, (rows, self.gate_up_proj.in_features), torch.bfloat16)
@@ -141,8 +141,9 @@ class Qwen3DecoderLayer:
         to ``forward`` (the GEMM output is rounded to bf16 before the bf16 add in both)."""
         q_fp8, a_scale = self.input_layernorm.quant_fp8(residual)
         self.self_attn.forward(None, batch, q_fp8=q_fp8, a_scale=a_scale, residual_inout=residual)
-        q_fp8, a_scale = self.post_attention_layernorm.quant_fp8(residual)
-        self.mlp.forward(None, q_fp8=q_fp8, a_scale=a_scale, residual_inout=residual)
+        row_amax = torch.empty(residual.shape[0], dtype=torch.float32, device=residual.device)
+        q_fp8, a_scale = self.post_attention_layernorm.quant_fp8(residual, zero=row_amax)
+        self.mlp.forward(None, q_fp8=q_fp8, a_scale=a_scale, residual_inout=residual, row_amax=row_amax)
         return residual
 
     def forward(self, x, residual, batch: ForwardBatch):

@@ -3,6 +3,8 @@
 
 from __future__ import annotations
 
+from typing import Optional
+
 import torch
 
 from flashrec_b200._lib import call, ptr, require_cuda, stream_ptr
@@ -10,7 +12,7 @@ from flashrec_b200._lib import call, ptr, require_cuda, stream_ptr
 _FP8 = torch.float8_e4m3fn
 
 
-def _launch(x, weight, eps, residual):
+def _launch(x, weight, eps, residual, zero=None):
     require_cuda(x, weight, residual)
     if x.dtype != torch.bfloat16:
         raise TypeError(f"rms_fp8: expected bfloat16 activations, got {x.dtype}")
@@ -29,8 +31,11 @@ def _launch(x, weight, eps, residual):
             r2 = r2.contiguous()
     q = torch.empty((rows, hidden), dtype=_FP8, device=x.device)
     scale = torch.empty((rows, 1), dtype=torch.float32, device=x.device)
-    call("fr_rms_quant_fp8", ptr(x2), ptr(r2), ptr(w), float(eps), ptr(q), ptr(scale), rows, hidden,
-         stream_ptr(x.device))
+    if zero is None:
+        call("fr_rms_quant_fp8", ptr(x2), ptr(r2), ptr(w), float(eps), ptr(q), ptr(scale), rows, hidden, stream_ptr(x.device))
+    else:
+        call("fr_rms_quant_zero_fp8", ptr(x2), ptr(r2), ptr(w), float(eps), ptr(q), ptr(scale), ptr(zero), rows, hidden,
+             stream_ptr(x.device))
     res_out = None
     if residual is not None:
         if r2.data_ptr() != residual.data_ptr():
@@ -41,8 +46,10 @@ def _launch(x, weight, eps, residual):
     return q, scale, res_out
 
 
-def rmsnorm_per_token_quant_fp8(x: torch.Tensor, weight: torch.Tensor, eps: float) -> tuple[torch.Tensor, torch.Tensor]:
-    q, scale, _ = _launch(x, weight, eps, None)
+def rmsnorm_per_token_quant_fp8(x: torch.Tensor, weight: torch.Tensor, eps: float,
+                                zero: Optional[torch.Tensor] = None) -> tuple[torch.Tensor, torch.Tensor]:
+    """``zero``: f32, one value per row, set to 0 by the same launch (``fr_rms_quant_zero_fp8``)."""
+    q, scale, _ = _launch(x, weight, eps, None, zero)
     return q, scale
 
 

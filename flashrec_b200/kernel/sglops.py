@@ -158,14 +158,15 @@ def interleave_gate_up(weight_nk: torch.Tensor, scale: torch.Tensor, block: int 
     return weight_nk.index_select(0, perm).contiguous(), scale.reshape(-1).index_select(0, perm).contiguous()
 
 
-def fp8_scaled_mm_silu_mul(a_fp8, b_interleaved_nk, scale_a, scale_b_interleaved, *, mode: int = 0):
+def fp8_scaled_mm_silu_mul(a_fp8, b_interleaved_nk, scale_a, scale_b_interleaved, *, mode: int = 0, row_amax=None):
     """gate_up GEMM with SwiGLU in the epilogue: returns ``(y bf16 [M, d], row_amax f32 [M])``,
-    bit-identical to ``silu_and_mul(fp8_scaled_mm(...))`` on the un-interleaved weight."""
+    bit-identical to ``silu_and_mul(fp8_scaled_mm(...))`` on the un-interleaved weight. ``row_amax``: zeros of a launch before
+    that become the maxima."""
     require_cuda(a_fp8, b_interleaved_nk, scale_a, scale_b_interleaved)
     m, k = int(a_fp8.shape[0]), int(a_fp8.shape[1])
     n = int(b_interleaved_nk.shape[0])
     y = torch.empty((m, n // 2), dtype=torch.bfloat16, device=a_fp8.device)
-    amax = torch.zeros(m, dtype=torch.float32, device=a_fp8.device)
+    amax = torch.zeros(m, dtype=torch.float32, device=a_fp8.device) if row_amax is None else row_amax
     sa = scale_a.reshape(-1).to(torch.float32).contiguous()
     call("fr_gemm_fp8_silu_mul", ptr(a_fp8), ptr(b_interleaved_nk), ptr(sa), ptr(scale_b_interleaved), ptr(y),
          ptr(amax), m, n, k, a_fp8.stride(0), b_interleaved_nk.stride(0), y.stride(0), int(mode),

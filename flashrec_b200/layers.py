@@ -137,10 +137,11 @@ class RMSNorm:
             return rmsnorm(x, self.weight, self.eps)
         return fused_add_rmsnorm(x, residual, self.weight, self.eps)
 
-    def quant_fp8(self, x: torch.Tensor, residual: Optional[torch.Tensor] = None):
-        """RMSNorm then per-token e4m3. With residual: fused add+norm+quant (layers/norm.py:28-42)."""
+    def quant_fp8(self, x: torch.Tensor, residual: Optional[torch.Tensor] = None, zero: Optional[torch.Tensor] = None):
+        """RMSNorm then per-token e4m3. With residual: fused add+norm+quant (layers/norm.py:28-42). ``zero`` (without
+        residual): f32 values of the rows that the launch sets to 0."""
         if residual is None:
-            return rmsnorm_per_token_quant_fp8(x, self.weight, self.eps)
+            return rmsnorm_per_token_quant_fp8(x, self.weight, self.eps, zero)
         return fused_add_rmsnorm_per_token_quant_fp8(x, residual, self.weight, self.eps)
 
 

@@ -50,6 +50,9 @@ int fr_device_status(int* status_out, int* site_out);
  * (kernel/rms_fp8.py:120-145). */
 int fr_rms_quant_fp8(const void* x, void* residual, const void* weight, float eps, void* q_out, float* scale_out,
                      int rows, int hidden, cudaStream_t stream);
+/* The same, and zero_out[row] = 0 (f32 [rows]): the row maxima that fr_gemm_fp8_silu_mul behind it raises. */
+int fr_rms_quant_zero_fp8(const void* x, void* residual, const void* weight, float eps, void* q_out, float* scale_out,
+                          float* zero_out, int rows, int hidden, cudaStream_t stream);
 
 /* bf16 RMSNorm (optionally residual += x first). y_out: bf16 [rows, hidden].
  * Reference: rmsnorm / fused_add_rmsnorm (kernel/sglops.py:34-61). */

@@ -38,6 +38,28 @@ def test_rms_quant_bit_exact(rows, hidden):
     assert r2.data_ptr() == r_dev.data_ptr()  # updated in place
 
 
+@pytest.mark.parametrize("rows,hidden", [(1, 2048), (2049, 1024), (7, 4096), (5, 384)])
+def test_rms_quant_clears_the_row_maxima_of_the_swiglu_product(rows, hidden):
+    """The norm's launch zeroes them, the product's raises them: as with maxima that start from a fill, in a row of launches too."""
+    from flashrec_b200.kernel.rms_fp8 import rmsnorm_per_token_quant_fp8
+    from flashrec_b200.kernel.sglops import fp8_scaled_mm_silu_mul
+
+    g = torch.Generator(device=DEV).manual_seed(rows)
+    x = torch.randn(rows, hidden, generator=g, device=DEV).bfloat16()
+    w = (1 + 0.1 * torch.randn(hidden, generator=g, device=DEV)).bfloat16()
+    gu = torch.randn(512, hidden, generator=g, device=DEV).to(torch.float8_e4m3fn)
+    sb = torch.rand(512, generator=g, device=DEV)
+    q, s = rmsnorm_per_token_quant_fp8(x, w, 1e-6)
+    y, amax = fp8_scaled_mm_silu_mul(q, gu, s, sb)
+    room = torch.full((rows + 2,), 7.0, device=DEV)
+    for _ in range(3):
+        q2, s2 = rmsnorm_per_token_quant_fp8(x, w, 1e-6, room[1:-1])
+        y2, amax2 = fp8_scaled_mm_silu_mul(q2, gu, s2, sb, row_amax=room[1:-1])
+    _eq_bytes(q2, q)
+    assert torch.equal(s2, s) and torch.equal(y2, y) and torch.equal(amax2, amax)
+    assert room[0] == 7.0 and room[-1] == 7.0
+
+
 def test_rms_quant_golden_reference_bytes():
     from flashrec_b200.kernel.rms_fp8 import fused_add_rmsnorm_per_token_quant_fp8, rmsnorm_per_token_quant_fp8
     from flashrec_b200.kernel.sglops import fused_add_rmsnorm, rmsnorm
