@@ -15,6 +15,7 @@ and replayed.
 from __future__ import annotations
 
 import ctypes
+import itertools
 from dataclasses import dataclass
 from typing import List, Optional, Sequence
 
@@ -457,6 +458,23 @@ class SidDecodeEngine:
             self.h_tokens.copy_(self.tok_planes[last], non_blocking=True)
             torch.cuda.current_stream(self.device).synchronize()
 
+    def _upload(self, *cols64, int32=()):
+        """Integer columns as int64 tensors (``int32``: a tuple of them as int32) on the device, each 16-byte aligned, in one copy
+        that the host does not wait for."""
+        n64, n32 = [(len(c) + 1) // 2 * 2 for c in cols64], [(len(c) + 3) // 4 * 4 for c in int32]
+        host = torch.empty(sum(n64) + sum(n32) // 2, dtype=torch.int64, pin_memory=True)
+        dev = torch.empty(host.shape, dtype=torch.int64, device=self.device)
+
+        def views(t):
+            wide, narrow = t[: sum(n64)].split(n64), t[sum(n64):].view(torch.int32).split(n32)
+            return [v[: len(c)] for v, c in zip(wide, cols64)], [v[: len(c)] for v, c in zip(narrow, int32)]
+
+        for v, c in zip(sum(views(host), []), (*cols64, *int32)):
+            v.copy_(torch.as_tensor(c))
+        dev.copy_(host, non_blocking=True)
+        wide, narrow = views(dev)
+        return *wide, narrow
+
     def prefill(self, chunk_tokens: Optional[int] = None) -> torch.Tensor:
         """Run the model over the prompts (seeded random token ids) so that the pool holds their real
         K/V instead of the synthetic fill. Request 0 computes the shared prefix, the others take it as a
@@ -478,7 +496,6 @@ class SidDecodeEngine:
         for r, plen in enumerate(self.prompt_lens):
             own = torch.randint(0, self.token_base, (plen - min(sp, plen),), generator=g)
             full_ids.append(torch.cat((shared_ids[: min(sp, plen)], own)))
-        table = self.req_to_token[self.rows:].cpu()
         chunk = int(chunk_tokens) if chunk_tokens else max(self.prompt_lens)
         if chunk <= 0:
             raise ValueError("chunk_tokens must be positive")
@@ -492,27 +509,29 @@ class SidDecodeEngine:
             reqs = [r for r in range(self.n) if done[r] < self.prompt_lens[r] and k >= first_pass[r]]
             ext = [min(chunk, self.prompt_lens[r] - done[r]) for r in reqs]
             seq_l = [done[r] + e for r, e in zip(reqs, ext)]
-            rows = self.prefill_rows[torch.tensor(reqs, dtype=torch.int64, device=dev)]
-            seq = torch.tensor(seq_l, dtype=torch.int32, device=dev)
+            # Everything the host knows of the pass goes up in one copy from pinned memory that nothing waits for, so that the
+            # host prepares a pass while the one before still runs; the new tokens' slots come from the gathered list on the device.
+            t, first = sum(ext), [0, *itertools.accumulate(seq_l)]
+            reqs_d, at, ids, positions, (seq, qo) = self._upload(
+                reqs, torch.cat([torch.arange(first[i] + done[r], first[i + 1]) for i, r in enumerate(reqs)]),
+                torch.cat([full_ids[r][done[r]: done[r] + e] for r, e in zip(reqs, ext)]),
+                torch.cat([torch.arange(done[r], done[r] + e) for r, e in zip(reqs, ext)]),
+                int32=(seq_l, [0, *itertools.accumulate(ext)]))
+            rows = self.prefill_rows[reqs_d]
             kv_indices = torch.empty(sum(seq_l), dtype=torch.int32, device=dev)
             kv_indptr = torch.empty(len(reqs) + 1, dtype=torch.int32, device=dev)
             kv_table_step(self.req_to_token, rows, seq, kv_indices, kv_indptr)  # plain gather
-            loc = torch.cat([table[r, done[r]: done[r] + e] for r, e in zip(reqs, ext)]).to(torch.int64)
-            qo = torch.zeros(len(reqs) + 1, dtype=torch.int32)
-            qo[1:] = torch.cumsum(torch.tensor(ext), 0)
             batch = ForwardBatch(
-                input_ids=torch.cat([full_ids[r][done[r]: done[r] + e] for r, e in zip(reqs, ext)]).to(dev),
-                req_pool_indices=rows, seq_lens=seq,
-                positions=torch.cat([torch.arange(done[r], done[r] + e) for r, e in zip(reqs, ext)]).to(dev),
-                out_cache_loc=loc.to(dev), is_prefill=True, kv_indices=kv_indices, kv_indptr=kv_indptr,
-                extend_prefix_lens=[done[r] for r in reqs], extend_seq_lens=ext, qo_indptr=qo.to(dev))
+                input_ids=ids, req_pool_indices=rows, seq_lens=seq, positions=positions,
+                out_cache_loc=kv_indices[at].to(torch.int64), is_prefill=True, kv_indices=kv_indices, kv_indptr=kv_indptr,
+                extend_prefix_lens=[done[r] for r in reqs], extend_seq_lens=ext, qo_indptr=qo)
             hidden = self.model.forward(batch)
             last = self.model.last_token_hidden(hidden, batch)
             for i, (r, e) in enumerate(zip(reqs, ext)):
                 done[r] += e
                 if done[r] == self.prompt_lens[r]:
                     last_hidden[r] = last[i]
-            self.prefill_tokens += int(qo[-1])
+            self.prefill_tokens += t
             k += 1
         self.prefill_passes = k
         self.prefill_hidden = last_hidden
