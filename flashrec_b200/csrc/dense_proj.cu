@@ -117,23 +117,38 @@ __device__ __forceinline__ void seg_write(const fr_out_segment& s, int64_t row, 
 // ---------------------------------------------------------------------------
 constexpr int kRowsThreads = 256;
 
-// ROWS weight rows (pointers) against MB activation rows, this warp's chunks of 256 columns
-template <typename T, int MB>
-__device__ __forceinline__ void rows_dot(const T* __restrict__ a, int64_t lda, const T* const (&w)[4], int K, int kwarp,
-                                         int ks, int M, float (&acc)[4][MB]) {
-  const int lane = threadIdx.x & 31;
-#pragma unroll 2
-  for (int k = kwarp * 256 + lane * 8; k < K; k += ks * 256) {
+// Four weight rows (pointers) against MB activation rows, this warp's chunks of 256 columns. The first P chunks of weights are loaded
+// by begin(), before griddepcontrol.wait, where the caller says that the launch ahead does not write them (FR_DENSE_LAID_OUT), so that
+// the products begin as soon as the activations are there. us per launch in a row of launches on new weights, P = 0 / chunks ahead,
+// one row: 32768 x 2048 25.6 / 23.6, 2048 x 2048 2.9 / 2.5, 8320 x 4096 14.2 / 13.1; f32 12288 x 2048 20.5 / 17.3. From three rows on
+// the registers for the weights cost more than that gave (eight rows of bf16 x 20480 x 2048 61.0 / 66.6).
+template <typename T, int MB, int P>
+struct RowsDot {
+  static constexpr int kVec = 8 * sizeof(T) / 16;  // 16-byte loads of a lane's eight columns
+  uint4 ahead[P > 0 ? P : 1][4][kVec];
+
+  static __device__ __forceinline__ void load(uint4 (&raw)[4][kVec], const T* const (&w)[4], int k) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int v = 0; v < kVec; ++v) raw[r][v] = __ldcs(reinterpret_cast<const uint4*>(w[r] + k) + v);
+  }
+  static __device__ __forceinline__ void add(const uint4 (&raw)[4][kVec], const T* __restrict__ a, int64_t lda, int k, int M,
+                                             float (&acc)[4][MB]) {
     float wv[4][8];
-    if constexpr (sizeof(T) == 2) {
-      uint4 raw[4];
 #pragma unroll
-      for (int r = 0; r < 4; ++r) raw[r] = __ldcs(reinterpret_cast<const uint4*>(w[r] + k));
+    for (int r = 0; r < 4; ++r) {
+      if constexpr (sizeof(T) == 2) {
+        unpack8(raw[r][0], wv[r]);
+      } else {
 #pragma unroll
-      for (int r = 0; r < 4; ++r) unpack8(raw[r], wv[r]);
-    } else {
-#pragma unroll
-      for (int r = 0; r < 4; ++r) load8(w[r] + k, wv[r]);
+        for (int v = 0; v < kVec; ++v) {
+          wv[r][4 * v] = __uint_as_float(raw[r][v].x);
+          wv[r][4 * v + 1] = __uint_as_float(raw[r][v].y);
+          wv[r][4 * v + 2] = __uint_as_float(raw[r][v].z);
+          wv[r][4 * v + 3] = __uint_as_float(raw[r][v].w);
+        }
+      }
     }
 #pragma unroll
     for (int m = 0; m < MB; ++m) {
@@ -145,21 +160,44 @@ __device__ __forceinline__ void rows_dot(const T* __restrict__ a, int64_t lda, c
         for (int i = 0; i < 8; ++i) acc[r][m] = fmaf(wv[r][i], av[i], acc[r][m]);
     }
   }
-}
+
+  __device__ __forceinline__ void begin(const T* const (&w)[4], int K, int kwarp, int ks) {
+#pragma unroll
+    for (int c = 0; c < P; ++c) {
+      const int k = (kwarp + c * ks) * 256 + (threadIdx.x & 31) * 8;
+      if (k < K) load(ahead[c], w, k);
+    }
+  }
+  __device__ __forceinline__ void finish(const T* __restrict__ a, int64_t lda, const T* const (&w)[4], int K, int kwarp, int ks, int M,
+                                         float (&acc)[4][MB]) {
+    const int k0 = kwarp * 256 + (threadIdx.x & 31) * 8;
+#pragma unroll
+    for (int c = 0; c < P; ++c)
+      if (k0 + c * ks * 256 < K) add(ahead[c], a, lda, k0 + c * ks * 256, M, acc);
+#pragma unroll 2
+    for (int k = k0 + P * ks * 256; k < K; k += ks * 256) {
+      uint4 raw[4][kVec];
+      load(raw, w, k);
+      add(raw, a, lda, k, M, acc);
+    }
+  }
+};
+template <typename T, bool AHEAD>
+constexpr int kRowsAhead = !AHEAD ? 0 : sizeof(T) == 2 ? 2 : 1;
 
 // Start four weight rows on their way into L2 (weights never change: this may run before griddepcontrol.wait, while
 // the previous kernel is still working).
 template <typename T>
-__device__ __forceinline__ void prefetch_rows(const T* const (&w)[4], int K, int kwarp, int ks) {
+__device__ __forceinline__ void prefetch_rows(const T* const (&w)[4], int K, int kwarp, int ks, int first) {  // columns from `first` on
   constexpr int kLine = 128 / sizeof(T);
   const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int r = 0; r < 4; ++r)
-    for (int k = (kwarp * 32 + lane) * kLine; k < K; k += ks * 32 * kLine)
+    for (int k = first + (kwarp * 32 + lane) * kLine; k < K; k += ks * 32 * kLine)
       asm volatile("prefetch.global.L2 [%0];" ::"l"(w[r] + k));
 }
 
-template <typename T, int MB>
+template <typename T, int MB, bool AHEAD>
 __global__ void __launch_bounds__(kRowsThreads)
 dense_rows_proj_kernel(const T* __restrict__ a, int64_t lda, const T* __restrict__ w, int64_t ldw, int M, int N, int K,
                        const __grid_constant__ Segs sg, int ks) {
@@ -173,6 +211,7 @@ dense_rows_proj_kernel(const T* __restrict__ a, int64_t lda, const T* __restrict
   int si = 0, c0 = 0;
   float acc[4][MB] = {};
   const T* wr[4] = {};
+  RowsDot<T, MB, kRowsAhead<T, AHEAD>> dot;
   if (live) {
     si = seg_of(sg, grp * 4);
     const fr_out_segment& s = sg.s[si];
@@ -189,11 +228,12 @@ dense_rows_proj_kernel(const T* __restrict__ a, int64_t lda, const T* __restrict
 #pragma unroll
       for (int r = 0; r < 4; ++r) wr[r] = w + static_cast<int64_t>(grp * 4 + r) * ldw;
     }
-    prefetch_rows<T>(wr, K, kwarp, ks);
+    dot.begin(wr, K, kwarp, ks);
+    prefetch_rows<T>(wr, K, kwarp, ks, kRowsAhead<T, AHEAD> * ks * 256);
   }
   ptx::griddep_wait();
   ptx::griddep_launch_dependents();
-  if (live) rows_dot<T, MB>(a, lda, wr, K, kwarp, ks, M, acc);
+  if (live) dot.finish(a, lda, wr, K, kwarp, ks, M, acc);
 #pragma unroll
   for (int r = 0; r < 4; ++r)
 #pragma unroll
@@ -222,7 +262,7 @@ dense_rows_proj_kernel(const T* __restrict__ a, int64_t lda, const T* __restrict
   }
 }
 
-template <typename T, int MB>
+template <typename T, int MB, bool AHEAD>
 __global__ void __launch_bounds__(kRowsThreads)
 dense_rows_gated_kernel(const __grid_constant__ Parts pt, float* __restrict__ x, int64_t ldx, int M, int N, T* __restrict__ copy,
                         int64_t ldc, int ks) {
@@ -237,23 +277,33 @@ dense_rows_gated_kernel(const __grid_constant__ Parts pt, float* __restrict__ x,
     for (int r = 0; r < 4; ++r)
       wr[r] = static_cast<const T*>(part.w) + static_cast<int64_t>(min(grp * 4 + r, N - 1)) * part.ldw;
   };
-  if (live) {
+  // One chunk of the last part ahead (in the models the longer one). More of them, or of two bf16 rows, cost CTAs per SM: us for one
+  // row, none / one / two and one of the first part: 2048 x (2048 + 6144) 8.3 / 7.5 / 9.4, 2048 x 6144 6.2 / 5.5 / 7.5,
+  // 4096 x 12288 24.5 / 20.0 / 19.0; two rows 9.4 / 11.0 / 10.4, 6.5 / 8.4 / 8.3, 23.0 / 22.8 / 21.9.
+  const int last = pt.n - 1;
+  constexpr int kAhead = AHEAD && (MB == 1 || sizeof(T) == 4) ? 1 : 0;
+  RowsDot<T, MB, 0> dot0;
+  RowsDot<T, MB, kAhead> dot1;
+  constexpr bool kLoop = MB > (sizeof(T) == 2 ? 2 : 4);  // see below
+  if (kLoop && live) {
     for (int p = 0; p < pt.n; ++p) {
       const T* wr[4];
       weight_rows(pt.p[p], wr);
-      prefetch_rows<T>(wr, pt.p[p].K, kwarp, ks);
+      prefetch_rows<T>(wr, pt.p[p].K, kwarp, ks, 0);
     }
+  } else if (live) {
+    const T* wr[4];
+    if (last > 0) {
+      weight_rows(pt.p[0], wr);
+      prefetch_rows<T>(wr, pt.p[0].K, kwarp, ks, 0);
+    }
+    weight_rows(pt.p[last], wr);
+    dot1.begin(wr, pt.p[last].K, kwarp, ks);
+    prefetch_rows<T>(wr, pt.p[last].K, kwarp, ks, kAhead * ks * 256);
   }
   ptx::griddep_wait();
   ptx::griddep_launch_dependents();
-  for (int p = 0; p < pt.n; ++p) {
-    const fr_gated_part& part = pt.p[p];
-    float acc[4][MB] = {};
-    if (live) {
-      const T* wr[4];
-      weight_rows(part, wr);
-      rows_dot<T, MB>(static_cast<const T*>(part.a), part.lda, wr, part.K, kwarp, ks, M, acc);
-    }
+  auto leave = [&](int p, const float (&acc)[4][MB]) {
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
@@ -261,6 +311,37 @@ dense_rows_gated_kernel(const __grid_constant__ Parts pt, float* __restrict__ x,
         const float v = warp_sum(acc[r][m]);
         if (lane == 0) red[warp][p][r * MB + m] = v;
       }
+  };
+  // Few rows: the parts one after the other, the second's loads on their way before the first's sums are joined. Many: a loop, which
+  // leaves the compiler room to keep two steps of loads in flight. us, loop / apart: one row, 2048 x 6144 8.4 / 6.2, two 9.8 / 6.5,
+  // three of f32 17.9 / 13.7; four of bf16 9.3 / 11.3, eight 18.0 / 19.8, eight of f32 x 4096 x 12288 66 / 76.
+  if constexpr (kLoop) {
+    for (int p = 0; p < pt.n; ++p) {
+      float acc[4][MB] = {};
+      if (live) {
+        const T* wr[4];
+        weight_rows(pt.p[p], wr);
+        RowsDot<T, MB, 0>().finish(static_cast<const T*>(pt.p[p].a), pt.p[p].lda, wr, pt.p[p].K, kwarp, ks, M, acc);
+      }
+      leave(p, acc);
+    }
+  } else {
+    if (last > 0) {
+      float acc[4][MB] = {};
+      const fr_gated_part& part = pt.p[0];
+      const T* wr[4];
+      weight_rows(part, wr);
+      if (live) dot0.finish(static_cast<const T*>(part.a), part.lda, wr, part.K, kwarp, ks, M, acc);
+      leave(0, acc);
+    }
+    {
+      float acc[4][MB] = {};
+      const fr_gated_part& part = pt.p[last];
+      const T* wr[4];
+      weight_rows(part, wr);
+      if (live) dot1.finish(static_cast<const T*>(part.a), part.lda, wr, part.K, kwarp, ks, M, acc);
+      leave(last, acc);
+    }
   }
   __syncthreads();
   if (!live || kwarp != 0 || lane >= 4 * MB) return;
@@ -1144,28 +1225,29 @@ static int rows_ks(int N, int K) {
 
 template <typename T>
 static int launch_rows_proj(const void* a, int64_t lda, const void* w, int64_t ldw, int M, int N, int K, const Segs& sg,
-                            cudaStream_t stream) {
+                            bool ahead, cudaStream_t stream) {
   const int ks = rows_ks(N, K);
   const int grid = ceil_div(ceil_div(N, 4), (kRowsThreads / 32) / ks);
   const T* A = static_cast<const T*>(a);
   const T* W = static_cast<const T*>(w);
-  if (M == 1) return launch_kernel(dense_rows_proj_kernel<T, 1>, grid, kRowsThreads, 0, stream, true, A, lda, W, ldw, M, N, K, sg, ks);
-  if (M == 2) return launch_kernel(dense_rows_proj_kernel<T, 2>, grid, kRowsThreads, 0, stream, true, A, lda, W, ldw, M, N, K, sg, ks);
-  if (M <= 4) return launch_kernel(dense_rows_proj_kernel<T, 4>, grid, kRowsThreads, 0, stream, true, A, lda, W, ldw, M, N, K, sg, ks);
-  return launch_kernel(dense_rows_proj_kernel<T, 8>, grid, kRowsThreads, 0, stream, true, A, lda, W, ldw, M, N, K, sg, ks);
+  auto go = [&](auto kernel) { return launch_kernel(kernel, grid, kRowsThreads, 0, stream, true, A, lda, W, ldw, M, N, K, sg, ks); };
+  if (M == 1) return ahead ? go(dense_rows_proj_kernel<T, 1, true>) : go(dense_rows_proj_kernel<T, 1, false>);
+  if (M == 2) return ahead ? go(dense_rows_proj_kernel<T, 2, true>) : go(dense_rows_proj_kernel<T, 2, false>);
+  return M <= 4 ? go(dense_rows_proj_kernel<T, 4, false>) : go(dense_rows_proj_kernel<T, 8, false>);
 }
 
 template <typename T>
-static int launch_rows_gated(const Parts& pt, float* x, int64_t ldx, int M, int N, void* copy_out, int64_t ldc, cudaStream_t stream) {
+static int launch_rows_gated(const Parts& pt, float* x, int64_t ldx, int M, int N, void* copy_out, int64_t ldc, bool ahead,
+                             cudaStream_t stream) {
   T* copy = static_cast<T*>(copy_out);
   int K = 0;
   for (int p = 0; p < pt.n; ++p) K = K > pt.p[p].K ? K : pt.p[p].K;
   const int ks = rows_ks(N, K);
   const int grid = ceil_div(ceil_div(N, 4), (kRowsThreads / 32) / ks);
-  if (M == 1) return launch_kernel(dense_rows_gated_kernel<T, 1>, grid, kRowsThreads, 0, stream, true, pt, x, ldx, M, N, copy, ldc, ks);
-  if (M == 2) return launch_kernel(dense_rows_gated_kernel<T, 2>, grid, kRowsThreads, 0, stream, true, pt, x, ldx, M, N, copy, ldc, ks);
-  if (M <= 4) return launch_kernel(dense_rows_gated_kernel<T, 4>, grid, kRowsThreads, 0, stream, true, pt, x, ldx, M, N, copy, ldc, ks);
-  return launch_kernel(dense_rows_gated_kernel<T, 8>, grid, kRowsThreads, 0, stream, true, pt, x, ldx, M, N, copy, ldc, ks);
+  auto go = [&](auto kernel) { return launch_kernel(kernel, grid, kRowsThreads, 0, stream, true, pt, x, ldx, M, N, copy, ldc, ks); };
+  if (M == 1) return ahead ? go(dense_rows_gated_kernel<T, 1, true>) : go(dense_rows_gated_kernel<T, 1, false>);
+  if (M == 2) return ahead ? go(dense_rows_gated_kernel<T, 2, true>) : go(dense_rows_gated_kernel<T, 2, false>);
+  return M <= 4 ? go(dense_rows_gated_kernel<T, 4, false>) : go(dense_rows_gated_kernel<T, 8, false>);
 }
 
 static bool operand_ok(const void* p, int64_t ld, int K) {
@@ -1233,6 +1315,12 @@ static int check_segs(const fr_out_segment* segs, int n_segs, int N, dense::Segs
   return FR_OK;
 }
 
+static bool take_laid_out(int* algo) {
+  if (*algo < 0 || (*algo & FR_DENSE_LAID_OUT) == 0) return false;
+  *algo &= ~FR_DENSE_LAID_OUT;
+  return true;
+}
+
 extern "C" int fr_dense_proj(int dtype, const void* a, int64_t lda, const void* w, int64_t ldw, int M, int N, int K,
                              const fr_out_segment* segs, int n_segs, int algo, cudaStream_t stream) {
   FR_CHECK_ARG((dtype == 0 || dtype == 1) && M >= 0 && N > 0);
@@ -1240,11 +1328,12 @@ extern "C" int fr_dense_proj(int dtype, const void* a, int64_t lda, const void* 
   FR_CHECK_ARG(dense::operand_ok(a, lda, K) && dense::operand_ok(w, ldw, K) && N % 4 == 0);
   dense::Segs sg{};
   if (check_segs(segs, n_segs, N, &sg) != FR_OK) return FR_ERR_BAD_ARG;
+  const bool ahead = take_laid_out(&algo);
   if (algo == 0) algo = dense::use_rows(dtype, M, N, K, false) ? 1 : 2;
   if (algo == 1) {
     FR_CHECK_SUPPORTED(M <= 8);
-    return dtype == 0 ? dense::launch_rows_proj<__nv_bfloat16>(a, lda, w, ldw, M, N, K, sg, stream)
-                      : dense::launch_rows_proj<float>(a, lda, w, ldw, M, N, K, sg, stream);
+    return dtype == 0 ? dense::launch_rows_proj<__nv_bfloat16>(a, lda, w, ldw, M, N, K, sg, ahead, stream)
+                      : dense::launch_rows_proj<float>(a, lda, w, ldw, M, N, K, sg, ahead, stream);
   }
   if (dtype == 1) {
     const float* A = static_cast<const float*>(a);
@@ -1327,11 +1416,12 @@ extern "C" int fr_dense_gated_add(int dtype, const fr_gated_part* parts, int n_p
     pt.p[p] = parts[p];
   }
   if (partials == nullptr) n_splits = 0;
+  const bool ahead = take_laid_out(&algo);
   if (algo == 0) algo = (M <= 8 && n_splits == 0) ? 1 : 2;
   if (algo == 1) {
     FR_CHECK_SUPPORTED(M <= 8 && n_splits == 0);
-    return dtype == 0 ? dense::launch_rows_gated<__nv_bfloat16>(pt, x, ldx, M, N, copy, ldc, stream)
-                      : dense::launch_rows_gated<float>(pt, x, ldx, M, N, copy, ldc, stream);
+    return dtype == 0 ? dense::launch_rows_gated<__nv_bfloat16>(pt, x, ldx, M, N, copy, ldc, ahead, stream)
+                      : dense::launch_rows_gated<float>(pt, x, ldx, M, N, copy, ldc, ahead, stream);
   }
   if (dtype == 1 && n_splits > 0) {
     int s0, s1;

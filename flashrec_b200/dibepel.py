@@ -198,7 +198,7 @@ class DibepelLayer:
         parts = [(o, self.o_w, g1)]
         if self.layer.ff is not None:
             parts.append((act, self.down_w, g2))
-        return gated_add(x, parts, few_rows=True)
+        return gated_add(x, parts, few_rows=True, laid_out=True)
 
 
 class DibepelForCausalLM:

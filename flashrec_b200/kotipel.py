@@ -305,7 +305,7 @@ class Mamba2Mixer(_Mixer):
         b, cc = xbc[:, m.inner:m.inner + keys], xbc[:, m.inner + keys:m.inner + 2 * keys]
         y = self.scan.forward(cc, b, xbc[:, :m.inner], dt, c.caches.state[c.run], c.batch, self.new(t, m.inner))
         o = group_norm(y, m.norm_groups, m.inner // m.norm_groups, self.norm, self.cfg.eps, self.new(t, m.inner), z, gate_first=True)
-        return Pending(gated_add(x, [(o, self.o_w, None)], few_rows=True))
+        return Pending(gated_add(x, [(o, self.o_w, None)], few_rows=True, laid_out=True))
 
 
 class KotipelLayer(_Mixer):
@@ -344,7 +344,7 @@ class KotipelLayer(_Mixer):
             act = self.new(t, self.ff_cols)
             self.gate_up(h, [act])
             copy = self.new(t, cfg.width) if self.side_embed is not None else None
-            pending = Pending(gated_add(x, [(act, self.down_w, None)], copy=copy, few_rows=True))
+            pending = Pending(gated_add(x, [(act, self.down_w, None)], copy=copy, few_rows=True, laid_out=True))
         if self.side_embed is not None:
             if self.layer.ff is None or not pending.empty:
                 copy = update_norm(x, eps, self.new(t, cfg.width), pending=pending)

@@ -80,6 +80,9 @@ class ColumnRange:
     up_bias: float = 0.0
 
 
+LAID_OUT = 16  # FR_DENSE_LAID_OUT: the weight may be read before the launch ahead on the stream has ended
+
+
 class MergedProjection:
     """All projections of one input as a single product: one weight ``[N, K]``, column ranges with their own
     epilogues (``fr_dense_proj``)."""
@@ -141,7 +144,7 @@ class MergedProjection:
             buf = torch.empty((n_splits, m, n0), dtype=torch.float32, device=a.device)
             call("fr_dense_proj_split", code, ptr(a), a.stride(0), ptr(w), w.stride(0), m, n0, k, segs, len(segs), ptr(buf), n_splits, s)
         else:
-            call("fr_dense_proj", code, ptr(a), a.stride(0), ptr(w), w.stride(0), m, n0, k, segs, len(segs), algo, s)
+            call("fr_dense_proj", code, ptr(a), a.stride(0), ptr(w), w.stride(0), m, n0, k, segs, len(segs), algo | LAID_OUT, s)
 
 
 @dataclass
@@ -153,10 +156,11 @@ class Partials:
 
 
 def gated_add(x: torch.Tensor, parts: Sequence[Tuple[torch.Tensor, torch.Tensor, Optional[torch.Tensor]]],
-              algo: int = 0, split: bool = True, copy: Optional[torch.Tensor] = None, few_rows: bool = False) -> Optional[Partials]:
+              algo: int = 0, split: bool = True, copy: Optional[torch.Tensor] = None, few_rows: bool = False,
+              laid_out: bool = False) -> Optional[Partials]:
     """``x += sum gate * (a @ w.T)`` over one or two ``(a, w, gate)`` parts; few-row products may come back as
     partials for the following ``rms_norm`` instead, with ``few_rows`` also those of up to 8 rows. ``copy`` gets the new x in
-    its own type (not with partials)."""
+    its own type (not with partials). ``laid_out``: the launch ahead on the stream does not write the weights."""
     require_cuda(x)
     m, n = int(x.shape[0]), int(x.shape[1])
     arr = (FrGatedPart * len(parts))()
@@ -172,7 +176,7 @@ def gated_add(x: torch.Tensor, parts: Sequence[Tuple[torch.Tensor, torch.Tensor,
     if n_splits > 0:
         copy = None
     call("fr_dense_gated_add", code, arr, len(parts), ptr(x), x.stride(0), m, n, ptr(buf), n_splits, ptr(copy),
-         copy.stride(0) if copy is not None else 0, algo, stream_ptr(x.device))
+         copy.stride(0) if copy is not None else 0, algo | (LAID_OUT if laid_out else 0), stream_ptr(x.device))
     return Partials(buf, n_splits) if n_splits > 0 else None
 
 

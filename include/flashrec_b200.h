@@ -548,7 +548,9 @@ struct fr_out_segment {
 
 /* z = a . w^T for one merged weight matrix, each column range leaving through its segment. a [M, K], w [N, K].
  * algo: 0 picks by shape; 1 = one warp per few weight rows (M <= 8); 2 = tcgen05 tiles (bf16), shared-memory
- * tiles (f32). */
+ * tiles (f32); | FR_DENSE_LAID_OUT: the launch ahead of this one on the stream does not write w, which may then be read before that
+ * launch has ended. */
+#define FR_DENSE_LAID_OUT 16
 int fr_dense_proj(int dtype, const void* a, int64_t lda, const void* w, int64_t ldw, int M, int N, int K,
                   const struct fr_out_segment* segs, int n_segs, int algo, cudaStream_t stream);
 
@@ -571,7 +573,7 @@ struct fr_gated_part {
  * [splits, M, N]) the K extent is split instead: partial s receives its share of the sum, x is left alone
  * and fr_lm_norm adds the partials in order. n_splits: 0 without partials; else as returned by
  * fr_dense_gated_add_splits or fr_dense_few_row_splits for the same shape. copy (or null, without partials): the new x rounded to dtype as well;
- * columns [N, ldc) are zeroed up to a multiple of 8. */
+ * columns [N, ldc) are zeroed up to a multiple of 8. algo: as for fr_dense_proj. */
 int fr_dense_gated_add(int dtype, const struct fr_gated_part* parts, int n_parts, float* x, int64_t ldx, int M, int N,
                        float* partials, int n_splits, void* copy, int64_t ldc, int algo, cudaStream_t stream);
 int fr_dense_gated_add_splits(int dtype, int M, int N, int K0, int K1);

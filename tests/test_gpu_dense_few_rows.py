@@ -179,3 +179,27 @@ def test_pairs_of_ctas(m, n, k):
     want = x.double() + gate.double() * ref + ref
     assert gated_add(x, [(a, w, gate), (a, w, None)], split=False) is None
     assert float((x.double() - want).abs().max()) < 2 * bound * float(want.abs().max())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("m,n,ks", [(1, 2056, (264, 520)), (2, 4096, (6144,)), (4, 520, (2048, 72)), (64, 2048, (2048, 6144)),
+                                    (130, 776, (1096,)), (700, 20480, (136,))])
+def test_weights_read_ahead_of_the_launch_before_keep_the_bits(dtype, m, n, ks):
+    """The activations come from a launch that ends while the product begins."""
+    from flashrec_b200.lm_layers import gated_add, rms_norm
+
+    h = [_rand(m, k, seed=k).float() for k in ks]
+    ws = [(_rand(n, k, seed=i) * k ** -0.5).to(dtype) for i, k in enumerate(ks)]
+    x0, got = torch.randn(m, n, device="cuda", generator=torch.Generator(device="cuda").manual_seed(5)), []
+    for laid_out in (True, False):
+        x = x0.clone()
+        for split in (False, True):
+            acts = [torch.empty(m, k, dtype=dtype, device="cuda") for k in ks]
+            for a, v, k in zip(acts, h, ks):
+                rms_norm(v, torch.ones(k, device="cuda"), 0.0, 1e-6, a)
+            p = gated_add(x, [(a, w, None) for a, w in zip(acts, ws)], few_rows=True, split=split, laid_out=laid_out)
+            if p is not None:
+                got.append(p.buf)
+        got.append(x)
+    for a, b in zip(got[: len(got) // 2], got[len(got) // 2:]):
+        assert torch.equal(a, b)
