@@ -62,8 +62,31 @@ __device__ __forceinline__ int64_t lower_bound(const int64_t* __restrict__ keys,
   return lo;
 }
 
+// The same with three keys in flight per round: half the rounds of latency. For threads that search alone (the winners' nodes); where
+// every thread has many to search the loads count, and lower_bound has fewer. With this, several warps to a beam and four candidates
+// in flight, a step of seven requests of 50 beams with 8192 codes a level takes 37 us instead of 135 (from full logits), one of 512
+// beams 54 instead of 58 (from records of the head's epilogue).
+__device__ __forceinline__ int64_t lower_bound_4(const int64_t* __restrict__ keys, int64_t n, int64_t key) {
+  int64_t lo = 0, hi = n;
+  while (hi - lo > 3) {
+    const int64_t step = (hi - lo) >> 2;  // lo < lo + step < lo + 2 step < lo + 3 step < hi
+    const int64_t k1 = __ldg(keys + lo + step), k2 = __ldg(keys + lo + 2 * step), k3 = __ldg(keys + lo + 3 * step);
+    if (k2 < key) {
+      if (k3 < key) lo += 3 * step + 1;
+      else { hi = lo + 3 * step; lo += 2 * step + 1; }
+    } else if (k1 < key) {
+      hi = lo + 2 * step;
+      lo += step + 1;
+    } else {
+      hi = lo + step;
+    }
+  }
+  while (lo < hi && __ldg(keys + lo) < key) ++lo;
+  return lo;
+}
+
 // The same for two keys by a whole warp: 32 places of each range at a time, so a million edges take four rounds of latency, not
-// twenty (the masks of 512 rows, 1M-item catalog: 26 -> 18 us).
+// twenty (the masks of 512 rows, 1M-item catalog: 26 -> 18 us, and 13.7 with four edges in flight).
 __device__ __forceinline__ void lower_bound_warp(const int64_t* __restrict__ keys, int64_t n, const int64_t (&key)[2], int64_t (&at)[2]) {
   const int lane = threadIdx.x & 31;
   int64_t lo[2] = {0, 0}, hi[2] = {n, n};
@@ -132,7 +155,7 @@ __device__ __forceinline__ int64_t trie_transition(const Trie& tr, int64_t old, 
   if (tr.kind == FR_TRIE_CSR) {
     if (tr.n_edges <= 0) return tr.invalid_node;
     const int64_t key = old * tr.vsz + rel;
-    const int64_t pos = lower_bound(tr.keys, tr.n_edges, key);
+    const int64_t pos = lower_bound_4(tr.keys, tr.n_edges, key);
     if (pos < tr.n_edges && __ldg(tr.keys + pos) == key) return __ldg(tr.child + pos);
     return tr.invalid_node;
   }
@@ -260,12 +283,26 @@ __device__ __forceinline__ void for_each_candidate(const StepParams& p, int n, b
     const uint2* cn = p.cand + static_cast<size_t>(n) * p.cand_cap;
     const int cnt = min(p.cand_count[n], p.cand_cap);
     const size_t row0 = static_cast<size_t>(n) * p.BW;
-    for (int i = threadIdx.x; i < cnt; i += kThreads) {
-      const uint2 rec = cn[i];
-      const uint32_t b = rec.y / static_cast<uint32_t>(p.idx_width);
-      const size_t row = row0 + b;
-      const float s = __fadd_rn(p.cum[row], __fsub_rn(__fsub_rn(__uint_as_float(rec.x), p.row_max[row]), p.row_logsum[row]));
-      if (s != p.neg_inf) f(compose(s, rec.y));
+    // four records at a time: a record's row leads to three more loads, and with one in flight per thread a pass over 62,000 records
+    // was 60 waits for two loads in a row
+    constexpr int kFlight = 4;
+    for (int i0 = threadIdx.x; i0 < cnt; i0 += kFlight * kThreads) {
+      uint2 rec[kFlight];
+      float cum[kFlight], mx[kFlight], ls[kFlight];
+#pragma unroll
+      for (int u = 0; u < kFlight; ++u) rec[u] = cn[min(i0 + u * kThreads, cnt - 1)];
+#pragma unroll
+      for (int u = 0; u < kFlight; ++u) {
+        const size_t row = row0 + rec[u].y / static_cast<uint32_t>(p.idx_width);
+        cum[u] = p.cum[row];
+        mx[u] = p.row_max[row];
+        ls[u] = p.row_logsum[row];
+      }
+#pragma unroll
+      for (int u = 0; u < kFlight; ++u) {
+        const float s = __fadd_rn(cum[u], __fsub_rn(__fsub_rn(__uint_as_float(rec[u].x), mx[u]), ls[u]));
+        if (i0 + u * kThreads < cnt && s != p.neg_inf) f(compose(s, rec[u].y));
+      }
     }
   } else if constexpr (!FULL) {
     const uint32_t M = static_cast<uint32_t>(p.BW) * p.C;
@@ -291,7 +328,9 @@ __device__ __forceinline__ void for_each_candidate(const StepParams& p, int n, b
     const Trie& tr = p.trie;
     const int64_t first_tok = p.level_tok_base + p.idx_base;  // token of this shard's local code 0
     const int64_t level_off = first_tok - tr.token_base;
-    for (int b = warp; b < p.BW; b += kThreads / 32) {
+    // fewer beams than warps (one, when a request starts from its prompt's last row): several warps to a beam
+    const int share = max(1, kThreads / 32 / p.BW), part = warp % share * 32 + lane, stride = share * 32;
+    for (int b = warp / share; b < p.BW; b += kThreads / 32 / share) {
       const size_t row = static_cast<size_t>(n) * p.BW + b;
       const float cumb = p.cum[row];
       if (cumb == p.neg_inf) continue;
@@ -302,18 +341,27 @@ __device__ __forceinline__ void for_each_candidate(const StepParams& p, int n, b
         // only the node's own edges can be legal: walk its slice of the sorted key array
         const int64_t k0 = node * tr.vsz + level_off;
         const int64_t e0 = rng[2 * b], e1 = rng[2 * b + 1];
-        for (int64_t e = e0 + lane; e < e1; e += 32) {
-          const int64_t c = __ldg(tr.keys + e) - k0;
-          const float s = __fadd_rn(cumb, __fsub_rn(__fsub_rn(lg[c], mx), ls));
-          if (s != p.neg_inf)
-            f(compose(s, static_cast<uint32_t>(static_cast<int64_t>(b) * p.idx_width + p.idx_base + c)));
+        constexpr int kFlight = 4;
+        for (int64_t e = e0 + part; e < e1; e += kFlight * stride) {
+          int64_t c[kFlight];
+          float l[kFlight];
+#pragma unroll
+          for (int u = 0; u < kFlight; ++u) c[u] = __ldg(tr.keys + min(e + u * stride, e1 - 1)) - k0;
+#pragma unroll
+          for (int u = 0; u < kFlight; ++u) l[u] = lg[c[u]];
+#pragma unroll
+          for (int u = 0; u < kFlight; ++u) {
+            const float s = __fadd_rn(cumb, __fsub_rn(__fsub_rn(l[u], mx), ls));
+            if (e + u * stride < e1 && s != p.neg_inf)
+              f(compose(s, static_cast<uint32_t>(static_cast<int64_t>(b) * p.idx_width + p.idx_base + c[u])));
+          }
         }
       } else if (tr.kind == FR_TRIE_BITMAP && node >= 0 && node < tr.n_rows) {
         // only the set bits of the node's row can be legal: walk them word by word (a node deep in
         // the trie has a handful of children among thousands of codes)
         const int64_t delta = level_off - __ldg(tr.level_off + node);  // bit index of this shard's code 0
         const uint32_t* bm = tr.bitmap + node * tr.words;
-        for (int w = lane; w < tr.words; w += 32) {
+        for (int w = part; w < tr.words; w += stride) {
           uint32_t bits = __ldg(bm + w);
           while (bits) {
             const int t = __ffs(bits) - 1;
@@ -326,7 +374,7 @@ __device__ __forceinline__ void for_each_candidate(const StepParams& p, int n, b
           }
         }
       } else {
-        for (int c = lane; c < p.C; c += 32) {
+        for (int c = part; c < p.C; c += stride) {
           if (!trie_allowed(tr, node, first_tok + c)) continue;
           const float s = __fadd_rn(cumb, __fsub_rn(__fsub_rn(lg[c], mx), ls));
           if (s != p.neg_inf)
@@ -411,8 +459,8 @@ __global__ void __launch_bounds__(kThreads, 1) beam_step_kernel(StepParams p) {
         int64_t e0 = -1, e1 = -1;
         if (node >= 0 && p.cum[row] != p.neg_inf) {
           const int64_t k0 = node * p.trie.vsz + level_off;
-          e0 = lower_bound(p.trie.keys, p.trie.n_edges, k0);
-          e1 = lower_bound(p.trie.keys, p.trie.n_edges, k0 + p.C);
+          e0 = lower_bound_4(p.trie.keys, p.trie.n_edges, k0);
+          e1 = lower_bound_4(p.trie.keys, p.trie.n_edges, k0 + p.C);
         }
         rng[2 * b] = e0;
         rng[2 * b + 1] = e1;
@@ -994,9 +1042,12 @@ __global__ void __launch_bounds__(256) row_mask_kernel(uint32_t* __restrict__ ma
     int64_t at[2];
     lower_bound_warp(tr.keys, tr.n_edges, ends, at);
     const int64_t e0 = at[0], e1 = at[1];
-    for (int64_t e = e0 + lane; e < e1; e += 32) {
-      const int64_t c = __ldg(tr.keys + e) - k0;
-      atomicOr(m + (c >> 5), 1u << (c & 31));
+    for (int64_t e = e0 + lane; e < e1; e += 128) {
+      int64_t c[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) c[u] = __ldg(tr.keys + min(e + u * 32, e1 - 1)) - k0;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) atomicOr(m + (c[u] >> 5), 1u << (c[u] & 31));  // the last edge again changes nothing
     }
     return;
   }

@@ -444,6 +444,33 @@ def test_sid_beam_step_full_width(layout, n, bw, kl):
         assert legal[live.numpy()].all()  # illegal-SID rate 0
 
 
+@pytest.mark.parametrize("layout", ["dense", "csr", "bitmap", None])
+@pytest.mark.parametrize("bw,k,level", [(1, 50, 0), (1, 700, 0), (2, 64, 1), (5, 50, 1), (12, 40, 1), (31, 100, 1), (33, 64, 1)])
+def test_sid_beam_step_of_few_beams(layout, bw, k, level):
+    """Several warps share a beam's codes, four at a time with a remainder; the winners' nodes by the search with three keys in flight."""
+    from flashrec_b200._lib import call, ptr, stream_ptr
+    from flashrec_b200.sid_decode import sid_beam_step
+    from flashrec_b200.trie import build_trie_arrays, trie_to_device
+
+    rng = np.random.default_rng(bw * 10 + level)
+    n, kl, base = 2, 517, 7000
+    items = np.stack([rng.integers(0, kl, 40000) for _ in range(3)], axis=1)
+    arrays = build_trie_arrays(items, [kl] * 3, base)
+    otr = O.OracleTrie(arrays.csr_keys, arrays.edge_child, arrays.vsz, base, arrays.invalid_node)
+    tr = trie_to_device(arrays, layout, DEV) if layout else None
+    first, past = int(arrays.level_start[level]), int(arrays.level_start[level + 1])
+    nodes = torch.from_numpy(rng.integers(first, past, (n, bw)))
+    cum = torch.from_numpy(rng.standard_normal((n, bw)).astype(np.float32))
+    logits = torch.from_numpy((3 * rng.standard_normal((n * bw, kl))).astype(np.float32))
+    lg, mx, ls = logits.to(DEV), torch.empty(n * bw, device=DEV), torch.empty(n * bw, device=DEV)
+    call("fr_logsumexp_rows", ptr(lg), lg.stride(0), ptr(mx), ptr(ls), None, 0, n * bw, kl, stream_ptr(lg.device))
+    k = min(k, bw * kl)
+    out = sid_beam_step(cum.to(DEV), lg, mx, ls, nodes.to(DEV), tr, base + kl * level, k)
+    ref = O.sid_beam_step(cum, logits, nodes, otr if layout else None, base + kl * level, k, stats=(mx.cpu(), ls.cpu()))
+    for name in ("vals", "indices", "parents", "tokens"):
+        assert torch.equal(getattr(out, name).cpu(), ref[name]), name
+
+
 def test_merge_shards_equals_unsharded():
     """Token-range sharded head: per-shard steps + merge == one unsharded step."""
     import ctypes
