@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(EpiCfg<EPI>::kThreads, 1)
 gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                 OutT* __restrict__ out, int64_t ldo, const float* __restrict__ scale_a,
                 const float* __restrict__ scale_b, const __nv_bfloat16* __restrict__ bias, int M, int N, int K,
-                unsigned int* __restrict__ row_amax, const uint16_t* __restrict__ silu_table, int* status) {
+                unsigned int* __restrict__ row_amax, const uint16_t* __restrict__ silu_table, bool ahead, int* status) {
   using C = Cfg<BLOCK_N>;
   constexpr int kEpiThreads = EpiCfg<EPI>::kEpiThreads;
   constexpr int kSplit = EpiCfg<EPI>::kWarps / 4;  // epilogue warps per lane quadrant
@@ -231,8 +231,17 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  // everything above touched only this CTA's shared / tensor memory: with a programmatic launch dependency it
-  // ran while the previous kernel of the stream was still finishing; global memory is touched from here on
+  // Everything above touched only this CTA's shared / tensor memory: with a programmatic launch dependency it
+  // ran while the previous kernel of the stream was still finishing. Weights that it does not write (FR_GEMM_LAID_OUT) fill the
+  // first tile's stages now; all other global memory is touched behind the wait. In a layer of 512 rows the launch ahead is a row
+  // kernel of 3 us beside which a CTA of this one fits, and the weights come from HBM: a wave of 84 such layers takes 7.70 ms, 7.90
+  // with the loads behind the wait.
+  const int pre = ahead && warp == 0 && static_cast<int>(blockIdx.x) < num_tiles ? min(C::kStages, num_kb) : 0;
+  for (int kb = 0; kb < pre; ++kb) {
+    ptx::mbar_expect_tx_one(bar_full + 8 * kb, C::kStageBytes);
+    ptx::tma_load_2d_one(base + kb * C::kStageBytes + C::kStageA, &tmap_b, kb * kBlockK,
+                         tile_coord(blockIdx.x, m_blocks, n_blocks).nb * BLOCK_N, bar_full + 8 * kb);
+  }
   ptx::griddep_wait();
   ptx::griddep_launch_dependents();
 
@@ -240,7 +249,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     // ------------------------------ TMA producer ---------------------------
     uint32_t stage = 0, phase = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+    int loaded = pre;  // k-blocks of this tile whose weights are on their way
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, loaded = 0) {
       const TileCoord tc = tile_coord(tile, m_blocks, n_blocks);
       const int m0 = tc.mb * kBlockM;
       const int n0 = tc.nb * BLOCK_N;
@@ -249,9 +259,11 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         if (!ok) break;
         const uint32_t sa = base + stage * C::kStageBytes;
         const uint32_t sbm = sa + C::kStageA;
-        ptx::mbar_expect_tx_one(bar_full + 8 * stage, C::kStageBytes);
+        if (kb >= loaded) {
+          ptx::mbar_expect_tx_one(bar_full + 8 * stage, C::kStageBytes);
+          ptx::tma_load_2d_one(sbm, &tmap_b, kb * kBlockK, n0, bar_full + 8 * stage);
+        }
         ptx::tma_load_2d_one(sa, &tmap_a, kb * kBlockK, m0, bar_full + 8 * stage);
-        ptx::tma_load_2d_one(sbm, &tmap_b, kb * kBlockK, n0, bar_full + 8 * stage);
         if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
       }
     }
@@ -453,7 +465,7 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                      const __grid_constant__ CUtensorMap tmap_out, const float* __restrict__ scale_a,
                      const float* __restrict__ scale_b, const __nv_bfloat16* __restrict__ bias, int M, int N, int K,
                      unsigned int* __restrict__ row_amax, const uint16_t* __restrict__ silu_table, const QkvRope rp,
-                     const HeadEpi hp, int* status) {
+                     const HeadEpi hp, bool ahead, int* status) {
   using C = PairCfg<EPI>;
   constexpr int BLOCK_N = C::kBlockN;
   constexpr int kEpiThreads = EpiCfg<EPI>::kEpiThreads;
@@ -513,14 +525,22 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
   ptx::cluster_wait();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  ptx::griddep_wait();  // see gemm_fp8_kernel
+  const int pre = ahead && warp == 0 && pair < num_tiles ? min(C::kStages, num_kb) : 0;  // see gemm_fp8_kernel
+  for (int kb = 0; kb < pre; ++kb) {
+    if (rank == 0) ptx::mbar_expect_tx_one(bar_full + 8 * kb, 2 * C::kStageBytes);
+    ptx::tma_load_2d_pair_one(base + kb * C::kStageBytes + C::kStageA, &tmap_b, kb * kBlockK,
+                              tile_coord(pair, m_blocks, n_blocks).nb * BLOCK_N + static_cast<int>(rank) * (BLOCK_N / 2),
+                              ptx::mapa(bar_full + 8 * kb, 0));
+  }
+  ptx::griddep_wait();
   ptx::griddep_launch_dependents();
 
   if (warp == 0) {
     // ------------------------------ TMA producer (both CTAs) ---------------
     uint32_t stage = 0, phase = 0;
     bool ok = true;
-    for (int tile = pair; tile < num_tiles && ok; tile += n_pairs) {
+    int loaded = pre;
+    for (int tile = pair; tile < num_tiles && ok; tile += n_pairs, loaded = 0) {
       const TileCoord tc = tile_coord(tile, m_blocks, n_blocks);
       const int m0 = tc.mb * (2 * kBlockM) + static_cast<int>(rank) * kBlockM;
       const int n0 = tc.nb * BLOCK_N + static_cast<int>(rank) * (BLOCK_N / 2);
@@ -529,9 +549,11 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         if (!ok) break;
         const uint32_t sa = base + stage * C::kStageBytes;
         const uint32_t full0 = ptx::mapa(bar_full + 8 * stage, 0);  // CTA 0 collects both CTAs' bytes
-        if (rank == 0) ptx::mbar_expect_tx_one(bar_full + 8 * stage, 2 * C::kStageBytes);
+        if (kb >= loaded) {
+          if (rank == 0) ptx::mbar_expect_tx_one(bar_full + 8 * stage, 2 * C::kStageBytes);
+          ptx::tma_load_2d_pair_one(sa + C::kStageA, &tmap_b, kb * kBlockK, n0, full0);
+        }
         ptx::tma_load_2d_pair_one(sa, &tmap_a, kb * kBlockK, m0, full0);
-        ptx::tma_load_2d_pair_one(sa + C::kStageA, &tmap_b, kb * kBlockK, n0, full0);
         if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
       }
     }
@@ -1116,7 +1138,7 @@ template <typename OutT, int EPI, int S, int TN>
 __global__ void __launch_bounds__(SplitCfg<TN>::kThreads, 1)
 gemm_fp8_splitk_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                        OutT* __restrict__ out, int64_t ldo, const float* __restrict__ scale_a,
-                       const float* __restrict__ scale_b, int M, int N, int K, int* status) {
+                       const float* __restrict__ scale_b, int M, int N, int K, bool ahead, int* status) {
   using C = SplitCfg<TN>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = ptx::smem_u32(smem_raw);
@@ -1159,7 +1181,12 @@ gemm_fp8_splitk_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  ptx::griddep_wait();  // see gemm_fp8_kernel
+  const int pre = ahead && warp == 0 ? min(C::kStages, per) : 0;  // see gemm_fp8_kernel
+  for (int i = 0; i < pre; ++i) {
+    ptx::mbar_expect_tx_one(bar_full + 8 * i, C::kStageBytes);
+    ptx::tma_load_2d_one(base + i * C::kStageBytes + C::kStageA, &tmap_b, (kb0 + i) * kBlockK, n0, bar_full + 8 * i);
+  }
+  ptx::griddep_wait();
   ptx::griddep_launch_dependents();
 
   if (warp == 0) {
@@ -1168,9 +1195,11 @@ gemm_fp8_splitk_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
       if (!ptx::mbar_wait_warp(bar_empty + 8 * stage, phase ^ 1u, abort_flag, status, 31)) break;
       const uint32_t sa = base + stage * C::kStageBytes;
       const int kx = (kb0 + i) * kBlockK;
-      ptx::mbar_expect_tx_one(bar_full + 8 * stage, C::kStageBytes);
+      if (i >= pre) {
+        ptx::mbar_expect_tx_one(bar_full + 8 * stage, C::kStageBytes);
+        ptx::tma_load_2d_one(sa + C::kStageA, &tmap_b, kx, n0, bar_full + 8 * stage);
+      }
       ptx::tma_load_2d_one(sa, &tmap_a, kx, m0, bar_full + 8 * stage);
-      ptx::tma_load_2d_one(sa + C::kStageA, &tmap_b, kx, n0, bar_full + 8 * stage);
       if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
     }
   } else if (warp == 1) {
@@ -1439,7 +1468,7 @@ static int pick_tile(int M, int N, int K, bool add) {
 
 template <int BLOCK_N, typename OutT, int EPI = 0>
 static int launch(const void* a, const void* b, const float* sa, const float* sb, const void* bias, void* out,
-                  int64_t ldo, int M, int N, int K, int64_t lda, int64_t ldb, cudaStream_t stream,
+                  int64_t ldo, int M, int N, int K, int64_t lda, int64_t ldb, bool ahead, cudaStream_t stream,
                   unsigned int* row_amax = nullptr) {
   using C = Cfg<BLOCK_N>;
   CUtensorMap ta, tb;
@@ -1465,7 +1494,7 @@ static int launch(const void* a, const void* b, const float* sa, const float* sb
   cfg.attrs = attr;
   cfg.numAttrs = fill_launch_attrs(attr, 1, use_pdl(M));
   if (cudaLaunchKernelEx(&cfg, kern, ta, tb, static_cast<OutT*>(out), ldo, sa, sb, static_cast<const __nv_bfloat16*>(bias),
-                         M, N, K, row_amax, table, status) != cudaSuccess) {
+                         M, N, K, row_amax, table, ahead, status) != cudaSuccess) {
     cudaGetLastError();
     return FR_ERR_CUDA;
   }
@@ -1474,7 +1503,7 @@ static int launch(const void* a, const void* b, const float* sa, const float* sb
 
 template <typename OutT, int EPI>
 static int launch_pair(const void* a, const void* b, const float* sa, const float* sb, const void* bias, void* out,
-                       int64_t ldo, int M, int N, int K, int64_t lda, int64_t ldb, cudaStream_t stream,
+                       int64_t ldo, int M, int N, int K, int64_t lda, int64_t ldb, bool ahead, cudaStream_t stream,
                        unsigned int* row_amax = nullptr, const QkvRope& rp = QkvRope{},
                        const HeadEpi& hp = HeadEpi{}) {
   using C = PairCfg<EPI>;
@@ -1507,7 +1536,7 @@ static int launch_pair(const void* a, const void* b, const float* sa, const floa
   cfg.attrs = attr;
   cfg.numAttrs = fill_launch_attrs(attr, 2, use_pdl(M));
   if (cudaLaunchKernelEx(&cfg, kern, ta, tb, to, sa, sb, static_cast<const __nv_bfloat16*>(bias), M, N, K, row_amax,
-                         table, rp, hp, status) != cudaSuccess) {
+                         table, rp, hp, ahead, status) != cudaSuccess) {
     cudaGetLastError();
     return FR_ERR_CUDA;
   }
@@ -1583,7 +1612,7 @@ static bool is_split_hint(int h) { return h == 1024 || h == 1024 + 128 || h == 1
 
 template <typename OutT, int EPI, int TN>
 static int launch_splitk_tn(const void* a, const void* b, const float* sa, const float* sb, void* out, int64_t ldo,
-                            int M, int N, int K, int64_t lda, int64_t ldb, int splits, cudaStream_t stream) {
+                            int M, int N, int K, int64_t lda, int64_t ldb, int splits, bool ahead, cudaStream_t stream) {
   using C = SplitCfg<TN>;
   CUtensorMap ta, tb;
   int st = make_tmap_u8(&ta, a, M, K, lda, kBlockM);
@@ -1591,7 +1620,7 @@ static int launch_splitk_tn(const void* a, const void* b, const float* sa, const
   st = make_tmap_u8(&tb, b, N, K, ldb, C::kTileN);
   if (st != FR_OK) return st;
   using Kern = void (*)(const CUtensorMap, const CUtensorMap, OutT*, int64_t, const float*, const float*, int, int, int,
-                        int*);
+                        bool, int*);
   Kern kern = nullptr;
   switch (splits) {
     case 1: kern = gemm_fp8_splitk_kernel<OutT, EPI, 1, TN>; break;
@@ -1613,7 +1642,7 @@ static int launch_splitk_tn(const void* a, const void* b, const float* sa, const
   cudaLaunchAttribute attr[2];
   cfg.attrs = attr;
   cfg.numAttrs = fill_launch_attrs(attr, splits, use_pdl(M));
-  if (cudaLaunchKernelEx(&cfg, kern, ta, tb, static_cast<OutT*>(out), ldo, sa, sb, M, N, K, status) != cudaSuccess) {
+  if (cudaLaunchKernelEx(&cfg, kern, ta, tb, static_cast<OutT*>(out), ldo, sa, sb, M, N, K, ahead, status) != cudaSuccess) {
     cudaGetLastError();
     return FR_ERR_CUDA;
   }
@@ -1622,10 +1651,10 @@ static int launch_splitk_tn(const void* a, const void* b, const float* sa, const
 
 template <typename OutT, int EPI>
 static int launch_splitk(const void* a, const void* b, const float* sa, const float* sb, void* out, int64_t ldo, int M,
-                         int N, int K, int64_t lda, int64_t ldb, SplitPlan plan, cudaStream_t stream) {
+                         int N, int K, int64_t lda, int64_t ldb, SplitPlan plan, bool ahead, cudaStream_t stream) {
   if (plan.tile_n == 128)
-    return launch_splitk_tn<OutT, EPI, 128>(a, b, sa, sb, out, ldo, M, N, K, lda, ldb, plan.splits, stream);
-  return launch_splitk_tn<OutT, EPI, 256>(a, b, sa, sb, out, ldo, M, N, K, lda, ldb, plan.splits, stream);
+    return launch_splitk_tn<OutT, EPI, 128>(a, b, sa, sb, out, ldo, M, N, K, lda, ldb, plan.splits, ahead, stream);
+  return launch_splitk_tn<OutT, EPI, 256>(a, b, sa, sb, out, ldo, M, N, K, lda, ldb, plan.splits, ahead, stream);
 }
 
 }  // namespace gemm
@@ -1633,7 +1662,7 @@ static int launch_splitk(const void* a, const void* b, const float* sa, const fl
 // The head GEMM with the SID-head epilogue (sid_head.cuh); called by fr_sid_head_topk.
 int launch_head_gemm(const void* a, const void* b, const float* sa, const float* sb, int M, int N, int K, int64_t lda,
                      int64_t ldb, const HeadEpi& hp, cudaStream_t stream) {
-  return gemm::launch_pair<float, 4>(a, b, sa, sb, nullptr, nullptr, 0, M, N, K, lda, ldb, stream, nullptr,
+  return gemm::launch_pair<float, 4>(a, b, sa, sb, nullptr, nullptr, 0, M, N, K, lda, ldb, false, stream, nullptr,
                                      gemm::QkvRope{}, hp);
 }
 
@@ -1641,11 +1670,18 @@ int launch_head_gemm(const void* a, const void* b, const float* sa, const float*
 
 using namespace fr;
 
+static bool take_laid_out(int* choice) {
+  if (*choice < 0 || (*choice & FR_GEMM_LAID_OUT) == 0) return false;
+  *choice &= ~FR_GEMM_LAID_OUT;
+  return true;
+}
+
 extern "C" int fr_gemm_fp8_w8a8(const void* a, const void* b, const float* scale_a, const float* scale_b,
                                 const void* bias, void* out, int out_is_f32, int M, int N, int K, int64_t lda,
                                 int64_t ldb, int64_t ldo, int block_n_hint, cudaStream_t stream) {
   FR_CHECK_ARG(M >= 0 && N > 0 && K > 0);
   if (M == 0) return FR_OK;
+  const bool ahead = take_laid_out(&block_n_hint);
   FR_CHECK_ARG(a && b && scale_a && scale_b && out);
   // TMA: 16-byte aligned base and row pitch; vector stores: 16-byte aligned output rows
   FR_CHECK_ARG(aligned16(a) && aligned16(b) && aligned16(out));
@@ -1656,22 +1692,22 @@ extern "C" int fr_gemm_fp8_w8a8(const void* a, const void* b, const float* scale
   if (bias == nullptr && (gemm::is_split_hint(block_n_hint) || block_n_hint == 0)) {
     const gemm::SplitPlan plan = gemm::split_plan_for_hint(block_n_hint, M, N, K);
     if (plan.splits >= 1)
-      return out_is_f32 ? gemm::launch_splitk<float, 0>(a, b, scale_a, scale_b, out, ldo, M, N, K, lda, ldb, plan,
+      return out_is_f32 ? gemm::launch_splitk<float, 0>(a, b, scale_a, scale_b, out, ldo, M, N, K, lda, ldb, plan, ahead,
                                                         stream)
                         : gemm::launch_splitk<__nv_bfloat16, 0>(a, b, scale_a, scale_b, out, ldo, M, N, K, lda, ldb,
-                                                                plan, stream);
+                                                                plan, ahead, stream);
   }
   int bn = block_n_hint;
   if (bn != 64 && bn != 128 && bn != 256 && bn != 512) bn = gemm::pick_tile(M, N, K, false);
   if (bn == 512) {
-    return out_is_f32 ? gemm::launch_pair<float, 0>(a, b, scale_a, scale_b, bias, out, ldo, M, N, K, lda, ldb, stream)
-                      : gemm::launch_pair<__nv_bfloat16, 0>(a, b, scale_a, scale_b, bias, out, ldo, M, N, K, lda, ldb,
+    return out_is_f32 ? gemm::launch_pair<float, 0>(a, b, scale_a, scale_b, bias, out, ldo, M, N, K, lda, ldb, ahead, stream)
+                      : gemm::launch_pair<__nv_bfloat16, 0>(a, b, scale_a, scale_b, bias, out, ldo, M, N, K, lda, ldb, ahead,
                                                             stream);
   }
 #define FR_GEMM_CASE(BN)                                                                                          \
   case BN:                                                                                                        \
-    return out_is_f32 ? gemm::launch<BN, float>(a, b, scale_a, scale_b, bias, out, ldo, M, N, K, lda, ldb, stream) \
-                      : gemm::launch<BN, __nv_bfloat16>(a, b, scale_a, scale_b, bias, out, ldo, M, N, K, lda, ldb, stream)
+    return out_is_f32 ? gemm::launch<BN, float>(a, b, scale_a, scale_b, bias, out, ldo, M, N, K, lda, ldb, ahead, stream) \
+                      : gemm::launch<BN, __nv_bfloat16>(a, b, scale_a, scale_b, bias, out, ldo, M, N, K, lda, ldb, ahead, stream)
   switch (bn) {
     FR_GEMM_CASE(256);
     FR_GEMM_CASE(128);
@@ -1687,15 +1723,16 @@ extern "C" int fr_gemm_fp8_silu_mul(const void* a, const void* b_interleaved, co
                                     int K, int64_t lda, int64_t ldb, int64_t ldo, int mode, cudaStream_t stream) {
   FR_CHECK_ARG(M >= 0 && N > 0 && K > 0);
   if (M == 0) return FR_OK;
+  const bool ahead = take_laid_out(&mode);
   FR_CHECK_ARG(a && b_interleaved && scale_a && scale_b_interleaved && y_out && row_amax);
   FR_CHECK_SUPPORTED(N % 256 == 0);
   FR_CHECK_ARG(aligned16(a) && aligned16(b_interleaved) && aligned16(y_out) && aligned16(scale_b_interleaved));
   FR_CHECK_ARG(lda >= K && ldb >= K && ldo >= N / 2 && lda % 16 == 0 && ldb % 16 == 0 && ldo % 8 == 0 && K % 16 == 0);
   if (mode == 2 || (mode == 0 && gemm::use_pair(M, N)))
     return gemm::launch_pair<__nv_bfloat16, 1>(a, b_interleaved, scale_a, scale_b_interleaved, nullptr, y_out, ldo, M,
-                                               N, K, lda, ldb, stream, reinterpret_cast<unsigned int*>(row_amax));
+                                               N, K, lda, ldb, ahead, stream, reinterpret_cast<unsigned int*>(row_amax));
   return gemm::launch<256, __nv_bfloat16, 1>(a, b_interleaved, scale_a, scale_b_interleaved, nullptr, y_out, ldo, M, N,
-                                             K, lda, ldb, stream, reinterpret_cast<unsigned int*>(row_amax));
+                                             K, lda, ldb, ahead, stream, reinterpret_cast<unsigned int*>(row_amax));
 }
 
 extern "C" int fr_gemm_fp8_w8a8_add(const void* a, const void* b, const float* scale_a, const float* scale_b,
@@ -1703,30 +1740,31 @@ extern "C" int fr_gemm_fp8_w8a8_add(const void* a, const void* b, const float* s
                                     int block_n_hint, cudaStream_t stream) {
   FR_CHECK_ARG(M >= 0 && N > 0 && K > 0);
   if (M == 0) return FR_OK;
+  const bool ahead = take_laid_out(&block_n_hint);
   FR_CHECK_ARG(a && b && scale_a && scale_b && residual_inout);
   FR_CHECK_ARG(aligned16(a) && aligned16(b) && aligned16(residual_inout));
   FR_CHECK_ARG(lda >= K && ldb >= K && ldr >= N && lda % 16 == 0 && ldb % 16 == 0 && ldr % 8 == 0 && K % 16 == 0);
   if (gemm::is_split_hint(block_n_hint) || block_n_hint == 0) {
     const gemm::SplitPlan plan = gemm::split_plan_for_hint(block_n_hint, M, N, K);
     if (plan.splits >= 1)
-      return gemm::launch_splitk<__nv_bfloat16, 2>(a, b, scale_a, scale_b, residual_inout, ldr, M, N, K, lda, ldb, plan,
+      return gemm::launch_splitk<__nv_bfloat16, 2>(a, b, scale_a, scale_b, residual_inout, ldr, M, N, K, lda, ldb, plan, ahead,
                                                    stream);
   }
   int bn = block_n_hint;
   if (bn != 64 && bn != 128 && bn != 256 && bn != 512) bn = gemm::pick_tile(M, N, K, true);
   if (bn == 512)
-    return gemm::launch_pair<__nv_bfloat16, 2>(a, b, scale_a, scale_b, nullptr, residual_inout, ldr, M, N, K, lda, ldb,
+    return gemm::launch_pair<__nv_bfloat16, 2>(a, b, scale_a, scale_b, nullptr, residual_inout, ldr, M, N, K, lda, ldb, ahead,
                                                stream);
   switch (bn) {
     case 256:
       return gemm::launch<256, __nv_bfloat16, 2>(a, b, scale_a, scale_b, nullptr, residual_inout, ldr, M, N, K, lda,
-                                                 ldb, stream);
+                                                 ldb, ahead, stream);
     case 128:
       return gemm::launch<128, __nv_bfloat16, 2>(a, b, scale_a, scale_b, nullptr, residual_inout, ldr, M, N, K, lda,
-                                                 ldb, stream);
+                                                 ldb, ahead, stream);
     case 64:
       return gemm::launch<64, __nv_bfloat16, 2>(a, b, scale_a, scale_b, nullptr, residual_inout, ldr, M, N, K, lda,
-                                                ldb, stream);
+                                                ldb, ahead, stream);
     default: break;
   }
   return FR_ERR_UNSUPPORTED;
@@ -1771,6 +1809,6 @@ extern "C" int fr_gemm_fp8_qkv_rope(const void* a, const void* b, const float* s
              reinterpret_cast<uintptr_t>(k_cache) % 32 == 0 && reinterpret_cast<uintptr_t>(v_cache) % 32 == 0 &&
              ck_s % 32 == 0 && ck_h % 32 == 0 && cv_s % 32 == 0 && cv_h % 32 == 0) ? 1 : 0;
   // the output tensor map of the launcher is not used by this epilogue; q_out gives it a valid target
-  return gemm::launch_pair<__nv_bfloat16, 3>(a, b, scale_a, scale_b, nullptr, q_out, ldq, M, N, K, lda, ldb, stream,
+  return gemm::launch_pair<__nv_bfloat16, 3>(a, b, scale_a, scale_b, nullptr, q_out, ldq, M, N, K, lda, ldb, false, stream,
                                              nullptr, rp);
 }

@@ -54,9 +54,9 @@ class Qwen3Attention:
         self.fuse_rope_gemm = False
         self.fuse_rope_min_rows = 2048
 
-    def forward(self, x, batch: ForwardBatch, *, q_fp8, a_scale, residual_inout=None) -> torch.Tensor:
+    def forward(self, x, batch: ForwardBatch, *, q_fp8, a_scale, residual_inout=None, laid_out: bool = False) -> torch.Tensor:
         """``residual_inout``: the o_proj GEMM adds its output to this bf16 residual stream in place
-        (and returns it) instead of returning the projection."""
+        (and returns it) instead of returning the projection. ``laid_out``: the launch ahead does not write the qkv weight."""
         t = int(q_fp8.shape[0])
         pool = self.attn.kv_pool
         # (worth it from a few thousand rows on; below that the two separate kernels are faster)
@@ -70,9 +70,9 @@ class Qwen3Attention:
             o = self.attn.forward(q, None, None, self.layer_id, batch, skip_store=True)
             if residual_inout is not None:
                 o_fp8, o_scale = per_token_quant_fp8(o.reshape(t, -1))
-                return self.o_proj.forward_fp8_add_(o_fp8, o_scale, residual_inout)
+                return self.o_proj.forward_fp8_add_(o_fp8, o_scale, residual_inout, laid_out=True)
             return self.o_proj(o.reshape(t, -1))
-        qkv = self.qkv_proj.forward_fp8(q_fp8, a_scale, (t, self.qkv_proj.in_features), torch.bfloat16)
+        qkv = self.qkv_proj.forward_fp8(q_fp8, a_scale, (t, self.qkv_proj.in_features), torch.bfloat16, laid_out)
         heads = qkv.view(t, self.num_qo + 2 * self.num_kv, self.head_dim)
         q = heads[:, : self.num_qo]
         k = heads[:, self.num_qo : self.num_qo + self.num_kv]
@@ -85,7 +85,7 @@ class Qwen3Attention:
         o = self.attn.forward(q, k, v, self.layer_id, batch, skip_store=True)
         if residual_inout is not None:
             o_fp8, o_scale = per_token_quant_fp8(o.reshape(t, -1))
-            return self.o_proj.forward_fp8_add_(o_fp8, o_scale, residual_inout)
+            return self.o_proj.forward_fp8_add_(o_fp8, o_scale, residual_inout, laid_out=True)
         return self.o_proj(o.reshape(t, -1))
 
 
@@ -112,18 +112,19 @@ class Qwen3MLP:
             self.gate_up_proj._fp8_weight = None
             self.gate_up_proj._fp8_scale = None
 
-    def forward(self, x, *, q_fp8, a_scale, residual_inout=None, row_amax=None) -> torch.Tensor:
+    def forward(self, x, *, q_fp8, a_scale, residual_inout=None, row_amax=None, laid_out: bool = False) -> torch.Tensor:
         """``residual_inout``: the down_proj GEMM adds its output to this bf16 residual stream in
-        place (and returns it) instead of returning the projection. ``row_amax``: zeros for the SwiGLU epilogue's maxima."""
+        place (and returns it) instead of returning the projection. ``row_amax``: zeros for the SwiGLU epilogue's maxima.
+        ``laid_out``: the launch ahead does not write the gate_up weight."""
         rows = int(q_fp8.shape[0])
         if self.fuse_silu_gemm and self._gu_w is not None:
-            y, amax = fp8_scaled_mm_silu_mul(q_fp8, self._gu_w, a_scale, self._gu_s, row_amax=row_amax)
+            y, amax = fp8_scaled_mm_silu_mul(q_fp8, self._gu_w, a_scale, self._gu_s, row_amax=row_amax, laid_out=laid_out)
             y_fp8, y_scale = quant_known_amax_fp8(y, amax)
         else:
             gu = self.gate_up_proj.forward_fp8(q_fp8, a_scale, (rows, self.gate_up_proj.in_features), torch.bfloat16)
             y_fp8, y_scale = silu_and_mul_per_token_quant_fp8(gu)
         if residual_inout is not None:
-            return self.down_proj.forward_fp8_add_(y_fp8, y_scale, residual_inout)
+            return self.down_proj.forward_fp8_add_(y_fp8, y_scale, residual_inout, laid_out=True)
         return self.down_proj.forward_fp8(y_fp8, y_scale, (rows, self.down_proj.in_features), torch.bfloat16)
 
 
@@ -140,10 +141,10 @@ class Qwen3DecoderLayer:
         and on exit, is updated in place, and each norm reads it without an add. Bit-identical
         to ``forward`` (the GEMM output is rounded to bf16 before the bf16 add in both)."""
         q_fp8, a_scale = self.input_layernorm.quant_fp8(residual)
-        self.self_attn.forward(None, batch, q_fp8=q_fp8, a_scale=a_scale, residual_inout=residual)
+        self.self_attn.forward(None, batch, q_fp8=q_fp8, a_scale=a_scale, residual_inout=residual, laid_out=True)
         row_amax = torch.empty(residual.shape[0], dtype=torch.float32, device=residual.device)
         q_fp8, a_scale = self.post_attention_layernorm.quant_fp8(residual, zero=row_amax)
-        self.mlp.forward(None, q_fp8=q_fp8, a_scale=a_scale, residual_inout=residual, row_amax=row_amax)
+        self.mlp.forward(None, q_fp8=q_fp8, a_scale=a_scale, residual_inout=residual, row_amax=row_amax, laid_out=True)
         return residual
 
     def forward(self, x, residual, batch: ForwardBatch):

@@ -14,6 +14,7 @@ from flashrec_b200 import _lib
 from flashrec_b200._lib import call, ptr, require_cuda, stream_ptr
 
 _FP8 = torch.float8_e4m3fn
+_LAID_OUT = 65536  # FR_GEMM_LAID_OUT
 
 
 def _rows2d(x: torch.Tensor, hidden: int) -> torch.Tensor:
@@ -84,10 +85,12 @@ def fp8_scaled_mm(
     bias: Optional[torch.Tensor] = None,
     *,
     block_n: int = 0,
+    laid_out: bool = False,
 ) -> torch.Tensor:
     """a: [M,K] e4m3 row-major, b: [K,N] e4m3 column-major (the ``.t()`` view of an
     [N,K] weight), scale_a: [M,1] or [M], scale_b: [N] (kernel/sglops.py:99-140).
-    ``out_dtype`` is bfloat16, or float32 (no bias) for the lm_head logits."""
+    ``out_dtype`` is bfloat16, or float32 (no bias) for the lm_head logits. ``laid_out``: the launch ahead on the stream does
+    not write ``b_fp8``, which may then be read before that launch has ended."""
     require_cuda(a_fp8, b_fp8, scale_a, scale_b, bias)
     if a_fp8.dtype != _FP8 or b_fp8.dtype != _FP8:
         raise TypeError("fp8_scaled_mm: operands must be float8_e4m3fn")
@@ -115,13 +118,13 @@ def fp8_scaled_mm(
         bias_c = bias.to(dtype=torch.bfloat16).contiguous()
     out = torch.empty((m, n), dtype=out_dtype, device=a.device)
     call("fr_gemm_fp8_w8a8", ptr(a), ptr(b_fp8), ptr(sa), ptr(sb), ptr(bias_c), ptr(out),
-         int(out_dtype == torch.float32), m, n, k, a.stride(0), b_fp8.stride(1), out.stride(0), int(block_n),
+         int(out_dtype == torch.float32), m, n, k, a.stride(0), b_fp8.stride(1), out.stride(0), int(block_n) | (_LAID_OUT if laid_out else 0),
          stream_ptr(a.device))
     return out
 
 
 def fp8_scaled_mm_add_(a_fp8: torch.Tensor, b_fp8: torch.Tensor, scale_a: torch.Tensor, scale_b: torch.Tensor,
-                       residual: torch.Tensor, block_n: int = 0) -> torch.Tensor:
+                       residual: torch.Tensor, block_n: int = 0, laid_out: bool = False) -> torch.Tensor:
     """``residual += fp8_scaled_mm(a, b, ..., bf16)`` in place, with the reference's roundings (the
     GEMM output rounded to bf16, then the bf16 sum): the add half of ``fused_add_rmsnorm`` that
     follows the o_proj / down_proj GEMMs (models/qwen3.py:205-214) folded into the GEMM epilogue.
@@ -140,7 +143,7 @@ def fp8_scaled_mm_add_(a_fp8: torch.Tensor, b_fp8: torch.Tensor, scale_a: torch.
     if sa.numel() != m or sb.numel() != n:
         raise ValueError("fp8_scaled_mm_add_: scale shapes do not match [M] / [N]")
     call("fr_gemm_fp8_w8a8_add", ptr(a), ptr(b_fp8), ptr(sa), ptr(sb), ptr(residual), m, n, k, a.stride(0),
-         b_fp8.stride(1), residual.stride(0), int(block_n), stream_ptr(a.device))
+         b_fp8.stride(1), residual.stride(0), int(block_n) | (_LAID_OUT if laid_out else 0), stream_ptr(a.device))
     return residual
 
 
@@ -158,7 +161,8 @@ def interleave_gate_up(weight_nk: torch.Tensor, scale: torch.Tensor, block: int 
     return weight_nk.index_select(0, perm).contiguous(), scale.reshape(-1).index_select(0, perm).contiguous()
 
 
-def fp8_scaled_mm_silu_mul(a_fp8, b_interleaved_nk, scale_a, scale_b_interleaved, *, mode: int = 0, row_amax=None):
+def fp8_scaled_mm_silu_mul(a_fp8, b_interleaved_nk, scale_a, scale_b_interleaved, *, mode: int = 0, row_amax=None,
+                           laid_out: bool = False):
     """gate_up GEMM with SwiGLU in the epilogue: returns ``(y bf16 [M, d], row_amax f32 [M])``,
     bit-identical to ``silu_and_mul(fp8_scaled_mm(...))`` on the un-interleaved weight. ``row_amax``: zeros of a launch before
     that become the maxima."""
@@ -169,7 +173,7 @@ def fp8_scaled_mm_silu_mul(a_fp8, b_interleaved_nk, scale_a, scale_b_interleaved
     amax = torch.zeros(m, dtype=torch.float32, device=a_fp8.device) if row_amax is None else row_amax
     sa = scale_a.reshape(-1).to(torch.float32).contiguous()
     call("fr_gemm_fp8_silu_mul", ptr(a_fp8), ptr(b_interleaved_nk), ptr(sa), ptr(scale_b_interleaved), ptr(y),
-         ptr(amax), m, n, k, a_fp8.stride(0), b_interleaved_nk.stride(0), y.stride(0), int(mode),
+         ptr(amax), m, n, k, a_fp8.stride(0), b_interleaved_nk.stride(0), y.stride(0), int(mode) | (_LAID_OUT if laid_out else 0),
          stream_ptr(a_fp8.device))
     return y, amax
 

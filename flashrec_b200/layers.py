@@ -101,23 +101,24 @@ class Linear:
         out_dtype = x.dtype if x.dtype == torch.bfloat16 else torch.bfloat16
         return self._fp8_mm(q, a_scale, orig, out_dtype)
 
-    def forward_fp8(self, q: torch.Tensor, a_scale: torch.Tensor, orig_shape: tuple, out_dtype: torch.dtype):
-        """GEMM from a pre-quantised activation. ``q`` is [M, K] e4m3 (layers/linear.py:134-142)."""
-        return self._fp8_mm(q, a_scale, orig_shape, out_dtype)
+    def forward_fp8(self, q: torch.Tensor, a_scale: torch.Tensor, orig_shape: tuple, out_dtype: torch.dtype, laid_out: bool = False):
+        """GEMM from a pre-quantised activation. ``q`` is [M, K] e4m3 (layers/linear.py:134-142). ``laid_out``: the launch ahead
+        on the stream does not write the weight."""
+        return self._fp8_mm(q, a_scale, orig_shape, out_dtype, laid_out)
 
-    def forward_fp8_add_(self, q: torch.Tensor, a_scale: torch.Tensor, residual: torch.Tensor) -> torch.Tensor:
+    def forward_fp8_add_(self, q: torch.Tensor, a_scale: torch.Tensor, residual: torch.Tensor, laid_out: bool = False) -> torch.Tensor:
         """``residual += self(q)`` in place on the bf16 residual stream [M, out_features] (bias-free layers)."""
         if not self._use_fp8:
             raise RuntimeError("Linear.load() has not been called")
         if self.bias is not None:
             raise RuntimeError("forward_fp8_add_: layers with a bias are not supported")
-        return fp8_scaled_mm_add_(q, self._fp8_weight, a_scale, self._fp8_scale, residual)
+        return fp8_scaled_mm_add_(q, self._fp8_weight, a_scale, self._fp8_scale, residual, laid_out=laid_out)
 
-    def _fp8_mm(self, q, a_scale, orig_shape, out_dtype):
+    def _fp8_mm(self, q, a_scale, orig_shape, out_dtype, laid_out=False):
         if not self._use_fp8:
             raise RuntimeError("Linear.load() has not been called")
         bias = self.bias.to(dtype=out_dtype) if self.bias is not None else None
-        out = fp8_scaled_mm(q, self._fp8_weight, a_scale, self._fp8_scale, out_dtype, bias)
+        out = fp8_scaled_mm(q, self._fp8_weight, a_scale, self._fp8_scale, out_dtype, bias, laid_out=laid_out)
         return out.view(*orig_shape[:-1], self.out_features)
 
 

@@ -93,9 +93,12 @@ int fr_silu_mul_bf16(const void* x, void* y_out, int rows, int d, cudaStream_t s
  * 512 = CTA pairs (cluster of 2, tcgen05 cta_group::2) on 256 x 256 tiles,
  * 1024 = split-K over a cluster of up to 8 CTAs per 128 x 256 or 128 x 128 tile (few rows, long K; no bias;
  * the tile width is chosen per shape, 1024 + 128 / 1024 + 256 name it).
+ * | FR_GEMM_LAID_OUT (also to the hint or mode of the two calls below that have one): the launch ahead of this
+ * one on the stream does not write b, which may then be read before that launch has ended.
  * Reports FR_ERR_TIMEOUT through fr_device_status if a pipeline wait gives up.
  * Reference: Linear.forward_fp8 -> fp8_scaled_mm (layers/linear.py:134-172,
  * kernel/sglops.py:99-140). */
+#define FR_GEMM_LAID_OUT 65536
 int fr_gemm_fp8_w8a8(const void* a, const void* b, const float* scale_a, const float* scale_b, const void* bias,
                      void* out, int out_is_f32, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldo,
                      int block_n_hint, cudaStream_t stream);

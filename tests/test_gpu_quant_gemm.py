@@ -471,3 +471,34 @@ def test_few_row_gemms_equal_across_tilings(m, n, k):
         r = res.to(DEV).clone()
         fp8_scaled_mm_add_(q, wq.t(), s, ws, r, block_n=hint)
         assert torch.equal(r, want), hint
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 256, 128), (130, 520, 336), (512, 2048, 6144), (700, 4096, 2048)])
+def test_weights_loaded_ahead_of_the_launch_before_keep_the_bits(m, n, k):
+    """Every tiling, K below and above what the stages hold, behind a quantiser that ends while the product begins."""
+    from flashrec_b200.kernel.sglops import fp8_scaled_mm, fp8_scaled_mm_add_, fp8_scaled_mm_silu_mul, per_token_quant_fp8
+
+    g = torch.Generator(device=DEV).manual_seed(m + k)
+    x = torch.randn(m, k, generator=g, device=DEV).bfloat16()
+    w = torch.randn(n, k, generator=g, device=DEV).to(torch.float8_e4m3fn)
+    sb = torch.rand(n, generator=g, device=DEV)
+    res = torch.randn(m, n, generator=g, device=DEV).bfloat16()
+
+    def products(laid_out):
+        outs = []
+        for block_n in (0, 64, 128, 256, 512, 1024, 1024 + 128, 1024 + 256):
+            q, s = per_token_quant_fp8(x)
+            outs.append(fp8_scaled_mm(q, w.t(), s, sb, torch.bfloat16, block_n=block_n, laid_out=laid_out))
+            q, s = per_token_quant_fp8(x)
+            outs.append(fp8_scaled_mm(q, w.t(), s, sb, torch.float32, block_n=block_n, laid_out=laid_out))
+            r = res.clone()
+            q, s = per_token_quant_fp8(x)
+            outs.append(fp8_scaled_mm_add_(q, w.t(), s, sb, r, block_n, laid_out=laid_out))
+        if n % 256 == 0:
+            for mode in (0, 1, 2):
+                q, s = per_token_quant_fp8(x)
+                outs += fp8_scaled_mm_silu_mul(q, w, s, sb, mode=mode, laid_out=laid_out)
+        return outs
+
+    for a, b in zip(products(True), products(False)):
+        assert torch.equal(a, b)
