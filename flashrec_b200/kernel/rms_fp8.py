@@ -31,6 +31,8 @@ def _launch(x, weight, eps, residual, zero=None):
             r2 = r2.contiguous()
     q = torch.empty((rows, hidden), dtype=_FP8, device=x.device)
     scale = torch.empty((rows, 1), dtype=torch.float32, device=x.device)
+    if zero is not None and (zero.dtype != torch.float32 or zero.numel() != rows or not zero.is_contiguous() or zero.device != x.device):
+        raise ValueError(f"rms_fp8: zero must be {rows} contiguous float32 values on {x.device}")
     if zero is None:
         call("fr_rms_quant_fp8", ptr(x2), ptr(r2), ptr(w), float(eps), ptr(q), ptr(scale), rows, hidden, stream_ptr(x.device))
     else:

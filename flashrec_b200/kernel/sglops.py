@@ -170,6 +170,9 @@ def fp8_scaled_mm_silu_mul(a_fp8, b_interleaved_nk, scale_a, scale_b_interleaved
     m, k = int(a_fp8.shape[0]), int(a_fp8.shape[1])
     n = int(b_interleaved_nk.shape[0])
     y = torch.empty((m, n // 2), dtype=torch.bfloat16, device=a_fp8.device)
+    if row_amax is not None and (row_amax.dtype != torch.float32 or row_amax.numel() != m or not row_amax.is_contiguous()
+                                 or row_amax.device != a_fp8.device):
+        raise ValueError(f"fp8_scaled_mm_silu_mul: row_amax must be {m} contiguous float32 values on {a_fp8.device}")
     amax = torch.zeros(m, dtype=torch.float32, device=a_fp8.device) if row_amax is None else row_amax
     sa = scale_a.reshape(-1).to(torch.float32).contiguous()
     call("fr_gemm_fp8_silu_mul", ptr(a_fp8), ptr(b_interleaved_nk), ptr(sa), ptr(scale_b_interleaved), ptr(y),

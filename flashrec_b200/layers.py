@@ -143,6 +143,8 @@ class RMSNorm:
         residual): f32 values of the rows that the launch sets to 0."""
         if residual is None:
             return rmsnorm_per_token_quant_fp8(x, self.weight, self.eps, zero)
+        if zero is not None:
+            raise ValueError("RMSNorm.quant_fp8: zero goes with a norm without residual")
         return fused_add_rmsnorm_per_token_quant_fp8(x, residual, self.weight, self.eps)
 
 

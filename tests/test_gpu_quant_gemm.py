@@ -58,6 +58,13 @@ def test_rms_quant_clears_the_row_maxima_of_the_swiglu_product(rows, hidden):
     _eq_bytes(q2, q)
     assert torch.equal(s2, s) and torch.equal(y2, y) and torch.equal(amax2, amax)
     assert room[0] == 7.0 and room[-1] == 7.0
+    for bad in (room, room[1:-1].double(), room.expand(rows, -1)[:, 0]):
+        if bad.numel() == rows and bad.dtype == torch.float32 and bad.is_contiguous():
+            continue
+        with pytest.raises(ValueError):
+            rmsnorm_per_token_quant_fp8(x, w, 1e-6, bad)
+        with pytest.raises(ValueError):
+            fp8_scaled_mm_silu_mul(q, gu, s, sb, row_amax=bad)
 
 
 def test_rms_quant_golden_reference_bytes():
