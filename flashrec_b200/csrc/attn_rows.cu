@@ -392,6 +392,10 @@ talk_rows_kernel(const __grid_constant__ fr_mix_attn a, int row0, int max_keys, 
   const int64_t t = row0 + static_cast<int64_t>(blockIdx.y);
   Place at;
   auto begin = [&] {
+    for (int e = tid; e < a.heads * REP; e += W * 32) {  // coefficient of source s in output o of this kv head
+      const int s = e / REP, o = e % REP;
+      cf[e] = o < rep ? a.coef[static_cast<int64_t>(g * rep + o) * a.heads + s] : 0.f;
+    }
     at = place_of(a, t, max_keys);
     for (int k0 = warp * 32, b = 0; k0 < at.n; k0 += W * 32, ++b) {
       const int x = slot_at(a, at, min(k0 + lane, at.n - 1));
@@ -402,10 +406,6 @@ talk_rows_kernel(const __grid_constant__ fr_mix_attn a, int row0, int max_keys, 
       }
     }
   };
-  for (int e = tid; e < a.heads * REP; e += W * 32) {  // coefficient of source s in output o of this kv head
-    const int s = e / REP, o = e % REP;
-    cf[e] = o < rep ? a.coef[static_cast<int64_t>(g * rep + o) * a.heads + s] : 0.f;
-  }
   if (early) begin();
   ptx::griddep_wait();
   ptx::griddep_launch_dependents();

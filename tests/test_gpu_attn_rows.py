@@ -152,3 +152,59 @@ def test_reads_before_the_launch_ahead_has_ended(kind, heads, kv, dim, vdim, len
 
     monkeypatch.setattr(lm_layers, "call", early)
     assert torch.equal(_run(kind, torch.bfloat16, heads, kv, dim, vdim, lens, 200, 0, 11), ref)
+
+
+def _decode(kind, heads, kv, dim, vdim, lens):
+    """A bound attention and a batch of one query per request, at the last of its ``lens`` tokens; pages lie one after the other."""
+    from flashrec_b200.core import ForwardBatch
+    from flashrec_b200.kvcache import CacheSpec
+    from flashrec_b200.lm_layers import MixAttention
+
+    n, pages = len(lens), [(m + PAGE - 1) // PAGE for m in lens]
+    table, at = torch.zeros((n + 1, max(pages) * PAGE), dtype=torch.int32), 0
+    for r, p in enumerate(pages):
+        table[r + 1, :p * PAGE] = torch.arange(at, at + p * PAGE)
+        at += p * PAGE
+    attn = MixAttention(kind, heads, kv, dim, vdim, dim ** -0.5, CacheSpec(0, 0, size=4096), eps=1e-5, lam=0.4, out_scale=0.8,
+                        coef=torch.zeros(heads, heads) if kind == "talk" else None)
+    attn.bind("cuda")
+    pos = torch.tensor([m - 1 for m in lens])
+    b = ForwardBatch(input_ids=None, req_pool_indices=torch.arange(1, n + 1).cuda(), seq_lens=None, positions=pos.cuda(),
+                     out_cache_loc=table[torch.arange(1, n + 1), pos].long().cuda(),
+                     tok_req=torch.arange(n, dtype=torch.int32).cuda(), n_row_tokens=n, max_pos=max(lens) - 1)
+    return attn, table.cuda(), b, at
+
+
+def _behind_each_other(step, inputs):
+    """``step`` over the inputs, queued behind a sleep, so that the GPU meets the launches without gaps."""
+    torch.cuda._sleep(20_000_000)
+    return [step(x) for x in inputs]
+
+
+@pytest.mark.parametrize("heads,kv,lens", [(8, 4, (300,)), (8, 8, (700, 33)), (16, 8, tuple(range(20, 420, 10)))])
+def test_coefficients_of_the_launch_ahead(heads, kv, lens):
+    """The mixing matrix comes from a product that lets its dependents start at its own beginning: the plain entry sees all of it."""
+    from flashrec_b200.lm_layers import MergedProjection
+
+    n, dim, depth = len(lens), 64, 8192
+    attn, table, b, slots = _decode("talk", heads, kv, dim, dim, lens)
+    g = torch.Generator(device="cuda").manual_seed(heads)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()  # noqa: E731
+    q, k, v = rnd(n, heads * dim), rnd(slots, kv * dim), rnd(slots, kv * dim)
+    proj = MergedProjection(depth)
+    proj.add("store_f32", rnd(heads, depth) * depth ** -0.5)
+    proj.finish(torch.bfloat16, "cuda")
+    torch.cuda.synchronize()
+    counters, inputs = torch.zeros(4096, dtype=torch.int32, device="cuda"), [rnd(heads, depth) for _ in range(24)]
+
+    def step(x, wait=False):
+        proj(x, [attn.coef])
+        if wait:
+            torch.cuda.synchronize()
+        return attn.forward(q, k, v, table, b, counters)
+
+    want = [step(x, wait=True) for x in inputs]
+    assert not torch.equal(want[0], want[1])
+    for _ in range(3):
+        for got, ref in zip(_behind_each_other(step, inputs), want):
+            assert torch.equal(got, ref)
