@@ -188,7 +188,7 @@ class DibepelLayer:
         if self.layer.ff is not None:
             act = outs[self.seg_ff] = new(self.ff_cols)
             g2 = outs[self.seg_g2] = new(cfg.width)
-        self.proj(h, outs, maps)
+        self.proj(h, outs, maps, laid_out=True)
         if self.conv_w is not None:
             q = new(self.attn.q_cols)
             nq, nk = self.attn.q_cols, self.spec.k_cols
@@ -254,7 +254,7 @@ class DibepelForCausalLM:
         h = torch.empty((n, ceil_to(self.cfg.width, 8)), dtype=self.dtype, device=self.device)
         rms_norm(x, self.final_norm, 1.0, self.cfg.eps, h, partials, rows)
         out = torch.empty((n, self.cfg.vocab), dtype=torch.float32, device=self.device)
-        self.head(h, [out])
+        self.head(h, [out], laid_out=True)
         return out
 
 

@@ -220,7 +220,7 @@ class _Mixer:
         y = split_product(a, p.weight[:w])
         if y is None:
             y = self.new(int(a.shape[0]), w)
-            p(a, [y])
+            p(a, [y], laid_out=True)
         return y
 
 
@@ -266,7 +266,7 @@ class ParallelMixer(_Mixer):
         rq, rk = self.new(t, g.heads * g.dim), self.new(t, g.heads * g.dim)
         rv, rg = self.new(t, g.heads * g.vdim), self.new(t, g.heads * g.vdim)
         gate, low = self.new(t, a.heads, f32), self.new(t, self.rank, f32)
-        self.proj(h, [q, k, vc, rq, rk, rv, rg, gate, low], [None, None, b.out_cache_loc] + [None] * 6)
+        self.proj(h, [q, k, vc, rq, rk, rv, rg, gate, low], [None, None, b.out_cache_loc] + [None] * 6, laid_out=True)
         if self.rotary not in c.tables:
             c.tables[self.rotary] = rotary_table(self.inv_freq, b.positions)
         qk_norm_rope(q, k, a.heads, a.kv_heads, a.dim, self.q_norm, self.k_norm, self.cfg.eps, c.tables[self.rotary], b, kc)
@@ -298,7 +298,7 @@ class Mamba2Mixer(_Mixer):
     def forward(self, x: torch.Tensor, h: torch.Tensor, c: _Context) -> Pending:
         m, t = self.m, int(x.shape[0])
         z, u, dt = self.new(t, m.inner), self.new(t, m.channels), self.new(t, m.heads, torch.float32)
-        self.proj(h, [z, u, dt])
+        self.proj(h, [z, u, dt], laid_out=True)
         xbc = self.new(t, m.channels)
         short_conv(u, self.conv_w, [(xbc, None, 0, m.channels)], c.caches.conv[c.run], c.batch, self.conv_b, silu=True)
         keys = m.groups * m.state
@@ -342,14 +342,14 @@ class KotipelLayer(_Mixer):
         if self.layer.ff is not None:
             h = update_norm(x, eps, self.new(t, cfg.width), self.norm2, pending=pending)
             act = self.new(t, self.ff_cols)
-            self.gate_up(h, [act])
+            self.gate_up(h, [act], laid_out=True)
             copy = self.new(t, cfg.width) if self.side_embed is not None else None
             pending = Pending(gated_add(x, [(act, self.down_w, None)], copy=copy, few_rows=True, laid_out=True))
         if self.side_embed is not None:
             if self.layer.ff is None or not pending.empty:
                 copy = update_norm(x, eps, self.new(t, cfg.width), pending=pending)
             g = self.new(t, int(self.side_embed.shape[1]))
-            self.side_gate(copy, [g], mul=(self.side_embed, c.batch.input_ids))
+            self.side_gate(copy, [g], mul=(self.side_embed, c.batch.input_ids), laid_out=True)
             pending = Pending(parts=[(self.product(g, self.side_proj), self.side_norm, 1.0)])
         return pending
 
@@ -410,7 +410,7 @@ class KotipelForCausalLM:
         h = torch.empty((n, ceil_to(self.cfg.width, 8)), dtype=self.dtype, device=self.device)
         update_norm(x, self.cfg.eps, h, self.final_norm, pending=pending, row_idx=rows)
         out = torch.empty((n, self.cfg.vocab), dtype=torch.float32, device=self.device)
-        self.head(h, [out])
+        self.head(h, [out], laid_out=True)
         return out
 
 

@@ -123,9 +123,10 @@ class MergedProjection:
 
     def __call__(self, a: torch.Tensor, outs: Sequence[torch.Tensor],
                  row_maps: Optional[Sequence[Optional[torch.Tensor]]] = None, algo: int = 0,
-                 mul: Optional[Tuple[torch.Tensor, torch.Tensor]] = None) -> None:
+                 mul: Optional[Tuple[torch.Tensor, torch.Tensor]] = None, laid_out: bool = False) -> None:
         """``a`` [M, lda >= K padded]; ``outs`` one 2-D tensor per range (rows are ``row_maps[i][m]`` if given);
-        ``mul`` = (table [rows, n], row of each m) of the ``gelu_mul`` ranges."""
+        ``mul`` = (table [rows, n], row of each m) of the ``gelu_mul`` ranges. ``laid_out``: the launch ahead on the stream does
+        not write the weight (``finish`` does, and so does a copy into it)."""
         require_cuda(a)
         segs = (FrOutSegment * len(self.ranges))()
         n0 = 0
@@ -144,7 +145,8 @@ class MergedProjection:
             buf = torch.empty((n_splits, m, n0), dtype=torch.float32, device=a.device)
             call("fr_dense_proj_split", code, ptr(a), a.stride(0), ptr(w), w.stride(0), m, n0, k, segs, len(segs), ptr(buf), n_splits, s)
         else:
-            call("fr_dense_proj", code, ptr(a), a.stride(0), ptr(w), w.stride(0), m, n0, k, segs, len(segs), algo | LAID_OUT, s)
+            call("fr_dense_proj", code, ptr(a), a.stride(0), ptr(w), w.stride(0), m, n0, k, segs, len(segs),
+                 algo | (LAID_OUT if laid_out else 0), s)
 
 
 @dataclass

@@ -63,7 +63,7 @@ class Qwen3LM:
 
     def logits(self, hidden: torch.Tensor, partials, rows: torch.Tensor) -> torch.Tensor:
         out = torch.empty((int(rows.numel()), self.vocab), dtype=torch.float32, device=self.device)
-        self.head(hidden.index_select(0, rows), [out])
+        self.head(hidden.index_select(0, rows), [out], laid_out=True)
         return out
 
 

@@ -169,6 +169,24 @@ def test_weight_layouts():
     assert starts == [0, 64, 192] and m.weight.shape == (224, 8)
 
 
+@pytest.mark.parametrize("algo", [0, 2])
+def test_projection_reads_its_weight_early_only_when_told(algo, monkeypatch):
+    """``finish`` and copies into the weight are launches too: nothing but the caller knows that none is directly ahead."""
+    from flashrec_b200 import lm_layers
+
+    m = MergedProjection(8)
+    m.add("store", torch.ones(1056, 8))  # too many columns to be split
+    m.finish(torch.float32, "cpu")
+    algos = []
+    monkeypatch.setattr(lm_layers, "require_cuda", lambda *t: None)
+    monkeypatch.setattr(lm_layers, "stream_ptr", lambda device: 0)
+    monkeypatch.setattr(lm_layers, "call", lambda name, *a: algos.append((name, a[-2])))
+    a, out = torch.ones(2, 8), torch.empty(2, 1056)
+    m(a, [out], algo=algo)
+    m(a, [out], algo=algo, laid_out=True)
+    assert algos == [("fr_dense_proj", algo), ("fr_dense_proj", algo | lm_layers.LAID_OUT)]
+
+
 def _fault(raw, what):
     bad = copy.deepcopy(raw)
     for e in bad["layers"]:

@@ -203,3 +203,36 @@ def test_weights_read_ahead_of_the_launch_before_keep_the_bits(dtype, m, n, ks):
         got.append(x)
     for a, b in zip(got[: len(got) // 2], got[len(got) // 2:]):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype,m", [(torch.bfloat16, 1), (torch.bfloat16, 2), (torch.bfloat16, 64), (torch.bfloat16, 600), (torch.float32, 1)])
+def test_projection_of_a_weight_that_the_launch_ahead_writes(dtype, m):
+    """The weight comes from a product that lets its dependents start at its own beginning: a projection whose caller does not
+    say that it lies there already sees all of it."""
+    from flashrec_b200.lm_layers import MergedProjection
+
+    n, k, depth = 1064, 512, 4096
+    proj = MergedProjection(k)
+    proj.add("store_f32", torch.zeros(n, k))
+    proj.finish(dtype, "cuda")
+    writer = MergedProjection(depth)
+    writer.add("store", _rand(k, depth, seed=1) * depth ** -0.5)
+    writer.finish(dtype, "cuda")
+    a = _rand(m, k, seed=2).to(dtype)
+    inputs = [_rand(n, depth, seed=10 + i).to(dtype) for i in range(16)]
+    torch.cuda.synchronize()
+
+    def step(x, wait=False):
+        writer(x, [proj.weight[:n]])
+        if wait:
+            torch.cuda.synchronize()
+        out = torch.empty(m, n, device="cuda")
+        proj(a, [out])
+        return out
+
+    want = [step(x, wait=True) for x in inputs]
+    assert not torch.equal(want[0], want[1])
+    for _ in range(3):
+        torch.cuda._sleep(20_000_000)  # the launches queue up and meet the GPU without gaps
+        for got, ref in zip([step(x) for x in inputs], want):
+            assert torch.equal(got, ref)
