@@ -1440,10 +1440,14 @@ static int forced_pair() {
 }
 
 // Tile choice: 64, 128 or 256 columns by 128 rows on one CTA, or 512 for 256 x 256 on a CTA pair, whichever is estimated to end
-// first: rounds of tiles over the SMs (pairs), each an epilogue share plus a time per k-block, fitted to launches of 64 to 8192
-// rows over N of 2048, 4096 and 8192 and K of 2048 and 6144 (in us; all within 15 %). All tiles give the same bits. Where it
-// departs from whole waves weighted by the tensor rate, which it replaces: 2048 rows x 2048 x 2048 with the residual 15.4 -> 12.3 us,
-// 6000 rows 34.4 -> 24.4, 2048 x 2048 x 6144 26.0 -> 22.2, 2048 x 4096 x 2048 18.5 -> 16.7.
+// first: rounds of tiles over the SMs (pairs), each an epilogue share plus a time per k-block, in us, fitted to launches of 64 to 8192
+// rows over N of 2048, 4096 and 8192 and K of 2048 and 6144. All tiles give the same bits. Over 64 to 16384 rows of ten N x K from
+// 1024 x 2048 to 12288 x 2048, with and without the residual, the choice takes 0.5 % more than the fastest of the four tiles in the
+// mean, 13 % at most, and at no size 2 % more than the rule that it replaces (whole waves weighted by the tensor rate): 2048 rows x
+// 2048 x 2048 with the residual 15.4 -> 12.3 us, 6000 rows 34.4 -> 24.4, 2048 x 2048 x 6144 26.0 -> 22.2, 2048 x 4096 x 2048 18.5 -> 16.7.
+// Pairs start at 5.6 us without the residual: at 5.0, which many rounds fit, a single round of them was underestimated by up to a tenth
+// and won where one CTA's tiles of 256 columns are faster (us, pair / one CTA: 512 rows x 6144 x 2048 11.9 / 11.5, 768 rows 12.2 / 11.3,
+// 512 rows x 8192 x 2048 12.3 / 11.9, 2048 rows x 2048 x 2048 11.8 / 11.1).
 static int pick_tile(int M, int N, int K, bool add) {
   if (forced_pair() == 1) return 512;
   const int tiles[4] = {64, 128, 256, 512};
@@ -1457,7 +1461,7 @@ static int pick_tile(int M, int N, int K, bool add) {
     if (pair && forced_pair() == 0) continue;
     const int64_t n = static_cast<int64_t>(ceil_div(M, pair ? 2 * kBlockM : kBlockM)) * ceil_div(N, pair ? 256 : tiles[i]);
     const int units = pair ? sm_count() / 2 : sm_count();
-    const double t = (pair ? 5.0 : 3.2) + static_cast<double>((n + units - 1) / units) * (epilogue[add][i] + per_kb[i] * kb);
+    const double t = (pair ? (add ? 5.0 : 5.6) : 3.2) + static_cast<double>((n + units - 1) / units) * (epilogue[add][i] + per_kb[i] * kb);
     if (best_tile == 0 || t < best) {
       best = t;
       best_tile = tiles[i];
