@@ -367,7 +367,8 @@ __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
 // y = bf16(silu(g) * u) of 2 N gate and up values in bf16 pairs, silu rounded to bf16 as silu_bf16 does; returns the pairs' largest
 // |y| (NaN left out). The rounding is known when the fast result, 24 fp32 ulp less and 24 ulp more, rounds to the same value both
 // times; pairs where it does not, and all pairs of a call with a gate below -60 (the exponential overflows from -88 on) or above 1e38 (its exponent does),
-// are read from the table. The products equal those of silu_mul_pack, except that results below 2^-126 are rounded once, not twice.
+// are read from the table. The products are those of silu_mul_pack to the last bit: two bf16 factors make at most 16 significant bits,
+// which fp32 holds exactly from 2^-134 on, so its rounding to bf16 is the only one there too; what is smaller becomes zero either way.
 template <int N>
 __device__ __forceinline__ uint32_t swiglu_pairs(const uint32_t (&g)[N], const uint32_t (&u)[N], const uint16_t* __restrict__ table,
                                                  uint32_t (&y)[N]) {

@@ -329,6 +329,26 @@ def test_gemm_silu_epilogue_every_gate(mode):
         assert torch.equal(y.view(torch.int16)[number], want.view(torch.int16)[number])
 
 
+@pytest.mark.parametrize("mode", [1, 2])
+@pytest.mark.parametrize("up", [1.9921875 * 2.0 ** -40, 1.3359375 * 2.0 ** -100, -1.0078125 * 2.0 ** -120, 1.6640625 * 2.0 ** -126, 127 * 2.0 ** -133])
+def test_gemm_silu_epilogue_smallest_results(mode, up):
+    """All gates times factors that bring the results to the subnormal numbers and below them: the unfused kernel's, bit for bit."""
+    from flashrec_b200.kernel.sglops import fp8_scaled_mm_silu_mul, interleave_gate_up, silu_and_mul
+
+    d, k = 65536, 16
+    gates = torch.arange(d, dtype=torch.int32, device=DEV).to(torch.int16).view(torch.bfloat16)
+    a, w = torch.zeros(1, k, device=DEV), torch.zeros(2 * d, k, device=DEV)
+    a[:, 0] = w[:, 0] = 1.0
+    wi, si = interleave_gate_up(w.to(torch.float8_e4m3fn), torch.cat((gates.float(), torch.full((d,), up, device=DEV))))
+    y, _ = fp8_scaled_mm_silu_mul(a.to(torch.float8_e4m3fn), wi, torch.ones(1, 1, device=DEV), si, mode=mode)
+    rows = gates.view(16, -1)
+    want = silu_and_mul(torch.cat((rows, torch.full_like(rows, up)), dim=1)).reshape(1, d)
+    number, small = ~want.isnan(), (want != 0) & (want.abs().float() < 2.0 ** -126)
+    assert int(small.sum()) > 100
+    assert torch.equal(y.isnan(), want.isnan())
+    assert torch.equal(y.view(torch.int16)[number], want.view(torch.int16)[number])
+
+
 @pytest.mark.parametrize("m,n,k", [(1500, 2048, 512), (700, 4104, 256), (3000, 1000, 2064), (257, 304, 6144)])
 def test_gemm_tile_choice_keeps_the_bits(m, n, k):
     """Every tile and the chosen one (none of these splits K by itself) give the same product and the same update."""
