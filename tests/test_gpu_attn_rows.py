@@ -208,3 +208,38 @@ def test_coefficients_of_the_launch_ahead(heads, kv, lens):
     for _ in range(3):
         for got, ref in zip(_behind_each_other(step, inputs), want):
             assert torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("kind", ["diff", "talk", "plain"])
+@pytest.mark.parametrize("lens", [(1100,), (1,), tuple(range(40, 440, 10))])
+def test_early_reads_behind_a_launch_that_writes(kind, lens):
+    """Queries, the rows' own keys and values and the heads' gates come, over the same buffers again and again, from a product that
+    lets its dependents start at its own beginning: the early entry's bits are those of the plain one behind a wait."""
+    from flashrec_b200.lm_layers import MergedProjection
+
+    n, heads, kv, dim, vdim, depth = len(lens), 8, 4, 64, 128, 4096
+    maps = 2 if kind == "diff" else 1
+    attn, table, b, slots = _decode(kind, heads, kv, dim, vdim, lens)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()  # noqa: E731
+    if kind == "talk":
+        attn.coef.copy_(0.5 * rnd(heads, heads).float())
+    q, k, v, gate = rnd(n, heads * maps * dim), rnd(slots, kv * maps * dim), rnd(slots, kv * vdim), torch.zeros(n, heads, device="cuda")
+    proj = MergedProjection(depth)
+    for cols, store in ((q.shape[1], "store"), (k.shape[1], "store"), (v.shape[1], "store"), (heads, "store_f32")):
+        proj.add(store, rnd(cols, depth) * 4 * depth ** -0.5)
+    proj.finish(torch.bfloat16, "cuda")
+    torch.cuda.synchronize()
+    counters, inputs = torch.zeros(4096, dtype=torch.int32, device="cuda"), [rnd(n, depth) for _ in range(24)]
+
+    def step(x, wait=False):
+        proj(x, [q, k, v, gate], [None, b.out_cache_loc, b.out_cache_loc, None], laid_out=True)
+        if wait:
+            torch.cuda.synchronize()
+        return attn.forward(q, k, v, table, b, counters, head_gate=gate if kind == "plain" else None, early=not wait)
+
+    want = [step(x, wait=True) for x in inputs]
+    assert not torch.equal(want[0], want[1])
+    for _ in range(3):
+        for got, ref in zip(_behind_each_other(step, inputs), want):
+            assert torch.equal(got, ref)
