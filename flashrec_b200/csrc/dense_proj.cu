@@ -281,7 +281,7 @@ dense_rows_gated_kernel(const __grid_constant__ Parts pt, float* __restrict__ x,
   // row, none / one / two and one of the first part: 2048 x (2048 + 6144) 8.3 / 7.5 / 9.4, 2048 x 6144 6.2 / 5.5 / 7.5,
   // 4096 x 12288 24.5 / 20.0 / 19.0; two rows 9.4 / 11.0 / 10.4, 6.5 / 8.4 / 8.3, 23.0 / 22.8 / 21.9.
   const int last = pt.n - 1;
-  constexpr int kAhead = AHEAD && (MB == 1 || sizeof(T) == 4) ? 1 : 0;
+  constexpr int kAhead = AHEAD ? 1 : 0;
   RowsDot<T, MB, 0> dot0;
   RowsDot<T, MB, kAhead> dot1;
   constexpr bool kLoop = MB > (sizeof(T) == 2 ? 2 : 4);  // see below
@@ -570,7 +570,6 @@ dense_finish_kernel(const float* __restrict__ partials, int n_splits, int M, int
 // ---------------------------------------------------------------------------
 constexpr int kBlockM = 128;
 constexpr int kBlockK = 64;  // bf16 elements: one 128-byte swizzle span
-constexpr int kUmmaK = 16;
 constexpr int kEpiWarps = 8;
 constexpr int kThreads = 64 + kEpiWarps * 32;
 enum Epi { kEpiSegs = 0, kEpiAdd = 1, kEpiPartial = 2 };
@@ -1264,7 +1263,8 @@ static int launch_rows_gated(const Parts& pt, float* x, int64_t ldx, int M, int 
   const int grid = ceil_div(ceil_div(N, 4), (kRowsThreads / 32) / ks);
   auto go = [&](auto kernel) { return launch_kernel(kernel, grid, kRowsThreads, 0, stream, true, pt, x, ldx, M, N, copy, ldc, ks); };
   if (M == 1) return ahead ? go(dense_rows_gated_kernel<T, 1, true>) : go(dense_rows_gated_kernel<T, 1, false>);
-  if (M == 2) return ahead ? go(dense_rows_gated_kernel<T, 2, true>) : go(dense_rows_gated_kernel<T, 2, false>);
+  constexpr bool kTwoAhead = sizeof(T) == 4;  // two bf16 rows load nothing ahead
+  if (M == 2) return ahead ? go(dense_rows_gated_kernel<T, 2, kTwoAhead>) : go(dense_rows_gated_kernel<T, 2, false>);
   return M <= 4 ? go(dense_rows_gated_kernel<T, 4, false>) : go(dense_rows_gated_kernel<T, 8, false>);
 }
 

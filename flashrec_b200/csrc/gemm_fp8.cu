@@ -147,8 +147,8 @@ __device__ __forceinline__ void scaled_pairs(const uint32_t (&r)[N], const float
 // SwiGLU on 16 gate / 16 up accumulator columns of one row (one thread): returns max|y| as a bf16 pair and
 // hands back the 16 bf16 results as two 16-byte pieces. About 15 instructions per result, two at a time where a packed form exists
 // (38 one by one, which held up the products: 12288 x 2048 columns, 512 rows 24.7 -> 19.9 us, 4096 rows 91.7 -> 78.8).
-// sbg / sbu: the 16 per-channel scales of the gate / up columns in global memory (16-byte
-// aligned; every thread reads the same addresses, so they come from L1). release_bar: 0, or the
+// sbg / sbu: the 16 per-channel scales of the gate / up columns in shared or global memory (16-byte
+// aligned; every thread reads the same addresses: one broadcast, or L1). release_bar: 0, or the
 // cluster address of the barrier to arrive on once the accumulator columns are in registers.
 __device__ __forceinline__ uint32_t swiglu16(uint32_t taddr_g, uint32_t taddr_u, const float* __restrict__ sbg,
                                              const float* __restrict__ sbu, float sa,
@@ -1413,22 +1413,6 @@ static bool use_pdl(int M) {
   if (forced >= 0) return forced == 1;
   return M <= 2048;
 }
-static int fill_launch_attrs(cudaLaunchAttribute* attr, int cluster, bool pdl) {
-  int n = 0;
-  if (cluster > 1) {
-    attr[n].id = cudaLaunchAttributeClusterDimension;
-    attr[n].val.clusterDim.x = cluster;
-    attr[n].val.clusterDim.y = 1;
-    attr[n].val.clusterDim.z = 1;
-    ++n;
-  }
-  if (pdl) {
-    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[n].val.programmaticStreamSerializationAllowed = 1;
-    ++n;
-  }
-  return n;
-}
 
 // FR_GEMM_PAIR=0/1 overrides the choice of CTA pairs; -1 without it.
 static int forced_pair() {
@@ -1489,20 +1473,8 @@ static int launch(const void* a, const void* b, const float* sa, const float* sb
   if (EPI == 1 && !table) return FR_ERR_CUDA;
   const int tiles = ceil_div(M, kBlockM) * ceil_div(N, BLOCK_N);
   const int grid = tiles < sm_count() ? tiles : sm_count();
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(EpiCfg<EPI>::kThreads);
-  cfg.dynamicSmemBytes = C::kSmemBytes;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
-  cfg.attrs = attr;
-  cfg.numAttrs = fill_launch_attrs(attr, 1, use_pdl(M));
-  if (cudaLaunchKernelEx(&cfg, kern, ta, tb, static_cast<OutT*>(out), ldo, sa, sb, static_cast<const __nv_bfloat16*>(bias),
-                         M, N, K, row_amax, table, ahead, status) != cudaSuccess) {
-    cudaGetLastError();
-    return FR_ERR_CUDA;
-  }
-  return FR_OK;
+  return launch_cluster(kern, grid, EpiCfg<EPI>::kThreads, C::kSmemBytes, stream, 1, use_pdl(M), ta, tb, static_cast<OutT*>(out), ldo,
+                        sa, sb, static_cast<const __nv_bfloat16*>(bias), M, N, K, row_amax, table, ahead, status);
 }
 
 template <typename OutT, int EPI>
@@ -1531,20 +1503,8 @@ static int launch_pair(const void* a, const void* b, const float* sa, const floa
   if (EPI == 1 && !table) return FR_ERR_CUDA;
   const int tiles = ceil_div(M, 2 * kBlockM) * ceil_div(N, C::kBlockN);
   const int pairs = tiles < sm_count() / 2 ? tiles : sm_count() / 2;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2 * pairs);
-  cfg.blockDim = dim3(EpiCfg<EPI>::kThreads);
-  cfg.dynamicSmemBytes = C::kSmemBytes;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
-  cfg.attrs = attr;
-  cfg.numAttrs = fill_launch_attrs(attr, 2, use_pdl(M));
-  if (cudaLaunchKernelEx(&cfg, kern, ta, tb, to, sa, sb, static_cast<const __nv_bfloat16*>(bias), M, N, K, row_amax,
-                         table, rp, hp, ahead, status) != cudaSuccess) {
-    cudaGetLastError();
-    return FR_ERR_CUDA;
-  }
-  return FR_OK;
+  return launch_cluster(kern, 2 * pairs, EpiCfg<EPI>::kThreads, C::kSmemBytes, stream, 2, use_pdl(M), ta, tb, to, sa, sb,
+                        static_cast<const __nv_bfloat16*>(bias), M, N, K, row_amax, table, rp, hp, ahead, status);
 }
 
 // SwiGLU epilogue: CTA pairs pay off once there are several waves of 256 x 256 tiles.
@@ -1638,19 +1598,8 @@ static int launch_splitk_tn(const void* a, const void* b, const float* sa, const
   int* status = device_status_ptr();
   if (!status) return FR_ERR_CUDA;
   const int tiles = ceil_div(M, C::kTileM) * ceil_div(N, C::kTileN);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(tiles * splits);
-  cfg.blockDim = dim3(C::kThreads);
-  cfg.dynamicSmemBytes = C::kSmemBytes;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
-  cfg.attrs = attr;
-  cfg.numAttrs = fill_launch_attrs(attr, splits, use_pdl(M));
-  if (cudaLaunchKernelEx(&cfg, kern, ta, tb, static_cast<OutT*>(out), ldo, sa, sb, M, N, K, ahead, status) != cudaSuccess) {
-    cudaGetLastError();
-    return FR_ERR_CUDA;
-  }
-  return FR_OK;
+  return launch_cluster(kern, tiles * splits, C::kThreads, C::kSmemBytes, stream, splits, use_pdl(M), ta, tb, static_cast<OutT*>(out), ldo,
+                        sa, sb, M, N, K, ahead, status);
 }
 
 template <typename OutT, int EPI>

@@ -78,11 +78,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 }
 
 // The same by a whole converged warp; all lanes get the same answer. The warps that load tiles and issue products run their loops
-// with all lanes, and the *_one functions below elect the lane that issues (the same one every time) in the same statement. In a
-// branch of one lane, of which the compiler does not know that it is one, every instruction with uniform operands (TMA,
-// tcgen05.mma, tcgen05.commit) becomes a walk over the active lanes: about 100 cycles each, 0.1 us and more per k-block of a product.
-// Before and after, same bits: FP8, 512 rows x 4096 x 2048 9.1 -> 7.7 us, 2048 x 6144 14.7 -> 12.7, 4096 rows x 4096 x 2048 32.8 -> 28.9;
-// bf16 update of 16 rows x 2048 x 8192 12.2 -> 9.9, projection of 8 rows x 20480 x 2048 24.4 -> 21.0.
+// with all lanes, and the *_one functions below elect the lane that issues (the same one every time) in the same statement. Before, a
+// branch of lane 0 held the loops, and an instruction in it took about 100 cycles to issue, 0.1 us and more per k-block of a product. The
+// likely reason is that TMA, tcgen05.mma and tcgen05.commit want operands that are uniform in the warp, and that nothing tells the
+// compiler that such a branch has one lane; what was measured are the times. Before and after, same bits: FP8, 512 rows x 4096 x 2048
+// 9.1 -> 7.7 us, 2048 x 6144 14.7 -> 12.7, 4096 rows x 4096 x 2048 32.8 -> 28.9; bf16 update of 16 rows x 2048 x 8192 12.2 -> 9.9,
+// projection of 8 rows x 20480 x 2048 24.4 -> 21.0.
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int site) {
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, site)) != 0;
 }
