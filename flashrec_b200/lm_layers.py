@@ -161,7 +161,7 @@ def gated_add(x: torch.Tensor, parts: Sequence[Tuple[torch.Tensor, torch.Tensor,
               algo: int = 0, split: bool = True, copy: Optional[torch.Tensor] = None, few_rows: bool = False,
               laid_out: bool = False) -> Optional[Partials]:
     """``x += sum gate * (a @ w.T)`` over one or two ``(a, w, gate)`` parts; few-row products may come back as
-    partials for the following ``rms_norm`` instead, with ``few_rows`` also those of up to 8 rows. ``copy`` gets the new x in
+    partials for the following ``rms_norm`` instead, with ``few_rows`` also those of up to 8 rows and float32 ones of 9 to 1024. ``copy`` gets the new x in
     its own type (not with partials). ``laid_out``: the launch ahead on the stream does not write the weights."""
     require_cuda(x)
     m, n = int(x.shape[0]), int(x.shape[1])
