@@ -462,3 +462,44 @@ def test_end_to_end_wave_against_the_oracle_with_its_own_attention_statistics():
     print("end-to-end wave, oracle attention: mean / max |score difference| per level "
           + ", ".join(f"{np.mean(x):.3f} / {np.max(x):.3f}" for x in diffs)
           + f"; 1e-3 rule: {viol} of {decided} decided positions differ")
+
+
+_EAGER_WAVES = """
+import sys
+import numpy as np, torch
+from flashrec_b200 import device_status
+from flashrec_b200.decoder import Qwen3Config
+from flashrec_b200.sid_decode import SidDecodeEngine
+from flashrec_b200.trie import build_trie_arrays, trie_to_device
+
+n, bw, prompt = map(int, sys.argv[1:])
+cfg = Qwen3Config(hidden_size=2048, num_attention_heads=16, num_key_value_heads=8, head_dim=128, intermediate_size=6144,
+                  num_hidden_layers=6, max_position_embeddings=1024, vocab_size=1000 + 768)
+rng = np.random.default_rng(0)
+sizes = [256, 256, 256]
+trie = trie_to_device(build_trie_arrays(np.stack([rng.integers(0, 256, 20000) for _ in sizes], 1), sizes, 1000), "csr", "cuda:0")
+eng = SidDecodeEngine(cfg, n, bw, [prompt - 3 * r for r in range(n)], sizes, 1000, trie, "cuda:0", shared_prefix=16, seed=1)
+waves = []
+for _ in range(4):
+    eng.run(host_io=False, _eager=True)
+    waves.append((eng.cum.clone(), eng.final_tokens.clone()))
+    assert device_status() == (0, 0)
+eng.capture()
+eng.run(host_io=False)
+assert device_status() == (0, 0)
+for cum, tokens in waves:
+    assert torch.equal(cum, eng.cum) and torch.equal(tokens, eng.final_tokens)
+"""
+
+
+@pytest.mark.parametrize("n,bw,prompt", [(1, 512, 640), (7, 50, 300)])
+def test_eager_waves_of_a_fresh_process(n, bw, prompt):
+    """A process's first waves, each kernel of a layer launched while the one ahead runs and the host in between: no wait of the
+    attention kernel or of a product gives up, and the bits are those of the graphs."""
+    import subprocess
+    import sys
+    from pathlib import Path
+
+    p = subprocess.run([sys.executable, "-c", _EAGER_WAVES, str(n), str(bw), str(prompt)], cwd=Path(__file__).resolve().parent.parent,
+                       capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0, p.stderr[-2000:]
